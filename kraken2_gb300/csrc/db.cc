@@ -134,8 +134,25 @@ k2g_status validate_parents(const uint64_t *parent, uint64_t n) {
 k2g_status upload_parents(k2g_db *db, const uint64_t *parent, uint64_t n) {
   std::vector<uint32_t> p32(n);
   for (uint64_t i = 0; i < n; i++) p32[i] = (uint32_t)parent[i];
-  K2G_CUDA_TRY(cudaMalloc(&db->d_parent, n * sizeof(uint32_t)));
-  K2G_CUDA_TRY(cudaMemcpy(db->d_parent, p32.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice));
+  // Preorder intervals: x is an ancestor of y (or y itself) exactly when y's
+  // number lies in x's interval.  parent[i] < i, so one pass from the back
+  // gives the subtree sizes and one from the front the numbers.
+  std::vector<uint2> span(n, make_uint2(0, 1));
+  for (uint64_t i = n; i-- > 1;) span[p32[i]].y += span[i].y;
+  std::vector<uint32_t> next(n, 1);
+  for (uint64_t i = 1; i < n; i++) {
+    const uint32_t pre = next[p32[i]], size = span[i].y;
+    next[p32[i]] += size;
+    next[i] = pre + 1;
+    span[i] = make_uint2(pre, pre + size);
+  }
+  // one allocation and one copy: the intervals, then the parents
+  std::vector<uint32_t> both(3 * n);
+  memcpy(both.data(), span.data(), n * sizeof(uint2));
+  memcpy(both.data() + 2 * n, p32.data(), n * sizeof(uint32_t));
+  K2G_CUDA_TRY(cudaMalloc(&db->d_span, 3 * n * sizeof(uint32_t)));
+  db->d_parent = reinterpret_cast<uint32_t *>(db->d_span + n);
+  K2G_CUDA_TRY(cudaMemcpy(db->d_span, both.data(), 3 * n * sizeof(uint32_t), cudaMemcpyHostToDevice));
   db->node_count = n;
   return K2G_OK;
 }
@@ -200,7 +217,7 @@ void destroy(k2g_db *db) {
   if (db->d_ext) cudaFree(db->d_ext);
   if (db->d_name_off) cudaFree(db->d_name_off);
   if (db->d_names) cudaFree(db->d_names);
-  if (db->d_parent) cudaFree(db->d_parent);
+  if (db->d_span) cudaFree(db->d_span);   // (d_parent lies in the same allocation)
   if (db->d_size) cudaFree(db->d_size);
   cudaSetDevice(cur);
   delete db;

@@ -18,6 +18,8 @@ __device__ __forceinline__ uint64_t murmur3(uint64_t k) {
 }
 
 
+__device__ __forceinline__ uint64_t min64(uint64_t a, uint64_t b) { return a < b ? a : b; }
+
 // n % d through the invariant-divisor magic (see DivMagic).
 __device__ __forceinline__ uint64_t fast_mod(uint64_t n, const DivMagic &m) {
   uint64_t t = __umul64hi(m.m, n);

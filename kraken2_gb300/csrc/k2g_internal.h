@@ -113,6 +113,8 @@ struct k2g_db {
   uint64_t *d_name_off = nullptr;
   char *d_names = nullptr;
   uint32_t *d_parent = nullptr;   // node_count entries
+  uint2 *d_span = nullptr;        // per node: preorder number, one past its subtree's last
+                                  // (d_parent follows in the same allocation)
   uint64_t *d_size = nullptr;     // device-side size counter used by builds
   k2g::DivMagic div{};
   bool owns_table = true;
@@ -141,6 +143,12 @@ k2g_status require_dna(const k2g_db *db);
 k2g_status classify_translated(const k2g_db *db, const k2g_reads *reads,
                                const k2g_classify_params *params, k2g_results *out,
                                cudaStream_t st);
+// Classification of short fragments in one launch, without device scratch
+// (warp_classify.cu): whether it takes a call, and the call itself.
+struct ClassifyArgs;
+bool warp_classify_takes(const ClassifyArgs &a, uint64_t max_len);
+cudaError_t warp_classify(const ClassifyArgs &a, const uint2 *span, uint64_t total_bases, int sms,
+                          cudaStream_t st);
 // Counts each kernel launch issued by the library (k2g_kernel_launches).
 void note_launches(uint64_t n = 1);
 // One round (< 2^30 pairs) of the order-exact build insert (build_ordered.cu).

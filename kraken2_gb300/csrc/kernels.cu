@@ -887,8 +887,12 @@ k2g_status k2g::classify_keyed(const k2g_db *db, const k2g_reads *reads,
     K2G_CUDA_TRY(cudaStreamSynchronize(st));
     total = ends[1] - ends[0];
   }
-  return run_classify(db, a, mode, reads->max_seq_len, total, st, state_key,
-                      db->tuning(params->paired != 0, total, reads->n_frags));
+  const Tuning tn = db->tuning(params->paired != 0, total, reads->n_frags);
+  if (mode == K2G_MODE_PIPELINED && tn.pipeline && warp_classify_takes(a, reads->max_seq_len)) {
+    K2G_CUDA_TRY(warp_classify(a, db->d_span, total, sm_count(db->device), st));
+    return K2G_OK;
+  }
+  return run_classify(db, a, mode, reads->max_seq_len, total, st, state_key, tn);
 }
 
 extern "C" k2g_status k2g_build_insert(k2g_db *db, const uint64_t *d_keys, const uint32_t *d_taxids,

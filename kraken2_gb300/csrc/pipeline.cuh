@@ -158,8 +158,6 @@ __device__ __forceinline__ void pipe_scan_emit(ScanLane<5> &s, const PipeArgs &p
   nst += is_key ? 1 : 0;
 }
 
-__device__ __forceinline__ uint64_t min64(uint64_t a, uint64_t b) { return a < b ? a : b; }
-
 // Four bases (one 32-bit word of the chunk) with a window of w = 5 l-mers:
 // the minimum over positions p-4..p is min(suffix minimum of the previous
 // word's candidates from p-4 on, prefix minimum of this word's up to p), so
