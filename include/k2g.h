@@ -195,17 +195,22 @@ typedef struct {
 typedef enum {
   K2G_MODE_PLAIN = 0,         /* fused kernel, one thread per fragment      */
   K2G_MODE_PERSISTENT = 1,    /* fused kernel, work-stealing lanes          */
-  K2G_MODE_PIPELINED = 2      /* scan / probe / resolve stages over
-                                 overlapping sub-batches (fastest); long
-                                 fragments go to the fused kernel, and a
-                                 batch averaging over 512 bases per
-                                 fragment runs it as K2G_MODE_PERSISTENT   */
+  K2G_MODE_PIPELINED = 2      /* the fastest form.  Tables with k - l = 4
+                                 (the default): one launch on the caller's
+                                 stream, a warp per group of fragments, long
+                                 single fragments in pieces.  Other tables:
+                                 scan / probe / resolve stages over
+                                 overlapping sub-batches; long fragments go
+                                 to the fused kernel, and a batch averaging
+                                 over 512 bases per fragment runs it as
+                                 K2G_MODE_PERSISTENT                       */
 } k2g_mode;
 
 /* Classifies a batch of fragments held in device memory.  Calls on one
  * stream run in order; calls on different streams may run at the same time
- * (up to eight streams per device get scratch of their own, further streams
- * share it and are serialised with their sharers), so a caller with several
+ * (the staged and fused kernels: up to eight streams per device get scratch
+ * of their own, further streams share it and are serialised with their
+ * sharers; the one-launch form needs none), so a caller with several
  * batches in flight overlaps one batch's tail with the next batch's work. */
 k2g_status k2g_classify(const k2g_db *db, const k2g_reads *reads,
                         const k2g_classify_params *params, k2g_results *out,
@@ -216,7 +221,9 @@ k2g_status k2g_classify(const k2g_db *db, const k2g_reads *reads,
  * prefetch distance at src/compact_hash.h:380-392).  Each table keeps one
  * set of values per (single-end or paired, length class) of a batch; every
  * k2g_classify call uses the set of its batch's class.  The values change
- * only how the work is scheduled, never a result.  A table starts with
+ * only how the work is scheduled, never a result.  The one-launch form of
+ * K2G_MODE_PIPELINED uses piece_len only (a warp's pieces are four times as
+ * long, up to 8192).  A table starts with
  * pipeline 1 for short batches and 0 otherwise, probe_split 2,
  * sub_batch_mb 256, piece_len 512 and graphs 0 in every class. */
 typedef struct {

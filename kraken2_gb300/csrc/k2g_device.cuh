@@ -27,6 +27,14 @@ __device__ __forceinline__ uint64_t fast_mod(uint64_t n, const DivMagic &m) {
   return n - q * m.d;
 }
 
+// n % d for d <= 2^63: n * inv / 2^64 is above n / d - 1 and not above n / d,
+// so the quotient is at most one short.  Fewer instructions than fast_mod
+// where the subtraction is a select.
+__device__ __forceinline__ uint64_t mod_once(uint64_t n, const DivMagic &m) {
+  const uint64_t r = n - __umul64hi(n, m.inv) * m.d;
+  return r >= m.d ? r - m.d : r;
+}
+
 // Read-only, L1-cached load of one table cell.
 __device__ __forceinline__ uint32_t load_cell(const uint32_t *p) { return __ldg(p); }
 

@@ -22,6 +22,7 @@ struct DivMagic {
   uint64_t d;
   uint64_t m;
   uint32_t sh1, sh2;
+  uint64_t inv;   // floor((2^64 - 1) / d), for mod_once
 };
 
 DivMagic make_div_magic(uint64_t d);
@@ -118,6 +119,7 @@ struct k2g_db {
   uint64_t *d_size = nullptr;     // device-side size counter used by builds
   k2g::DivMagic div{};
   bool owns_table = true;
+  bool counted = false;           // among the databases that keep the scratch pool alive
   // scheduling values per (paired, length class); guarded by tune_mu
   mutable std::mutex tune_mu;
   k2g::Tuning tune[2][K2G_LEN_CLASSES] = {
@@ -143,12 +145,17 @@ k2g_status require_dna(const k2g_db *db);
 k2g_status classify_translated(const k2g_db *db, const k2g_reads *reads,
                                const k2g_classify_params *params, k2g_results *out,
                                cudaStream_t st);
-// Classification of short fragments in one launch, without device scratch
-// (warp_classify.cu): whether it takes a call, and the call itself.
+// Classification by warps on the caller's stream (warp_classify.cu): whether
+// it takes a call, and the call itself.
 struct ClassifyArgs;
 bool warp_classify_takes(const ClassifyArgs &a, uint64_t max_len);
-cudaError_t warp_classify(const ClassifyArgs &a, const uint2 *span, uint64_t total_bases, int sms,
-                          cudaStream_t st);
+cudaError_t warp_classify(const ClassifyArgs &a, const uint2 *span, uint64_t max_len, uint64_t total_bases,
+                          uint32_t piece_len, int device, int sms, cudaStream_t st);
+// Device scratch of one call, allocated on its stream (given back by
+// cudaFreeAsync), and the databases that keep the pool alive (scratch.cu).
+cudaError_t scratch_alloc(void **p, size_t bytes, int device, cudaStream_t st);
+void scratch_db_opened(int device);
+void scratch_db_closed(int device);
 // Counts each kernel launch issued by the library (k2g_kernel_launches).
 void note_launches(uint64_t n = 1);
 // One round (< 2^30 pairs) of the order-exact build insert (build_ordered.cu).

@@ -888,8 +888,9 @@ k2g_status k2g::classify_keyed(const k2g_db *db, const k2g_reads *reads,
     total = ends[1] - ends[0];
   }
   const Tuning tn = db->tuning(params->paired != 0, total, reads->n_frags);
-  if (mode == K2G_MODE_PIPELINED && tn.pipeline && warp_classify_takes(a, reads->max_seq_len)) {
-    K2G_CUDA_TRY(warp_classify(a, db->d_span, total, sm_count(db->device), st));
+  if (mode == K2G_MODE_PIPELINED && warp_classify_takes(a, reads->max_seq_len)) {
+    K2G_CUDA_TRY(warp_classify(a, db->d_span, reads->max_seq_len, total, tn.piece_len, db->device,
+                               sm_count(db->device), st));
     return K2G_OK;
   }
   return run_classify(db, a, mode, reads->max_seq_len, total, st, state_key, tn);

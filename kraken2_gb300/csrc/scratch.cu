@@ -1,0 +1,63 @@
+// Device scratch of single calls: stream-ordered allocations from a memory
+// pool of the library's own, one per device.  A call allocates on its stream
+// and gives the memory back on it, so calls on any streams and threads share
+// the pool safely, and a captured call's allocations become part of its
+// graph.  The pool keeps up to kKeep bytes between calls (a pool that keeps
+// nothing maps the memory anew after every synchronisation, about 0.8 ms a
+// call) and gives everything back when the device's last database is closed.
+#include <cuda_runtime.h>
+
+#include <mutex>
+
+#include "k2g_internal.h"
+
+namespace k2g {
+namespace {
+
+constexpr uint64_t kKeep = 256ull << 20;
+
+struct Pool {
+  std::mutex mu;
+  cudaMemPool_t pool = nullptr;
+  int dbs = 0;
+};
+Pool g_pools[64];
+
+}  // namespace
+
+cudaError_t scratch_alloc(void **p, size_t bytes, int device, cudaStream_t st) {
+  Pool &d = g_pools[device & 63];
+  {
+    std::lock_guard<std::mutex> lock(d.mu);
+    if (!d.pool) {
+      cudaMemPoolProps props = {};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.handleTypes = cudaMemHandleTypeNone;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = device;
+      cudaError_t e = cudaMemPoolCreate(&d.pool, &props);
+      if (e != cudaSuccess) {
+        d.pool = nullptr;
+        return e;
+      }
+      uint64_t keep = kKeep;
+      e = cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+      if (e != cudaSuccess) return e;
+    }
+  }
+  return cudaMallocFromPoolAsync(p, bytes ? bytes : 1, d.pool, st);
+}
+
+void scratch_db_opened(int device) {
+  Pool &d = g_pools[device & 63];
+  std::lock_guard<std::mutex> lock(d.mu);
+  d.dbs++;
+}
+
+void scratch_db_closed(int device) {
+  Pool &d = g_pools[device & 63];
+  std::lock_guard<std::mutex> lock(d.mu);
+  if (--d.dbs == 0 && d.pool) cudaMemPoolTrimTo(d.pool, 0);
+}
+
+}  // namespace k2g

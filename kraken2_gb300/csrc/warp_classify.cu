@@ -1,19 +1,35 @@
-// The one-launch classification of short fragments (warp_classify.cuh).
+// The one-launch classification of short fragments, and long fragments in
+// pieces (warp_classify.cuh).
 #include <algorithm>
 
 #include "k2g_internal.h"
 #include "warp_classify.cuh"
 
 namespace k2g {
+namespace {
 
-template <bool WIDE, bool HITS>
-static cudaError_t launch_warp(const WcArgs &wa, cudaStream_t st) {
-  const uint64_t blocks = (wa.n_groups + kWcWarps - 1) / kWcWarps;
-  warp_classify_kernel<WIDE, HITS>
+// Nominal length of a warp's piece, in tuned piece lengths (those are for one
+// lane): 2,048 bases by default.  A warp takes about 30 us for that beside
+// the others of its SM, so the last pieces to run do not keep the device long.
+constexpr uint32_t kWarpPieces = 4;
+
+template <bool WIDE, bool HITS, bool LONG>
+cudaError_t launch_warp(const WcArgs &wa, cudaStream_t st) {
+  const uint64_t blocks = (wa.piece_slots + wa.n_groups + kWcWarps - 1) / kWcWarps;
+  warp_classify_kernel<WIDE, HITS, LONG>
       <<<(unsigned)blocks, kWcWarps * 32, kWcWarps * sizeof(WcShared), st>>>(wa);
   note_launches();
   return cudaGetLastError();
 }
+
+template <bool LONG>
+cudaError_t launch(const WcArgs &wa, cudaStream_t st) {
+  const bool hits = wa.a.hit_keys != nullptr;
+  if (wa.a.table.wide) return hits ? launch_warp<true, true, LONG>(wa, st) : launch_warp<true, false, LONG>(wa, st);
+  return hits ? launch_warp<false, true, LONG>(wa, st) : launch_warp<false, false, LONG>(wa, st);
+}
+
+}  // namespace
 
 bool warp_classify_takes(const ClassifyArgs &a, uint64_t max_len) {
   // (a walk that goes on keeps its sector's number in 32 bits)
@@ -21,21 +37,51 @@ bool warp_classify_takes(const ClassifyArgs &a, uint64_t max_len) {
   return a.scan.w == 5 && a.scan.revcom_version != 0 && max_len <= kWcMaxLen && sectors < (1ull << 32);
 }
 
-cudaError_t warp_classify(const ClassifyArgs &a, const uint2 *span, uint64_t total_bases, int sms,
-                          cudaStream_t st) {
-  WcArgs wa{a, span, 0, 0};
+cudaError_t warp_classify(const ClassifyArgs &a, const uint2 *span, uint64_t max_len, uint64_t total_bases,
+                          uint32_t piece_len, int device, int sms, cudaStream_t st) {
+  WcArgs wa{a, span, 0, 0, 0};
+  // Single fragments of two pieces and more are cut (quick mode stops inside
+  // a fragment, and a pair carries a mate border: those stay whole).
+  const uint32_t piece = std::min(kWarpPieces * piece_len, kPieceLenMax);
+  const bool split = !a.cls.paired && !a.cls.quick && max_len >= 2ull * piece;
   // Fragments per group: as many as keep every warp slot of the device busy
-  // (24 warps per SM are resident), up to about 1,600 bases (their entries
-  // fill the shared-memory list once).
+  // (kWcWarps * kWcBlocks per SM), up to about 1,600 bases (their entries
+  // fill the shared-memory list once); 4 where long fragments are cut, since
+  // the average says nothing of the others then.
   const double avg = (double)total_bases / (double)a.n_frags;
-  while ((2u << wa.log_reads) <= (uint32_t)kWcReads &&
-         (a.n_frags >> (wa.log_reads + 1)) >= (uint64_t)sms * 24 &&
-         avg * (double)(2u << wa.log_reads) <= 1600.0)
+  while ((2u << wa.log_reads) <= (uint32_t)(split ? 4 : kWcReads) &&
+         (a.n_frags >> (wa.log_reads + 1)) >= (uint64_t)sms * kWcWarps * kWcBlocks &&
+         (split || avg * (double)(2u << wa.log_reads) <= 1600.0))
     wa.log_reads++;
   wa.n_groups = (a.n_frags + (1ull << wa.log_reads) - 1) >> wa.log_reads;
-  const bool hits = a.hit_keys != nullptr;
-  if (a.table.wide) return hits ? launch_warp<true, true>(wa, st) : launch_warp<true, false>(wa, st);
-  return hits ? launch_warp<false, true>(wa, st) : launch_warp<false, false>(wa, st);
+  if (!split) return launch<false>(wa, st);
+
+  const uint64_t pc = split_pieces_cap(total_bases, piece), fc = split_frags_cap(total_bases, piece);
+  const size_t at_pieces = 64, at_frags = at_pieces + pc * sizeof(SplitPiece),
+               at_mark = at_frags + fc * sizeof(SplitFrag);
+  unsigned char *mem = nullptr;
+  cudaError_t e = scratch_alloc(reinterpret_cast<void **>(&mem), at_mark + a.n_frags, device, st);
+  if (e != cudaSuccess) return e;
+  SplitBufs b{mem + at_mark, reinterpret_cast<SplitPiece *>(mem + at_pieces), pc,
+              reinterpret_cast<SplitFrag *>(mem + at_frags), fc, nullptr, nullptr,
+              reinterpret_cast<unsigned long long *>(mem), piece};
+  e = cudaMemsetAsync(mem, 0, at_frags, st);
+  if (e == cudaSuccess) e = split_plan(a, b, sms, st);
+  if (e == cudaSuccess) {
+    wa.a.pieces = b.pieces;
+    wa.a.n_pieces = b.ctr;
+    wa.a.split_mark = b.mark;
+    wa.piece_slots = pc;
+    e = launch<true>(wa, st);
+  }
+  if (e == cudaSuccess) {
+    const uint64_t blocks = std::min<uint64_t>((fc + kMergeWarps - 1) / kMergeWarps, (uint64_t)sms * 12);
+    warp_merge_kernel<<<(unsigned)blocks, kMergeWarps * 32, 0, st>>>(a, span, b);
+    note_launches();
+    e = cudaGetLastError();
+  }
+  const cudaError_t ef = cudaFreeAsync(mem, st);
+  return e != cudaSuccess ? e : ef;
 }
 
 }  // namespace k2g

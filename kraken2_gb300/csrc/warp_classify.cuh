@@ -2,7 +2,7 @@
 //
 // A group is up to kWcReads consecutive fragments.  Its warp runs the whole
 // path -- scan, table lookups, hit lists, ResolveTree -- with everything in
-// between in registers and 9.4 KB of shared memory, so a call is one launch
+// between in registers and 8 KB of shared memory, so a call is one launch
 // with no device scratch:
 //   pack     16 bases per lane to 2-bit words in shared memory: forward
 //            (first base high) and complement (first base low), so that an
@@ -13,9 +13,10 @@
 //            minima come from prefix and suffix minima of blocks of four.
 //            The starts of token groups (src/classify.cc:797-838) become
 //            entries (key, fragment, token position) in token order;
-//   probe    one entry per lane, four table sectors in flight per lane; walks
+//   probe    one entry per lane, three table sectors in flight per lane; walks
 //            that leave their home sector are listed and finished together
-//            (src/compact_hash.h:355-392);
+//            (src/compact_hash.h:355-392; a sector of every listed walk at a
+//            time, all lanes in step, was 13 % slower);
 //   replay   32 entries at a time: equal neighbours join into hit-list runs
 //            (src/classify.cc:950-991), every finished run adds its tokens to
 //            its fragment's taxon map, hits are counted by ballots;
@@ -33,19 +34,21 @@
 #pragma once
 
 #include "classify_core.cuh"
+#include "classify_split.h"
 
 namespace k2g {
 
-constexpr int kWcWarps = 2;           // warps per block
+// Warps per block and blocks per SM, and table sectors in flight per lane of
+// a probe: 2 x 14 and 3.  On 2M x 150 bp reads, 4 GB table: 2.30 ms; 2 x 12
+// and 4: 2.37, 2 x 12 and 5: 2.51, 2 x 16 and 2 (with half the entries): 2.38.
+constexpr int kWcWarps = 2, kWcBlocks = 14;
 constexpr int kWcReads = 8;           // most fragments per group
-constexpr int kWcEntries = 352;       // entries held before a probe and replay
-constexpr int kWcSlots = 256;         // taxon map slots per warp, shared out among its fragments
+constexpr int kWcEntries = 320;       // entries held before a probe and replay
+constexpr int kWcLogSlots = 7, kWcSlots = 1 << kWcLogSlots;   // taxon map slots per warp, shared out among its fragments
 constexpr int kWcWindow = 2048;       // bases packed at a time
 constexpr int kWcPos = 8;             // l-mer positions per lane
-// Longest sequence the one-launch path takes (a lane group walks a sequence
-// at about 70 bases per microsecond, so this bounds a warp's time to about
-// 0.1 ms).
-constexpr uint64_t kWcMaxLen = 8192;
+// Longest sequence taken: token positions of a fragment fit kEPosBits.
+constexpr uint64_t kWcMaxLen = 1ull << 26;
 
 // Entry kinds (two bits of an entry's meta word: kind, fragment, position).
 enum : uint32_t { E_KEY = 0, E_AMBIG = 1, E_BORDER = 2, E_CONT = 3 };
@@ -56,6 +59,11 @@ struct WcArgs {
   const uint2 *span;      // per taxon: preorder number, one past its subtree's last
   uint32_t log_reads;     // fragments per group = 1 << log_reads <= kWcReads
   uint64_t n_groups;
+  // Pieces of long fragments (classify_split.h), one warp each, before the
+  // groups: a piece's tokens are those of a read of its own that starts k - 1
+  // bases before its cut.  a.pieces and a.n_pieces say which slots hold one;
+  // the groups pass over the fragments in a.split_mark.
+  uint64_t piece_slots;
 };
 
 // One warp's shared memory.
@@ -178,25 +186,37 @@ __device__ __forceinline__ uint32_t wc_walk(const TableView &t, uint64_t hc, uin
   return 0;
 }
 
-// Adds n tokens of a taxon to fragment r's part of the warp's taxon map.
-__device__ __forceinline__ void wc_count(WcShared &s, uint32_t log_slots, uint32_t r, uint32_t taxon,
-                                         uint32_t n) {
-  const uint32_t mask = (1u << log_slots) - 1u, base = r << log_slots;
-  uint32_t i = ((taxon * 0x9E3779B1u) >> 16) & mask;
-  for (uint32_t probes = 0; probes <= mask; probes++) {
-    const uint32_t old = atomicCAS(&s.mkey[base + i], 0u, taxon);
-    if (old == 0) {
-      atomicAdd(&s.n_taxa[r], 1u);
-      s.a_slot[r] = base + i;
+// A taxon -> tokens map: open addressing over `mask` + 1 slots, key 0 empty.
+struct WcMap {
+  uint32_t *key, *cnt;
+  uint32_t mask, step;   // slot i at key[i * step], cnt[i * step]
+  __device__ __forceinline__ uint32_t home(uint32_t taxon) const { return ((taxon * 0x9E3779B1u) >> 16) & mask; }
+  // Adds n tokens; the slot, kOld | the slot where the taxon was there
+  // already, or ~0 when the map is full.
+  static constexpr uint32_t kOld = 0x80000000u;
+  __device__ __forceinline__ uint32_t add(uint32_t taxon, uint32_t n) const {
+    uint32_t i = home(taxon);
+    for (uint32_t probes = 0; probes <= mask; probes++) {
+      const uint32_t old = atomicCAS(&key[i * step], 0u, taxon);
+      if (old == 0 || old == taxon) {
+        atomicAdd(&cnt[i * step], n);
+        return old ? i | kOld : i;
+      }
+      i = (i + 1) & mask;
     }
-    if (old == 0 || old == taxon) {
-      atomicAdd(&s.mcnt[base + i], n);
-      return;
-    }
-    i = (i + 1) & mask;
+    return 0xFFFFFFFFu;
   }
-  atomicOr(&s.over, 1u << r);   // resolved from the fragment's runs
-}
+  __device__ __forceinline__ uint32_t get(uint32_t taxon) const {
+    uint32_t i = home(taxon);
+    for (uint32_t probes = 0; probes <= mask; probes++) {
+      const uint32_t k = key[i * step];
+      if (k == taxon) return cnt[i * step];
+      if (k == 0) return 0;
+      i = (i + 1) & mask;
+    }
+    return 0;
+  }
+};
 
 __device__ __forceinline__ bool in_span(uint2 s, uint32_t pre) { return s.x <= pre && pre < s.y; }
 
@@ -205,22 +225,22 @@ __device__ __forceinline__ bool in_span(uint2 s, uint32_t pre) { return s.x <= p
 // until the tokens of its subtree reach `required` (sum_of and in_tree give
 // the tokens of a taxon and of a subtree).
 template <class SumOf, class InTree>
-__device__ __forceinline__ uint32_t wc_climb(const ClassifyArgs &a, const uint2 *span, uint32_t from,
+__device__ __forceinline__ uint32_t wc_climb(const uint32_t *parent, const uint2 *span, uint32_t from,
                                              uint32_t hi, uint32_t required, SumOf sum_of,
                                              InTree in_tree) {
   uint32_t call = from;
-  while (call && hi >= __ldg(&span[call].y)) call = __ldg(a.parent + call);
+  while (call && hi >= __ldg(&span[call].y)) call = __ldg(parent + call);
   uint32_t score = sum_of(call);
   while (call && score < required) {
     score = in_tree(__ldg(span + call));
     if (score >= required) break;
-    call = __ldg(a.parent + call);
+    call = __ldg(parent + call);
   }
   return call;
 }
 
 // ResolveTree over `many` <= 32 distinct taxa, in the first lanes (t = 0: none).
-__device__ __forceinline__ uint32_t wc_resolve(const ClassifyArgs &a, const uint2 *span, uint32_t t,
+__device__ __forceinline__ uint32_t wc_resolve(const uint32_t *parent, const uint2 *span, uint32_t t,
                                                uint32_t n, int many, uint32_t required) {
   const uint2 sp = t ? __ldg(span + t) : make_uint2(0xFFFFFFFFu, 0u);
   uint32_t score = 0;
@@ -236,57 +256,120 @@ __device__ __forceinline__ uint32_t wc_resolve(const ClassifyArgs &a, const uint
   const uint32_t at = __ballot_sync(0xffffffffu, top && sp.x == lo);
   const uint32_t from = __shfl_sync(0xffffffffu, t, __ffs(at) - 1);
   return wc_climb(
-      a, span, from, hi, required,
+      parent, span, from, hi, required,
       [&](uint32_t x) { return __reduce_add_sync(0xffffffffu, t && t == x ? n : 0u); },
       [&](uint2 x) { return __reduce_add_sync(0xffffffffu, t && in_span(x, sp.x) ? n : 0u); });
 }
 
-// ResolveTree over a list of (taxon, tokens) items, zero taxa skipped and
-// taxa possibly repeated: a fragment with more taxa than lanes (its map) or
-// than map slots (its hit-list runs).  Quadratic in the items, spread over
-// the lanes; such fragments are rare.
-template <class Item>
-__device__ __noinline__ uint32_t wc_resolve_items(const ClassifyArgs &a, const uint2 *span,
-                                                  uint32_t count, uint32_t required, Item item) {
-  const uint32_t lane = threadIdx.x & 31;
-  uint32_t best = 0, lo = 0xFFFFFFFFu, hi = 0, from = 0;
-  for (uint32_t i0 = 0; i0 < count; i0 += 32) {
-    const uint2 it = i0 + lane < count ? item(i0 + lane) : make_uint2(0, 0);
-    const uint32_t pre = it.x ? __ldg(&span[it.x].x) : 0;
-    uint32_t score = 0;
-    for (uint32_t j = 0; j < count; j++) {
-      const uint2 o = item(j);
-      if (o.x && it.x && in_span(__ldg(span + o.x), pre)) score += o.y;
-    }
-    if (it.x && score > best) {
-      best = score;
+// The highest score seen by a lane, and the taxa that reach it.
+struct WcBest {
+  uint32_t score = 0, lo = 0xFFFFFFFFu, hi = 0, from = 0;
+  __device__ __forceinline__ void see(uint32_t taxon, uint32_t pre, uint32_t s) {
+    if (s > score) {
+      score = s;
       lo = hi = pre;
-      from = it.x;
-    } else if (it.x && score == best) {
+      from = taxon;
+    } else if (s == score) {
       if (pre < lo) {
         lo = pre;
-        from = it.x;
+        from = taxon;
       }
       hi = max(hi, pre);
     }
   }
-  const uint32_t most = __reduce_max_sync(0xffffffffu, best);
-  if (!most) return 0;
-  const uint32_t all_lo = __reduce_min_sync(0xffffffffu, best == most ? lo : 0xFFFFFFFFu);
-  hi = __reduce_max_sync(0xffffffffu, best == most ? hi : 0u);
-  const uint32_t at = __ballot_sync(0xffffffffu, best == most && lo == all_lo);
-  from = __shfl_sync(0xffffffffu, from, __ffs(at) - 1);
+  // the same over the warp; false when nothing was seen
+  __device__ __forceinline__ bool join() {
+    const uint32_t most = __reduce_max_sync(0xffffffffu, score);
+    if (!most) return false;
+    const uint32_t all_lo = __reduce_min_sync(0xffffffffu, score == most ? lo : 0xFFFFFFFFu);
+    hi = __reduce_max_sync(0xffffffffu, score == most ? hi : 0u);
+    const uint32_t at = __ballot_sync(0xffffffffu, score == most && lo == all_lo);
+    from = __shfl_sync(0xffffffffu, from, __ffs(at) - 1);
+    return true;
+  }
+};
+
+// ResolveTree over a map of any size, a taxon per lane at a time: its score
+// from its path to the root.
+static __device__ __noinline__ uint32_t wc_resolve_map(const uint32_t *parent, const uint2 *span, WcMap m,
+                                                       uint32_t required) {
+  const uint32_t lane = threadIdx.x & 31;
+  WcBest best;
+  for (uint32_t i = lane; i <= m.mask; i += 32) {
+    const uint32_t t = m.key[i * m.step];
+    if (!t) continue;
+    uint32_t score = 0;
+    for (uint32_t x = t; x; x = __ldg(parent + x)) score += m.get(x);
+    best.see(t, __ldg(&span[t].x), score);
+  }
+  __syncwarp();
+  if (!best.join()) return 0;
+  return wc_climb(parent, span, best.from, best.hi, required, [&](uint32_t x) { return x ? m.get(x) : 0u; },
+                  [&](uint2 x) {
+                    uint32_t sum = 0;
+                    for (uint32_t i = lane; i <= m.mask; i += 32) {
+                      const uint32_t t = m.key[i * m.step];
+                      if (t && in_span(x, __ldg(&span[t].x))) sum += m.cnt[i * m.step];
+                    }
+                    __syncwarp();
+                    return __reduce_add_sync(0xffffffffu, sum);
+                  });
+}
+
+// A hit-list run as this warp wrote it.
+__device__ __forceinline__ uint2 wc_run(const uint64_t *runs, uint32_t i) {
+  const uint64_t x = *const_cast<const volatile uint64_t *>(runs + i);
+  const uint32_t t = (uint32_t)(x >> 32);
+  return make_uint2(t < K2G_CODE_AMBIGUOUS ? t : 0u, (uint32_t)x);
+}
+
+// ResolveTree from a fragment's runs, for one with more taxa than any map at
+// hand holds: quadratic in the runs, spread over the lanes.
+static __device__ __noinline__ uint32_t wc_resolve_runs(const uint32_t *parent, const uint2 *span,
+                                                        const uint64_t *runs, uint32_t count,
+                                                        uint32_t required) {
+  const uint32_t lane = threadIdx.x & 31;
+  WcBest best;
+  for (uint32_t i0 = 0; i0 < count; i0 += 32) {
+    const uint2 it = i0 + lane < count ? wc_run(runs, i0 + lane) : make_uint2(0, 0);
+    const uint32_t pre = it.x ? __ldg(&span[it.x].x) : 0;
+    uint32_t score = 0;
+    for (uint32_t j = 0; j < count; j++) {
+      const uint2 o = wc_run(runs, j);
+      if (o.x && it.x && in_span(__ldg(span + o.x), pre)) score += o.y;
+    }
+    if (it.x) best.see(it.x, pre, score);
+  }
+  if (!best.join()) return 0;
   auto sum = [&](auto pick) {
     uint32_t s = 0;
     for (uint32_t i = lane; i < count; i += 32) {
-      const uint2 o = item(i);
+      const uint2 o = wc_run(runs, i);
       if (o.x && pick(o.x)) s += o.y;
     }
+    __syncwarp();
     return __reduce_add_sync(0xffffffffu, s);
   };
-  return wc_climb(
-      a, span, from, hi, required, [&](uint32_t x) { return sum([&](uint32_t t) { return t == x; }); },
-      [&](uint2 x) { return sum([&](uint32_t t) { return in_span(x, __ldg(&span[t].x)); }); });
+  return wc_climb(parent, span, best.from, best.hi, required,
+                  [&](uint32_t x) { return sum([&](uint32_t t) { return t == x; }); },
+                  [&](uint2 x) { return sum([&](uint32_t t) { return in_span(x, __ldg(&span[t].x)); }); });
+}
+
+// ResolveTree over a map of `taxa` > 0 taxa in shared memory; `list` holds 32.
+__device__ __forceinline__ uint32_t wc_resolve_slots(const uint32_t *parent, const uint2 *span, const WcMap &m,
+                                                     uint32_t taxa, uint2 *list, uint32_t required) {
+  if (taxa > 32) return wc_resolve_map(parent, span, m, required);
+  const uint32_t lane = threadIdx.x & 31, lt = (1u << lane) - 1u;
+  int n = 0;
+  for (uint32_t i0 = 0; i0 <= m.mask; i0 += 32) {
+    const uint32_t t = i0 + lane <= m.mask ? m.key[i0 + lane] : 0;
+    const uint32_t b = __ballot_sync(0xffffffffu, t != 0);
+    if (t) list[n + __popc(b & lt)] = make_uint2(t, m.cnt[i0 + lane]);
+    n += __popc(b);
+  }
+  __syncwarp();
+  const uint2 x = (int)lane < n ? list[lane] : make_uint2(0, 0);
+  return wc_resolve(parent, span, x.x, x.y, n, required);
 }
 
 // ---- the kernel --------------------------------------------------------------
@@ -299,6 +382,7 @@ struct Wc {
   const uint32_t lt;            // lanes below
   uint64_t f0;                  // first fragment of the group
   uint32_t log_slots;           // taxon map slots per fragment
+  uint32_t first_pos;           // position of a fragment's first token
   uint32_t key_shift;           // keys are held in the top bits
   uint64_t toggle_top;
   // carried from one replay to the next (the same in all lanes): the run
@@ -311,9 +395,15 @@ struct Wc {
     return *reinterpret_cast<const uint64_t *>(&s.entry[i]);
   }
 
-  // Get() for every key entry.
+  __device__ __forceinline__ WcMap map_of(uint32_t r) const {
+    return WcMap{s.mkey + (r << log_slots), s.mcnt + (r << log_slots), (1u << log_slots) - 1u, 1u};
+  }
+
+  // Get() for every key entry: the home sectors of all, then the next sector
+  // of every walk that goes on, and so on (about one walk in five leaves its
+  // home sector at load 0.7, and one in four of those goes on again).
   __device__ __forceinline__ void probe(int ne) {
-    constexpr int B = 4;
+    constexpr int B = 3;
     constexpr uint32_t N = WIDE ? 4 : 8, kLogN = WIDE ? 2 : 3;
     const TableView &t = a.table;
     uint16_t *list = reinterpret_cast<uint16_t *>(s.be);
@@ -321,6 +411,7 @@ struct Wc {
     // look empty, so an absent key found there is looked up once more
     const uint64_t partial = t.capacity & (N - 1) ? t.capacity & ~(uint64_t)(N - 1) : ~0ull;
     int n_list = 0;
+    bool redo = false;
 #pragma unroll 1
     for (int i0 = 0; i0 < ne; i0 += 32 * B) {
       uint64_t hc[B], idx[B];
@@ -333,7 +424,7 @@ struct Wc {
         hc[b] = murmur3(key_of(top));
         // a subsampled minimizer (-M) is not looked up: its value is 0
         const bool look = top != ~0ull && hc[b] >= a.scan.min_hash;
-        idx[b] = look ? fast_mod(hc[b], t.div) : 0;
+        idx[b] = look ? mod_once(hc[b], t.div) : 0;
         ask |= look ? 1u << b : 0u;
         sec[b] = wc_load<WIDE>(t, idx[b] & ~(uint64_t)(N - 1));
       }
@@ -350,6 +441,7 @@ struct Wc {
         // a walk that goes on leaves its sector's number instead of a value
         if (look) s.entry[i].w = on ? (uint32_t)(base >> kLogN) : v;
         n_list += __popc(m);
+        redo |= again;
       }
     }
     __syncwarp();
@@ -482,9 +574,9 @@ struct Wc {
       if (j < nh) nx = *reinterpret_cast<const uint2 *>(&s.entry[j]);
       const bool ends = j < n_items && it.y != 0xFFFFFFFFu && (j < nh || last);
       const uint32_t start = it.y & below(kEPosBits), r = (it.y >> kEPosBits) & 7u;
-      // runs of the fragment before this one (its first run starts at 0)
+      // runs of the fragment before this one (its first run starts at first_pos)
       const uint32_t le = lt | (1u << lane);
-      const uint32_t firsts = __ballot_sync(0xffffffffu, j < n_items && it.y != 0xFFFFFFFFu && start == 0);
+      const uint32_t firsts = __ballot_sync(0xffffffffu, j < n_items && it.y != 0xFFFFFFFFu && start == first_pos);
       const uint32_t rank = (firsts & le) ? (uint32_t)(lane - last_bit(firsts & le)) : open_rank + (uint32_t)lane;
       if (ends) {
         const bool same = (nx.y >> kEPosBits) == (it.y >> kEPosBits);
@@ -493,7 +585,15 @@ struct Wc {
         if (at < a.runs_cap) a.runs[at] = ((uint64_t)it.x << 32) | n;
         else atomicOr(a.status, STATUS_RUNS_OVERFLOW);
         if (!same) s.n_runs[r] = rank + 1;
-        if (it.x && it.x < K2G_CODE_AMBIGUOUS) wc_count(s, log_slots, r, it.x, n);
+        if (it.x && it.x < K2G_CODE_AMBIGUOUS) {
+          const uint32_t slot = map_of(r).add(it.x, n);
+          if (slot == 0xFFFFFFFFu) {
+            atomicOr(&s.over, 1u << r);   // resolved from the fragment's runs
+          } else if (!(slot & WcMap::kOld)) {
+            atomicAdd(&s.n_taxa[r], 1u);
+            s.a_slot[r] = (r << log_slots) + slot;
+          }
+        }
       }
       const int tail = min(31, n_items - 1 - j0);
       const uint32_t tail_rank = __shfl_sync(0xffffffffu, rank, tail);
@@ -511,37 +611,60 @@ struct Wc {
   }
 };
 
-template <bool WIDE, bool HITS>
-__global__ void __launch_bounds__(kWcWarps * 32, 12) warp_classify_kernel(WcArgs wa) {
+// LONG: the call's long fragments come as pieces.
+template <bool WIDE, bool HITS, bool LONG>
+__global__ void __launch_bounds__(kWcWarps * 32, kWcBlocks) warp_classify_kernel(WcArgs wa) {
   extern __shared__ __align__(16) unsigned char smem[];
   const ClassifyArgs &a = wa.a;
-  const uint64_t group = blockIdx.x * (uint64_t)kWcWarps + (threadIdx.x >> 5);
-  if (group >= wa.n_groups) return;   // the whole warp; the block has no barriers
+  // (whole warps return: the block has no barriers)
+  const uint64_t task = blockIdx.x * (uint64_t)kWcWarps + (threadIdx.x >> 5);
+  bool piece = false;
+  uint64_t f0 = 0;
+  uint32_t hi = 0, first_pos = 0;     // of a piece: the k-mers ending at k - 1 + first_pos .. hi - 1
+  if constexpr (LONG) {
+    piece = task < wa.piece_slots;
+    if (task >= wa.piece_slots + wa.n_groups || (piece && task >= (uint64_t)*a.n_pieces)) return;
+    f0 = (task - wa.piece_slots) << wa.log_reads;
+    if (piece) {
+      f0 = a.pieces[task].frag;
+      first_pos = a.pieces[task].lo - (uint32_t)(a.scan.k - 1);
+      hi = a.pieces[task].hi;
+      if (!hi) return;
+    }
+  } else {
+    if (task >= wa.n_groups) return;
+    f0 = task << wa.log_reads;
+  }
   WcShared &s = reinterpret_cast<WcShared *>(smem)[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const uint32_t lt = (1u << lane) - 1u, le = lt | (1u << lane);
   const int k = a.scan.k, l = a.scan.l;
-  const uint64_t f0 = group << wa.log_reads;
-  const int nr = (int)min((uint64_t)1 << wa.log_reads, a.n_frags - f0);
+  const int nr = piece ? 1 : (int)min((uint64_t)1 << wa.log_reads, a.n_frags - f0);
   const int per = a.cls.paired ? 2 : 1, ns = nr * per;
   const uint32_t key_shift = 64u - 2u * (uint32_t)l;
-  Wc<WIDE, HITS> w{a, s, lane, lt, f0, 8u - wa.log_reads, key_shift, a.scan.toggle << key_shift};
+  Wc<WIDE, HITS> w{a, s, lane, lt, f0, piece ? kWcLogSlots : kWcLogSlots - wa.log_reads, first_pos, key_shift,
+                   a.scan.toggle << key_shift};
   const uint64_t mask_top = (a.scan.spaced_mask ? a.scan.spaced_mask & a.scan.lmer_mask : a.scan.lmer_mask)
                             << key_shift;
 
   // ---- the group's sequences: lane i holds sequence i
-  const uint64_t o = lane <= ns ? a.seq_off[f0 * per + lane] : 0;
+  uint64_t o = lane <= ns ? a.seq_off[f0 * per + (piece ? 0 : lane)] : 0;
+  const uint64_t runs_at = o;
+  if (piece) o += lane ? hi : first_pos;
   const uint64_t o0 = __shfl_sync(0xffffffffu, o, 0);
   const uint64_t o_end = __shfl_sync(0xffffffffu, o, ns);
   const uint64_t o_next = __shfl_down_sync(0xffffffffu, o, 1);
-  const uint32_t len = lane < ns ? (uint32_t)(o_next - o) : 0;
+  // (a fragment that its pieces carry has no part in the group)
+  bool mine = lane < ns;
+  if constexpr (LONG) mine = mine && (piece || !a.split_mark[f0 + lane / per]);
+  const uint32_t len = mine ? (uint32_t)(o_next - o) : 0;
   const uint32_t kmers = len >= (uint32_t)k ? len - (uint32_t)k + 1 : 0;
   const bool mate2 = per == 2 && (lane & 1);
   const uint32_t mate1_kmers = __shfl_up_sync(0xffffffffu, kmers, 1);
   const uint32_t mate2_kmers = __shfl_down_sync(0xffffffffu, kmers, 1);
   // work items: 8 positions each from the first l-mer's end on; a second
   // mate without k-mers keeps one item for the mate border
-  const uint32_t items = kmers ? (len - (uint32_t)(l - 1) + kWcPos - 1) / kWcPos : (mate2 && lane < ns ? 1u : 0u);
+  const uint32_t items = kmers ? (len - (uint32_t)(l - 1) + kWcPos - 1) / kWcPos : (mate2 && mine ? 1u : 0u);
   uint32_t incl = items;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
@@ -561,11 +684,11 @@ __global__ void __launch_bounds__(kWcWarps * 32, 12) warp_classify_kernel(WcArgs
   const uint32_t stream_end = lead + (uint32_t)(o_end - o0);
   if (items)
     s.seq[__popc(busy & lt)] = make_uint4(lead + (uint32_t)(o - o0), len, first_item,
-                                          (uint32_t)(lane / per) | (mate2 ? 8u | ((mate1_kmers + 1) << 4) : 0u));
+                                          (uint32_t)(lane / per) | (mate2 ? 8u | ((mate1_kmers + 1) << 4) : first_pos << 4));
   if (lane < ns && lane % per == 0) {
     const int r = lane / per;
-    s.run_base[r] = o + 2 * (f0 + r + a.frag_off);
-    s.tokens[r] = per == 2 ? kmers + 1 + mate2_kmers : kmers;
+    s.run_base[r] = runs_at + 2 * (f0 + r + a.frag_off) + first_pos;
+    s.tokens[r] = per == 2 ? kmers + 1 + mate2_kmers : first_pos + kmers;
     s.hits[r] = 0;
     s.n_runs[r] = 0;
     s.n_taxa[r] = 0;
@@ -585,16 +708,17 @@ __global__ void __launch_bounds__(kWcWarps * 32, 12) warp_classify_kernel(WcArgs
   uint64_t seen_min = 0;              // last unambiguous minimizer, and its sequence
   uint32_t seen_seq = 0xFFFFFFFFu;
   int ne = 0;
+  bool own0 = true;                   // lane 0's item is not a repeated one
+  (void)own0;
   bool done = n_items == 0;
   while (!done) {
     bool full = false;
 #pragma unroll 1
     while (!done && !full) {
       // item of this lane: the sequence whose first item is the last at or
-      // before it.  From the second pass on lane 0 repeats the item before,
-      // for the lane above.
+      // before it.  A pass that goes on inside a sequence repeats the item
+      // before in lane 0, for the lane above.
       const uint32_t g = g0 + (uint32_t)lane;
-      const bool in = g < n_items, own = in && (lane > 0 || g0 == 0);
       const uint32_t rel = first_item - g0;   // (wraps for earlier sequences)
       const uint32_t starts = __reduce_or_sync(0xffffffffu, rel < 32 ? 1u << rel : 0u);
       const uint32_t before = __popc(__ballot_sync(0xffffffffu, first_item < g0));
@@ -640,6 +764,16 @@ __global__ void __launch_bounds__(kWcWarps * 32, 12) warp_classify_kernel(WcArgs
         }
         __syncwarp();
       }
+      // (items behind a gap that the window does not reach wait for a later pass)
+      bool in = g < n_items;
+      int n_in = 32;
+      if constexpr (LONG) {
+        in = in && q0 + kWcPos <= (int)win_hi;
+        n_in = __popc(__ballot_sync(0xffffffffu, in));
+      } else {
+        own0 = g0 == 0;
+      }
+      const bool own = in && (lane > 0 || own0);
       // candidates of the 8 positions, in the top 2l bits
       uint64_t c[kWcPos];
       {
@@ -705,11 +839,11 @@ __global__ void __launch_bounds__(kWcWarps * 32, 12) warp_classify_kernel(WcArgs
         for (int j = 1; j < kWcPos; j++) start |= m[j] != m[j - 1] ? 1u << j : 0u;
         if (head) start |= 1u << (k - l);   // a sequence's first minimizer is new
         start &= emit;
-        next_min = __shfl_sync(0xffffffffu, m[7], 31);
-        next_seq = __shfl_sync(0xffffffffu, sq, 31);
+        next_min = __shfl_sync(0xffffffffu, m[7], n_in - 1);
+        next_seq = __shfl_sync(0xffffffffu, sq, n_in - 1);
       } else {
         // the repeated lane's first minima miss the candidates before it
-        const uint32_t clear = emit & ~amb & (lane == 0 && g0 ? 0xF0u : 0xFFu);
+        const uint32_t clear = emit & ~amb & (lane == 0 && !own0 ? 0xF0u : 0xFFu);
         uint64_t lm = 0;
 #pragma unroll
         for (int j = 0; j < kWcPos; j++) lm = (clear >> j) & 1u ? m[j] : lm;
@@ -744,8 +878,8 @@ __global__ void __launch_bounds__(kWcWarps * 32, 12) warp_classify_kernel(WcArgs
       if (!own) start = 0;
       // entries in token order
       const bool border = own && head && (seq.w & 8u);
-      const uint32_t mine = __popc(start) + (border ? 1u : 0u);
-      uint32_t upto = mine;
+      const uint32_t adds = __popc(start) + (border ? 1u : 0u);
+      uint32_t upto = adds;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
         const uint32_t x = __shfl_up_sync(0xffffffffu, upto, d);
@@ -754,7 +888,7 @@ __global__ void __launch_bounds__(kWcWarps * 32, 12) warp_classify_kernel(WcArgs
       const int total = (int)__shfl_sync(0xffffffffu, upto, 31);
       full = ne + total > kWcEntries;   // the pass is redone after a replay
       if (!full) {
-        uint4 *at = s.entry + (uint32_t)ne + upto - mine;
+        uint4 *at = s.entry + (uint32_t)ne + upto - adds;
         const uint32_t rtag = (seq.w & 7u) << kEPosBits;
         const uint32_t meta = rtag + (seq.w >> 4) + (uint32_t)(p0 - (k - 1));
         if (border) *at++ = make_uint4(~0u, ~0u, (E_BORDER << 30) | rtag | ((seq.w >> 4) - 1), 0);
@@ -774,8 +908,9 @@ __global__ void __launch_bounds__(kWcWarps * 32, 12) warp_classify_kernel(WcArgs
         ne += total;
         seen_min = next_min;
         seen_seq = next_seq;
-        done = g0 + 32 >= n_items;
-        g0 += 31;
+        done = g0 + (uint32_t)n_in >= n_items;
+        if constexpr (LONG) own0 = n_in < 32 && ((starts >> n_in) & 1u);   // the next item begins a sequence
+        g0 += (uint32_t)n_in - (LONG && own0 ? 0u : 1u);
       }
     }
     __syncwarp();
@@ -785,10 +920,21 @@ __global__ void __launch_bounds__(kWcWarps * 32, 12) warp_classify_kernel(WcArgs
     ne = 0;
   }
 
+  if (LONG && piece) {   // the merge resolves its fragment
+    if (lane == 0) {
+      SplitPiece &pc = a.pieces[task];
+      pc.hit_groups = s.hits[0];
+      pc.tokens = s.tokens[0] - first_pos;
+      pc.n_runs = s.n_runs[0];
+    }
+    return;
+  }
+
   // ---- calls
-  const uint32_t slots = 1u << w.log_slots;
   uint32_t call = 0, required = 0, taxa = 0;
-  if (lane < nr) {
+  bool out = lane < nr;
+  if constexpr (LONG) out = out && !a.split_mark[f0 + lane];
+  if (out) {
     const uint32_t total = s.tokens[lane] - (a.cls.paired ? 1u : 0u);
     required = (uint32_t)ceil(__dmul_rn(a.cls.confidence, (double)total));
     taxa = (s.over >> lane) & 1u ? 0xFFFFFFFFu : s.n_taxa[lane];
@@ -799,39 +945,40 @@ __global__ void __launch_bounds__(kWcWarps * 32, 12) warp_classify_kernel(WcArgs
     }
   }
   for (uint32_t todo = __ballot_sync(0xffffffffu, taxa > 1); todo; todo &= todo - 1) {
-    const int r = __ffs(todo) - 1;
+    const uint32_t r = (uint32_t)__ffs(todo) - 1;
     const uint32_t need = __shfl_sync(0xffffffffu, required, r), many = __shfl_sync(0xffffffffu, taxa, r);
+    // (the entries are done with: their memory serves as scratch)
+    uint2 *list = reinterpret_cast<uint2 *>(s.entry);
     uint32_t got = 0;
-    if (many == 0xFFFFFFFFu) {
+    if (many != 0xFFFFFFFFu) {
+      got = wc_resolve_slots(a.parent, wa.span, w.map_of(r), many, list, need);
+    } else {
+      // more taxa than its share of the map: count its runs into a larger one
+      constexpr uint32_t kBig = 512;
+      static_assert(32 * sizeof(uint2) + kBig * 8 <= sizeof(s.entry), "scratch");
+      uint32_t *mem = reinterpret_cast<uint32_t *>(list + 32);
+      const WcMap big{mem, mem + kBig, kBig - 1, 1};
+      for (uint32_t i = lane; i < 2 * kBig; i += 32) mem[i] = 0;
+      __syncwarp();
       const uint64_t base = s.run_base[r];
       const uint32_t n = base >= a.runs_cap ? 0u : (uint32_t)min((uint64_t)s.n_runs[r], a.runs_cap - base);
-      const uint64_t *runs = a.runs + base;
-      got = wc_resolve_items(a, wa.span, n, need, [runs](uint32_t i) {
-        const uint64_t x = *const_cast<const volatile uint64_t *>(runs + i);
-        const uint32_t t = (uint32_t)(x >> 32);
-        return make_uint2(t < K2G_CODE_AMBIGUOUS ? t : 0u, (uint32_t)x);
-      });
-    } else if (many > 32) {
-      const uint32_t *mk = s.mkey + r * slots, *mc = s.mcnt + r * slots;
-      got = wc_resolve_items(a, wa.span, slots, need, [mk, mc](uint32_t i) { return make_uint2(mk[i], mc[i]); });
-    } else {
-      // the fragment's taxa, one per lane (the entries are done with)
-      uint2 *list = reinterpret_cast<uint2 *>(s.entry) + 32 * r;
-      int n_list = 0;
-      for (uint32_t i0 = 0; i0 < slots; i0 += 32) {
-        const uint32_t at = (uint32_t)r * slots + i0 + (uint32_t)lane;
-        const uint32_t t = s.mkey[at];
-        const uint32_t b = __ballot_sync(0xffffffffu, t != 0);
-        if (t) list[n_list + __popc(b & lt)] = make_uint2(t, s.mcnt[at]);
-        n_list += __popc(b);
+      uint32_t added = 0;
+      bool full = false;
+      for (uint32_t i = lane; i < n; i += 32) {
+        const uint2 x = wc_run(a.runs + base, i);
+        const uint32_t slot = x.x ? big.add(x.x, x.y) : WcMap::kOld;
+        full |= slot == 0xFFFFFFFFu;
+        added += slot < kBig ? 1u : 0u;
       }
       __syncwarp();
-      const uint2 x = lane < n_list ? list[lane] : make_uint2(0, 0);
-      got = wc_resolve(a, wa.span, x.x, x.y, n_list, need);
+      added = __reduce_add_sync(0xffffffffu, added);
+      if (__any_sync(0xffffffffu, full)) got = wc_resolve_runs(a.parent, wa.span, a.runs + base, n, need);
+      else got = wc_resolve_slots(a.parent, wa.span, big, added, list, need);
     }
-    if (lane == r) call = got;
+    __syncwarp();
+    if (lane == (int)r) call = got;
   }
-  if (lane < nr) {
+  if (out) {
     const uint64_t f = f0 + lane;
     const uint32_t groups = s.hits[lane];
     if ((int32_t)groups < a.cls.min_hit_groups) call = 0;
@@ -840,6 +987,138 @@ __global__ void __launch_bounds__(kWcWarps * 32, 12) warp_classify_kernel(WcArgs
     if (a.hitlist_off) a.hitlist_off[f] = s.run_base[lane];
     if (a.hitlist_len) a.hitlist_len[f] = s.n_runs[lane];
     if (call && a.taxon_reads) atomicAdd(a.taxon_reads + call, 1ull);
+  }
+}
+
+// ---- the fragments their pieces carried ---------------------------------------
+
+constexpr int kMergeWarps = 4;
+constexpr uint32_t kMergeSlots = 512;
+
+struct MergeShared {
+  uint32_t mkey[kMergeSlots], mcnt[kMergeSlots];
+  uint2 list[32];
+};
+
+// One warp per fragment.  The pieces' runs lie in the fragment's run region,
+// shifted by the tokens before each piece; they are moved to the front in
+// place (a run is never written behind where it is read: a piece has no more
+// runs than tokens), equal runs that meet at a cut joining as they would have
+// in one pass.  The runs are counted into a taxon map on the way.
+static __global__ void __launch_bounds__(kMergeWarps * 32)
+warp_merge_kernel(ClassifyArgs a, const uint2 *span, SplitBufs b) {
+  __shared__ MergeShared shared[kMergeWarps];
+  MergeShared &s = shared[threadIdx.x >> 5];
+  const uint32_t lane = threadIdx.x & 31;
+  const uint64_t n_split = min((uint64_t)b.ctr[1], b.frags_cap);
+  const uint32_t k = (uint32_t)a.scan.k;
+  const WcMap small{s.mkey, s.mcnt, kMergeSlots - 1, 1};
+  for (uint64_t sid = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; sid < n_split;
+       sid += ((uint64_t)gridDim.x * blockDim.x) >> 5) {
+    const SplitFrag sf = b.frags[sid];
+    if (!sf.n) continue;
+    const uint64_t f = sf.frag, o0 = a.seq_off[f], len = a.seq_off[f + 1] - o0;
+    const uint64_t base = o0 + 2 * (f + a.frag_off);
+    for (uint32_t i = lane; i < kMergeSlots; i += 32) s.mkey[i] = s.mcnt[i] = 0;
+    __syncwarp();
+    uint32_t hits = 0, w = 0, added = 0;
+    bool full = false, have = false;
+    uint64_t open = 0;   // the last run so far, not written yet
+    for (uint32_t j = 0; j < sf.n; j++) {
+      const SplitPiece &pc = b.pieces[sf.first + j];
+      hits += pc.hit_groups;
+      const uint64_t from = base + (pc.lo - (k - 1));
+      // (past runs_cap nothing was written, and the overflow was flagged)
+      const uint32_t n = from >= a.runs_cap ? 0u : (uint32_t)min((uint64_t)pc.n_runs, a.runs_cap - from);
+      constexpr uint32_t U = 4;
+      for (uint32_t i0 = 0; i0 < n; i0 += 32 * U) {
+        uint64_t x[U];
+#pragma unroll
+        for (uint32_t u = 0; u < U; u++) {
+          const uint32_t i = i0 + 32 * u + lane;
+          x[u] = i < n ? a.runs[from + i] : 0;
+        }
+        __syncwarp();
+        // the first of these joins the open run or follows it
+        const uint64_t head = __shfl_sync(0xffffffffu, x[0], 0);
+        const bool joins = have && (uint32_t)(head >> 32) == (uint32_t)(open >> 32);
+        const uint32_t m = min(32 * U, n - i0);
+        if (have && !joins) {
+          if (lane == 0) a.runs[base + w] = open;
+          w++;
+        }
+        const uint64_t first = joins ? open + (uint32_t)head : head;
+        // all but the last are final
+#pragma unroll
+        for (uint32_t u = 0; u < U; u++) {
+          const uint32_t i = 32 * u + lane;
+          if (i + 1 < m) a.runs[base + w + i] = i ? x[u] : first;
+          const uint32_t t = (uint32_t)(x[u] >> 32);
+          if (i < m && t && t < K2G_CODE_AMBIGUOUS) {
+            const uint32_t slot = small.add(t, (uint32_t)x[u]);
+            full |= slot == 0xFFFFFFFFu;
+            added += slot < kMergeSlots ? 1u : 0u;
+          }
+        }
+        w += m - 1;
+        uint64_t last = first;
+#pragma unroll
+        for (uint32_t u = 0; u < U; u++) {
+          const uint64_t y = __shfl_sync(0xffffffffu, x[u], (m - 1) & 31);
+          if (m > 1 && (m - 1) >> 5 == u) last = y;
+        }
+        open = last;
+        have = true;
+        __syncwarp();
+      }
+    }
+    if (have) {
+      if (base + w < a.runs_cap) {
+        if (lane == 0) a.runs[base + w] = open;
+      } else if (lane == 0) {
+        atomicOr(a.status, STATUS_RUNS_OVERFLOW);
+      }
+      w++;
+    }
+    __syncwarp();
+    const uint32_t total = (uint32_t)(len - (k - 1));
+    const uint32_t required = (uint32_t)ceil(__dmul_rn(a.cls.confidence, (double)total));
+    added = __reduce_add_sync(0xffffffffu, added);
+    uint32_t call = 0;
+    if (__any_sync(0xffffffffu, full)) {
+      // too many taxa for the map: one in the unused part of the run region
+      const uint64_t end = min(base + len + 2, a.runs_cap), free0 = base + w;
+      const uint64_t room = end > free0 ? end - free0 : 0;
+      uint32_t slots = 32;
+      while (slots < 65536 && 2ull * slots <= room) slots *= 2;
+      const uint32_t n = base >= a.runs_cap ? 0u : (uint32_t)min((uint64_t)w, a.runs_cap - base);
+      bool over = slots > room;
+      if (!over) {
+        uint32_t *mem = reinterpret_cast<uint32_t *>(a.runs + free0);
+        const WcMap big{mem, mem + 1, slots - 1, 2};
+        for (uint32_t i = lane; i < slots; i += 32) a.runs[free0 + i] = 0;
+        __syncwarp();
+        for (uint32_t i = lane; i < n; i += 32) {
+          const uint2 x = wc_run(a.runs + base, i);
+          if (x.x && big.add(x.x, x.y) == 0xFFFFFFFFu) over = true;
+        }
+        __syncwarp();
+        over = __any_sync(0xffffffffu, over);
+        if (!over) call = wc_resolve_map(a.parent, span, big, required);
+      }
+      if (over) call = wc_resolve_runs(a.parent, span, a.runs + base, n, required);
+    } else if (added) {
+      call = wc_resolve_slots(a.parent, span, small, added, s.list, required);
+    }
+    if ((int32_t)hits < a.cls.min_hit_groups) call = 0;
+    if (lane == 0) {
+      a.call[f] = call;
+      if (a.hit_groups) a.hit_groups[f] = hits;
+      if (a.hitlist_off) a.hitlist_off[f] = base;
+      if (a.hitlist_len) a.hitlist_len[f] = w;
+      if (call && a.taxon_reads) atomicAdd(a.taxon_reads + call, 1ull);
+    }
+    __syncwarp();
   }
 }
 

@@ -19,7 +19,8 @@ MASK, TOGGLE = 0x3ffffffff3333333, 0xe37e28c4271b5a2d
 ACGT = np.frombuffer(b"ACGT", np.uint8)
 # around: k; 8 positions a lane; 32 lanes a pass; the 352 entries; the packed window
 EDGES = [0, 1, 30, 31, 34, 35, 36, 38, 39, 42, 43, 46, 47, 62, 63, 100, 150, 151, 250, 286, 287, 294,
-         295, 301, 534, 535, 1100, 2032, 2047, 2048, 2049, 2100, 4096, 8192]
+         295, 301, 534, 535, 1100, 2032, 2047, 2048, 2049, 2100, 4095, 4096, 4097, 8192, 20_000]
+CUT = 4096    # single fragments from here on are cut into pieces (not in quick mode)
 
 _cache = {}
 
@@ -102,9 +103,12 @@ def check(db, o, bases, q, off, n, params, mode=k2g.MODE_PIPELINED):
     got, want = r.runs[idx], runs[odx]
     assert np.array_equal(got >> np.uint64(32), want["code"].astype(np.uint64) & np.uint64(0xFFFFFFFF))
     assert np.array_equal(got & np.uint64(0xFFFFFFFF), want["count"].astype(np.uint64))
-    # nothing is written outside the fragments' runs
+    # nothing is written outside the runs of fragments that stay whole
     untouched = np.ones(len(r.runs), bool)
     untouched[idx] = False
+    if not params.get("paired") and not params.get("quick"):
+        for f in np.flatnonzero(np.diff(off.astype(np.int64)) >= CUT):
+            untouched[int(off[f]) + 2 * f:int(off[f + 1]) + 2 * f + 2] = False
     assert not r.runs[untouched].any()
     assert np.array_equal(r.taxon_reads, np.bincount(calls[calls > 0].astype(np.int64), minlength=len(r.taxon_reads)))
 
@@ -136,6 +140,45 @@ def test_groups_of_several_fragments_equal_the_oracle(n, hi, paired):
     lens = np.random.default_rng(n).integers(0, hi + 1, n * (2 if paired else 1))
     bases, q, off = batch(genome, [int(x) for x in lens], n)
     check(db, o, bases, q, off, n, dict(confidence=0.1, min_hit_groups=2, paired=paired))
+
+
+@pytest.mark.parametrize("piece_len", [256, 512, 8192])
+@pytest.mark.parametrize("params", [dict(confidence=0.0, min_hit_groups=0),
+                                    dict(confidence=0.2, min_hit_groups=2, min_quality=15)],
+                         ids=["plain", "quality"])
+def test_long_reads_in_pieces_equal_the_oracle(params, piece_len):
+    """Reads built to stress the cuts (test_gpu_split.py), and the -K counters
+    of their events against those of whole fragments."""
+    from kraken_io import GOLDEN, golden_db
+    from test_gpu_counters import classify_with_events
+    from test_gpu_split import long_reads, use_piece
+    db = k2g.Database.open(os.path.join(GOLDEN, "db_a"))
+    use_piece(db, piece_len)
+    b = long_reads(31, n=50, quals="min_quality" in params, piece=4 * piece_len if piece_len < 2048 else 8192)
+    g = golden_db("db_a")
+    o = oracle.Oracle(g.hash.cells, g.hash.capacity, g.hash.key_bits, g.hash.value_bits, g.taxo.parent,
+                      oracle.index_opts(g.opts.k, g.opts.l, g.opts.spaced_seed_mask, g.opts.toggle_mask))
+    r = classify_batch(db, b, params, mode=k2g.MODE_PIPELINED)
+    assert r.status == 0
+    calls, hg, nr, runs, base = o.classify(b.bases, b.quals, b.seq_off, b.n_frags, threads=4, **params)
+    assert np.array_equal(r.call[:b.n_frags], calls.astype(np.uint32))
+    assert np.array_equal(r.hit_groups[:b.n_frags], hg.astype(np.uint32))
+    for i in range(b.n_frags):
+        want = [(int(x["code"]), int(x["count"])) for x in runs[int(base[i]):int(base[i]) + int(nr[i])]]
+        assert r.runs_of(i) == want, i
+    b.blocks = (np.arange(b.n_frags) // 7).astype(np.uint32)
+    outs = []
+    for mode in (k2g.MODE_PIPELINED, k2g.MODE_PLAIN):
+        c = k2g.Counters(db)
+        reads, res, tr, keep = classify_with_events(db, b, dict(quick=False, paired=False, min_quality=0, **{
+            k: v for k, v in params.items() if k != "min_quality"}), mode)
+        c.add(reads, res)
+        outs.append(c.finish())
+        c.close()
+        del keep
+    for x, y in zip(*outs):
+        assert np.array_equal(x, y)
+    db.close()
 
 
 @pytest.mark.parametrize("capacity", [5, 8, 13, 61])
