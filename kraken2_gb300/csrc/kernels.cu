@@ -828,28 +828,8 @@ extern "C" k2g_status k2g_classify(const k2g_db *db, const k2g_reads *reads,
   return k2g::classify_keyed(db, reads, params, out, mode, stream, stream);
 }
 
-k2g_status k2g::classify_keyed(const k2g_db *db, const k2g_reads *reads,
-                               const k2g_classify_params *params, k2g_results *out, int mode,
-                               void *stream, const void *state_key) {
-  if (!db || !reads || !params || !out) return fail(K2G_ERR_ARG, "null argument");
-  if (!reads->n_frags) return K2G_OK;
-  if (!reads->d_bases || !reads->d_seq_off || !out->d_call || !out->d_runs || !out->d_status)
-    return fail(K2G_ERR_ARG, "missing required buffer");
-  if (params->confidence < 0 || params->confidence > 1)
-    return fail(K2G_ERR_ARG, "confidence threshold must be in [0, 1]");
-  if (!db->opts.dna_db) {   // translated search (translated.cu)
-    K2G_CUDA_TRY(cudaSetDevice(db->device));
-    return classify_translated(db, reads, params, out, (cudaStream_t)stream);
-  }
-  if (out->d_hit_keys && (!out->d_hit_taxa || !out->d_hit_order || !out->d_hits_used))
-    return fail(K2G_ERR_ARG, "incomplete hit event buffers");
-  if (reads->max_seq_len >= (1ull << 31)) return fail(K2G_ERR_ARG, "sequence too long");
-  // Bases are read as the 16-byte aligned chunks that contain them (such a
-  // chunk never leaves the allocation); qualities must share that alignment.
-  if (reads->d_quals && (((uintptr_t)reads->d_bases - (uintptr_t)reads->d_quals) & 15u))
-    return fail(K2G_ERR_ARG, "d_bases and d_quals must have the same alignment modulo 16");
-  K2G_CUDA_TRY(cudaSetDevice(db->device));
-  ClassifyArgs a{};
+void k2g::set_classify_args(ClassifyArgs &a, const k2g_db *db, const k2g_reads *reads,
+                            const k2g_classify_params *params, const k2g_results *out) {
   a.table = db->table_view();
   a.scan = db->scan_view();
   a.cls.confidence = params->confidence;
@@ -876,6 +856,31 @@ k2g_status k2g::classify_keyed(const k2g_db *db, const k2g_reads *reads,
   a.hits_cap = out->hits_cap;
   a.hits_used = reinterpret_cast<unsigned long long *>(out->d_hits_used);
   a.status = out->d_status;
+}
+
+k2g_status k2g::classify_keyed(const k2g_db *db, const k2g_reads *reads,
+                               const k2g_classify_params *params, k2g_results *out, int mode,
+                               void *stream, const void *state_key) {
+  if (!db || !reads || !params || !out) return fail(K2G_ERR_ARG, "null argument");
+  if (!reads->n_frags) return K2G_OK;
+  if (!reads->d_bases || !reads->d_seq_off || !out->d_call || !out->d_runs || !out->d_status)
+    return fail(K2G_ERR_ARG, "missing required buffer");
+  if (params->confidence < 0 || params->confidence > 1)
+    return fail(K2G_ERR_ARG, "confidence threshold must be in [0, 1]");
+  if (!db->opts.dna_db) {   // translated search (translated.cu)
+    K2G_CUDA_TRY(cudaSetDevice(db->device));
+    return classify_translated(db, reads, params, out, (cudaStream_t)stream);
+  }
+  if (out->d_hit_keys && (!out->d_hit_taxa || !out->d_hit_order || !out->d_hits_used))
+    return fail(K2G_ERR_ARG, "incomplete hit event buffers");
+  if (reads->max_seq_len >= (1ull << 31)) return fail(K2G_ERR_ARG, "sequence too long");
+  // Bases are read as the 16-byte aligned chunks that contain them (such a
+  // chunk never leaves the allocation); qualities must share that alignment.
+  if (reads->d_quals && (((uintptr_t)reads->d_bases - (uintptr_t)reads->d_quals) & 15u))
+    return fail(K2G_ERR_ARG, "d_bases and d_quals must have the same alignment modulo 16");
+  K2G_CUDA_TRY(cudaSetDevice(db->device));
+  ClassifyArgs a{};
+  set_classify_args(a, db, reads, params, out);
   cudaStream_t st = (cudaStream_t)stream;
   uint64_t total = reads->total_bases;
   if (!total) {

@@ -1,5 +1,6 @@
-// Translated search on the GPU: one thread per fragment runs the host/device
-// core of translated.cuh (six frames, protein scanner, tokens, ResolveTree,
+// Translated search on the GPU.  Tables with the default window go to the
+// warp form (warp_translated.cuh); for others one thread per fragment runs
+// the host/device core of translated.cuh (six frames, protein scanner, tokens, ResolveTree,
 // hit-list runs), looking keys up in the resident table.  It serves
 // k2g_classify (and the host-buffer paths above it) for protein tables; its
 // outputs follow the nucleotide path's layout: fragment i's runs at
@@ -12,6 +13,7 @@
 #include "k2g_device.cuh"
 #include "k2g_internal.h"
 #include "translated.cuh"
+#include "warp_translated.cuh"
 
 namespace k2g {
 namespace {
@@ -91,12 +93,50 @@ __global__ void translated_kernel(TxArgs a) {
   }
 }
 
+template <bool WIDE, bool HITS>
+cudaError_t launch_warp(const TxWarpArgs &wa, cudaStream_t st) {
+  const uint64_t blocks = (wa.n_groups + kWcWarps - 1) / kWcWarps;
+  warp_translated_kernel<WIDE, HITS><<<(unsigned)blocks, kWcWarps * 32, kWcWarps * sizeof(TxShared), st>>>(wa);
+  note_launches();
+  return cudaGetLastError();
+}
+
+// The warp form (warp_translated.cuh) takes the default window (k - l = 3);
+// it reads bases and qualities as the same 16-byte chunks.
+bool warp_takes(const TableView &t, const ScanView &sv, const k2g_reads *reads,
+                const k2g_classify_params *params) {
+  const uint64_t max_len = reads->max_seq_len;
+  if (reads->d_quals && params->min_quality > 0 &&
+      (((uintptr_t)reads->d_bases - (uintptr_t)reads->d_quals) & 15u))
+    return false;
+  // (a walk that goes on keeps its sector's number in 32 bits)
+  return sv.w == 4 && max_len <= kTxMaxLen && t.capacity / (t.wide ? 4 : 8) < (1ull << 32);
+}
+
 }  // namespace
 
 k2g_status classify_translated(const k2g_db *db, const k2g_reads *reads,
                                const k2g_classify_params *params, k2g_results *out,
                                cudaStream_t st) {
   const ScanView sv = db->scan_view();
+  if (!reads->max_seq_len) return fail(K2G_ERR_ARG, "max_seq_len is needed for translated search");
+  if (reads->max_seq_len > (1u << 30)) return fail(K2G_ERR_ARG, "sequence too long");
+  int sms = 0;
+  K2G_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, db->device));
+  if (warp_takes(db->table_view(), sv, reads, params)) {
+    ClassifyArgs c{};
+    set_classify_args(c, db, reads, params, out);
+    TxWarpArgs wa{c, db->d_span, 0, 0, reads->max_seq_len};
+    // two single fragments to a warp where that keeps every warp slot busy
+    // and their entries fit the list (0.8 a base)
+    if (!params->paired && reads->max_seq_len <= 200 && reads->n_frags / 2 >= (uint64_t)sms * kWcWarps * 10)
+      wa.log_reads = 1;
+    wa.n_groups = (reads->n_frags + (1ull << wa.log_reads) - 1) >> wa.log_reads;
+    const bool hits = c.hit_keys != nullptr;
+    const cudaError_t e = c.table.wide ? (hits ? launch_warp<true, true>(wa, st) : launch_warp<true, false>(wa, st))
+                                       : (hits ? launch_warp<false, true>(wa, st) : launch_warp<false, false>(wa, st));
+    return e == cudaSuccess ? K2G_OK : cuda_fail(e, "warp_translated_kernel");
+  }
   TxArgs a{};
   a.table = db->table_view();
   a.p.k = sv.k;
@@ -129,8 +169,6 @@ k2g_status classify_translated(const k2g_db *db, const k2g_reads *reads,
   a.hits_cap = out->hits_cap;
   a.hits_used = reinterpret_cast<unsigned long long *>(out->d_hits_used);
   a.status = out->d_status;
-  if (!reads->max_seq_len) return fail(K2G_ERR_ARG, "max_seq_len is needed for translated search");
-  if (reads->max_seq_len > (1u << 30)) return fail(K2G_ERR_ARG, "sequence too long");
   // per-thread scratch: six frames and the masked mate; a taxon map with
   // room for every lookup of the longest fragment (or every taxon)
   const uint64_t max_len = reads->max_seq_len;
@@ -143,8 +181,6 @@ k2g_status classify_translated(const k2g_db *db, const k2g_reads *reads,
   while (cap < 2 * std::min(lookups, taxa)) cap <<= 1;
   a.map_cap = (uint32_t)cap;
   const uint64_t per_thread = a.frame_bytes + 12ull * a.map_cap;
-  int sms = 0;
-  K2G_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, db->device));
   constexpr uint64_t kScratchBudget = 2ull << 30;
   uint64_t threads = std::min<uint64_t>({reads->n_frags, (uint64_t)sms * 512,
                                          std::max<uint64_t>(32, kScratchBudget / per_thread)});
@@ -152,7 +188,7 @@ k2g_status classify_translated(const k2g_db *db, const k2g_reads *reads,
   const unsigned block = 128;
   threads = (std::max<uint64_t>(threads, 1) + block - 1) / block * block;
   void *scratch = nullptr;
-  K2G_CUDA_TRY(cudaMallocAsync(&scratch, threads * per_thread, st));
+  K2G_CUDA_TRY(scratch_alloc(&scratch, threads * per_thread, db->device, st));
   a.frames = static_cast<uint8_t *>(scratch);
   a.maps = reinterpret_cast<uint32_t *>(a.frames + threads * a.frame_bytes);
   translated_kernel<<<(unsigned)(threads / block), block, 0, st>>>(a);

@@ -66,23 +66,29 @@ struct WcArgs {
   uint64_t piece_slots;
 };
 
-// One warp's shared memory.
-struct WcShared {
+// One warp's shared memory: what every form of the classification uses ...
+struct WcBase {
   // An entry: key (two words, in the top bits; ~0 where nothing is looked
   // up), meta, value.  The replay then keeps its run heads (code, meta) in
   // the first two words.
   uint4 entry[kWcEntries];
-  // Packed bases; after a scan the same words list the entries whose walk
-  // goes on (16 bits each).
-  uint32_t be[kWcWindow / 16 + 4];
-  uint32_t le[kWcWindow / 16 + 4];    // [3] holds the window's first word
-  uint32_t inv[kWcWindow / 32 + 4];   // bit per base: not A/C/G/T; [2] is the first word
   uint32_t mkey[kWcSlots], mcnt[kWcSlots];
   uint4 seq[2 * kWcReads];            // sequences with work: start, length, first item, fragment and tokens before
+                                      // (bit 3 of the last: a border comes first)
   uint64_t run_base[kWcReads];
   uint32_t tokens[kWcReads], hits[kWcReads], n_runs[kWcReads];
   uint32_t n_taxa[kWcReads], a_slot[kWcReads];   // taxa of the map, and a slot of them
   uint32_t over, stopped;             // fragment bits
+};
+
+// ... and the packed bases of the nucleotide scan.  After a scan the same
+// words list the entries whose walk goes on (16 bits each).
+struct WcShared : WcBase {
+  static constexpr bool kFrames = false;
+  uint32_t be[kWcWindow / 16 + 4];
+  uint32_t le[kWcWindow / 16 + 4];    // [3] holds the window's first word
+  uint32_t inv[kWcWindow / 32 + 4];   // bit per base: not A/C/G/T; [2] is the first word
+  __device__ __forceinline__ uint16_t *list() { return reinterpret_cast<uint16_t *>(be); }
 };
 
 __device__ __forceinline__ uint32_t below(int n) { return n >= 32 ? 0xFFFFFFFFu : (1u << n) - 1u; }
@@ -374,10 +380,10 @@ __device__ __forceinline__ uint32_t wc_resolve_slots(const uint32_t *parent, con
 
 // ---- the kernel --------------------------------------------------------------
 
-template <bool WIDE, bool HITS>
+template <bool WIDE, bool HITS, class Shared>
 struct Wc {
   const ClassifyArgs &a;
-  WcShared &s;
+  Shared &s;
   const int lane;
   const uint32_t lt;            // lanes below
   uint64_t f0;                  // first fragment of the group
@@ -390,6 +396,103 @@ struct Wc {
   // and the value of the last key
   uint32_t open_code = 0, open_meta = 0xFFFFFFFFu, open_rank = 0, key_taxon = 0;
 
+  // the last unambiguous minimizer of the scan, and its sequence
+  uint64_t seen_min = 0;
+  uint32_t seen_seq = 0xFFFFFFFFu;
+
+  // Where token groups start among the lane's positions, given their window
+  // minima, which of them end a k-mer (emit) and which of those k-mers are
+  // ambiguous.  head: the lane's first position is its sequence's first;
+  // repeated: lane 0 repeats the item before the pass, its first k - l minima
+  // miss the candidates before it; sq: the lane's sequence; n_in: lanes with
+  // an item.  cont: starts that continue the last key's taxon.  next_*: the
+  // scan state after the pass.
+  __device__ __forceinline__ uint32_t starts(const uint64_t (&m)[kWcPos], uint32_t emit, uint32_t amb, bool head,
+                                             bool repeated, bool dirty, uint32_t sq, int n_in, uint32_t skip,
+                                             uint32_t &cont, uint64_t &next_min, uint32_t &next_seq) const {
+    uint32_t start = 0;
+    next_min = seen_min;
+    next_seq = seen_seq;
+    if (!dirty) {
+      const uint64_t pm = __shfl_up_sync(0xffffffffu, m[7], 1);
+      start = m[0] != pm ? 1u : 0u;
+#pragma unroll
+      for (int j = 1; j < kWcPos; j++) start |= m[j] != m[j - 1] ? 1u << j : 0u;
+      if (head) start |= 1u << skip;   // a sequence's first minimizer is new
+      start &= emit;
+      next_min = __shfl_sync(0xffffffffu, m[7], n_in - 1);
+      next_seq = __shfl_sync(0xffffffffu, sq, n_in - 1);
+      return start;
+    }
+    const uint32_t clear = emit & ~amb & (lane == 0 && repeated ? 0xFFu << skip : 0xFFu);
+    uint64_t lm = 0;
+#pragma unroll
+    for (int j = 0; j < kWcPos; j++) lm = (clear >> j) & 1u ? m[j] : lm;
+    // the last unambiguous minimizer before this lane, in its sequence
+    const uint32_t have = __ballot_sync(0xffffffffu, clear != 0);
+    const int src = (have & lt) ? last_bit(have & lt) : 0;
+    uint64_t run_min = __shfl_sync(0xffffffffu, lm, src);
+    uint32_t run_seq = __shfl_sync(0xffffffffu, sq, src);
+    if (!(have & lt)) {
+      run_min = seen_min;
+      run_seq = seen_seq;
+    }
+    bool known = run_seq == sq && !head;
+    bool prev_amb = (__shfl_up_sync(0xffffffffu, amb, 1) >> (kWcPos - 1)) & 1u;
+    bool fresh = head;
+#pragma unroll
+    for (int j = 0; j < kWcPos; j++) {
+      const bool is_amb = (amb >> j) & 1u, at = (emit >> j) & 1u;
+      const bool is_new = !is_amb && !(known && run_min == m[j]);
+      if (at && (fresh || is_amb != prev_amb || is_new)) start |= 1u << j;
+      if (!is_amb && !is_new) cont |= 1u << j;
+      known = known || (at && !is_amb);
+      run_min = at && !is_amb ? m[j] : run_min;
+      fresh = fresh && !at;
+      prev_amb = at ? is_amb : prev_amb;
+    }
+    if (have) {
+      next_min = __shfl_sync(0xffffffffu, lm, last_bit(have));
+      next_seq = __shfl_sync(0xffffffffu, sq, last_bit(have));
+    }
+    return start;
+  }
+
+  // Appends the lanes' token groups to the entries, in token order; false
+  // (and nothing appended) when they do not fit.  tag: the sequence's word
+  // (WcBase::seq); tok0: the token position of the lane's first position.
+  __device__ __forceinline__ bool add(int &ne, const uint64_t (&m)[kWcPos], uint32_t start, uint32_t amb,
+                                      uint32_t cont, bool border, uint32_t tag, uint32_t tok0, bool dirty) {
+    const uint32_t adds = __popc(start) + (border ? 1u : 0u);
+    uint32_t upto = adds;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t x = __shfl_up_sync(0xffffffffu, upto, d);
+      if (lane >= d) upto += x;
+    }
+    const int total = (int)__shfl_sync(0xffffffffu, upto, 31);
+    if (ne + total > kWcEntries) return false;
+    uint4 *at = s.entry + (uint32_t)ne + upto - adds;
+    const uint32_t rtag = (tag & 7u) << kEPosBits;
+    const uint32_t meta = rtag + tok0;
+    if (border) *at++ = make_uint4(~0u, ~0u, (E_BORDER << 30) | rtag | ((tag >> 4) - 1), 0);
+    if (!dirty) {
+#pragma unroll
+      for (int j = 0; j < kWcPos; j++)
+        if ((start >> j) & 1u) *at++ = make_uint4((uint32_t)m[j], (uint32_t)(m[j] >> 32), meta + j, 0);
+    } else {
+#pragma unroll
+      for (int j = 0; j < kWcPos; j++) {
+        const bool is_amb = (amb >> j) & 1u, is_cont = (cont >> j) & 1u;
+        const uint64_t key = is_amb || is_cont ? ~0ull : m[j];
+        const uint32_t kind = is_amb ? E_AMBIG << 30 : is_cont ? E_CONT << 30 : 0u;
+        if ((start >> j) & 1u) *at++ = make_uint4((uint32_t)key, (uint32_t)(key >> 32), kind | (meta + j), 0);
+      }
+    }
+    ne += total;
+    return true;
+  }
+
   __device__ __forceinline__ uint64_t key_of(uint64_t top) const { return (top ^ toggle_top) >> key_shift; }
   __device__ __forceinline__ uint64_t top_of(int i) const {
     return *reinterpret_cast<const uint64_t *>(&s.entry[i]);
@@ -399,14 +502,13 @@ struct Wc {
     return WcMap{s.mkey + (r << log_slots), s.mcnt + (r << log_slots), (1u << log_slots) - 1u, 1u};
   }
 
-  // Get() for every key entry: the home sectors of all, then the next sector
-  // of every walk that goes on, and so on (about one walk in five leaves its
-  // home sector at load 0.7, and one in four of those goes on again).
+  // Get() for every key entry: the home sectors of all, then the walks that
+  // go on (about one in five at load 0.7).
   __device__ __forceinline__ void probe(int ne) {
     constexpr int B = 3;
     constexpr uint32_t N = WIDE ? 4 : 8, kLogN = WIDE ? 2 : 3;
     const TableView &t = a.table;
-    uint16_t *list = reinterpret_cast<uint16_t *>(s.be);
+    uint16_t *list = s.list();
     // the table's last sector where it is a partial one: its padding cells
     // look empty, so an absent key found there is looked up once more
     const uint64_t partial = t.capacity & (N - 1) ? t.capacity & ~(uint64_t)(N - 1) : ~0ull;
@@ -487,6 +589,12 @@ struct Wc {
     }
   }
 
+  // (a border between frames, or between mates)
+  __device__ __forceinline__ uint32_t border_code(uint32_t r, uint32_t pos) const {
+    if constexpr (Shared::kFrames) return pos == s.mate_pos[r] ? K2G_CODE_MATE_BORDER : K2G_CODE_FRAME_BORDER;
+    else return K2G_CODE_MATE_BORDER;
+  }
+
   // Quick mode: the lookup whose hit reaches the minimum ends its fragment;
   // it and everything after it leave no tokens.  Returns whether the entry
   // stands; `hit` is cleared where it does not (the ending lookup keeps its
@@ -547,7 +655,7 @@ struct Wc {
       if constexpr (HITS) emit_events(event, i, r, where & below(kEPosBits), v, events);
       if (hit) atomicAdd(&s.hits[r], 1u);
       const uint32_t code = kind == E_AMBIG    ? K2G_CODE_AMBIGUOUS
-                            : kind == E_BORDER ? K2G_CODE_MATE_BORDER
+                            : kind == E_BORDER ? border_code(r, where & below(kEPosBits))
                                                : v;
       const uint32_t acts = __ballot_sync(0xffffffffu, act);
       const int prev = (acts & lt) ? last_bit(acts & lt) : -1;
@@ -582,7 +690,10 @@ struct Wc {
         const bool same = (nx.y >> kEPosBits) == (it.y >> kEPosBits);
         const uint32_t n = (same ? nx.y & below(kEPosBits) : s.tokens[r]) - start;
         const uint64_t at = s.run_base[r] + rank;
-        if (at < a.runs_cap) a.runs[at] = ((uint64_t)it.x << 32) | n;
+        bool room = at < a.runs_cap;
+        // (six frames can have more runs than their fragment's region holds)
+        if constexpr (Shared::kFrames) room = room && rank < s.room[r];
+        if (room) a.runs[at] = ((uint64_t)it.x << 32) | n;
         else atomicOr(a.status, STATUS_RUNS_OVERFLOW);
         if (!same) s.n_runs[r] = rank + 1;
         if (it.x && it.x < K2G_CODE_AMBIGUOUS) {
@@ -608,6 +719,65 @@ struct Wc {
       }
     }
     __syncwarp();
+  }
+
+  // The calls and outputs of the group's fragments: lane r writes fragment r
+  // where `out` says so; total: the tokens its confidence counts.
+  __device__ __forceinline__ void finish(const uint2 *span, bool out, uint64_t total) {
+    uint32_t call = 0, required = 0, taxa = 0;
+    if (out) {
+      required = (uint32_t)ceil(__dmul_rn(a.cls.confidence, (double)total));
+      taxa = (s.over >> lane) & 1u ? 0xFFFFFFFFu : s.n_taxa[lane];
+      // one taxon: it, or nothing (its ancestors hold no more tokens)
+      if (taxa == 1) {
+        const uint32_t at = s.a_slot[lane];
+        call = s.mcnt[at] >= required ? s.mkey[at] : 0u;
+      }
+    }
+    for (uint32_t todo = __ballot_sync(0xffffffffu, taxa > 1); todo; todo &= todo - 1) {
+      const uint32_t r = (uint32_t)__ffs(todo) - 1;
+      const uint32_t need = __shfl_sync(0xffffffffu, required, r), many = __shfl_sync(0xffffffffu, taxa, r);
+      // (the entries are done with: their memory serves as scratch)
+      uint2 *list = reinterpret_cast<uint2 *>(s.entry);
+      uint32_t got = 0;
+      if (many != 0xFFFFFFFFu) {
+        got = wc_resolve_slots(a.parent, span, map_of(r), many, list, need);
+      } else {
+        // more taxa than its share of the map: count its runs into a larger one
+        constexpr uint32_t kBig = 512;
+        static_assert(32 * sizeof(uint2) + kBig * 8 <= sizeof(s.entry), "scratch");
+        uint32_t *mem = reinterpret_cast<uint32_t *>(list + 32);
+        const WcMap big{mem, mem + kBig, kBig - 1, 1};
+        for (uint32_t i = lane; i < 2 * kBig; i += 32) mem[i] = 0;
+        __syncwarp();
+        const uint64_t base = s.run_base[r];
+        const uint32_t n = base >= a.runs_cap ? 0u : (uint32_t)min((uint64_t)s.n_runs[r], a.runs_cap - base);
+        uint32_t added = 0;
+        bool full = false;
+        for (uint32_t i = lane; i < n; i += 32) {
+          const uint2 x = wc_run(a.runs + base, i);
+          const uint32_t slot = x.x ? big.add(x.x, x.y) : WcMap::kOld;
+          full |= slot == 0xFFFFFFFFu;
+          added += slot < kBig ? 1u : 0u;
+        }
+        __syncwarp();
+        added = __reduce_add_sync(0xffffffffu, added);
+        if (__any_sync(0xffffffffu, full)) got = wc_resolve_runs(a.parent, span, a.runs + base, n, need);
+        else got = wc_resolve_slots(a.parent, span, big, added, list, need);
+      }
+      __syncwarp();
+      if (lane == (int)r) call = got;
+    }
+    if (out) {
+      const uint64_t f = f0 + lane;
+      const uint32_t groups = s.hits[lane];
+      if ((int32_t)groups < a.cls.min_hit_groups) call = 0;
+      a.call[f] = call;
+      if (a.hit_groups) a.hit_groups[f] = groups;
+      if (a.hitlist_off) a.hitlist_off[f] = s.run_base[lane];
+      if (a.hitlist_len) a.hitlist_len[f] = s.n_runs[lane];
+      if (call && a.taxon_reads) atomicAdd(a.taxon_reads + call, 1ull);
+    }
   }
 };
 
@@ -642,7 +812,7 @@ __global__ void __launch_bounds__(kWcWarps * 32, kWcBlocks) warp_classify_kernel
   const int nr = piece ? 1 : (int)min((uint64_t)1 << wa.log_reads, a.n_frags - f0);
   const int per = a.cls.paired ? 2 : 1, ns = nr * per;
   const uint32_t key_shift = 64u - 2u * (uint32_t)l;
-  Wc<WIDE, HITS> w{a, s, lane, lt, f0, piece ? kWcLogSlots : kWcLogSlots - wa.log_reads, first_pos, key_shift,
+  Wc<WIDE, HITS, WcShared> w{a, s, lane, lt, f0, piece ? kWcLogSlots : kWcLogSlots - wa.log_reads, first_pos, key_shift,
                    a.scan.toggle << key_shift};
   const uint64_t mask_top = (a.scan.spaced_mask ? a.scan.spaced_mask & a.scan.lmer_mask : a.scan.lmer_mask)
                             << key_shift;
@@ -705,8 +875,6 @@ __global__ void __launch_bounds__(kWcWarps * 32, kWcBlocks) warp_classify_kernel
   uint32_t g0 = 0;                    // first item of the pass
   uint32_t win_lo = 0, win_hi = 0;    // bases packed in shared memory
   bool dirty = false;                 // ambiguous bases seen in the group
-  uint64_t seen_min = 0;              // last unambiguous minimizer, and its sequence
-  uint32_t seen_seq = 0xFFFFFFFFu;
   int ne = 0;
   bool own0 = true;                   // lane 0's item is not a repeated one
   (void)own0;
@@ -828,86 +996,17 @@ __global__ void __launch_bounds__(kWcWarps * 32, kWcBlocks) warp_classify_kernel
         m[6] = min64(t2, u2);
         m[7] = min64(c[3], u3);
       }
-      // starts of token groups
-      uint32_t start = 0, cont = 0;
-      uint64_t next_min = seen_min;
-      uint32_t next_seq = seen_seq;
-      if (!dirty) {
-        const uint64_t pm = __shfl_up_sync(0xffffffffu, m[7], 1);
-        start = m[0] != pm ? 1u : 0u;
-#pragma unroll
-        for (int j = 1; j < kWcPos; j++) start |= m[j] != m[j - 1] ? 1u << j : 0u;
-        if (head) start |= 1u << (k - l);   // a sequence's first minimizer is new
-        start &= emit;
-        next_min = __shfl_sync(0xffffffffu, m[7], n_in - 1);
-        next_seq = __shfl_sync(0xffffffffu, sq, n_in - 1);
-      } else {
-        // the repeated lane's first minima miss the candidates before it
-        const uint32_t clear = emit & ~amb & (lane == 0 && !own0 ? 0xF0u : 0xFFu);
-        uint64_t lm = 0;
-#pragma unroll
-        for (int j = 0; j < kWcPos; j++) lm = (clear >> j) & 1u ? m[j] : lm;
-        // the last unambiguous minimizer before this lane, in its sequence
-        const uint32_t have = __ballot_sync(0xffffffffu, clear != 0);
-        const int src = (have & lt) ? last_bit(have & lt) : 0;
-        uint64_t run_min = __shfl_sync(0xffffffffu, lm, src);
-        uint32_t run_seq = __shfl_sync(0xffffffffu, sq, src);
-        if (!(have & lt)) {
-          run_min = seen_min;
-          run_seq = seen_seq;
-        }
-        bool known = run_seq == sq && !head;
-        bool prev_amb = (__shfl_up_sync(0xffffffffu, amb, 1) >> (kWcPos - 1)) & 1u;
-        bool fresh = head;
-#pragma unroll
-        for (int j = 0; j < kWcPos; j++) {
-          const bool is_amb = (amb >> j) & 1u, at = (emit >> j) & 1u;
-          const bool is_new = !is_amb && !(known && run_min == m[j]);
-          if (at && (fresh || is_amb != prev_amb || is_new)) start |= 1u << j;
-          if (!is_amb && !is_new) cont |= 1u << j;
-          known = known || (at && !is_amb);
-          run_min = at && !is_amb ? m[j] : run_min;
-          fresh = fresh && !at;
-          prev_amb = at ? is_amb : prev_amb;
-        }
-        if (have) {
-          next_min = __shfl_sync(0xffffffffu, lm, last_bit(have));
-          next_seq = __shfl_sync(0xffffffffu, sq, last_bit(have));
-        }
-      }
+      // token groups
+      uint32_t cont = 0;
+      uint64_t next_min;
+      uint32_t next_seq;
+      uint32_t start = w.starts(m, emit, amb, head, !own0, dirty, sq, n_in, (uint32_t)(k - l), cont, next_min, next_seq);
       if (!own) start = 0;
-      // entries in token order
-      const bool border = own && head && (seq.w & 8u);
-      const uint32_t adds = __popc(start) + (border ? 1u : 0u);
-      uint32_t upto = adds;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t x = __shfl_up_sync(0xffffffffu, upto, d);
-        if (lane >= d) upto += x;
-      }
-      const int total = (int)__shfl_sync(0xffffffffu, upto, 31);
-      full = ne + total > kWcEntries;   // the pass is redone after a replay
-      if (!full) {
-        uint4 *at = s.entry + (uint32_t)ne + upto - adds;
-        const uint32_t rtag = (seq.w & 7u) << kEPosBits;
-        const uint32_t meta = rtag + (seq.w >> 4) + (uint32_t)(p0 - (k - 1));
-        if (border) *at++ = make_uint4(~0u, ~0u, (E_BORDER << 30) | rtag | ((seq.w >> 4) - 1), 0);
-        if (!dirty) {
-#pragma unroll
-          for (int j = 0; j < kWcPos; j++)
-            if ((start >> j) & 1u) *at++ = make_uint4((uint32_t)m[j], (uint32_t)(m[j] >> 32), meta + j, 0);
-        } else {
-#pragma unroll
-          for (int j = 0; j < kWcPos; j++) {
-            const bool is_amb = (amb >> j) & 1u, is_cont = (cont >> j) & 1u;
-            const uint64_t key = is_amb || is_cont ? ~0ull : m[j];
-            const uint32_t kind = is_amb ? E_AMBIG << 30 : is_cont ? E_CONT << 30 : 0u;
-            if ((start >> j) & 1u) *at++ = make_uint4((uint32_t)key, (uint32_t)(key >> 32), kind | (meta + j), 0);
-          }
-        }
-        ne += total;
-        seen_min = next_min;
-        seen_seq = next_seq;
+      const uint32_t tok0 = (seq.w >> 4) + (uint32_t)(p0 - (k - 1));
+      full = !w.add(ne, m, start, amb, cont, own && head && (seq.w & 8u), seq.w, tok0, dirty);
+      if (!full) {   // (else the pass is redone after a replay)
+        w.seen_min = next_min;
+        w.seen_seq = next_seq;
         done = g0 + (uint32_t)n_in >= n_items;
         if constexpr (LONG) own0 = n_in < 32 && ((starts >> n_in) & 1u);   // the next item begins a sequence
         g0 += (uint32_t)n_in - (LONG && own0 ? 0u : 1u);
@@ -930,64 +1029,11 @@ __global__ void __launch_bounds__(kWcWarps * 32, kWcBlocks) warp_classify_kernel
     return;
   }
 
-  // ---- calls
-  uint32_t call = 0, required = 0, taxa = 0;
   bool out = lane < nr;
   if constexpr (LONG) out = out && !a.split_mark[f0 + lane];
-  if (out) {
-    const uint32_t total = s.tokens[lane] - (a.cls.paired ? 1u : 0u);
-    required = (uint32_t)ceil(__dmul_rn(a.cls.confidence, (double)total));
-    taxa = (s.over >> lane) & 1u ? 0xFFFFFFFFu : s.n_taxa[lane];
-    // one taxon: it, or nothing (its ancestors hold no more tokens)
-    if (taxa == 1) {
-      const uint32_t at = s.a_slot[lane];
-      call = s.mcnt[at] >= required ? s.mkey[at] : 0u;
-    }
-  }
-  for (uint32_t todo = __ballot_sync(0xffffffffu, taxa > 1); todo; todo &= todo - 1) {
-    const uint32_t r = (uint32_t)__ffs(todo) - 1;
-    const uint32_t need = __shfl_sync(0xffffffffu, required, r), many = __shfl_sync(0xffffffffu, taxa, r);
-    // (the entries are done with: their memory serves as scratch)
-    uint2 *list = reinterpret_cast<uint2 *>(s.entry);
-    uint32_t got = 0;
-    if (many != 0xFFFFFFFFu) {
-      got = wc_resolve_slots(a.parent, wa.span, w.map_of(r), many, list, need);
-    } else {
-      // more taxa than its share of the map: count its runs into a larger one
-      constexpr uint32_t kBig = 512;
-      static_assert(32 * sizeof(uint2) + kBig * 8 <= sizeof(s.entry), "scratch");
-      uint32_t *mem = reinterpret_cast<uint32_t *>(list + 32);
-      const WcMap big{mem, mem + kBig, kBig - 1, 1};
-      for (uint32_t i = lane; i < 2 * kBig; i += 32) mem[i] = 0;
-      __syncwarp();
-      const uint64_t base = s.run_base[r];
-      const uint32_t n = base >= a.runs_cap ? 0u : (uint32_t)min((uint64_t)s.n_runs[r], a.runs_cap - base);
-      uint32_t added = 0;
-      bool full = false;
-      for (uint32_t i = lane; i < n; i += 32) {
-        const uint2 x = wc_run(a.runs + base, i);
-        const uint32_t slot = x.x ? big.add(x.x, x.y) : WcMap::kOld;
-        full |= slot == 0xFFFFFFFFu;
-        added += slot < kBig ? 1u : 0u;
-      }
-      __syncwarp();
-      added = __reduce_add_sync(0xffffffffu, added);
-      if (__any_sync(0xffffffffu, full)) got = wc_resolve_runs(a.parent, wa.span, a.runs + base, n, need);
-      else got = wc_resolve_slots(a.parent, wa.span, big, added, list, need);
-    }
-    __syncwarp();
-    if (lane == (int)r) call = got;
-  }
-  if (out) {
-    const uint64_t f = f0 + lane;
-    const uint32_t groups = s.hits[lane];
-    if ((int32_t)groups < a.cls.min_hit_groups) call = 0;
-    a.call[f] = call;
-    if (a.hit_groups) a.hit_groups[f] = groups;
-    if (a.hitlist_off) a.hitlist_off[f] = s.run_base[lane];
-    if (a.hitlist_len) a.hitlist_len[f] = s.n_runs[lane];
-    if (call && a.taxon_reads) atomicAdd(a.taxon_reads + call, 1ull);
-  }
+  uint64_t total = 0;
+  if (out) total = s.tokens[lane] - (a.cls.paired ? 1u : 0u);
+  w.finish(wa.span, out, total);
 }
 
 // ---- the fragments their pieces carried ---------------------------------------
