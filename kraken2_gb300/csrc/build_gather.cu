@@ -13,6 +13,8 @@
 // i >= 1 also reports the minimizer of its first k - l l-mers (bases i ..
 // i + k - 2) as an unambiguous one, when those bases are A/C/G/T.  That
 // value is part of the block's set too.  Here, for a whole batch at once:
+// (Tables with the default window take the shorter way of build_blocks.cuh
+// for steps 1 to 4.)
 //   1. chunk_kernel: one thread per chunk of at most kChunk k-mer starts
 //      (chunks never cross a block) scans the chunk's bases and writes its
 //      candidate minimizers and their count.  A k-mer whose minimizer equals
@@ -95,11 +97,12 @@ __device__ __forceinline__ bool keep(const ScanView &sv, uint32_t sample_below, 
 
 template <int W>
 __global__ void chunk_kernel(ScanView sv, const uint8_t *bases, const Chunk *chunks,
-                             uint64_t n_chunks, uint64_t *cand, uint32_t *counts,
-                             uint32_t sample_below) {
+                             uint64_t n_chunks, uint64_t *cand, uint32_t *counts, const uint32_t *offs,
+                             uint32_t sample_below, bool only_starts) {
   const uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   if (c >= n_chunks) return;
   const Chunk ch = chunks[c];
+  if (only_starts && ch.kind != kSubblockStart) return;   // (block_scan_kernel has the others)
   const int k = sv.k, l = sv.l;
   const bool sub = ch.kind == kSubblockStart;
   const uint64_t start = ch.kind == kContinues ? ch.pos - 1 : ch.pos;
@@ -114,7 +117,10 @@ __global__ void chunk_kernel(ScanView sv, const uint8_t *bases, const Chunk *chu
   bool prev_ok = false;    // the previous k-mer of the block is unambiguous
   uint64_t prev_min = 0;
   uint32_t cnt = 0;
-  uint64_t *out = cand + ch.slot;
+  // counted first (cand null), then written back to back at offs; or in one
+  // go, to places of the chunk's own
+  const bool write = cand != nullptr;
+  uint64_t *out = write ? cand + (offs ? offs[c] : ch.slot) : nullptr;
   const int bits = sv.protein ? 4 : 2;
   for (uint32_t p = 0; p < len; p++) {
     const uint32_t byte = __ldg(seq + p);
@@ -140,20 +146,37 @@ __global__ void chunk_kernel(ScanView sv, const uint8_t *bases, const Chunk *chu
     const bool amb = (int32_t)p - last_amb <= amb_span;
     const uint64_t m = win.min(sv.w) ^ sv.toggle;
     const bool own = start + p - (k - 1) >= ch.pos;   // not the previous block k-mer
-    if (own && !amb && !(prev_ok && prev_min == m) && keep(sv, sample_below, m)) out[cnt++] = m;
+    if (own && !amb && !(prev_ok && prev_min == m) && keep(sv, sample_below, m)) {
+      if (write) out[cnt] = m;
+      cnt++;
+    }
     prev_ok = !amb;
     prev_min = m;
   }
   if (sub && last_amb < 0) {   // bases i .. i + k - 2 all A/C/G/T
     const uint64_t m = win.min(sv.w) ^ sv.toggle;
-    if (keep(sv, sample_below, m)) out[cnt++] = m;
+    if (keep(sv, sample_below, m)) {
+      if (write) out[cnt] = m;
+      cnt++;
+    }
   }
   counts[c] = cnt;
 }
 
+// Whether the warp scan and the block sort take a table's k-mers.
+bool scans_by_warps(const ScanView &sv) { return sv.w == 5 && !sv.protein && sv.revcom_version != 0; }
+
+}  // namespace
+}  // namespace k2g
+
+#include "build_blocks.cuh"
+
+namespace k2g {
+namespace {
+
 // One warp per chunk: its candidates, with its block number, at offs[c].
 __global__ void compact_kernel(const Chunk *chunks, uint64_t n_chunks, const uint64_t *cand,
-                               const uint32_t *counts, const uint32_t *offs, uint64_t *keys,
+                               const uint32_t *counts, const uint32_t *offs, bool packed, uint64_t *keys,
                                uint32_t *blocks) {
   const uint64_t c = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint32_t lane = threadIdx.x & 31;
@@ -161,7 +184,7 @@ __global__ void compact_kernel(const Chunk *chunks, uint64_t n_chunks, const uin
   const Chunk ch = chunks[c];
   const uint32_t n = counts[c], o = offs[c];
   for (uint32_t i = lane; i < n; i += 32) {
-    keys[o + i] = cand[ch.slot + i];
+    keys[o + i] = cand[(packed ? o : ch.slot) + i];
     blocks[o + i] = ch.block;
   }
 }
@@ -300,9 +323,10 @@ __global__ void unique_kernel(const uint64_t *keys, const uint32_t *blocks, uint
 
 template <int W>
 void launch_chunks(const ScanView &sv, const uint8_t *bases, const Chunk *chunks, uint64_t n,
-                   uint64_t *cand, uint32_t *counts, uint32_t sample_below, cudaStream_t st) {
-  chunk_kernel<W><<<(unsigned)((n + 127) / 128), 128, 0, st>>>(sv, bases, chunks, n, cand, counts,
-                                                                sample_below);
+                   uint64_t *cand, uint32_t *counts, const uint32_t *offs, uint32_t sample_below,
+                   bool only_starts, cudaStream_t st) {
+  chunk_kernel<W><<<(unsigned)((n + 127) / 128), 128, 0, st>>>(sv, bases, chunks, n, cand, counts, offs,
+                                                                sample_below, only_starts);
   note_launches();
 }
 
@@ -318,16 +342,24 @@ __global__ void key_unique_kernel(const uint64_t *keys, uint64_t n, const uint32
   if (i < n && (i == 0 || keys[i] != keys[i - 1])) out[pos[i]] = keys[i];
 }
 
-// Device buffers of one call, freed together.
+// Device buffers of one call, given back together on its stream.
 struct Scratch {
+  int device;
+  cudaStream_t st;
   std::vector<void *> ptrs;
-  ~Scratch() {
-    for (void *p : ptrs) cudaFree(p);
+  ~Scratch() { keep_only(nullptr, nullptr); }
+  void keep_only(const void *a, const void *b) {
+    std::vector<void *> kept;
+    for (void *p : ptrs) {
+      if (p == a || p == b) kept.push_back(p);
+      else cudaFreeAsync(p, st);
+    }
+    ptrs.swap(kept);
   }
   template <class T>
   cudaError_t get(T **p, uint64_t count) {
     *p = nullptr;
-    cudaError_t e = cudaMalloc(reinterpret_cast<void **>(p), std::max<uint64_t>(count, 1) * sizeof(T));
+    cudaError_t e = scratch_alloc(reinterpret_cast<void **>(p), std::max<uint64_t>(count, 1) * sizeof(T), device, st);
     if (e == cudaSuccess) ptrs.push_back(*p);
     return e;
   }
@@ -340,11 +372,15 @@ struct StreamGuard {
   }
 };
 
-// A batch's candidates, compacted on the device.
+// A batch's candidates on the device: chunk c has counts[c], offs[c] of the
+// others before them, at cand + offs[c] (packed) or cand + chunks[c].slot.
 struct Gathered {
-  uint64_t *keys = nullptr;      // n candidate minimizers
-  uint32_t *blocks = nullptr;    // the block of each
-  uint64_t n = 0;
+  uint64_t n = 0, n_chunks = 0;
+  bool packed = false;
+  Chunk *chunks = nullptr;
+  uint64_t *cand = nullptr;
+  uint32_t *counts = nullptr, *offs = nullptr;
+  uint64_t largest = 0;          // most candidates a block can have
   std::vector<uint32_t> block_taxon;
 };
 
@@ -370,13 +406,17 @@ k2g_status gather(const k2g_db *db, const char *bases, const uint64_t *seq_off,
       const uint64_t finish = std::min(j + block_size + k - 1, len);
       const uint32_t blk = (uint32_t)g.block_taxon.size();
       const size_t before = chunks.size();
+      uint64_t most = be > j ? be - j : 0;
       for (uint64_t c = j; c < be; c += kChunk)
         chunks.push_back(Chunk{s0 + c, s0 + c, (uint32_t)std::min<uint64_t>(kChunk, be - c), blk,
                                c == j ? kOpensBlock : kContinues, 0u});
       if (sv.k > sv.l)
         for (uint64_t sb = j; sb < finish; sb += subblock_size)
-          if (sb >= 1 && sb + k - 1 <= finish)
+          if (sb >= 1 && sb + k - 1 <= finish) {
             chunks.push_back(Chunk{s0 + sb, extra_slot++, 1u, blk, kSubblockStart, 0u});
+            most++;
+          }
+      g.largest = std::max(g.largest, most);
       if (chunks.size() > before) g.block_taxon.push_back(taxids ? taxids[i] : 1u);
       if (block_size > len) break;
     }
@@ -386,22 +426,36 @@ k2g_status gather(const k2g_db *db, const char *bases, const uint64_t *seq_off,
   const uint64_t nc = chunks.size();
   uint8_t *d_bases;
   Chunk *d_chunks;
-  uint64_t *d_cand;
+  uint64_t *d_cand = nullptr;
   uint32_t *d_counts, *d_offs, *d_sums;
   K2G_CUDA_TRY(s.get(&d_bases, total + 8));
   K2G_CUDA_TRY(s.get(&d_chunks, nc));
-  K2G_CUDA_TRY(s.get(&d_cand, extra_slot));
   K2G_CUDA_TRY(s.get(&d_counts, nc));
   K2G_CUDA_TRY(s.get(&d_offs, nc));
   K2G_CUDA_TRY(s.get(&d_sums, nc / rsort::kScanChunk + 2));
   K2G_CUDA_TRY(cudaMemcpyAsync(d_bases, bases + base0, total, cudaMemcpyHostToDevice, st));
   K2G_CUDA_TRY(cudaMemcpyAsync(d_chunks, chunks.data(), nc * sizeof(Chunk), cudaMemcpyHostToDevice, st));
-  switch (sv.w) {
-    case 1: launch_chunks<1>(sv, d_bases, d_chunks, nc, d_cand, d_counts, sample_below, st); break;
-    case 5: launch_chunks<5>(sv, d_bases, d_chunks, nc, d_cand, d_counts, sample_below, st); break;
-    case 7: launch_chunks<7>(sv, d_bases, d_chunks, nc, d_cand, d_counts, sample_below, st); break;
-    default: launch_chunks<0>(sv, d_bases, d_chunks, nc, d_cand, d_counts, sample_below, st); break;
-  }
+  const bool by_warps = scans_by_warps(sv), starts = extra_slot > total;
+  // one pass over the chunks: counts (cand null), or the candidates too
+  auto scan = [&](const uint32_t *offs) {
+    if (by_warps) {
+      const unsigned grid = (unsigned)((nc + kScanWarps - 1) / kScanWarps);
+      if (d_cand)
+        block_scan_kernel<true><<<grid, kScanWarps * 32, 0, st>>>(sv, d_bases, d_chunks, nc, d_cand, d_counts, offs, sample_below);
+      else
+        block_scan_kernel<false><<<grid, kScanWarps * 32, 0, st>>>(sv, d_bases, d_chunks, nc, nullptr, d_counts, nullptr, sample_below);
+      note_launches();
+    }
+    if (by_warps && !starts) return;
+    switch (sv.w) {
+      case 1: launch_chunks<1>(sv, d_bases, d_chunks, nc, d_cand, d_counts, offs, sample_below, by_warps, st); break;
+      case 5: launch_chunks<5>(sv, d_bases, d_chunks, nc, d_cand, d_counts, offs, sample_below, by_warps, st); break;
+      case 7: launch_chunks<7>(sv, d_bases, d_chunks, nc, d_cand, d_counts, offs, sample_below, by_warps, st); break;
+      default: launch_chunks<0>(sv, d_bases, d_chunks, nc, d_cand, d_counts, offs, sample_below, by_warps, st); break;
+    }
+  };
+  if (!by_warps) K2G_CUDA_TRY(s.get(&d_cand, extra_slot));
+  scan(nullptr);
   K2G_CUDA_TRY(cudaGetLastError());
   K2G_CUDA_TRY(cudaMemcpyAsync(d_offs, d_counts, nc * 4, cudaMemcpyDeviceToDevice, st));
   K2G_CUDA_TRY(rsort::exclusive_scan(d_offs, nc, d_sums, st));
@@ -410,13 +464,70 @@ k2g_status gather(const k2g_db *db, const char *bases, const uint64_t *seq_off,
   K2G_CUDA_TRY(cudaMemcpyAsync(&last[1], d_counts + nc - 1, 4, cudaMemcpyDeviceToHost, st));
   K2G_CUDA_TRY(cudaStreamSynchronize(st));
   g.n = (uint64_t)last[0] + last[1];
-  if (!g.n) return K2G_OK;
-  K2G_CUDA_TRY(s.get(&g.keys, g.n));
-  K2G_CUDA_TRY(s.get(&g.blocks, g.n));
-  compact_kernel<<<(unsigned)((nc * 32 + 255) / 256), 256, 0, st>>>(d_chunks, nc, d_cand, d_counts,
-                                                                       d_offs, g.keys, g.blocks);
+  if (by_warps && g.n) {
+    K2G_CUDA_TRY(s.get(&d_cand, g.n));
+    scan(d_offs);
+    K2G_CUDA_TRY(cudaGetLastError());
+    g.packed = true;
+  }
+  g.n_chunks = nc;
+  g.chunks = d_chunks;
+  g.cand = d_cand;
+  g.counts = d_counts;
+  g.offs = d_offs;
+  return K2G_OK;
+}
+
+// The candidates back to back, with the block of each.
+k2g_status compact(const Gathered &g, Scratch &s, uint64_t **keys, uint32_t **blocks, cudaStream_t st) {
+  K2G_CUDA_TRY(s.get(keys, g.n));
+  K2G_CUDA_TRY(s.get(blocks, g.n));
+  compact_kernel<<<(unsigned)((g.n_chunks * 32 + 255) / 256), 256, 0, st>>>(g.chunks, g.n_chunks, g.cand, g.counts,
+                                                                       g.offs, g.packed, *keys, *blocks);
   note_launches();
   K2G_CUDA_TRY(cudaGetLastError());
+  return K2G_OK;
+}
+
+// The distinct (block, minimizer) pairs in the build's order, blocks sorted
+// in shared memory (build_blocks.cuh).
+k2g_status sort_blocks(const Gathered &g, Scratch &s, const uint32_t *block_taxon, uint64_t **keys,
+                       uint32_t **taxa, uint64_t *n, cudaStream_t st) {
+  const uint32_t nb = (uint32_t)g.block_taxon.size();
+  uint32_t *first, *distinct, *place, *sums;
+  K2G_CUDA_TRY(s.get(&first, nb + 1));
+  K2G_CUDA_TRY(s.get(&distinct, nb));
+  K2G_CUDA_TRY(s.get(&place, nb));
+  K2G_CUDA_TRY(s.get(&sums, nb / rsort::kScanChunk + 2));
+  K2G_CUDA_TRY(s.get(keys, g.n));
+  K2G_CUDA_TRY(s.get(taxa, g.n));
+  const uint32_t nc = (uint32_t)g.n_chunks;
+  K2G_CUDA_TRY(cudaMemcpyAsync(first + nb, &nc, 4, cudaMemcpyHostToDevice, st));
+  block_first_kernel<<<(unsigned)((g.n_chunks + 255) / 256), 256, 0, st>>>(g.chunks, g.n_chunks, first);
+  note_launches();
+  // most blocks have a third as many candidates as k-mers: three thread
+  // blocks to an SM for those, one for the others
+  const uint32_t caps[3] = {0, kSmallBlock, kLargeBlock};
+  for (int i = 1; i < 3; i++) {
+    if (i > 1 && g.largest <= caps[i - 1]) break;
+    const size_t smem = block_sort_smem(caps[i]);
+    K2G_CUDA_TRY(cudaFuncSetAttribute(block_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    block_sort_kernel<<<nb, kSortThreads, smem, st>>>(first, g.cand, g.counts, g.offs, caps[i - 1], caps[i],
+                                                      distinct);
+    note_launches();
+    K2G_CUDA_TRY(cudaGetLastError());
+  }
+  K2G_CUDA_TRY(cudaMemcpyAsync(place, distinct, nb * 4ull, cudaMemcpyDeviceToDevice, st));
+  K2G_CUDA_TRY(rsort::exclusive_scan(place, nb, sums, st));
+  block_pack_kernel<<<(unsigned)((nb * 32ull + 255) / 256), 256, 0, st>>>(first, g.offs, g.cand, distinct, place, nb,
+                                                                         block_taxon, *keys, *taxa);
+  note_launches();
+  K2G_CUDA_TRY(cudaGetLastError());
+  uint32_t last[2] = {0, 0};
+  K2G_CUDA_TRY(cudaMemcpyAsync(&last[0], place + nb - 1, 4, cudaMemcpyDeviceToHost, st));
+  K2G_CUDA_TRY(cudaMemcpyAsync(&last[1], distinct + nb - 1, 4, cudaMemcpyDeviceToHost, st));
+  K2G_CUDA_TRY(cudaStreamSynchronize(st));
+  *n = (uint64_t)last[0] + last[1];
   return K2G_OK;
 }
 
@@ -437,31 +548,45 @@ extern "C" k2g_status k2g_build_sequences(k2g_db *db, const char *bases, const u
   StreamGuard guard;
   K2G_CUDA_TRY(cudaStreamCreateWithFlags(&guard.s, cudaStreamNonBlocking));
   cudaStream_t st = guard.s;
-  Scratch s;
+  Scratch s{db->device, st};
   Gathered g;
   k2g_status r = gather(db, bases, seq_off, taxids, n_seqs, block_size, subblock_size, 0, s, st, g);
   if (r != K2G_OK || !g.n) return r;
   const uint64_t n = g.n, nb = g.block_taxon.size();
   const int key_bits = db->scan_view().l * (db->opts.dna_db ? 2 : 4);
 
-  uint64_t *d_k1;
-  uint32_t *d_v1, *d_hist, *d_hsums, *d_btax;
+  uint32_t *d_btax;
+  K2G_CUDA_TRY(s.get(&d_btax, nb));
+  K2G_CUDA_TRY(cudaMemcpyAsync(d_btax, g.block_taxon.data(), nb * 4, cudaMemcpyHostToDevice, st));
+  // (a thread block holds the candidates of a sequence block up to 25,600,
+  // at least those of 16,384 k-mer starts; larger ones go to radix passes)
+  if (scans_by_warps(db->scan_view()) && g.largest <= kLargeBlock) {
+    uint64_t *keys = nullptr, n_pairs = 0;
+    uint32_t *taxa = nullptr;
+    r = sort_blocks(g, s, d_btax, &keys, &taxa, &n_pairs, st);
+    s.keep_only(keys, taxa);   // (the insert needs as much again)
+    if (r == K2G_OK) r = k2g_build_insert(db, keys, taxa, n_pairs, ordered, st);
+    if (r == K2G_OK && n_keys) *n_keys = n_pairs;
+    return r;
+  }
+  uint64_t *g_keys, *d_k1;
+  uint32_t *g_blocks, *d_v1, *d_hist, *d_hsums;
+  r = compact(g, s, &g_keys, &g_blocks, st);
+  if (r != K2G_OK) return r;
   const uint32_t ntiles = (uint32_t)((n + kPTile - 1) / kPTile);
   const uint64_t hist_n = 256ull * ntiles;
   K2G_CUDA_TRY(s.get(&d_k1, n));
   K2G_CUDA_TRY(s.get(&d_v1, n));
   K2G_CUDA_TRY(s.get(&d_hist, hist_n));
   K2G_CUDA_TRY(s.get(&d_hsums, (hist_n + rsort::kScanChunk - 1) / rsort::kScanChunk + 1));
-  K2G_CUDA_TRY(s.get(&d_btax, nb));
-  K2G_CUDA_TRY(cudaMemcpyAsync(d_btax, g.block_taxon.data(), nb * 4, cudaMemcpyHostToDevice, st));
 
   // passes: minimizer bytes (2l bits), zone, block bytes
   std::vector<Digit> passes;
   for (int sh = 0; sh < key_bits; sh += 8) passes.push_back(Digit{0, sh});
   passes.push_back(Digit{1, 0});
   for (int sh = 0; sh < 32 && (nb - 1) >> sh; sh += 8) passes.push_back(Digit{2, sh});
-  uint64_t *ka = g.keys, *kb = d_k1;
-  uint32_t *va = g.blocks, *vb = d_v1;
+  uint64_t *ka = g_keys, *kb = d_k1;
+  uint32_t *va = g_blocks, *vb = d_v1;
   for (const Digit &dg : passes) {
     pair_hist_kernel<<<ntiles, kPThreads, 0, st>>>(ka, va, n, dg, d_hist, ntiles);
     note_launches();
@@ -509,21 +634,24 @@ extern "C" k2g_status k2g_sample_minimizers(const k2g_db *db, const char *bases,
   StreamGuard guard;
   K2G_CUDA_TRY(cudaStreamCreateWithFlags(&guard.s, cudaStreamNonBlocking));
   cudaStream_t st = guard.s;
-  Scratch s;
+  Scratch s{db->device, st};
   Gathered g;
   // whole sequences: one block, no subblocks (MinimizerScanner::LoadSequence(seq))
   const uint64_t whole = UINT64_MAX / 4;
   k2g_status r = gather(db, bases, seq_off, nullptr, n_seqs, whole, whole, sample_below, s, st, g);
   if (r != K2G_OK || !g.n) return r;
   const uint64_t n = g.n;
-  uint64_t *d_alt, *sorted = nullptr;
+  uint64_t *g_keys, *d_alt, *sorted = nullptr;
+  uint32_t *g_blocks;
+  r = compact(g, s, &g_keys, &g_blocks, st);
+  if (r != K2G_OK) return r;
   uint32_t *d_hist, *d_hsums, *d_flag, *d_fsums;
   K2G_CUDA_TRY(s.get(&d_alt, n));
   K2G_CUDA_TRY(s.get(&d_hist, rsort::hist_entries(n)));
   K2G_CUDA_TRY(s.get(&d_hsums, rsort::sum_entries(n) + 1));
-  K2G_CUDA_TRY(rsort::sort_u64(g.keys, d_alt, n, db->scan_view().l * (db->opts.dna_db ? 2 : 4),
+  K2G_CUDA_TRY(rsort::sort_u64(g_keys, d_alt, n, db->scan_view().l * (db->opts.dna_db ? 2 : 4),
                                d_hist, d_hsums, st, &sorted));
-  uint64_t *d_out = sorted == g.keys ? d_alt : g.keys;
+  uint64_t *d_out = sorted == g_keys ? d_alt : g_keys;
   K2G_CUDA_TRY(s.get(&d_flag, n));
   K2G_CUDA_TRY(s.get(&d_fsums, (n + rsort::kScanChunk - 1) / rsort::kScanChunk + 1));
   const unsigned gr = (unsigned)((n + 255) / 256);

@@ -277,9 +277,15 @@ int bits_of(uint64_t x) {
 
 template <class T>
 struct DevBuf {
+  int device;
+  cudaStream_t st;
   T *p = nullptr;
-  ~DevBuf() { if (p) cudaFree(p); }
-  cudaError_t alloc(uint64_t n) { return cudaMalloc(&p, std::max<uint64_t>(n, 1) * sizeof(T)); }
+  DevBuf(int d, cudaStream_t s) : device(d), st(s) {}
+  DevBuf(const DevBuf &) = delete;
+  ~DevBuf() { if (p) cudaFreeAsync(p, st); }
+  cudaError_t alloc(uint64_t n) {
+    return scratch_alloc(reinterpret_cast<void **>(&p), std::max<uint64_t>(n, 1) * sizeof(T), device, st);
+  }
 };
 
 }  // namespace
@@ -293,11 +299,12 @@ k2g_status insert_ordered(k2g_db *db, typename C::T *cells, const uint64_t *d_ke
   const TableView t = db->table_view();
   const uint64_t cap = db->capacity;
   if (bits_of(cap) + kIndexBits > 64) return fail(K2G_ERR_UNSUPPORTED, "table too large for the ordered insert");
-  DevBuf<T> snap;
-  DevBuf<uint32_t> occ, status;
-  DevBuf<uint64_t> keys, alt, flags, scratch;
-  DevBuf<uint32_t> hist, sums;
-  DevBuf<unsigned long long> ctr;
+  const int dev = db->device;
+  DevBuf<T> snap(dev, st);
+  DevBuf<uint32_t> occ(dev, st), status(dev, st);
+  DevBuf<uint64_t> keys(dev, st), alt(dev, st), flags(dev, st), scratch(dev, st);
+  DevBuf<uint32_t> hist(dev, st), sums(dev, st);
+  DevBuf<unsigned long long> ctr(dev, st);
   K2G_CUDA_TRY(snap.alloc(cap));
   K2G_CUDA_TRY(occ.alloc((cap + 31) / 32));
   K2G_CUDA_TRY(status.alloc(1));
@@ -320,7 +327,10 @@ k2g_status insert_ordered(k2g_db *db, typename C::T *cells, const uint64_t *d_ke
   note_launches(2);
   K2G_CUDA_TRY(cudaGetLastError());
   uint64_t *sorted = nullptr;
-  K2G_CUDA_TRY(rsort::sort_u64(keys.p, alt.p, n, 64, hist.p, sums.p, st, &sorted));
+  // by cluster start alone: the list positions below it are in order already,
+  // and the sort is stable (pairs that are not inserted have all bits set,
+  // above any cell number)
+  K2G_CUDA_TRY(rsort::sort_u64(keys.p, alt.p, n, kIndexBits + bits_of(cap), hist.p, sums.p, st, &sorted, kIndexBits));
   // 3. per-cluster replays
   K2G_CUDA_TRY(flags.alloc(kFlagCap));
   replay_kernel<C><<<grid(db->device, n), 256, 0, st>>>(v, sorted, n, flags.p, ctr.p);

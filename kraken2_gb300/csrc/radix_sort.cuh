@@ -179,13 +179,13 @@ inline cudaError_t exclusive_scan(uint32_t *v, uint64_t n, uint32_t *sums, cudaS
   return cudaGetLastError();
 }
 
-// Sorts keys[0, n) by bits [0, nbits); *result receives keys or alt,
+// Sorts keys[0, n) by bits [first_bit, nbits), stably; *result receives keys or alt,
 // whichever holds the sorted keys.  n must stay below 2^32.
 inline cudaError_t sort_u64(uint64_t *keys, uint64_t *alt, uint64_t n, int nbits, uint32_t *hist,
-                            uint32_t *sums, cudaStream_t st, uint64_t **result) {
+                            uint32_t *sums, cudaStream_t st, uint64_t **result, int first_bit = 0) {
   uint64_t *a = keys, *b = alt;
   const uint32_t ntiles = (uint32_t)((n + kTile - 1) / kTile);
-  for (int shift = 0; shift < nbits && n > 1; shift += 8) {
+  for (int shift = first_bit; shift < nbits && n > 1; shift += 8) {
     hist_kernel<<<ntiles, kThreads, 0, st>>>(a, n, shift, hist, ntiles);
     note_launches();
     cudaError_t e = exclusive_scan(hist, (uint64_t)kRadix * ntiles, sums, st);

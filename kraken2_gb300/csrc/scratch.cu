@@ -14,7 +14,7 @@
 namespace k2g {
 namespace {
 
-constexpr uint64_t kKeep = 256ull << 20;
+constexpr uint64_t kKeep = 1ull << 30;
 
 struct Pool {
   std::mutex mu;

@@ -139,6 +139,25 @@ __device__ __forceinline__ uint32_t wc_low_quality(const uint4 &q, uint32_t qthr
   return bad;
 }
 
+// Window minima: m[j] of the five candidates ending at position j, the first
+// four positions' reaching into the lane below.
+__device__ __forceinline__ void wc_window5(const uint64_t (&c)[kWcPos], uint64_t (&m)[kWcPos]) {
+  const uint64_t s6 = min64(c[6], c[7]), s5 = min64(c[5], s6), s4 = min64(c[4], s5);
+  const uint64_t p3 = __shfl_up_sync(0xffffffffu, c[7], 1), p2 = __shfl_up_sync(0xffffffffu, s6, 1),
+                 p1 = __shfl_up_sync(0xffffffffu, s5, 1), p0 = __shfl_up_sync(0xffffffffu, s4, 1);
+  const uint64_t q1 = min64(c[0], c[1]), q2 = min64(q1, c[2]), q3 = min64(q2, c[3]);
+  m[0] = min64(p0, c[0]);
+  m[1] = min64(p1, q1);
+  m[2] = min64(p2, q2);
+  m[3] = min64(p3, q3);
+  const uint64_t t2 = min64(c[2], c[3]), t1 = min64(c[1], t2);
+  const uint64_t u1 = min64(c[4], c[5]), u2 = min64(u1, c[6]), u3 = min64(u2, c[7]);
+  m[4] = min64(q3, c[4]);
+  m[5] = min64(t1, u1);
+  m[6] = min64(t2, u2);
+  m[7] = min64(c[3], u3);
+}
+
 // The walk of CompactHashTable::Get over one 32-byte sector of the table:
 // the value where it ends (0: absent), or kWalkOn.  Cells [off, lim) count.
 constexpr uint32_t kWalkOn = 0xFFFFFFFFu;
@@ -978,24 +997,8 @@ __global__ void __launch_bounds__(kWcWarps * 32, kWcBlocks) warp_classify_kernel
           if ((v >> (36 + j - k)) & am) amb |= 1u << j;
         }
       }
-      // window minima: five candidates ending at each position
       uint64_t m[kWcPos];
-      {
-        const uint64_t s6 = min64(c[6], c[7]), s5 = min64(c[5], s6), s4 = min64(c[4], s5);
-        const uint64_t p3 = __shfl_up_sync(0xffffffffu, c[7], 1), p2 = __shfl_up_sync(0xffffffffu, s6, 1),
-                       p1 = __shfl_up_sync(0xffffffffu, s5, 1), p0m = __shfl_up_sync(0xffffffffu, s4, 1);
-        const uint64_t q1 = min64(c[0], c[1]), q2 = min64(q1, c[2]), q3 = min64(q2, c[3]);
-        m[0] = min64(p0m, c[0]);
-        m[1] = min64(p1, q1);
-        m[2] = min64(p2, q2);
-        m[3] = min64(p3, q3);
-        const uint64_t t2 = min64(c[2], c[3]), t1 = min64(c[1], t2);
-        const uint64_t u1 = min64(c[4], c[5]), u2 = min64(u1, c[6]), u3 = min64(u2, c[7]);
-        m[4] = min64(q3, c[4]);
-        m[5] = min64(t1, u1);
-        m[6] = min64(t2, u2);
-        m[7] = min64(c[3], u3);
-      }
+      wc_window5(c, m);
       // token groups
       uint32_t cont = 0;
       uint64_t next_min;
