@@ -11,6 +11,7 @@
 #include "classify_split.h"
 #include "k2g_internal.h"
 #include "pipeline.cuh"
+#include "warp_classify.cuh"
 
 namespace k2g {
 // compiled in classify_w5.cu / classify_misc.cu
@@ -75,32 +76,71 @@ k2g_status max_table_value(const k2g_db *db, uint32_t *out) {
 // Lookup: KeyValueStore::GetBatch
 // ---------------------------------------------------------------------------
 
-__global__ void lookup_kernel(TableView t, const uint64_t *keys, uint32_t *vals, uint64_t n) {
-  constexpr int B = 4;
-  uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  if (t.wide) {   // 40-bit cells
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += stride)
-      vals[i] = table_get_wide(t, murmur3(keys[i]));
-    return;
-  }
-  for (uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i0 < n; i0 += stride * B) {
-    uint64_t hc[B], idx[B];
-    Sector sec[B];
+// A tile of kLookupThreads x K keys per block: all home sectors first, then
+// the walks that go on (one in five at load 0.7) from a list in shared memory,
+// a thread each -- in their own threads they kept whole warps waiting for a
+// few lanes.  Bound by the random sectors: 16.8M keys, 2 GB table 0.67 ->
+// 0.40 ms (54 G sectors/s).
+constexpr int kLookupThreads = 256;
+
+template <bool WIDE, int K>
+__global__ void __launch_bounds__(kLookupThreads)
+lookup_kernel(TableView t, const uint64_t *keys, uint32_t *vals, uint64_t n) {
+  constexpr uint32_t N = WIDE ? 4 : 8, kLogN = WIDE ? 2 : 3;
+  __shared__ uint4 list[kLookupThreads * K];   // hash, key of the tile, sector
+  __shared__ uint32_t n_list;
+  if (threadIdx.x == 0) n_list = 0;
+  __syncthreads();
+  const uint64_t i0 = blockIdx.x * (uint64_t)(kLookupThreads * K) + threadIdx.x;
+  uint64_t hc[K], idx[K];
+  Sector sec[K];
 #pragma unroll
-    for (int b = 0; b < B; b++) {
-      uint64_t i = i0 + b * stride;
-      if (i < n) {
-        hc[b] = murmur3(keys[i]);
-        idx[b] = fast_mod(hc[b], t.div);
-        sec[b] = load_sector(t.cells, idx[b] & ~7ull);
-      }
-    }
-#pragma unroll
-    for (int b = 0; b < B; b++) {
-      uint64_t i = i0 + b * stride;
-      if (i < n) vals[i] = probe_sectors(t, hc[b], idx[b], sec[b]);
-    }
+  for (int b = 0; b < K; b++) {
+    const uint64_t i = i0 + b * kLookupThreads;
+    hc[b] = i < n ? murmur3(__ldcs(keys + i)) : 0;
+    idx[b] = mod_once(hc[b], t.div);
+    sec[b] = wc_load<WIDE>(t, idx[b] & ~(uint64_t)(N - 1));
   }
+#pragma unroll
+  for (int b = 0; b < K; b++) {
+    const uint64_t i = i0 + b * kLookupThreads;
+    const uint64_t base = idx[b] & ~(uint64_t)(N - 1), left = t.capacity - base;
+    const uint32_t v = wc_sector<WIDE>(t, sec[b], hc[b], (uint32_t)idx[b] & (N - 1), left < N ? (uint32_t)left : N);
+    if (i >= n) continue;
+    if (v != kWalkOn) __stcs(vals + i, v);
+    else
+      list[atomicAdd(&n_list, 1u)] = make_uint4((uint32_t)hc[b], (uint32_t)(hc[b] >> 32),
+                                                threadIdx.x + b * kLookupThreads, (uint32_t)(base >> kLogN));
+  }
+  __syncthreads();
+  const uint64_t tile = blockIdx.x * (uint64_t)(kLookupThreads * K);
+  for (uint32_t e = threadIdx.x; e < n_list; e += kLookupThreads) {
+    const uint4 x = list[e];
+    const uint64_t base = (uint64_t)x.w << kLogN;
+    vals[tile + x.z] = wc_walk<WIDE>(t, ((uint64_t)x.y << 32) | x.x, base + N >= t.capacity ? 0 : base + N);
+  }
+}
+
+// Tables with 2^32 sectors and more: a walk per thread.
+__global__ void lookup_large_kernel(TableView t, const uint64_t *keys, uint32_t *vals, uint64_t n) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += stride)
+    vals[i] = table_get(t, keys[i]);
+}
+
+template <bool WIDE>
+static void launch_lookup(const TableView &t, const uint64_t *keys, uint32_t *vals, uint64_t n, int sms,
+                          cudaStream_t st) {
+  // A table within L2 is bound by instructions: three keys a thread share
+  // them better (2M keys, 8 MB: 28 against 31 us) where that still gives every
+  // SM its eight blocks.  Beyond L2 one key a thread leaves more warps, and so
+  // loads, in flight (16.8M keys, 2 GB: 404 against 414 us).
+  constexpr int K = 3;
+  constexpr uint64_t kL2 = 126ull << 20;
+  if (t.capacity * (WIDE ? 8 : 4) <= kL2 && n >= (uint64_t)sms * 8 * kLookupThreads * K)
+    lookup_kernel<WIDE, K><<<(unsigned)((n + kLookupThreads * K - 1) / (kLookupThreads * K)), kLookupThreads, 0, st>>>(t, keys, vals, n);
+  else
+    lookup_kernel<WIDE, 1><<<(unsigned)((n + kLookupThreads - 1) / kLookupThreads), kLookupThreads, 0, st>>>(t, keys, vals, n);
 }
 
 // ---------------------------------------------------------------------------
@@ -703,9 +743,12 @@ extern "C" k2g_status k2g_lookup(const k2g_db *db, const uint64_t *d_keys, uint3
   if (!n) return K2G_OK;
   K2G_CUDA_TRY(cudaSetDevice(db->device));
   cudaStream_t st = (cudaStream_t)stream;
-  uint64_t blocks = std::min<uint64_t>((n + 1023) / 1024, (uint64_t)sm_count(db->device) * 16);
-  lookup_kernel<<<(unsigned)std::max<uint64_t>(1, blocks), 256, 0, st>>>(db->table_view(), d_keys,
-                                                                          d_vals, n);
+  const TableView t = db->table_view();
+  const int sms = sm_count(db->device);
+  if (t.capacity / (t.wide ? 4 : 8) >= (1ull << 32))
+    lookup_large_kernel<<<(unsigned)std::min<uint64_t>((n + 255) / 256, (uint64_t)sms * 8), 256, 0, st>>>(t, d_keys, d_vals, n);
+  else if (t.wide) launch_lookup<true>(t, d_keys, d_vals, n, sms, st);
+  else launch_lookup<false>(t, d_keys, d_vals, n, sms, st);
   note_launches();
   K2G_CUDA_TRY(cudaGetLastError());
   return K2G_OK;
