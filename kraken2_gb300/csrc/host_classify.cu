@@ -1,10 +1,11 @@
 // k2g_classify_host: classification of reads held in host memory.
 //
-// The input is cut into chunks.  Each chunk is copied in, classified and its
-// results copied out on one of two streams, so the copies of one chunk
-// overlap the kernels of the other.  Hit-list runs are compacted on the
-// device (exclusive scan of the per-fragment run counts, then a gather) so
-// only the used runs cross back to the host.
+// The input is cut into chunks of about an eighth of the call.  Each chunk is
+// copied in, classified and its results copied out on one of three streams,
+// so its copies overlap the kernels of the others, and the host waits for a
+// chunk only when the two after it are under way.  Hit-list runs are
+// compacted on the device (exclusive scan of the per-fragment run counts,
+// then a gather) so only the used runs cross back to the host.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -69,15 +70,29 @@ __global__ void scan_sums_kernel(uint64_t *sums, uint64_t nb, uint64_t *total) {
   if (threadIdx.x == 0) *total = carry;
 }
 
-// Adds block offsets and gathers each fragment's runs into the dense array.
+// Adds block offsets and gathers each fragment's runs into the dense array: a
+// thread copies a short list, a warp the long ones of its 32 fragments one
+// after another (a thread each for all took 0.72 ms for 120k fragments of up
+// to 50 kb).
+constexpr uint32_t kShortList = 16;
+
 __global__ void gather_runs_kernel(const uint64_t *sparse, const uint64_t *seq_off, int per,
                                    const uint32_t *len, uint64_t *excl, const uint64_t *sums,
                                    uint64_t n, uint64_t *dense) {
-  uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  uint64_t o = excl[i] + sums[i / kScanBlock];
-  const uint64_t src = seq_off[i * per] + 2 * i;
-  for (uint32_t r = 0; r < len[i]; r++) dense[o + r] = sparse[src + r];
+  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+  const uint32_t lane = threadIdx.x & 31;
+  const bool in = i < n;
+  const uint32_t m = in ? len[i] : 0;
+  const uint64_t to = in ? excl[i] + sums[i / kScanBlock] : 0, from = in ? seq_off[i * per] + 2 * i : 0;
+  if (m <= kShortList)
+    for (uint32_t r = 0; r < m; r++) dense[to + r] = sparse[from + r];
+  for (uint32_t todo = __ballot_sync(0xffffffffu, m > kShortList); todo; todo &= todo - 1) {
+    const int who = __ffs(todo) - 1;
+    const uint32_t k = __shfl_sync(0xffffffffu, m, who);
+    const uint64_t o = __shfl_sync(0xffffffffu, to, who), src = __shfl_sync(0xffffffffu, from, who);
+#pragma unroll 4
+    for (uint32_t r = lane; r < k; r += 32) dense[o + r] = sparse[src + r];
+  }
 }
 
 __global__ void rebase_kernel(uint64_t *off, uint64_t n, uint64_t base) {
@@ -129,22 +144,25 @@ struct Slot {
   cudaEvent_t done = nullptr;
   char *bases = nullptr, *quals = nullptr;
   uint64_t *off = nullptr;
-  uint32_t *call = nullptr, *hg = nullptr, *hlen = nullptr, *status = nullptr;
+  uint32_t *call = nullptr, *hg = nullptr, *hlen = nullptr;
   uint64_t *sparse = nullptr, *dense = nullptr, *excl = nullptr, *sums = nullptr;
-  uint64_t *total = nullptr;       // device
-  uint64_t *h_total = nullptr;     // pinned
+  uint64_t *total = nullptr;       // device: runs of the chunk, then its status word
+  uint64_t *h_total = nullptr;     // the same, pinned
   // add_kmer events (only with counters)
   uint64_t *hit_keys = nullptr, *hit_order = nullptr, *hits_used = nullptr;
   uint32_t *hit_taxa = nullptr, *blocks = nullptr;
   uint64_t cap_bases = 0, cap_frags = 0, cap_quals = 0, cap_hits = 0;
-  // chunk bookkeeping for the deferred runs copy
-  bool pending = false;
-  uint64_t f0 = 0, nf = 0;
+  // the chunk under way
+  bool copied = false;             // results on their way out
+  uint64_t f0 = 0, nf = 0, max_len = 0;
+  k2g_reads rd{};
+  k2g_results rs{};
 };
+constexpr int kSlots = 3;
 
 struct HostCache {
   std::mutex mu;
-  Slot slots[2];
+  Slot slots[kSlots];
   unsigned long long *taxon_reads = nullptr;
   uint64_t taxon_cap = 0;
 };
@@ -164,9 +182,8 @@ cudaError_t fit_slot(Slot &s, uint64_t bb, uint64_t fb, int per, bool quals, uin
   if (!s.st) {
     TRY(cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking));
     TRY(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
-    TRY(cudaHostAlloc(&s.h_total, 8, cudaHostAllocDefault));
-    TRY(cudaMalloc(&s.status, 4));
-    TRY(cudaMalloc(&s.total, 8));
+    TRY(cudaHostAlloc(&s.h_total, 16, cudaHostAllocDefault));
+    TRY(cudaMalloc(&s.total, 16));
     TRY(cudaMalloc(&s.hits_used, 8));
   }
   if (bb > s.cap_bases || fb > s.cap_frags) {
@@ -219,9 +236,9 @@ uint64_t cut_by_bases(const uint64_t *seq_off, int per, uint64_t f, uint64_t n,
 
 }  // namespace
 
-// Host-buffer classification over double-buffered chunks.  With counters,
-// chunks end at reader-block boundaries (frag_block) and each chunk's
-// add_kmer events are folded in after it is classified.
+// Host-buffer classification over chunks.  With counters, chunks end at
+// reader-block boundaries (frag_block) and each chunk's add_kmer events are
+// folded in after it is classified.
 static k2g_status host_classify(const k2g_db *db, const char *bases, const char *quals,
                                 const uint64_t *seq_off, uint64_t n_frags,
                                 const uint32_t *frag_block, k2g_counters *counters,
@@ -237,8 +254,15 @@ static k2g_status host_classify(const k2g_db *db, const char *bases, const char 
   K2G_CUDA_TRY(cudaSetDevice(db->device));
   const int per = params->paired ? 2 : 1;
 
-  // chunk plan: ~256 MB of bases (64 MB with hit events) or 2M fragments
-  const uint64_t max_bases = counters ? 64ull << 20 : 256ull << 20, max_frags = 2ull << 20;
+  // Chunk plan: about an eighth of the call (a quarter with hit events, whose
+  // counting makes the host wait), 16 MB of bases at least -- below that a
+  // chunk's launches and copies outweigh what overlaps -- and 128 MB (64 MB
+  // with hit events) or 2M fragments at most.  2M x 150 bp: 8 chunks 3.5 ms,
+  // 2 of 256 MB 5.6.
+  const uint64_t all_bases = seq_off[n_frags * per] - seq_off[0];
+  const uint64_t max_bases = std::min<uint64_t>(counters ? 64ull << 20 : 128ull << 20,
+                                                std::max<uint64_t>(16ull << 20, all_bases / (counters ? 4 : 8) + 1)),
+                 max_frags = 2ull << 20;
   std::vector<uint64_t> cuts{0};
   while (cuts.back() < n_frags) {
     const uint64_t f = cuts.back();
@@ -271,133 +295,161 @@ static k2g_status host_classify(const k2g_db *db, const char *bases, const char 
   HostCache &hc = g_host[db->device & 63];
   std::lock_guard<std::mutex> lock(hc.mu);
   Slot *slots = hc.slots;
-  k2g_status status = K2G_OK;
-#define SLOT_TRY(call_)                                     \
-  do {                                                      \
-    cudaError_t _e = (call_);                               \
-    if (_e != cudaSuccess) return cuda_fail((int)_e, #call_); \
-  } while (0)
-  for (int i = 0; i < 2; i++)
-    SLOT_TRY(fit_slot(slots[i], chunk_bases, chunk_frags, per, quals != nullptr, hits_cap));
+  const size_t n_chunks = cuts.size() - 1;
+  // (a third slot as large as one huge sequence would be memory for nothing)
+  const size_t n_slots = chunk_bases > (256ull << 20) ? 2 : kSlots;
+  const int used = (int)std::min(n_chunks, n_slots);
+  for (int i = 0; i < used; i++)
+    K2G_CUDA_TRY(fit_slot(slots[i], chunk_bases, chunk_frags, per, quals != nullptr, hits_cap));
   unsigned long long *d_taxon_reads = nullptr;
   if (taxon_reads) {
     if (hc.taxon_cap < db->node_count) {
-      SLOT_TRY(regrow(hc.taxon_reads, db->node_count));
+      K2G_CUDA_TRY(regrow(hc.taxon_reads, db->node_count));
       hc.taxon_cap = db->node_count;
     }
     d_taxon_reads = hc.taxon_reads;
-    SLOT_TRY(cudaMemset(d_taxon_reads, 0, db->node_count * 8));
+    // zeroed before any stream's first chunk
+    K2G_CUDA_TRY(cudaMemsetAsync(d_taxon_reads, 0, db->node_count * 8, slots[0].st));
+    K2G_CUDA_TRY(cudaEventRecord(slots[0].done, slots[0].st));
+    for (int i = 1; i < used; i++) K2G_CUDA_TRY(cudaStreamWaitEvent(slots[i].st, slots[0].done, 0));
   }
 
+  // Stage 1 of chunk c: copy in.  (Blocks first: they often lie in pageable
+  // memory, where the call returns only when the stream has got to the copy.)
+  auto copy_in = [&](size_t c) -> k2g_status {
+    Slot &s = slots[c % n_slots];
+    const uint64_t f0 = cuts[c], nf = cuts[c + 1] - f0;
+    const uint64_t b0 = seq_off[f0 * per], nb = seq_off[(f0 + nf) * per] - b0;
+    s.f0 = f0;
+    s.nf = nf;
+    if (counters) {
+      K2G_CUDA_TRY(cudaMemcpyAsync(s.blocks, frag_block + f0, nf * 4, cudaMemcpyHostToDevice, s.st));
+      K2G_CUDA_TRY(cudaMemsetAsync(s.hits_used, 0, 8, s.st));
+    }
+    K2G_CUDA_TRY(cudaMemcpyAsync(s.off, seq_off + f0 * per, (nf * per + 1) * 8,
+                                 cudaMemcpyHostToDevice, s.st));
+    K2G_CUDA_TRY(cudaMemcpyAsync(s.bases, bases + b0, nb, cudaMemcpyHostToDevice, s.st));
+    if (quals) K2G_CUDA_TRY(cudaMemcpyAsync(s.quals, quals + b0, nb, cudaMemcpyHostToDevice, s.st));
+    K2G_CUDA_TRY(cudaMemsetAsync(s.total, 0, 16, s.st));
+    // longest sequence of the chunk (while the copies run)
+    s.max_len = 0;
+    for (uint64_t i = f0 * per; i < (f0 + nf) * per; i++)
+      s.max_len = std::max(s.max_len, seq_off[i + 1] - seq_off[i]);
+    return K2G_OK;
+  };
+  // Stage 2: classify.
+  auto classify = [&](size_t c) -> k2g_status {
+    Slot &s = slots[c % n_slots];
+    const uint64_t f0 = s.f0, nf = s.nf, b0 = seq_off[f0 * per], nb = seq_off[(f0 + nf) * per] - b0;
+    // (after the copies: a kernel waits for the blocks of the chunk before,
+    // and copies behind it would too)
+    rebase_kernel<<<(unsigned)((nf * per + 1 + 255) / 256), 256, 0, s.st>>>(s.off, nf * per + 1, b0);
+    note_launches();
+    s.rd = k2g_reads{};
+    s.rd.d_bases = s.bases;
+    s.rd.d_quals = quals ? s.quals : nullptr;
+    s.rd.d_seq_off = s.off;
+    s.rd.n_frags = nf;
+    s.rd.max_seq_len = s.max_len;
+    s.rd.total_bases = nb;
+    s.rd.frag_base = f0;
+    s.rs = k2g_results{};
+    s.rs.d_call = s.call;
+    s.rs.d_hit_groups = s.hg;
+    s.rs.d_hitlist_len = s.hlen;
+    s.rs.d_runs = s.sparse;
+    s.rs.runs_cap = s.cap_bases + 2 * s.cap_frags + 8;
+    s.rs.d_taxon_reads = reinterpret_cast<uint64_t *>(d_taxon_reads);
+    s.rs.d_status = reinterpret_cast<uint32_t *>(s.total + 1);
+    if (counters) {
+      s.rd.d_frag_block = s.blocks;
+      s.rs.d_hit_keys = s.hit_keys;
+      s.rs.d_hit_taxa = s.hit_taxa;
+      s.rs.d_hit_order = s.hit_order;
+      s.rs.hits_cap = s.cap_hits;
+      s.rs.d_hits_used = s.hits_used;
+    }
+    // short-read chunks share one execution state (in order, as overlapping
+    // them only adds interference); long-read chunks overlap their tails
+    // (the one-launch form has no state)
+    const void *key = long_batch(nb, nf) ? (const void *)s.st : (const void *)&hc;
+    return classify_keyed(db, &s.rd, params, &s.rs, K2G_MODE_PIPELINED, s.st, key);
+  };
+  // Stage 3: count the events, compact the runs, copy the fixed-size results.
+  auto copy_out = [&](size_t c) -> k2g_status {
+    Slot &s = slots[c % n_slots];
+    if (counters) {
+      const k2g_status r = k2g_counters_add(counters, &s.rd, &s.rs, s.st);
+      if (r != K2G_OK) return r;
+    }
+    const k2g_status r = compact_runs(s.sparse, s.off, per, s.hlen, s.nf, s.excl, s.sums, s.total, s.dense, s.st);
+    if (r != K2G_OK) return r;
+    K2G_CUDA_TRY(cudaMemcpyAsync(s.h_total, s.total, 16, cudaMemcpyDeviceToHost, s.st));
+    K2G_CUDA_TRY(cudaEventRecord(s.done, s.st));
+    K2G_CUDA_TRY(cudaMemcpyAsync(call + s.f0, s.call, s.nf * 4, cudaMemcpyDeviceToHost, s.st));
+    if (hit_groups)
+      K2G_CUDA_TRY(cudaMemcpyAsync(hit_groups + s.f0, s.hg, s.nf * 4, cudaMemcpyDeviceToHost, s.st));
+    if (hitlist_len)
+      K2G_CUDA_TRY(cudaMemcpyAsync(hitlist_len + s.f0, s.hlen, s.nf * 4, cudaMemcpyDeviceToHost, s.st));
+    s.copied = true;
+    return K2G_OK;
+  };
+  // Stage 4: copy the runs, whose number the host now knows (chunk order).
   uint64_t runs_written = 0;
-  // Copies the runs of a finished chunk (needs its run total on the host).
-  auto drain = [&](Slot &s) -> k2g_status {
-    if (!s.pending) return K2G_OK;
-    cudaError_t e = cudaEventSynchronize(s.done);
+  auto copy_runs = [&](size_t c) -> k2g_status {
+    Slot &s = slots[c % n_slots];
+    if (!s.copied) return K2G_OK;
+    const cudaError_t e = cudaEventSynchronize(s.done);
+    s.copied = false;
     if (e != cudaSuccess) return cuda_fail(e, "chunk completion");
-    s.pending = false;
-    uint32_t st_word = 0;
-    e = cudaMemcpy(&st_word, s.status, 4, cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return cuda_fail(e, "status readback");
-    if (st_word) return fail(K2G_ERR_CAPACITY, "classification buffer overflow");
-    uint64_t nr = *s.h_total;
+    if ((uint32_t)s.h_total[1]) return fail(K2G_ERR_CAPACITY, "classification buffer overflow");
+    const uint64_t nr = s.h_total[0];
     if (runs) {
       if (runs_written + nr > runs_cap) return fail(K2G_ERR_CAPACITY, "runs buffer too small");
-      e = cudaMemcpy(runs + runs_written, s.dense, nr * 8, cudaMemcpyDeviceToHost);
-      if (e != cudaSuccess) return cuda_fail(e, "runs copy");
+      K2G_CUDA_TRY(cudaMemcpyAsync(runs + runs_written, s.dense, nr * 8, cudaMemcpyDeviceToHost, s.st));
     }
     runs_written += nr;
     return K2G_OK;
   };
-  // On an error, let the chunks in flight finish before the slots are reused.
-  auto settle = [&]() {
-    for (int i = 0; i < 2; i++) {
-      if (slots[i].st) cudaStreamSynchronize(slots[i].st);
-      slots[i].pending = false;
+  auto all_chunks = [&]() -> k2g_status {
+    // with counters, stage 3 of a chunk makes the host wait for its kernels:
+    // the next chunk's are in the queue and the copies of the one after it on
+    // their way before that (1M x 150 bp: 4.2 -> 2.9 ms)
+    const size_t lag = counters ? 1 : 0, ahead = counters && n_slots > 2 ? 1 : 0;
+    for (size_t c = 0; c < n_chunks + ahead + lag; c++) {
+      k2g_status r = K2G_OK;
+      if (ahead && c >= ahead && c - ahead < n_chunks) r = classify(c - ahead);
+      if (r == K2G_OK && c < n_chunks) {
+        if (c >= n_slots) r = copy_runs(c - n_slots);
+        if (r == K2G_OK) r = copy_in(c);
+        if (r == K2G_OK && !ahead) r = classify(c);
+      }
+      if (r == K2G_OK && c >= ahead + lag) r = copy_out(c - ahead - lag);
+      if (r != K2G_OK) return r;
     }
+    for (size_t c = n_chunks > n_slots ? n_chunks - n_slots : 0; c < n_chunks; c++) {
+      const k2g_status r = copy_runs(c);
+      if (r != K2G_OK) return r;
+    }
+    return K2G_OK;
   };
-
-  for (size_t c = 0; c + 1 < cuts.size(); c++) {
-    Slot &s = slots[c & 1];
-    status = drain(s);
-    if (status != K2G_OK) { settle(); return status; }
-    const uint64_t f0 = cuts[c], nf = cuts[c + 1] - f0;
-    const uint64_t b0 = seq_off[f0 * per], nb = seq_off[(f0 + nf) * per] - b0;
-    // longest sequence of this chunk (overlaps the previous chunk's work)
-    uint64_t max_len = 0;
-    for (uint64_t i = f0 * per; i < (f0 + nf) * per; i++)
-      max_len = std::max(max_len, seq_off[i + 1] - seq_off[i]);
-    SLOT_TRY(cudaMemcpyAsync(s.bases, bases + b0, nb, cudaMemcpyHostToDevice, s.st));
-    if (quals) SLOT_TRY(cudaMemcpyAsync(s.quals, quals + b0, nb, cudaMemcpyHostToDevice, s.st));
-    SLOT_TRY(cudaMemcpyAsync(s.off, seq_off + f0 * per, (nf * per + 1) * 8,
-                             cudaMemcpyHostToDevice, s.st));
-    note_launches();
-    rebase_kernel<<<(unsigned)((nf * per + 1 + 255) / 256), 256, 0, s.st>>>(s.off, nf * per + 1, b0);
-    SLOT_TRY(cudaMemsetAsync(s.status, 0, 4, s.st));
-    k2g_reads rd{};
-    rd.d_bases = s.bases;
-    rd.d_quals = quals ? s.quals : nullptr;
-    rd.d_seq_off = s.off;
-    rd.n_frags = nf;
-    rd.max_seq_len = max_len;
-    rd.total_bases = nb;
-    rd.frag_base = f0;
-    k2g_results rs{};
-    rs.d_call = s.call;
-    rs.d_hit_groups = s.hg;
-    rs.d_hitlist_len = s.hlen;
-    rs.d_runs = s.sparse;
-    rs.runs_cap = s.cap_bases + 2 * s.cap_frags + 8;
-    rs.d_taxon_reads = reinterpret_cast<uint64_t *>(d_taxon_reads);
-    rs.d_status = s.status;
-    if (counters) {
-      SLOT_TRY(cudaMemcpyAsync(s.blocks, frag_block + f0, nf * 4, cudaMemcpyHostToDevice, s.st));
-      SLOT_TRY(cudaMemsetAsync(s.hits_used, 0, 8, s.st));
-      rd.d_frag_block = s.blocks;
-      rs.d_hit_keys = s.hit_keys;
-      rs.d_hit_taxa = s.hit_taxa;
-      rs.d_hit_order = s.hit_order;
-      rs.hits_cap = s.cap_hits;
-      rs.d_hits_used = s.hits_used;
-    }
-    // short-read chunks share one execution state (in order, as overlapping
-    // them only adds interference); long-read chunks overlap their tails
-    const void *key = long_batch(nb, nf) ? (const void *)s.st : (const void *)&hc;
-    status = classify_keyed(db, &rd, params, &rs, K2G_MODE_PIPELINED, s.st, key);
-    if (status != K2G_OK) { settle(); return status; }
-    if (counters) {
-      status = k2g_counters_add(counters, &rd, &rs, s.st);
-      if (status != K2G_OK) { settle(); return status; }
-    }
-    status = compact_runs(s.sparse, s.off, per, s.hlen, nf, s.excl, s.sums, s.total, s.dense, s.st);
-    if (status != K2G_OK) { settle(); return status; }
-    SLOT_TRY(cudaMemcpyAsync(s.h_total, s.total, 8, cudaMemcpyDeviceToHost, s.st));
-    SLOT_TRY(cudaMemcpyAsync(call + f0, s.call, nf * 4, cudaMemcpyDeviceToHost, s.st));
-    if (hit_groups)
-      SLOT_TRY(cudaMemcpyAsync(hit_groups + f0, s.hg, nf * 4, cudaMemcpyDeviceToHost, s.st));
-    if (hitlist_len)
-      SLOT_TRY(cudaMemcpyAsync(hitlist_len + f0, s.hlen, nf * 4, cudaMemcpyDeviceToHost, s.st));
-    SLOT_TRY(cudaEventRecord(s.done, s.st));
-    s.pending = true;
-    s.f0 = f0;
-    s.nf = nf;
-    // keep chunk order for the runs: drain the other slot (older chunk) now
-    Slot &o = slots[(c + 1) & 1];
-    status = drain(o);
-    if (status != K2G_OK) { settle(); return status; }
+  const k2g_status status = all_chunks();
+  // every copy is done (on an error too: the slots are free for the next call)
+  cudaError_t e = cudaSuccess;
+  for (int i = 0; i < used; i++) {
+    const cudaError_t es = cudaStreamSynchronize(slots[i].st);
+    if (es != cudaSuccess) e = es;
+    slots[i].copied = false;
   }
-  for (size_t c = cuts.size() - 1; c < cuts.size() + 1; c++) {
-    status = drain(slots[c & 1]);
-    if (status != K2G_OK) { settle(); return status; }
-  }
+  if (status != K2G_OK) return status;
+  if (e != cudaSuccess) return cuda_fail(e, "host classification");
   if (taxon_reads) {
     std::vector<uint64_t> tr(db->node_count);
-    SLOT_TRY(cudaMemcpy(tr.data(), d_taxon_reads, db->node_count * 8, cudaMemcpyDeviceToHost));
+    K2G_CUDA_TRY(cudaMemcpy(tr.data(), d_taxon_reads, db->node_count * 8, cudaMemcpyDeviceToHost));
     for (uint64_t i = 0; i < db->node_count; i++) taxon_reads[i] += tr[i];
   }
   if (n_runs) *n_runs = runs_written;
   return K2G_OK;
-#undef SLOT_TRY
 }
 
 extern "C" k2g_status k2g_classify_host(const k2g_db *db, const char *bases, const char *quals,
