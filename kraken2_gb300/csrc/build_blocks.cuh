@@ -7,11 +7,11 @@
 //                       candidates and then to write them back to back (a
 //                       place for every k-mer would be three times the
 //                       memory, and mapping it costs more than the scan);
-//   block_sort_kernel   one thread block per sequence block: its candidates
-//                       to shared memory by zone (MurmurHash3 mod 256, the
-//                       order's first key, so about 22 candidates a zone at
-//                       the default block size), each zone ranked and freed
-//                       of repeats by one warp;
+//   bucket_sort_kernel  (bucket_sort.cuh) one thread block per sequence block:
+//                       its candidates to shared memory by zone (MurmurHash3
+//                       mod 256, the order's first key, so about 22
+//                       candidates a zone at the default block size), each
+//                       zone ranked and freed of repeats by one warp;
 //   block_pack_kernel   the blocks' lists back to back, with their taxa.
 //
 // This replaces eleven radix passes over all (minimizer, block) pairs: for 48
@@ -19,6 +19,7 @@
 // 0.8 ms now; a candidate is written once, read twice and moved once.
 #pragma once
 
+#include "bucket_sort.cuh"
 #include "warp_classify.cuh"
 
 namespace k2g {
@@ -163,163 +164,20 @@ block_scan_kernel(ScanView sv, const uint8_t *bases, const Chunk *chunks, uint64
   }
 }
 
-constexpr int kSortThreads = 512;
-constexpr int kZones = 256;
-constexpr uint32_t kSmallBlock = 8064;    // candidates; three thread blocks to an SM
-constexpr uint32_t kLargeBlock = 25600;   // 200 KB of keys
-
-inline size_t block_sort_smem(uint32_t cap) { return (size_t)cap * 8 + kZones * 12 + 16; }
-
-// First chunk of every sequence block, by chunk order (block_first[n_blocks]
-// = n_chunks is set by the host).
-__global__ void block_first_kernel(const Chunk *chunks, uint64_t n_chunks, uint32_t *block_first) {
+// Where every sequence block's candidates start: chunks lie block after block.
+// (start[n_blocks] is set by the host.)
+__global__ void block_start_kernel(const Chunk *chunks, uint64_t n_chunks, const uint32_t *offs, uint32_t *start) {
   const uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  if (c < n_chunks && (c == 0 || chunks[c].block != chunks[c - 1].block)) block_first[chunks[c].block] = (uint32_t)c;
-}
-
-// Distinct candidates of a zone holding more than 128 keys, one after
-// another from the smallest (warp-wide); out may be null (count only).
-__device__ __forceinline__ uint32_t select_distinct(const uint64_t *z, uint32_t n, uint64_t *out) {
-  const uint32_t lane = threadIdx.x & 31;
-  uint64_t last = 0;
-  uint32_t d = 0;
-  for (;;) {
-    uint64_t best = ~0ull;
-    for (uint32_t i = lane; i < n; i += 32) {
-      const uint64_t x = z[i];
-      if ((!d || x > last) && x < best) best = x;
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) best = min64(best, __shfl_xor_sync(0xffffffffu, best, o));
-    if (best == ~0ull) return d;   // (a minimizer has at most 62 bits)
-    if (out && lane == 0) out[d] = best;
-    last = best;
-    d++;
-  }
-}
-
-// Blocks with lo < candidates <= cap, in place; the others return.
-__global__ void __launch_bounds__(kSortThreads)
-block_sort_kernel(const uint32_t *block_first, uint64_t *cand, const uint32_t *counts, const uint32_t *offs,
-                  uint32_t lo, uint32_t cap, uint32_t *n_distinct) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  uint64_t *key = reinterpret_cast<uint64_t *>(smem);
-  uint32_t *hist = reinterpret_cast<uint32_t *>(smem + (size_t)cap * 8), *first = hist + kZones, *dist = first + kZones;
-  const uint32_t b = blockIdx.x, c0 = block_first[b], c1 = block_first[b + 1];
-  const uint32_t base = offs[c0], n = offs[c1 - 1] + counts[c1 - 1] - base;
-  if (n <= lo && lo) return;
-  if (n > cap) return;
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = kSortThreads / 32;
-  if (!n) {
-    if (threadIdx.x == 0) n_distinct[b] = 0;
-    return;
-  }
-  for (uint32_t i = threadIdx.x; i < kZones; i += kSortThreads) hist[i] = 0;
-  __syncthreads();
-  const uint64_t *x = cand + base;
-  for (uint32_t i = threadIdx.x; i < n; i += kSortThreads) atomicAdd(&hist[murmur3(x[i]) & 0xFFu], 1u);
-  __syncthreads();
-  auto scan = [&](const uint32_t *in, uint32_t *out) {   // exclusive, by the first warp
-    uint32_t carry = 0;
-    for (int i0 = 0; i0 < kZones; i0 += 32) {
-      const uint32_t v = in[i0 + lane];
-      uint32_t x = v;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if ((int)lane >= o) x += y;
-      }
-      out[i0 + lane] = carry + x - v;
-      carry += __shfl_sync(0xffffffffu, x, 31);
-    }
-    return carry;
-  };
-  if (warp == 0) scan(hist, first);
-  __syncthreads();
-  for (uint32_t i = threadIdx.x; i < kZones; i += kSortThreads) dist[i] = first[i];   // cursors
-  __syncthreads();
-  for (uint32_t i = threadIdx.x; i < n; i += kSortThreads) {
-    const uint64_t v = x[i];
-    key[atomicAdd(&dist[murmur3(v) & 0xFFu], 1u)] = v;
-  }
-  __syncthreads();
-  // every zone sorted in place, repeats dropped
-  for (uint32_t z = warp; z < kZones; z += warps) {
-    const uint32_t m = hist[z];
-    uint64_t *zk = key + first[z];
-    uint32_t d = 0;
-    if (m <= 32) {
-      const uint64_t v = lane < m ? zk[lane] : ~0ull;
-      uint32_t less = 0;
-      bool again = false;
-      for (uint32_t j = 0; j < m; j++) {
-        const uint64_t x = __shfl_sync(0xffffffffu, v, j);
-        less |= x < v ? 1u << j : 0u;
-        again |= x == v && j < lane;
-      }
-      const bool own = lane < m && !again;
-      const uint32_t keepers = __ballot_sync(0xffffffffu, own);
-      __syncwarp();
-      if (own) zk[__popc(less & keepers)] = v;
-      d = __popc(keepers);
-    } else if (m <= 128) {
-      uint64_t v[4];
-      uint32_t own = 0, rank[4] = {0, 0, 0, 0};
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        const uint32_t i = 32 * t + lane;
-        v[t] = i < m ? zk[i] : ~0ull;
-        bool again = i >= m;
-        for (uint32_t j = 0; j < i && j < m; j++) again |= zk[j] == v[t];
-        own |= again ? 0u : 1u << t;
-      }
-      __syncwarp();
-      uint32_t keepers[4];
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        keepers[t] = __ballot_sync(0xffffffffu, (own >> t) & 1u);
-        d += __popc(keepers[t]);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-        for (uint32_t k = keepers[u]; k; k &= k - 1) {
-          const uint64_t x = zk[32 * u + __ffs(k) - 1];
-#pragma unroll
-          for (int t = 0; t < 4; t++) rank[t] += x < v[t] ? 1u : 0u;
-        }
-      __syncwarp();
-#pragma unroll
-      for (int t = 0; t < 4; t++)
-        if ((own >> t) & 1u) zk[rank[t]] = v[t];
-    } else {
-      d = select_distinct(zk, m, nullptr);
-    }
-    __syncwarp();
-    if (lane == 0) dist[z] = d;
-  }
-  __syncthreads();
-  __shared__ uint32_t place[kZones];
-  if (warp == 0) {
-    const uint32_t total = scan(dist, place);
-    if (lane == 0) n_distinct[b] = total;
-  }
-  __syncthreads();
-  for (uint32_t z = warp; z < kZones; z += warps) {
-    uint64_t *out = cand + base + place[z];
-    const uint64_t *zk = key + first[z];
-    if (hist[z] > 128) select_distinct(zk, hist[z], out);
-    else
-      for (uint32_t i = lane; i < dist[z]; i += 32) out[i] = zk[i];
-  }
+  if (c < n_chunks && (c == 0 || chunks[c].block != chunks[c - 1].block)) start[chunks[c].block] = offs[c];
 }
 
 // One warp per sequence block: its list to its place, and its taxon.
-__global__ void block_pack_kernel(const uint32_t *block_first, const uint32_t *offs, const uint64_t *sorted,
-                                  const uint32_t *n_distinct, const uint32_t *place, uint32_t n_blocks,
-                                  const uint32_t *block_taxon, uint64_t *out_keys, uint32_t *out_taxa) {
+__global__ void block_pack_kernel(const uint32_t *start, const uint64_t *sorted, const uint32_t *n_distinct,
+                                  const uint32_t *place, uint32_t n_blocks, const uint32_t *block_taxon,
+                                  uint64_t *out_keys, uint32_t *out_taxa) {
   const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (b >= n_blocks) return;
-  const uint64_t *x = sorted + offs[block_first[b]];
+  const uint64_t *x = sorted + start[b];
   const uint32_t n = n_distinct[b], o = place[b], t = block_taxon[b];
   for (uint32_t i = lane; i < n; i += 32) {
     out_keys[o + i] = x[i];

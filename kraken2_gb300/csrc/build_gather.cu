@@ -494,32 +494,21 @@ k2g_status compact(const Gathered &g, Scratch &s, uint64_t **keys, uint32_t **bl
 k2g_status sort_blocks(const Gathered &g, Scratch &s, const uint32_t *block_taxon, uint64_t **keys,
                        uint32_t **taxa, uint64_t *n, cudaStream_t st) {
   const uint32_t nb = (uint32_t)g.block_taxon.size();
-  uint32_t *first, *distinct, *place, *sums;
+  uint32_t *first, *distinct, *place, *sums;   // (first: where a block's candidates start)
   K2G_CUDA_TRY(s.get(&first, nb + 1));
   K2G_CUDA_TRY(s.get(&distinct, nb));
   K2G_CUDA_TRY(s.get(&place, nb));
   K2G_CUDA_TRY(s.get(&sums, nb / rsort::kScanChunk + 2));
   K2G_CUDA_TRY(s.get(keys, g.n));
   K2G_CUDA_TRY(s.get(taxa, g.n));
-  const uint32_t nc = (uint32_t)g.n_chunks;
-  K2G_CUDA_TRY(cudaMemcpyAsync(first + nb, &nc, 4, cudaMemcpyHostToDevice, st));
-  block_first_kernel<<<(unsigned)((g.n_chunks + 255) / 256), 256, 0, st>>>(g.chunks, g.n_chunks, first);
+  const uint32_t total = (uint32_t)g.n;
+  K2G_CUDA_TRY(cudaMemcpyAsync(first + nb, &total, 4, cudaMemcpyHostToDevice, st));
+  block_start_kernel<<<(unsigned)((g.n_chunks + 255) / 256), 256, 0, st>>>(g.chunks, g.n_chunks, g.offs, first);
   note_launches();
-  // most blocks have a third as many candidates as k-mers: three thread
-  // blocks to an SM for those, one for the others
-  const uint32_t caps[3] = {0, kSmallBlock, kLargeBlock};
-  for (int i = 1; i < 3; i++) {
-    if (i > 1 && g.largest <= caps[i - 1]) break;
-    const size_t smem = block_sort_smem(caps[i]);
-    K2G_CUDA_TRY(cudaFuncSetAttribute(block_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    block_sort_kernel<<<nb, kSortThreads, smem, st>>>(first, g.cand, g.counts, g.offs, caps[i - 1], caps[i],
-                                                      distinct);
-    note_launches();
-    K2G_CUDA_TRY(cudaGetLastError());
-  }
+  K2G_CUDA_TRY(bucket_sort(first, nb, g.largest, g.cand, distinct, ZoneMurmur{}, st));
   K2G_CUDA_TRY(cudaMemcpyAsync(place, distinct, nb * 4ull, cudaMemcpyDeviceToDevice, st));
   K2G_CUDA_TRY(rsort::exclusive_scan(place, nb, sums, st));
-  block_pack_kernel<<<(unsigned)((nb * 32ull + 255) / 256), 256, 0, st>>>(first, g.offs, g.cand, distinct, place, nb,
+  block_pack_kernel<<<(unsigned)((nb * 32ull + 255) / 256), 256, 0, st>>>(first, g.cand, distinct, place, nb,
                                                                          block_taxon, *keys, *taxa);
   note_launches();
   K2G_CUDA_TRY(cudaGetLastError());

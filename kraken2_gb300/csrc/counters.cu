@@ -31,6 +31,7 @@
 
 #include "k2g_device.cuh"
 #include "k2g_internal.h"
+#include "bucket_sort.cuh"
 #include "radix_sort.cuh"
 
 namespace k2g {
@@ -405,6 +406,7 @@ struct k2g_counters {
   int tbits = 0;                       // bits of a preorder number
   std::vector<uint32_t> parent;        // host copy of the taxonomy
   std::vector<uint32_t> pre, end;      // DFS preorder numbers and subtree ends
+  void *d_mem = nullptr;               // holds the next four and d_ctr
   uint32_t *d_pre = nullptr, *d_end = nullptr, *d_node_of = nullptr;
   uint64_t *d_nobs = nullptr;          // add_kmer calls per taxon
   uint8_t *d_dense = nullptr;          // some block's sketch of the taxon went dense
@@ -428,30 +430,35 @@ struct k2g_counters {
 namespace k2g {
 namespace {
 
+// Buffers come from the device's scratch pool, on the calling stream: every
+// entry point leaves its stream synchronised, so the next may use another.
+// (cudaMalloc and cudaFree here stopped all other streams.)
 template <class T>
-cudaError_t reserve(T *&p, uint64_t &cap, uint64_t want) {
+cudaError_t reserve(k2g_counters *c, cudaStream_t st, T *&p, uint64_t &cap, uint64_t want) {
   if (cap >= want && p) return cudaSuccess;
-  if (p) cudaFree(p);
+  if (p) cudaFreeAsync(p, st);
   p = nullptr;
   cap = 0;
   const uint64_t n = std::max<uint64_t>(want + want / 4, 1024);
-  cudaError_t e = cudaMalloc(&p, n * sizeof(T));
+  const cudaError_t e = scratch_alloc(reinterpret_cast<void **>(&p), n * sizeof(T), c->device, st);
   if (e == cudaSuccess) cap = n;
   return e;
 }
 
 // Grows a buffer keeping its first `used` entries.
 template <class T>
-cudaError_t reserve_keep(T *&p, uint64_t &cap, uint64_t want, uint64_t used, cudaStream_t st) {
+cudaError_t reserve_keep(k2g_counters *c, cudaStream_t st, T *&p, uint64_t &cap, uint64_t want, uint64_t used) {
   if (cap >= want && p) return cudaSuccess;
   T *q = nullptr;
   const uint64_t n = std::max<uint64_t>(want + want / 2, 1024);
-  cudaError_t e = cudaMalloc(&q, n * sizeof(T));
+  cudaError_t e = scratch_alloc(reinterpret_cast<void **>(&q), n * sizeof(T), c->device, st);
   if (e != cudaSuccess) return e;
   if (used) e = cudaMemcpyAsync(q, p, used * sizeof(T), cudaMemcpyDeviceToDevice, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (e != cudaSuccess) { cudaFree(q); return e; }
-  if (p) cudaFree(p);
+  if (e != cudaSuccess) {
+    cudaFreeAsync(q, st);
+    return e;
+  }
+  if (p) cudaFreeAsync(p, st);
   p = q;
   cap = n;
   return cudaSuccess;
@@ -475,9 +482,9 @@ int grid_for(int device, uint64_t n) {
 k2g_status sort_keys(k2g_counters *c, uint64_t *&keys, uint64_t &keys_cap, uint64_t *&alt,
                      uint64_t &alt_cap, uint64_t n, int nbits, cudaStream_t st) {
   if (n >= (1ull << 32)) return fail(K2G_ERR_BUDGET, "more than 2^32 keys to sort");
-  K2G_CUDA_TRY(reserve(alt, alt_cap, n));
-  K2G_CUDA_TRY(reserve(c->d_hist, c->hist_cap, rsort::hist_entries(n)));
-  K2G_CUDA_TRY(reserve(c->d_sums, c->sums_cap, rsort::sum_entries(n) + 1));
+  K2G_CUDA_TRY(reserve(c, st, alt, alt_cap, n));
+  K2G_CUDA_TRY(reserve(c, st, c->d_hist, c->hist_cap, rsort::hist_entries(n)));
+  K2G_CUDA_TRY(reserve(c, st, c->d_sums, c->sums_cap, rsort::sum_entries(n) + 1));
   uint64_t *res = nullptr;
   K2G_CUDA_TRY(rsort::sort_u64(keys, alt, n, nbits, c->d_hist, c->d_sums, st, &res));
   if (res != keys) {
@@ -497,14 +504,14 @@ k2g_status sort_unique(k2g_counters *c, uint64_t *&keys, uint64_t &keys_cap, uin
   k2g_status s = sort_keys(c, keys, keys_cap, alt, alt_cap, n, nbits, st);
   if (s != K2G_OK) return s;
   const uint64_t tiles = (n + rsort::kTile - 1) / rsort::kTile;
-  K2G_CUDA_TRY(reserve(c->d_hist, c->hist_cap, tiles + 1));
-  K2G_CUDA_TRY(reserve(c->d_sums, c->sums_cap, rsort::sum_entries(n) + 1));
+  K2G_CUDA_TRY(reserve(c, st, c->d_hist, c->hist_cap, tiles + 1));
+  K2G_CUDA_TRY(reserve(c, st, c->d_sums, c->sums_cap, rsort::sum_entries(n) + 1));
   run_count_kernel<<<(unsigned)tiles, rsort::kThreads, 0, st>>>(keys, n, c->d_hist);
   note_launches();
   K2G_CUDA_TRY(cudaGetLastError());
   K2G_CUDA_TRY(cudaMemsetAsync(c->d_hist + tiles, 0, sizeof(uint32_t), st));
   K2G_CUDA_TRY(rsort::exclusive_scan(c->d_hist, tiles + 1, c->d_sums, st));
-  K2G_CUDA_TRY(reserve(alt, alt_cap, n));
+  K2G_CUDA_TRY(reserve(c, st, alt, alt_cap, n));
   run_write_kernel<<<(unsigned)tiles, rsort::kThreads, 0, st>>>(keys, n, c->d_hist, alt);
   note_launches();
   K2G_CUDA_TRY(cudaGetLastError());
@@ -517,12 +524,130 @@ k2g_status sort_unique(k2g_counters *c, uint64_t *&keys, uint64_t &keys_cap, uin
   return K2G_OK;
 }
 
+// The accumulator's keys are dealt into buckets by two kernels, each thread
+// block on one slice of the keys with a counter per bucket in shared memory
+// (a global atomic per key, counting and dealing, took 0.50 ms each for 28M
+// keys): the first adds up the buckets' sizes, the second takes a place in
+// every bucket for its slice's keys and then writes them there, in any order.
+constexpr int kDealThreads = 1024;
+constexpr int kDealBits = 15;   // 2^15 counters are 128 KB
+
+__device__ __forceinline__ void count_slice(const uint64_t *k, uint64_t i0, uint64_t i1, int shift, uint32_t nb,
+                                            uint32_t *h) {
+  for (uint32_t b = threadIdx.x; b < nb; b += kDealThreads) h[b] = 0;
+  __syncthreads();
+#pragma unroll 4
+  for (uint64_t i = i0 + threadIdx.x; i < i1; i += kDealThreads) atomicAdd(&h[k[i] >> shift], 1u);
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(kDealThreads)
+bucket_count_kernel(const uint64_t *k, uint64_t n, uint64_t slice, int shift, uint32_t nb, uint32_t *count) {
+  extern __shared__ uint32_t h[];
+  const uint64_t i0 = min(n, blockIdx.x * slice), i1 = min(n, i0 + slice);
+  count_slice(k, i0, i1, shift, nb, h);
+  for (uint32_t b = threadIdx.x; b < nb; b += kDealThreads)
+    if (h[b]) atomicAdd(&count[b], h[b]);
+}
+
+__global__ void __launch_bounds__(kDealThreads)
+bucket_deal_kernel(const uint64_t *k, uint64_t n, uint64_t slice, int shift, uint32_t nb, uint32_t *cursor,
+                   uint64_t *out) {
+  extern __shared__ uint32_t h[];
+  const uint64_t i0 = min(n, blockIdx.x * slice), i1 = min(n, i0 + slice);
+  count_slice(k, i0, i1, shift, nb, h);
+  for (uint32_t b = threadIdx.x; b < nb; b += kDealThreads)
+    if (h[b]) h[b] = atomicAdd(&cursor[b], h[b]);
+  __syncthreads();
+#pragma unroll 4
+  for (uint64_t i = i0 + threadIdx.x; i < i1; i += kDealThreads) {
+    const uint64_t x = k[i];
+    out[atomicAdd(&h[x >> shift], 1u)] = x;
+  }
+}
+
+__global__ void bucket_largest_kernel(const uint32_t *count, uint32_t n, uint32_t *largest) {
+  uint32_t m = 0;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) m = max(m, count[i]);
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) atomicMax(largest, m);
+}
+
+// One warp per bucket: its distinct keys to their place.
+__global__ void bucket_pack_kernel(const uint32_t *start, const uint64_t *sorted, const uint32_t *n_distinct,
+                                   const uint32_t *place, uint32_t n_buckets, uint64_t *out) {
+  const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (b >= n_buckets) return;
+  const uint64_t *x = sorted + start[b];
+  const uint32_t n = n_distinct[b], o = place[b];
+  for (uint32_t i = lane; i < n; i += 32) out[o + i] = x[i];
+}
+
+// Sorts the accumulator and drops repeats.  Encodings are hash bits, so their
+// top bits deal the keys evenly into buckets that fit shared memory (2,250 to
+// 4,500 keys each): one pass to count, one to deal, one to sort, instead of
+// six radix passes of two each.  A minimizer seen so often that its bucket is
+// too large, or more keys than 2^15 buckets take, leave the radix sort.
 k2g_status compact_acc(k2g_counters *c, cudaStream_t st) {
   if (c->acc_used == c->acc_compact) return K2G_OK;   // already sorted and unique
-  uint64_t n = 0;
-  k2g_status s = sort_unique(c, c->d_acc, c->acc_cap, c->d_alt, c->alt_cap, c->acc_used,
-                             32 + c->tbits, st, &n);
-  if (s != K2G_OK) return s;
+  const uint64_t total = c->acc_used;
+  int bits = 0;
+  while (bits < kDealBits && (total >> bits) > 4500) bits++;
+  const uint32_t nb = 1u << bits;
+  uint64_t n = total;
+  bool sorted = false;
+  if (total >= 2 && total < (1ull << 32) && (total >> bits) <= 6000) {
+    const int shift = c->tbits + 32 - bits;
+    uint32_t *mem = nullptr;   // start[nb + 1], cursors and places[nb + 1], distinct[nb], largest, scan sums
+    const uint64_t words = 3ull * nb + 2 + 1 + nb / rsort::kScanChunk + 2;
+    K2G_CUDA_TRY(reserve(c, st, c->d_alt, c->alt_cap, total));
+    K2G_CUDA_TRY(scratch_alloc(reinterpret_cast<void **>(&mem), words * 4, c->device, st));
+    uint32_t *start = mem, *place = start + nb + 1, *distinct = place + nb + 1, *largest = distinct + nb, *sums = largest + 1;
+    uint32_t most = 0;
+    auto by_buckets = [&]() -> k2g_status {
+      K2G_CUDA_TRY(cudaMemsetAsync(mem, 0, words * 4, st));
+      int sms = 0;
+      K2G_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+      // (a slice of several keys per counter)
+      const uint64_t slice = std::max<uint64_t>((total + sms - 1) / sms, 4096);
+      const unsigned g = (unsigned)((total + slice - 1) / slice);
+      const int smem = (int)(nb * 4);
+      K2G_CUDA_TRY(cudaFuncSetAttribute(bucket_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 << kDealBits));
+      K2G_CUDA_TRY(cudaFuncSetAttribute(bucket_deal_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 << kDealBits));
+      bucket_count_kernel<<<g, kDealThreads, smem, st>>>(c->d_acc, total, slice, shift, nb, start);
+      bucket_largest_kernel<<<(nb + 255) / 256, 256, 0, st>>>(start, nb, largest);
+      note_launches(2);
+      K2G_CUDA_TRY(rsort::exclusive_scan(start, nb + 1, sums, st));
+      K2G_CUDA_TRY(cudaMemcpyAsync(place, start, nb * 4ull, cudaMemcpyDeviceToDevice, st));
+      bucket_deal_kernel<<<g, kDealThreads, smem, st>>>(c->d_acc, total, slice, shift, nb, place, c->d_alt);
+      note_launches();
+      K2G_CUDA_TRY(cudaGetLastError());
+      K2G_CUDA_TRY(cudaMemcpyAsync(&most, largest, 4, cudaMemcpyDeviceToHost, st));
+      K2G_CUDA_TRY(cudaStreamSynchronize(st));
+      if (most > kLargeBlock) return K2G_OK;
+      K2G_CUDA_TRY(bucket_sort(start, nb, most, c->d_alt, distinct, ZoneBits{shift - 8}, st));
+      K2G_CUDA_TRY(cudaMemcpyAsync(place, distinct, nb * 4ull, cudaMemcpyDeviceToDevice, st));
+      K2G_CUDA_TRY(cudaMemsetAsync(place + nb, 0, 4, st));
+      K2G_CUDA_TRY(rsort::exclusive_scan(place, nb + 1, sums, st));
+      bucket_pack_kernel<<<(unsigned)((nb * 32ull + 255) / 256), 256, 0, st>>>(start, c->d_alt, distinct, place, nb,
+                                                                              c->d_acc);
+      note_launches();
+      K2G_CUDA_TRY(cudaGetLastError());
+      uint32_t got = 0;
+      K2G_CUDA_TRY(cudaMemcpyAsync(&got, place + nb, 4, cudaMemcpyDeviceToHost, st));
+      K2G_CUDA_TRY(cudaStreamSynchronize(st));
+      n = got;
+      sorted = true;
+      return K2G_OK;
+    };
+    const k2g_status s = by_buckets();
+    cudaFreeAsync(mem, st);
+    if (s != K2G_OK) return s;
+  }
+  if (!sorted) {
+    k2g_status s = sort_unique(c, c->d_acc, c->acc_cap, c->d_alt, c->alt_cap, total, 32 + c->tbits, st, &n);
+    if (s != K2G_OK) return s;
+  }
   c->acc_used = c->acc_compact = n;
   unsigned long long v = n;
   K2G_CUDA_TRY(cudaMemcpyAsync(c->d_ctr, &v, sizeof(v), cudaMemcpyHostToDevice, st));
@@ -581,6 +706,7 @@ extern "C" k2g_status k2g_counters_create(const k2g_db *db, k2g_counters **out) 
   auto c = new k2g_counters();
   c->db = db;
   c->device = db->device;
+  scratch_opened(c->device);
   c->node_count = db->node_count;
   c->tbits = bits_for(db->node_count);
   auto bad = [&](k2g_status s) { k2g_counters_destroy(c); return s; };
@@ -620,21 +746,26 @@ extern "C" k2g_status k2g_counters_create(const k2g_db *db, k2g_counters **out) 
   }
   c->pre = pre;
   c->end = end;
-  uint64_t dummy = 0;
-  if ((e = cudaMalloc(&c->d_pre, n * 4)) != cudaSuccess ||
-      (e = cudaMalloc(&c->d_end, n * 4)) != cudaSuccess ||
-      (e = cudaMalloc(&c->d_node_of, n * 4)) != cudaSuccess ||
-      (e = cudaMalloc(&c->d_nobs, n * 8)) != cudaSuccess ||
-      (e = cudaMalloc(&c->d_dense, n)) != cudaSuccess ||
-      (e = cudaMalloc(&c->d_ctr, 4 * sizeof(unsigned long long))) != cudaSuccess ||
-      (e = cudaMemcpy(c->d_pre, pre.data(), n * 4, cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaMemcpy(c->d_end, end.data(), n * 4, cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaMemcpy(c->d_node_of, node_of.data(), n * 4, cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaMemset(c->d_nobs, 0, n * 8)) != cudaSuccess ||
+  // one allocation, zeroed; the counts first (8-byte aligned)
+  unsigned char *mem = nullptr;
+  const size_t head = 4 * sizeof(unsigned long long), tables = head + n * 8, total = tables + 12 * n + n;
+  if ((e = scratch_alloc_now(reinterpret_cast<void **>(&mem), total, c->device)) == cudaSuccess) {
+    c->d_mem = mem;
+    c->d_ctr = reinterpret_cast<unsigned long long *>(mem);
+    c->d_nobs = reinterpret_cast<uint64_t *>(mem + head);
+    c->d_pre = reinterpret_cast<uint32_t *>(mem + tables);
+    c->d_end = c->d_pre + n;
+    c->d_node_of = c->d_end + n;
+    c->d_dense = reinterpret_cast<uint8_t *>(c->d_node_of + n);
+  }
+  std::vector<uint32_t> all(3 * n);
+  std::copy(pre.begin(), pre.end(), all.begin());
+  std::copy(end.begin(), end.end(), all.begin() + n);
+  std::copy(node_of.begin(), node_of.end(), all.begin() + 2 * n);
+  if (e != cudaSuccess || (e = cudaMemset(mem, 0, tables)) != cudaSuccess ||
       (e = cudaMemset(c->d_dense, 0, n)) != cudaSuccess ||
-      (e = cudaMemset(c->d_ctr, 0, 4 * sizeof(unsigned long long))) != cudaSuccess)
+      (e = cudaMemcpy(c->d_pre, all.data(), 12 * n, cudaMemcpyHostToDevice)) != cudaSuccess)
     return bad(cuda_fail(e, "counter set-up"));
-  (void)dummy;
   // a quarter of the free memory for the accumulator and its sort buffer
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 1ull << 32;
@@ -647,11 +778,10 @@ extern "C" k2g_status k2g_counters_create(const k2g_db *db, k2g_counters **out) 
 extern "C" k2g_status k2g_counters_destroy(k2g_counters *c) {
   if (!c) return K2G_OK;
   cudaSetDevice(c->device);
-  void *bufs[] = {c->d_pre, c->d_end, c->d_node_of, c->d_nobs, c->d_dense, c->d_ctr, c->d_acc,
-                  c->d_alt, c->d_reset, c->d_stop, c->d_seg, c->d_big_taxon, c->d_big_d,
+  void *bufs[] = {c->d_mem, c->d_acc, c->d_alt, c->d_reset, c->d_stop, c->d_seg, c->d_big_taxon, c->d_big_d,
                   c->d_big_last_enc, c->d_big_last, c->d_bkeys, c->d_balt, c->d_hist, c->d_sums};
-  for (void *p : bufs)
-    if (p) cudaFree(p);
+  for (void *p : bufs) scratch_free_now(p, c->device);
+  scratch_closed(c->device);
   delete c;
   return K2G_OK;
 }
@@ -685,12 +815,12 @@ extern "C" k2g_status k2g_counters_add(k2g_counters *c, const k2g_reads *reads,
     if (s != K2G_OK) return s;
     if (c->acc_used + n_ev >= (1ull << 32)) return fail(K2G_ERR_BUDGET, "too many distinct minimizers");
   }
-  K2G_CUDA_TRY(reserve_keep(c->d_acc, c->acc_cap, c->acc_used + n_ev, c->acc_used, st));
-  K2G_CUDA_TRY(reserve(c->d_reset, c->frag_cap, nf));
-  K2G_CUDA_TRY(reserve(c->d_stop, c->stop_cap, nf));
-  K2G_CUDA_TRY(reserve(c->d_seg, c->seg_cap, c->node_count * nblk));
+  K2G_CUDA_TRY(reserve_keep(c, st, c->d_acc, c->acc_cap, c->acc_used + n_ev, c->acc_used));
+  K2G_CUDA_TRY(reserve(c, st, c->d_reset, c->frag_cap, nf));
+  K2G_CUDA_TRY(reserve(c, st, c->d_stop, c->stop_cap, nf));
+  K2G_CUDA_TRY(reserve(c, st, c->d_seg, c->seg_cap, c->node_count * nblk));
   const uint64_t big_cap = n_ev / kSparseLimit + 1;
-  K2G_CUDA_TRY(reserve(c->d_big_taxon, c->big_cap, big_cap));
+  K2G_CUDA_TRY(reserve(c, st, c->d_big_taxon, c->big_cap, big_cap));
   K2G_CUDA_TRY(cudaMemsetAsync(c->d_reset, 0, nf, st));
   K2G_CUDA_TRY(cudaMemsetAsync(c->d_stop, 0xFF, nf * 4, st));
   K2G_CUDA_TRY(cudaMemsetAsync(c->d_seg, 0, c->node_count * nblk * 4, st));
@@ -715,10 +845,10 @@ extern "C" k2g_status k2g_counters_add(k2g_counters *c, const k2g_reads *reads,
 
   if (n_big) {
     // exact distinct counts of the segments that can reach the sparse limit
-    K2G_CUDA_TRY(reserve(c->d_big_d, c->big_d_cap, n_big));
-    K2G_CUDA_TRY(reserve(c->d_big_last_enc, c->big_enc_cap, n_big));
-    K2G_CUDA_TRY(reserve(c->d_big_last, c->big_last_cap, n_big));
-    K2G_CUDA_TRY(reserve(c->d_bkeys, c->bkeys_cap, n_ev));
+    K2G_CUDA_TRY(reserve(c, st, c->d_big_d, c->big_d_cap, n_big));
+    K2G_CUDA_TRY(reserve(c, st, c->d_big_last_enc, c->big_enc_cap, n_big));
+    K2G_CUDA_TRY(reserve(c, st, c->d_big_last, c->big_last_cap, n_big));
+    K2G_CUDA_TRY(reserve(c, st, c->d_bkeys, c->bkeys_cap, n_ev));
     K2G_CUDA_TRY(cudaMemsetAsync(c->d_big_d, 0, n_big * 4, st));
     K2G_CUDA_TRY(cudaMemsetAsync(c->d_big_last, 0, n_big * 8, st));
     big_gather_kernel<<<g, 256, 0, st>>>(ev, c->d_seg, c->d_bkeys, c->d_ctr + 2, c->d_big_last);
@@ -786,11 +916,11 @@ extern "C" k2g_status k2g_counters_import(k2g_counters *c, const uint64_t *entri
     if (c->acc_used + n_entries >= (1ull << 32)) return fail(K2G_ERR_BUDGET, "too many distinct minimizers");
   }
   const uint64_t n = c->node_count;
-  K2G_CUDA_TRY(reserve_keep(c->d_acc, c->acc_cap, c->acc_used + n_entries, c->acc_used, st));
+  K2G_CUDA_TRY(reserve_keep(c, st, c->d_acc, c->acc_cap, c->acc_used + n_entries, c->acc_used));
   uint64_t *d_nobs = nullptr;
   uint8_t *d_dense = nullptr;
-  cudaError_t e = cudaMalloc(&d_nobs, n * 8);
-  if (e == cudaSuccess) e = cudaMalloc(&d_dense, n);
+  cudaError_t e = scratch_alloc((void **)&d_nobs, n * 8, c->device, st);
+  if (e == cudaSuccess) e = scratch_alloc((void **)&d_dense, n, c->device, st);
   if (e == cudaSuccess && n_entries)
     e = cudaMemcpyAsync(c->d_acc + c->acc_used, entries, n_entries * 8, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_nobs, taxon_kmers, n * 8, cudaMemcpyHostToDevice, st);
@@ -804,8 +934,8 @@ extern "C" k2g_status k2g_counters_import(k2g_counters *c, const uint64_t *entri
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(c->d_ctr, &fill, sizeof(fill), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  if (d_nobs) cudaFree(d_nobs);
-  if (d_dense) cudaFree(d_dense);
+  if (d_nobs) cudaFreeAsync(d_nobs, st);
+  if (d_dense) cudaFreeAsync(d_dense, st);
   if (e != cudaSuccess) return cuda_fail(e, "k2g_counters_import");
   c->acc_used += n_entries;   // sorted and de-duplicated with the rest at the next compaction
   return K2G_OK;
@@ -860,16 +990,16 @@ extern "C" k2g_status k2g_counters_finish(k2g_counters *c, uint64_t *taxon_kmers
   uint32_t *d_hot = nullptr, *d_cos = nullptr, *d_regs = nullptr, *d_hist = nullptr;
   auto release = [&]() {
     for (void *p : {(void *)d_node, (void *)d_hot, (void *)d_cos, (void *)d_regs, (void *)d_hist})
-      if (p) cudaFree(p);
+      if (p) cudaFreeAsync(p, st);
   };
   std::vector<uint32_t> hist(n * kHist);
   cudaError_t e = cudaSuccess;
   do {
-    if ((e = cudaMalloc(&d_node, n * sizeof(uint4))) != cudaSuccess) break;
-    if ((e = cudaMalloc(&d_hot, kHot * 4)) != cudaSuccess) break;
-    if ((e = cudaMalloc(&d_cos, std::max<uint64_t>(nd, 1) * 4)) != cudaSuccess) break;
-    if ((e = cudaMalloc(&d_regs, std::max<uint64_t>(nd, 1) * (4ull << kHllP))) != cudaSuccess) break;
-    if ((e = cudaMalloc(&d_hist, n * kHist * 4)) != cudaSuccess) break;
+    if ((e = scratch_alloc((void **)&d_node, n * sizeof(uint4), c->device, st)) != cudaSuccess) break;
+    if ((e = scratch_alloc((void **)&d_hot, kHot * 4, c->device, st)) != cudaSuccess) break;
+    if ((e = scratch_alloc((void **)&d_cos, std::max<uint64_t>(nd, 1) * 4, c->device, st)) != cudaSuccess) break;
+    if ((e = scratch_alloc((void **)&d_regs, std::max<uint64_t>(nd, 1) * (4ull << kHllP), c->device, st)) != cudaSuccess) break;
+    if ((e = scratch_alloc((void **)&d_hist, n * kHist * 4, c->device, st)) != cudaSuccess) break;
     if ((e = cudaMemcpyAsync(d_node, node.data(), n * sizeof(uint4), cudaMemcpyHostToDevice, st)) != cudaSuccess) break;
     if ((e = cudaMemcpyAsync(d_hot, hot.data(), kHot * 4, cudaMemcpyHostToDevice, st)) != cudaSuccess) break;
     if (nd && (e = cudaMemcpyAsync(d_cos, clade_of_slot.data(), nd * 4, cudaMemcpyHostToDevice, st)) != cudaSuccess) break;

@@ -220,7 +220,7 @@ void destroy(k2g_db *db) {
   if (db->d_names) cudaFree(db->d_names);
   if (db->d_span) cudaFree(db->d_span);   // (d_parent lies in the same allocation)
   if (db->d_size) cudaFree(db->d_size);
-  if (db->counted) scratch_db_closed(db->device);
+  if (db->counted) scratch_closed(db->device);
   cudaSetDevice(cur);
   delete db;
 }
@@ -411,7 +411,7 @@ extern "C" k2g_status k2g_db_open(const char *hash_k2d, const char *taxo_k2d,
   }
   ce = cudaMemcpy(db->d_size, &db->size, 8, cudaMemcpyHostToDevice);
   if (ce != cudaSuccess) { destroy(db.release()); return cuda_fail(ce, "size upload"); }
-  scratch_db_opened(db->device);
+  scratch_opened(db->device);
   db->counted = true;
   *out = db.release();
   return K2G_OK;
@@ -448,7 +448,7 @@ extern "C" k2g_status k2g_db_create(const k2g_index_options *opts, uint64_t capa
   else K2G_CUDA_TRY(cudaMemset(db->d_cells, 0, capacity * sizeof(uint32_t)));
   K2G_CUDA_TRY(cudaMemset(db->d_size, 0, 8));
   db->size = 0;
-  scratch_db_opened(db->device);
+  scratch_opened(db->device);
   db->counted = true;
   *out = db.release();
   return K2G_OK;

@@ -154,10 +154,14 @@ bool warp_classify_takes(const ClassifyArgs &a, uint64_t max_len);
 cudaError_t warp_classify(const ClassifyArgs &a, const uint2 *span, uint64_t max_len, uint64_t total_bases,
                           uint32_t piece_len, int device, int sms, cudaStream_t st);
 // Device scratch of one call, allocated on its stream (given back by
-// cudaFreeAsync), and the databases that keep the pool alive (scratch.cu).
+// cudaFreeAsync), and the objects that keep the pool's memory (scratch.cu).
 cudaError_t scratch_alloc(void **p, size_t bytes, int device, cudaStream_t st);
-void scratch_db_opened(int device);
-void scratch_db_closed(int device);
+// The same for memory of an object that outlives calls: usable on any stream
+// when it returns; freed once nothing uses it any more.
+cudaError_t scratch_alloc_now(void **p, size_t bytes, int device);
+void scratch_free_now(void *p, int device);
+void scratch_opened(int device);
+void scratch_closed(int device);
 // Counts each kernel launch issued by the library (k2g_kernel_launches).
 void note_launches(uint64_t n = 1);
 // One round (< 2^30 pairs) of the order-exact build insert (build_ordered.cu).

@@ -1,10 +1,11 @@
-// Device scratch of single calls: stream-ordered allocations from a memory
-// pool of the library's own, one per device.  A call allocates on its stream
+// Device scratch of single calls, and the counters' buffers: stream-ordered
+// allocations from a memory pool of the library's own, one per device.  A call allocates on its stream
 // and gives the memory back on it, so calls on any streams and threads share
 // the pool safely, and a captured call's allocations become part of its
 // graph.  The pool keeps up to kKeep bytes between calls (a pool that keeps
 // nothing maps the memory anew after every synchronisation, about 0.8 ms a
-// call) and gives everything back when the device's last database is closed.
+// call) and gives everything back when the device's last database or counter
+// set is closed.
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -19,7 +20,8 @@ constexpr uint64_t kKeep = 1ull << 30;
 struct Pool {
   std::mutex mu;
   cudaMemPool_t pool = nullptr;
-  int dbs = 0;
+  cudaStream_t st = nullptr;   // for memory that no call's stream owns
+  int users = 0;               // open databases and counter sets
 };
 Pool g_pools[64];
 
@@ -48,16 +50,36 @@ cudaError_t scratch_alloc(void **p, size_t bytes, int device, cudaStream_t st) {
   return cudaMallocFromPoolAsync(p, bytes ? bytes : 1, d.pool, st);
 }
 
-void scratch_db_opened(int device) {
+cudaError_t scratch_alloc_now(void **p, size_t bytes, int device) {
   Pool &d = g_pools[device & 63];
-  std::lock_guard<std::mutex> lock(d.mu);
-  d.dbs++;
+  {
+    std::lock_guard<std::mutex> lock(d.mu);
+    if (!d.st) {
+      const cudaError_t e = cudaStreamCreateWithFlags(&d.st, cudaStreamNonBlocking);
+      if (e != cudaSuccess) return e;
+    }
+  }
+  const cudaError_t e = scratch_alloc(p, bytes, device, d.st);
+  return e != cudaSuccess ? e : cudaStreamSynchronize(d.st);
 }
 
-void scratch_db_closed(int device) {
+void scratch_free_now(void *p, int device) {
+  if (p) cudaFreeAsync(p, g_pools[device & 63].st);
+}
+
+void scratch_opened(int device) {
   Pool &d = g_pools[device & 63];
   std::lock_guard<std::mutex> lock(d.mu);
-  if (--d.dbs == 0 && d.pool) cudaMemPoolTrimTo(d.pool, 0);
+  d.users++;
+}
+
+void scratch_closed(int device) {
+  Pool &d = g_pools[device & 63];
+  std::lock_guard<std::mutex> lock(d.mu);
+  if (--d.users == 0 && d.pool) {
+    if (d.st) cudaStreamSynchronize(d.st);
+    cudaMemPoolTrimTo(d.pool, 0);
+  }
 }
 
 }  // namespace k2g
