@@ -24,11 +24,11 @@ def make(lens, seed):
     t = torch()
     mins, amb = t.zeros(4_000_000, dtype=t.int64, device="cuda"), t.zeros(4_000_000, dtype=t.uint8, device="cuda")
     st = t.cuda.current_stream().cuda_stream
-    db.scan(to_dev(bases[:4_000_016]).data_ptr(), to_dev(np.array([0, 4_000_000], np.uint64)).data_ptr(), 1,
-            mins.data_ptr(), amb.data_ptr(), st)
+    d_b, d_o = to_dev(bases[:4_000_016]), to_dev(np.array([0, 4_000_000], np.uint64))
+    db.scan(d_b.data_ptr(), d_o.data_ptr(), 1, mins.data_ptr(), amb.data_ptr(), st)
     keys = np.unique(mins.cpu().numpy()[:3_999_900:4])[:600_000]
-    db.build_insert(to_dev(keys.view(np.uint64)).data_ptr(),
-                    to_dev(rng.integers(1, NODES, len(keys)).astype(np.uint32)).data_ptr(), len(keys), False, st)
+    d_k, d_t = to_dev(keys.view(np.uint64)), to_dev(rng.integers(1, NODES, len(keys)).astype(np.uint32))
+    db.build_insert(d_k.data_ptr(), d_t.data_ptr(), len(keys), False, st)
     t.cuda.synchronize()
     # every chunk meets stored k-mers
     bases = np.resize(bases[:4_000_000], int(off[-1]) + 16)

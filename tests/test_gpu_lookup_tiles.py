@@ -22,8 +22,8 @@ def test_lookups_equal_the_oracle(capacity, load, n, wide):
     db = k2g.Database.create(k2g.IndexOptions(35, 31, 0, 0, 1, 1, 0), capacity, kb, 10, parent)
     stored = rng.integers(0, 2**62, int(capacity * load), dtype=np.int64).astype(np.uint64)
     taxa = rng.integers(1, nodes, len(stored)).astype(np.uint32)
-    db.build_insert(to_dev(stored).data_ptr(), to_dev(taxa).data_ptr(), len(stored), False,
-                    t.cuda.current_stream().cuda_stream)
+    d_stored, d_taxa = to_dev(stored), to_dev(taxa)
+    db.build_insert(d_stored.data_ptr(), d_taxa.data_ptr(), len(stored), False, t.cuda.current_stream().cuda_stream)
     keys = np.where(rng.random(n) < 0.6, stored[rng.integers(0, len(stored), n)],
                     rng.integers(0, 2**62, n, dtype=np.int64).astype(np.uint64))
     d_keys = to_dev(keys)
