@@ -12,6 +12,8 @@
 namespace k2g {
 k2g_status exclusive_scan_u32(const uint32_t *d_in, uint64_t n, uint64_t *d_out, uint64_t *d_sums,
                               uint64_t *d_total, cudaStream_t st);
+k2g_status block_scan_u32(const uint32_t *d_in, uint64_t n, uint64_t *d_out, uint64_t *d_sums, uint64_t *d_total,
+                          cudaStream_t st);
 }
 
 using namespace k2g;
@@ -119,12 +121,12 @@ extern "C" k2g_status k2g_format_lines_host(const k2g_db *db, const k2g_lines *i
   if (s != K2G_OK) return s;
   int sms = 0;
   K2G_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, (uint64_t)sms * 8));
-  line_len_kernel<<<grid, 256, 0, st>>>(v, static_cast<uint32_t *>(fc.len.p));
+  const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + kThreads - 1) / kThreads, (uint64_t)sms * 8));
+  line_len_kernel<<<grid, kThreads, 0, st>>>(v, static_cast<uint32_t *>(fc.len.p));
   note_launches();
   K2G_CUDA_TRY(cudaGetLastError());
   uint64_t *d_line_off = static_cast<uint64_t *>(fc.line_off.p);
-  s = exclusive_scan_u32(static_cast<const uint32_t *>(fc.len.p), n, d_line_off, d_sums, d_total, st);
+  s = block_scan_u32(static_cast<const uint32_t *>(fc.len.p), n, d_line_off, d_sums, d_total, st);
   if (s != K2G_OK) return s;
   uint64_t total = 0;
   unsigned int bad = 0;
@@ -139,7 +141,8 @@ extern "C" k2g_status k2g_format_lines_host(const k2g_db *db, const k2g_lines *i
   if (total > text_cap) return fail(K2G_ERR_CAPACITY, "text buffer too small for the lines");
   if (!text) return fail(K2G_ERR_ARG, "null text buffer");
   K2G_CUDA_TRY(fc.out.need(total));
-  line_write_kernel<<<grid, 256, 0, st>>>(v, d_line_off, static_cast<char *>(fc.out.p));
+  line_write_kernel<<<grid, kThreads, 0, st>>>(v, static_cast<const uint32_t *>(fc.len.p), d_line_off, d_sums, d_total,
+                                               static_cast<char *>(fc.out.p), total);
   note_launches();
   K2G_CUDA_TRY(cudaGetLastError());
   K2G_CUDA_TRY(cudaMemcpyAsync(text, fc.out.p, total, cudaMemcpyDeviceToHost, st));

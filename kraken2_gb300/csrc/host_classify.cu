@@ -105,14 +105,26 @@ __global__ void add_block_base_kernel(uint64_t *out, const uint64_t *sums, uint6
   if (i < n) out[i] += sums[i / kScanBlock];
 }
 
-k2g_status exclusive_scan_u32(const uint32_t *d_in, uint64_t n, uint64_t *d_out, uint64_t *d_sums,
-                              uint64_t *d_total, cudaStream_t st) {
+// Exclusive scan whose value i is d_out[i] + d_sums[i / 1024].
+k2g_status block_scan_u32(const uint32_t *d_in, uint64_t n, uint64_t *d_out, uint64_t *d_sums, uint64_t *d_total,
+                          cudaStream_t st) {
   if (!n) return K2G_OK;
   uint64_t nb = (n + kScanBlock - 1) / kScanBlock;
   scan_blocks_kernel<<<(unsigned)nb, kScanBlock, 0, st>>>(d_in, d_out, d_sums, n);
   scan_sums_kernel<<<1, kScanBlock, 0, st>>>(d_sums, nb, d_total);
+  note_launches(2);
+  K2G_CUDA_TRY(cudaGetLastError());
+  return K2G_OK;
+}
+static_assert(kScanBlock == 1024, "users of block_scan_u32 add d_sums[i >> 10]");
+
+k2g_status exclusive_scan_u32(const uint32_t *d_in, uint64_t n, uint64_t *d_out, uint64_t *d_sums,
+                              uint64_t *d_total, cudaStream_t st) {
+  if (!n) return K2G_OK;
+  const k2g_status s = block_scan_u32(d_in, n, d_out, d_sums, d_total, st);
+  if (s != K2G_OK) return s;
   add_block_base_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d_out, d_sums, n);
-  note_launches(3);
+  note_launches();
   K2G_CUDA_TRY(cudaGetLastError());
   return K2G_OK;
 }

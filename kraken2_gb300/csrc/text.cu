@@ -24,17 +24,23 @@
 // (an unfinished reader block) followed by the new chunk.
 //   1. '\n' positions: per-tile counts, a scan, and an ordered write.
 //   2. per line: its role (header, sequence, '+', quality), the bytes it
-//      adds to the sequence, and whether it breaks the form.
-//   3. scans of the sequence bytes and of the header flags place every
-//      record's sequence and give every header its record number.
-//   4. per record: the name and the sequence offset; then one thread cuts
-//      reader blocks (LoadBlock: sequence bytes up to 3 MiB; LoadBatch: a
-//      record count) and keeps the whole blocks.
+//      adds to the sequence, and whether it breaks the form; per tile of
+//      lines, the sums of the bytes and of the headers.
+//   3. a scan of these sums, and how many records are complete and of the
+//      strict form.
+//   4. per line: where its bytes go; per record: the name and the sequence
+//      offset; then one thread cuts reader blocks (LoadBlock: sequence bytes
+//      up to 3 MiB; LoadBatch: a record count) and keeps the whole blocks.
 //   5. the kept sequences are gathered into one array (-Q masking on the
 //      way), classified (k2g_classify's pipelined path), and their kraken
 //      lines are formatted (lines.cuh) from the window's names.
 // Whatever follows the kept blocks is copied to the front of the other
 // window buffer for the next call.
+//
+// The host waits twice per call: for the counts that step 5's launches need,
+// and for the results.  Steps 1 to 4 take their counts from device memory
+// (waiting for the number of lines and of records in between, with scans of
+// three launches each, took 0.26 ms of a 32 MB chunk's 0.62; 0.14 of 0.44 now).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -45,8 +51,8 @@
 #include "lines.cuh"
 
 namespace k2g {
-k2g_status exclusive_scan_u32(const uint32_t *d_in, uint64_t n, uint64_t *d_out, uint64_t *d_sums,
-                              uint64_t *d_total, cudaStream_t st);
+k2g_status block_scan_u32(const uint32_t *d_in, uint64_t n, uint64_t *d_out, uint64_t *d_sums, uint64_t *d_total,
+                          cudaStream_t st);
 }
 
 using namespace k2g;
@@ -57,9 +63,11 @@ constexpr uint32_t kTile = 16384;          // window bytes per newline-count blo
 constexpr int kTileThreads = 256;          // 64 contiguous bytes per thread
 constexpr uint64_t kMaxChunk = 1ull << 30;
 constexpr unsigned long long kNone = ~0ull;
+constexpr uint32_t kLineTile = 1024;       // lines per block of the line kernels
+constexpr int kLineThreads = 256;
+constexpr uint32_t kHeader = 0xFFFFFFFFu;  // contrib of a header line
 
-// Counters a call's kernels fill in (one per call, zeroed first except
-// first_bad, which starts at kNone).
+// What a call's kernels find (set up by tile_scan_kernel).
 struct ParseInfo {
   unsigned long long first_bad;   // first line outside the strict form
   unsigned long long max_len;     // longest kept sequence
@@ -71,14 +79,26 @@ struct ParseInfo {
   unsigned long long valid;       // records before the first line outside the form
   unsigned long long classified;  // kept fragments with a call
   unsigned long long all;         // the input ends with the last valid record
+  unsigned long long n_nl, n_lines;        // (0 when too_many)
+  unsigned long long too_many;    // more lines than the buffers hold
+  unsigned long long n_hdr;       // header lines
+  unsigned long long contrib;     // sequence bytes of all lines
+  uint64_t text_len;              // bytes of the kraken lines
+  uint32_t status;                // k2g_classify's
+  unsigned int bad;               // the formatter's
 };
 
 struct Window {
   const char *win;
   uint64_t len;                   // window bytes
   const uint32_t *nl;             // '\n' positions
-  uint64_t n_nl, n_lines;
+  const ParseInfo *info;
   int fastq, at_eof;
+  uint64_t n_nl, n_lines;         // the info's (load)
+  __device__ __forceinline__ void load() {
+    n_nl = info->n_nl;
+    n_lines = info->n_lines;
+  }
   __device__ __forceinline__ uint64_t start(uint64_t k) const { return k ? (uint64_t)nl[k - 1] + 1 : 0; }
   __device__ __forceinline__ uint64_t end(uint64_t k) const { return k < n_nl ? (uint64_t)nl[k] : len; }
 };
@@ -152,107 +172,227 @@ __global__ void __launch_bounds__(kTileThreads) nl_write_kernel(const char *win,
     if (out < nl_cap) nl[out] = (uint32_t)(base + (uint64_t)(__ffsll((long long)mask) - 1));
 }
 
-// Per line: header flag, sequence bytes, and the strict-form check.
-__global__ void line_kernel(Window wd, uint32_t *contrib, uint32_t *hflag, ParseInfo *info) {
-  const char *w = wd.win;
-  for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < wd.n_lines;
-       k += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t s = wd.start(k), e = wd.end(k);
-    const unsigned char c0 = e > s ? (unsigned char)w[s] : '\n';
-    uint32_t add = 0, hdr = 0;
-    bool bad = false;
-    if (wd.fastq) {
-      switch (k & 3) {
-        case 0:
-          hdr = 1;
-          bad = c0 != '@';
-          // an input that ends inside a record: the caller's reader decides
-          bad |= wd.at_eof && k + 4 > wd.n_lines;
-          break;
-        case 1:
-          bad = e == s || c0 == '>' || c0 == '+' || c0 == '@';
-          add = line_bytes(w, s, e);
-          break;
-        case 2:
-          bad = c0 != '+';
-          break;
-        default:
-          bad = line_bytes(w, s, e) != line_bytes(w, wd.start(k - 2), wd.end(k - 2));
-      }
-    } else {
-      hdr = c0 == '>';
-      if (!hdr) {
-        bad = k == 0 || c0 == '@' || c0 == '+' || (e - s == 1 && c0 == '\r');
-        add = e > s ? line_bytes(w, s, e) : 0;
-      }
+// Exclusive scan of load(0 .. n) into store(i, value) by one block of
+// kScanThreads; returns the total.
+constexpr int kScanThreads = 1024;
+constexpr int kScanPer = 4;
+
+template <class Load, class Store>
+__device__ __forceinline__ uint64_t scan_by_block(uint64_t n, Load load, Store store) {
+  __shared__ uint64_t tot[32];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint64_t carry = 0;
+  for (uint64_t base = 0; base < n; base += kScanThreads * kScanPer) {
+    const uint64_t i = base + threadIdx.x * (uint64_t)kScanPer;
+    uint64_t v[kScanPer], sum = 0;
+#pragma unroll
+    for (int u = 0; u < kScanPer; u++) {
+      v[u] = i + u < n ? load(i + u) : 0;
+      sum += v[u];
     }
-    if (bad) atomicMin(&info->first_bad, (unsigned long long)k);
-    contrib[k] = add;
-    hflag[k] = hdr;
+    auto scan_warp = [&](uint64_t x) {
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint64_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if ((int)lane >= o) x += y;
+      }
+      return x;
+    };
+    const uint64_t x = scan_warp(sum);
+    if (lane == 31) tot[w] = x;
+    __syncthreads();
+    if (w == 0) tot[lane] = scan_warp(tot[lane]);
+    __syncthreads();
+    uint64_t before = carry + (w ? tot[w - 1] : 0) + x - sum;
+#pragma unroll
+    for (int u = 0; u < kScanPer; u++) {
+      if (i + u < n) store(i + u, before);
+      before += v[u];
+    }
+    carry += tot[31];
+    __syncthreads();
+  }
+  return carry;
+}
+
+// One block: where each tile's '\n' positions go, and a fresh info.
+__global__ void __launch_bounds__(kScanThreads) tile_scan_kernel(const char *win, uint64_t len, const uint32_t *tile_cnt,
+                                                                 uint64_t tiles, uint64_t *tile_off, int at_eof,
+                                                                 uint64_t line_cap, ParseInfo *info) {
+  const uint64_t n_nl = scan_by_block(tiles, [&](uint64_t i) { return (uint64_t)tile_cnt[i]; },
+                                      [&](uint64_t i, uint64_t x) { tile_off[i] = x; });
+  if (threadIdx.x == 0) {
+    ParseInfo p{};
+    p.first_bad = kNone;
+    p.n_nl = n_nl;
+    // the last line counts when the input ends without a '\n'
+    p.n_lines = n_nl + (at_eof && win[len - 1] != '\n' ? 1 : 0);
+    if (p.n_lines > line_cap) {
+      p.too_many = 1;
+      p.n_nl = p.n_lines = 0;
+    }
+    *info = p;
   }
 }
 
+// Per line: its sequence bytes (kHeader: a header line) and the strict-form
+// check.  Per tile of lines: (headers << 32 | sequence bytes).
+__global__ void __launch_bounds__(kLineThreads) line_kernel(Window wd, uint32_t *contrib, uint64_t *tile_sum,
+                                                            ParseInfo *info) {
+  __shared__ uint64_t s_sum[kLineThreads / 32];
+  wd.load();
+  const char *w = wd.win;
+  for (uint64_t t0 = blockIdx.x * (uint64_t)kLineTile; t0 < wd.n_lines; t0 += gridDim.x * (uint64_t)kLineTile) {
+    uint64_t sum = 0;
+    for (uint64_t k = t0 + threadIdx.x; k < min(t0 + kLineTile, wd.n_lines); k += kLineThreads) {
+      const uint64_t s = wd.start(k), e = wd.end(k);
+      const unsigned char c0 = e > s ? (unsigned char)w[s] : '\n';
+      uint32_t add = 0;
+      bool bad = false;
+      if (wd.fastq) {
+        switch (k & 3) {
+          case 0:
+            add = kHeader;
+            bad = c0 != '@';
+            // an input that ends inside a record: the caller's reader decides
+            bad |= wd.at_eof && k + 4 > wd.n_lines;
+            break;
+          case 1:
+            bad = e == s || c0 == '>' || c0 == '+' || c0 == '@';
+            add = line_bytes(w, s, e);
+            break;
+          case 2:
+            bad = c0 != '+';
+            break;
+          default:
+            bad = line_bytes(w, s, e) != line_bytes(w, wd.start(k - 2), wd.end(k - 2));
+        }
+      } else if (c0 == '>') {
+        add = kHeader;
+      } else {
+        bad = k == 0 || c0 == '@' || c0 == '+' || (e - s == 1 && c0 == '\r');
+        add = e > s ? line_bytes(w, s, e) : 0;
+      }
+      if (bad) atomicMin(&info->first_bad, (unsigned long long)k);
+      contrib[k] = add;
+      sum += add == kHeader ? 1ull << 32 : add;
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    __syncthreads();   // (the tile before is done with)
+    if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = sum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int i = 1; i < kLineThreads / 32; i++) sum += s_sum[i];
+      tile_sum[t0 / kLineTile] = sum;
+    }
+  }
+}
+
+// One block: the sums before each tile of lines; the totals; how many records
+// are valid and complete.
+__global__ void __launch_bounds__(kScanThreads) line_scan_kernel(Window wd, const uint32_t *contrib, uint64_t *tile_sum,
+                                                                 ParseInfo *info) {
+  wd.load();
+  const uint64_t tiles = (wd.n_lines + kLineTile - 1) / kLineTile;
+  const uint64_t total = scan_by_block(tiles, [&](uint64_t i) { return tile_sum[i]; },
+                                       [&](uint64_t i, uint64_t x) { tile_sum[i] = x; });
+  const unsigned long long fb = info->first_bad;
+  const uint64_t n_hdr = total >> 32;
+  uint64_t complete, limit;
+  if (wd.fastq) {
+    complete = wd.n_lines / 4;
+    limit = fb == kNone ? complete : fb / 4;
+  } else {
+    complete = limit = wd.at_eof ? n_hdr : (n_hdr ? n_hdr - 1 : 0);
+    if (fb != kNone) {
+      // a bad line is never a header: it belongs to the record before it
+      const uint64_t t0 = fb / kLineTile * kLineTile, k = t0 + threadIdx.x;   // (kLineTile == kScanThreads)
+      const uint64_t rank = (tile_sum[fb / kLineTile] >> 32) + __syncthreads_count(k < fb && contrib[k] == kHeader);
+      limit = rank ? rank - 1 : 0;
+    }
+  }
+  if (threadIdx.x == 0) {
+    info->n_hdr = n_hdr;
+    info->contrib = total & 0xFFFFFFFFull;
+    info->valid = min(complete, limit);
+    info->all = fb == kNone && wd.at_eof;   // the input ends with record `valid`
+  }
+}
+static_assert(kLineTile == kScanThreads, "line_scan_kernel looks at a tile's lines by threads");
+
 struct RecordOut {
+  uint32_t *line_pos;             // where each line's bytes go in the gathered array
   k2g_name_ref *refs;             // name of each record (window positions)
   uint64_t *seq_off;              // start of each record's sequence in the gathered array
   uint32_t *rec_line;             // header line of each record
   uint64_t cap;
 };
 
-// Per header line: record number, name and sequence offset.
-__global__ void record_kernel(Window wd, const uint32_t *hflag, const uint64_t *line_pos,
-                              const uint64_t *hdr_rank, RecordOut ro) {
+// Per line: where its bytes go; per header line: record number, name and
+// sequence offset.  (The lengths of all sequences end at seq_off[n_hdr].)
+__global__ void __launch_bounds__(kLineThreads) record_kernel(Window wd, const uint32_t *contrib, const uint64_t *tile_sum,
+                                                              RecordOut ro) {
+  __shared__ uint64_t s_sum[kLineThreads / 32];
+  constexpr int kPer = kLineTile / kLineThreads;
+  wd.load();
   const char *w = wd.win;
-  for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < wd.n_lines;
-       k += (uint64_t)gridDim.x * blockDim.x) {
-    if (!hflag[k]) continue;
-    const uint64_t j = hdr_rank[k];
-    if (j >= ro.cap) continue;
-    const uint64_t s = wd.start(k), e = wd.end(k);
-    uint64_t p = s + 1;
-    while (p < e && !is_space((unsigned char)w[p])) p++;
-    ro.refs[j].pos = s + 1;
-    ro.refs[j].len = (uint32_t)(p - s - 1);
-    ro.seq_off[j] = line_pos[k];
-    ro.rec_line[j] = (uint32_t)k;
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (blockIdx.x == 0 && threadIdx.x == 0) ro.seq_off[wd.info->n_hdr] = wd.info->contrib;
+  for (uint64_t t0 = blockIdx.x * (uint64_t)kLineTile; t0 < wd.n_lines; t0 += gridDim.x * (uint64_t)kLineTile) {
+    const uint64_t k0 = t0 + threadIdx.x * kPer;
+    uint32_t c[kPer];
+    uint64_t sum = 0;
+#pragma unroll
+    for (int u = 0; u < kPer; u++) {
+      c[u] = k0 + u < wd.n_lines ? contrib[k0 + u] : 0;
+      sum += c[u] == kHeader ? 1ull << 32 : c[u];
+    }
+    uint64_t x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint64_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if ((int)lane >= o) x += y;
+    }
+    __syncthreads();   // (the tile before is done with)
+    if (lane == 31) s_sum[warp] = x;
+    __syncthreads();
+    uint64_t before = tile_sum[t0 / kLineTile] + x - sum;
+    for (uint32_t i = 0; i < warp; i++) before += s_sum[i];
+#pragma unroll
+    for (int u = 0; u < kPer; u++) {
+      const uint64_t k = k0 + u;
+      if (k >= wd.n_lines) break;
+      ro.line_pos[k] = (uint32_t)before;
+      if (c[u] != kHeader) {
+        before += c[u];
+        continue;
+      }
+      const uint64_t j = before >> 32;
+      before += 1ull << 32;
+      if (j >= ro.cap) continue;
+      const uint64_t s = wd.start(k), e = wd.end(k);
+      uint64_t p = s + 1;
+      while (p < e && !is_space((unsigned char)w[p])) p++;
+      ro.refs[j].pos = s + 1;
+      ro.refs[j].len = (uint32_t)(p - s - 1);
+      ro.seq_off[j] = before & 0xFFFFFFFFull;
+      ro.rec_line[j] = (uint32_t)k;
+    }
   }
 }
 
 struct CutArgs {
   Window wd;
-  const uint32_t *hflag;
-  const uint64_t *line_pos, *hdr_rank;
-  uint64_t n_hdr, contrib_total;
   uint64_t block_bytes, block_records;
   int interleaved;
-  uint64_t *seq_off;              // [cap + 1]
+  const uint64_t *seq_off;
   const uint32_t *rec_line;
   uint64_t *block_start;          // [block_cap + 1]
   uint64_t block_cap;
   const uint32_t *rnext;          // LoadBlock: the record after the block starting at r
   ParseInfo *info;
 };
-
-// One thread: how many records are valid and complete, and the sequence end
-// of the last of them.
-__global__ void valid_kernel(CutArgs a) {
-  if (blockIdx.x || threadIdx.x) return;
-  const Window &wd = a.wd;
-  const unsigned long long fb = a.info->first_bad;
-  uint64_t complete, limit;
-  if (wd.fastq) {
-    complete = wd.n_lines / 4;
-    limit = fb == kNone ? complete : fb / 4;
-  } else {
-    complete = wd.at_eof ? a.n_hdr : (a.n_hdr ? a.n_hdr - 1 : 0);
-    // a bad line is never a header: it belongs to the record before it
-    limit = fb == kNone ? complete : (a.hdr_rank[fb] ? a.hdr_rank[fb] - 1 : 0);
-  }
-  const uint64_t valid = complete < limit ? complete : limit;
-  a.seq_off[valid] = valid < a.n_hdr ? a.line_pos[a.rec_line[valid]] : a.contrib_total;
-  a.info->valid = valid;
-  a.info->all = fb == kNone && wd.at_eof;   // the input ends with record `valid`
-}
 
 constexpr uint32_t kNoEnd = 0xFFFFFFFFu;
 
@@ -283,7 +423,8 @@ __global__ void block_end_kernel(const uint64_t *seq_off, uint64_t block_bytes,
 // src/seqreader.h:101-163) from record 0, following rnext for LoadBlock.
 __global__ void cut_kernel(CutArgs a) {
   if (blockIdx.x || threadIdx.x) return;
-  const Window &wd = a.wd;
+  Window wd = a.wd;
+  wd.load();
   const uint64_t valid = a.info->valid;
   const bool all = a.info->all != 0;
   uint64_t take = 0, nb = 0;
@@ -310,10 +451,10 @@ __global__ void cut_kernel(CutArgs a) {
   a.info->bases = a.seq_off[a.interleaved ? 2 * frags : frags];
   // the window bytes of the kept records: up to the next header, or to the
   // end of the last whole line when every record was kept
-  a.info->consumed = take < a.n_hdr   ? wd.start(a.rec_line[take])
-                     : take == 0      ? 0
+  a.info->consumed = take < a.info->n_hdr ? wd.start(a.rec_line[take])
+                     : take == 0          ? 0
                      : wd.n_lines > wd.n_nl ? wd.len
-                                      : wd.start(wd.n_lines);
+                                          : wd.start(wd.n_lines);
 }
 
 // Per kept fragment: its reader block and the longest sequence.
@@ -341,12 +482,12 @@ __global__ void frag_kernel(const uint64_t *seq_off, const uint64_t *block_start
 // One warp per sequence line of a kept record: its bytes to the gathered
 // array; with min_quality, FASTQ bases whose quality byte (signed) minus '!'
 // is below it become 'x' (MaskLowQualityBases, src/classify.cc:1061-1071).
-__global__ void gather_kernel(Window wd, const uint32_t *contrib, const uint64_t *line_pos,
-                              const uint32_t *rec_line, const uint64_t n_hdr, const ParseInfo *info,
-                              int min_quality, char *bases) {
-  const uint64_t take = info->n_take;
+__global__ void gather_kernel(Window wd, const uint32_t *contrib, const uint32_t *line_pos,
+                              const uint32_t *rec_line, int min_quality, char *bases) {
+  wd.load();
+  const uint64_t take = wd.info->n_take;
   if (!take) return;
-  const uint64_t stop = take < n_hdr ? rec_line[take] : wd.n_lines;
+  const uint64_t stop = take < wd.info->n_hdr ? rec_line[take] : wd.n_lines;
   const int lane = threadIdx.x & 31;
   const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
   const uint64_t first = rec_line[0];
@@ -355,21 +496,28 @@ __global__ void gather_kernel(Window wd, const uint32_t *contrib, const uint64_t
     const uint64_t k = wd.fastq ? 4 * u + 1 : first + u;
     if (k >= stop) break;
     const uint32_t n = contrib[k];
-    if (!n) continue;
+    if (!n || n == kHeader) continue;
     const char *src = wd.win + wd.start(k);
     char *dst = bases + line_pos[k];
     if (wd.fastq && min_quality > 0) {
       const signed char *q = reinterpret_cast<const signed char *>(wd.win + wd.start(k + 2));
       for (uint32_t j = lane; j < n; j += 32) dst[j] = (int)q[j] - '!' < min_quality ? 'x' : src[j];
     } else {
-      for (uint32_t j = lane; j < n; j += 32) dst[j] = src[j];
+      constexpr int kAhead = 4;   // loads in flight per lane
+      for (uint32_t j = lane; j < n; j += 32 * kAhead) {
+        char c[kAhead];
+#pragma unroll
+        for (int t = 0; t < kAhead; t++) c[t] = j + 32 * t < n ? src[j + 32 * t] : 0;
+#pragma unroll
+        for (int t = 0; t < kAhead; t++)
+          if (j + 32 * t < n) dst[j + 32 * t] = c[t];
+      }
     }
   }
 }
 
-__global__ void count_classified_kernel(const uint32_t *call, const ParseInfo *info_in,
-                                        ParseInfo *info) {
-  const uint64_t n = info_in->n_frags;
+__global__ void count_classified_kernel(const uint32_t *call, ParseInfo *info) {
+  const uint64_t n = info->n_frags;
   unsigned c = 0;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x)
@@ -415,8 +563,8 @@ struct k2g_text {
   bool handed_off = false;
   uint32_t next_block = 0;
   uint64_t next_frag = 0;
-  DBuf<uint32_t> tile_cnt, nl, contrib, hflag, rec_line, block, call, hlen, status, rnext;
-  DBuf<uint64_t> tile_off, sums, total, line_pos, hdr_rank, seq_off, block_start, runs;
+  DBuf<uint32_t> tile_cnt, nl, contrib, line_pos, rec_line, block, call, hlen, rnext;
+  DBuf<uint64_t> tile_off, sums, line_sum, seq_off, block_start, runs;
   DBuf<k2g_name_ref> refs;
   DBuf<char> bases;
   DBuf<unsigned long long> taxon_reads;
@@ -428,7 +576,6 @@ struct k2g_text {
   int text_cur = 0;               // the buffer of the last call
   cudaStream_t fetch_st = nullptr;
   cudaEvent_t text_free[2] = {nullptr, nullptr};   // the last copy out of each buffer
-  DBuf<unsigned int> bad;
   DBuf<ParseInfo> info;
   ParseInfo *h_info = nullptr;    // pinned
   uint64_t text_len = 0;          // kraken-line bytes of the last call, in `text`
@@ -453,13 +600,11 @@ k2g_status text_alloc(k2g_text *t) {
   const uint64_t tiles = W / kTile + 2;
   K2G_CUDA_TRY(t->tile_cnt.need(tiles));
   K2G_CUDA_TRY(t->tile_off.need(tiles));
-  K2G_CUDA_TRY(t->sums.need(t->line_cap / 1024 + 2));
-  K2G_CUDA_TRY(t->total.need(2));
+  K2G_CUDA_TRY(t->sums.need(t->rec_cap / 1024 + 2));
+  K2G_CUDA_TRY(t->line_sum.need(t->line_cap / kLineTile + 2));
   K2G_CUDA_TRY(t->nl.need(t->line_cap));
   K2G_CUDA_TRY(t->contrib.need(t->line_cap));
-  K2G_CUDA_TRY(t->hflag.need(t->line_cap));
   K2G_CUDA_TRY(t->line_pos.need(t->line_cap));
-  K2G_CUDA_TRY(t->hdr_rank.need(t->line_cap));
   K2G_CUDA_TRY(t->refs.need(t->rec_cap));
   K2G_CUDA_TRY(t->rec_line.need(t->rec_cap + 1));
   K2G_CUDA_TRY(t->seq_off.need(t->rec_cap + 2));
@@ -470,12 +615,10 @@ k2g_status text_alloc(k2g_text *t) {
   K2G_CUDA_TRY(t->call.need(t->rec_cap));
   K2G_CUDA_TRY(t->hlen.need(t->rec_cap));
   K2G_CUDA_TRY(t->runs.need(W + 2 * t->rec_cap + 8));
-  K2G_CUDA_TRY(t->status.need(1));
   K2G_CUDA_TRY(t->taxon_reads.need(t->db->node_count));
   K2G_CUDA_TRY(cudaMemset(t->taxon_reads.p, 0, t->db->node_count * 8));
   K2G_CUDA_TRY(t->line_len.need(t->rec_cap));
   K2G_CUDA_TRY(t->line_off.need(t->rec_cap));
-  K2G_CUDA_TRY(t->bad.need(1));
   K2G_CUDA_TRY(t->info.need(1));
   K2G_CUDA_TRY(t->hits_used.need(1));
   K2G_CUDA_TRY(cudaStreamCreateWithFlags(&t->copy_st, cudaStreamNonBlocking));
@@ -488,12 +631,12 @@ k2g_status text_alloc(k2g_text *t) {
 void text_free(k2g_text *t) {
   if (t->st) cudaStreamSynchronize(t->st);
   for (auto &b : t->win) b.free();
-  t->tile_cnt.free(); t->nl.free(); t->contrib.free(); t->hflag.free(); t->rec_line.free();
-  t->block.free(); t->rnext.free(); t->call.free(); t->hlen.free(); t->status.free();
-  t->tile_off.free(); t->sums.free(); t->total.free(); t->line_pos.free(); t->hdr_rank.free();
+  t->tile_cnt.free(); t->nl.free(); t->contrib.free(); t->line_pos.free(); t->rec_line.free();
+  t->block.free(); t->rnext.free(); t->call.free(); t->hlen.free();
+  t->tile_off.free(); t->sums.free(); t->line_sum.free();
   t->seq_off.free(); t->block_start.free(); t->runs.free(); t->refs.free(); t->bases.free();
   t->taxon_reads.free(); t->hit_keys.free(); t->hit_order.free(); t->hits_used.free();
-  t->hit_taxa.free(); t->line_len.free(); t->line_off.free(); t->bad.free();
+  t->hit_taxa.free(); t->line_len.free(); t->line_off.free();
   t->info.free();
   if (t->copy_st) cudaStreamSynchronize(t->copy_st);
   if (t->fetch_st) cudaStreamSynchronize(t->fetch_st);
@@ -613,83 +756,42 @@ extern "C" k2g_status k2g_text_classify(k2g_text *t, const char *chunk, uint64_t
 
   // 1. line ends
   const uint64_t tiles = (W + kTile - 1) / kTile;
+  ParseInfo *info = t->info.p;
   nl_count_kernel<<<(unsigned)tiles, kTileThreads, 0, st>>>(win, W, t->tile_cnt.p);
-  k2g_status s = exclusive_scan_u32(t->tile_cnt.p, tiles, t->tile_off.p, t->sums.p, t->total.p, st);
-  if (s != K2G_OK) return s;
+  tile_scan_kernel<<<1, kScanThreads, 0, st>>>(win, W, t->tile_cnt.p, tiles, t->tile_off.p, at_eof ? 1 : 0,
+                                               t->line_cap, info);
   nl_write_kernel<<<(unsigned)tiles, kTileThreads, 0, st>>>(win, W, t->tile_off.p, t->nl.p,
                                                             t->line_cap);
-  note_launches(2);
-  K2G_CUDA_TRY(cudaGetLastError());
-  uint64_t n_nl = 0;
-  K2G_CUDA_TRY(cudaMemcpyAsync(&n_nl, t->total.p, 8, cudaMemcpyDeviceToHost, st));
-  K2G_CUDA_TRY(cudaStreamSynchronize(st));
-  // the last line counts when the input ends without a '\n'
-  char last = len ? chunk[len - 1] : '\n';
-  if (!len) {   // only held bytes: the last one is on the device
-    K2G_CUDA_TRY(cudaMemcpyAsync(&last, win + W - 1, 1, cudaMemcpyDeviceToHost, st));
-    K2G_CUDA_TRY(cudaStreamSynchronize(st));
-  }
-  const uint64_t n_lines = n_nl + (at_eof && last != '\n' ? 1 : 0);
-  if (n_lines > t->line_cap) return hand_off(0);   // lines too short for the buffers
-
-  Window wd{win, W, t->nl.p, n_nl, n_lines, t->format, at_eof ? 1 : 0};
-  ParseInfo init{};
-  init.first_bad = kNone;
-  K2G_CUDA_TRY(cudaMemcpyAsync(t->info.p, &init, sizeof(init), cudaMemcpyHostToDevice, st));
-  // 2. line roles
-  if (n_lines) {
-    line_kernel<<<grid_for(t, n_lines, 256), 256, 0, st>>>(wd, t->contrib.p, t->hflag.p, t->info.p);
-    note_launches();
-    K2G_CUDA_TRY(cudaGetLastError());
-  }
+  // 2. line roles (lines are W / 80 or so; any grid does)
+  Window wd{win, W, t->nl.p, info, t->format, at_eof ? 1 : 0, 0, 0};
+  const unsigned g_lines = grid_for(t, W / 64 + 1, kLineTile), g_recs = grid_for(t, W / 256 + 1, 256);
+  line_kernel<<<g_lines, kLineThreads, 0, st>>>(wd, t->contrib.p, t->line_sum.p, info);
   // 3. sequence placement and record numbers
-  uint64_t *d_tot = t->total.p;
-  s = exclusive_scan_u32(t->contrib.p, n_lines, t->line_pos.p, t->sums.p, d_tot, st);
-  if (s != K2G_OK) return s;
-  uint64_t totals[2] = {0, 0};
-  K2G_CUDA_TRY(cudaMemcpyAsync(&totals[0], d_tot, 8, cudaMemcpyDeviceToHost, st));
-  s = exclusive_scan_u32(t->hflag.p, n_lines, t->hdr_rank.p, t->sums.p, d_tot + 1, st);
-  if (s != K2G_OK) return s;
-  K2G_CUDA_TRY(cudaMemcpyAsync(&totals[1], d_tot + 1, 8, cudaMemcpyDeviceToHost, st));
-  K2G_CUDA_TRY(cudaStreamSynchronize(st));
-  if (!n_lines) totals[0] = totals[1] = 0;
-  const uint64_t contrib_total = totals[0], n_hdr = totals[1];
-  if (n_hdr > t->rec_cap) return hand_off(0);
+  line_scan_kernel<<<1, kScanThreads, 0, st>>>(wd, t->contrib.p, t->line_sum.p, info);
   // 4. records and reader blocks
-  RecordOut ro{t->refs.p, t->seq_off.p, t->rec_line.p, t->rec_cap};
-  if (n_lines) {
-    record_kernel<<<grid_for(t, n_lines, 256), 256, 0, st>>>(wd, t->hflag.p, t->line_pos.p,
-                                                            t->hdr_rank.p, ro);
-    note_launches();
-  }
-  CutArgs ca{wd, t->hflag.p, t->line_pos.p, t->hdr_rank.p, n_hdr, contrib_total,
-             t->cfg.block_bytes, t->cfg.block_records, t->cfg.interleaved ? 1 : 0,
-             t->seq_off.p, t->rec_line.p, t->block_start.p, t->block_cap, t->rnext.p,
-             t->info.p};
-  valid_kernel<<<1, 1, 0, st>>>(ca);
+  RecordOut ro{t->line_pos.p, t->refs.p, t->seq_off.p, t->rec_line.p, t->rec_cap};
+  record_kernel<<<g_lines, kLineThreads, 0, st>>>(wd, t->contrib.p, t->line_sum.p, ro);
+  CutArgs ca{wd, t->cfg.block_bytes, t->cfg.block_records, t->cfg.interleaved ? 1 : 0,
+             t->seq_off.p, t->rec_line.p, t->block_start.p, t->block_cap, t->rnext.p, info};
   if (!t->cfg.block_records) {
-    block_end_kernel<<<grid_for(t, n_hdr, 256), 256, 0, st>>>(t->seq_off.p, t->cfg.block_bytes,
-                                                               t->info.p, t->rnext.p);
+    block_end_kernel<<<g_recs, 256, 0, st>>>(t->seq_off.p, t->cfg.block_bytes, info, t->rnext.p);
     note_launches();
   }
   cut_kernel<<<1, 1, 0, st>>>(ca);
-  note_launches();
-  frag_kernel<<<grid_for(t, n_hdr, 256), 256, 0, st>>>(t->seq_off.p, t->block_start.p,
-                                                        t->next_block, t->cfg.interleaved ? 1 : 0,
-                                                        t->block.p, t->info.p);
-  note_launches(2);
+  frag_kernel<<<g_recs, 256, 0, st>>>(t->seq_off.p, t->block_start.p, t->next_block,
+                                      t->cfg.interleaved ? 1 : 0, t->block.p, info);
+  note_launches(8);
   K2G_CUDA_TRY(cudaGetLastError());
-  K2G_CUDA_TRY(cudaMemcpyAsync(t->h_info, t->info.p, sizeof(ParseInfo), cudaMemcpyDeviceToHost, st));
+  K2G_CUDA_TRY(cudaMemcpyAsync(t->h_info, info, sizeof(ParseInfo), cudaMemcpyDeviceToHost, st));
   K2G_CUDA_TRY(cudaStreamSynchronize(st));
   const ParseInfo pi = *t->h_info;
+  if (pi.too_many) return hand_off(0);   // lines too short for the buffers
   const uint64_t nf = pi.n_frags;
   // 5. gather, classify, count and format
   if (nf) {
     gather_kernel<<<grid_for(t, pi.n_take * 32, 256), 256, 0, st>>>(
-        wd, t->contrib.p, t->line_pos.p, t->rec_line.p, n_hdr, t->info.p,
-        t->params.min_quality, t->bases.p);
+        wd, t->contrib.p, t->line_pos.p, t->rec_line.p, t->params.min_quality, t->bases.p);
     note_launches();
-    K2G_CUDA_TRY(cudaMemsetAsync(t->status.p, 0, 4, st));
     k2g_classify_params cp = t->params;
     cp.min_quality = 0;   // masked while gathering
     k2g_reads rd{};
@@ -706,7 +808,7 @@ extern "C" k2g_status k2g_text_classify(k2g_text *t, const char *chunk, uint64_t
     rs.d_runs = t->runs.p;
     rs.runs_cap = t->runs.cap;
     rs.d_taxon_reads = reinterpret_cast<uint64_t *>(t->taxon_reads.p);
-    rs.d_status = t->status.p;
+    rs.d_status = &info->status;
     if (counters) {
       const uint64_t hits = pi.bases + 4 * nf + 16;
       K2G_CUDA_TRY(t->hit_keys.need(hits));
@@ -719,18 +821,26 @@ extern "C" k2g_status k2g_text_classify(k2g_text *t, const char *chunk, uint64_t
       rs.hits_cap = t->hit_keys.cap;
       rs.d_hits_used = t->hits_used.p;
     }
-    s = classify_keyed(t->db, &rd, &cp, &rs, K2G_MODE_PIPELINED, st, st);
+    k2g_status s = classify_keyed(t->db, &rd, &cp, &rs, K2G_MODE_PIPELINED, st, st);
     if (s != K2G_OK) return s;
     if (counters) {
       s = k2g_counters_add(counters, &rd, &rs, st);
       if (s != K2G_OK) return s;
     }
-    count_classified_kernel<<<grid_for(t, nf, 256), 256, 0, st>>>(t->call.p, t->info.p, t->info.p);
+    count_classified_kernel<<<grid_for(t, nf, 256), 256, 0, st>>>(t->call.p, info);
     note_launches();
     K2G_CUDA_TRY(cudaGetLastError());
-    uint64_t text_total = 0;
+    lines::LinesView v{};
+    const unsigned g = grid_for(t, nf, lines::kThreads);
+    const int c = t->text_cur ^ 1;   // the other buffer than the last call's
+    // (writes nothing where the buffer is too small)
+    auto write_lines = [&]() {
+      lines::line_write_kernel<<<g, lines::kThreads, 0, st>>>(v, t->line_len.p, t->line_off.p, t->sums.p, &info->text_len,
+                                                              t->text[c].p, t->text[c].cap);
+      note_launches();
+      return cudaGetLastError();
+    };
     if (t->cfg.lines) {
-      lines::LinesView v{};
       v.call = t->call.p;
       v.hlen = t->hlen.p;
       v.run_start = nullptr;   // runs where k2g_classify wrote them
@@ -743,7 +853,7 @@ extern "C" k2g_status k2g_text_classify(k2g_text *t, const char *chunk, uint64_t
       v.text_len = W;
       v.n_runs = t->runs.cap;
       v.node_count = t->db->node_count;
-      v.bad = t->bad.p;
+      v.bad = &info->bad;
       v.ext = t->db->d_ext;
       v.name_off = t->db->d_name_off;
       v.names = t->db->d_names;
@@ -752,32 +862,28 @@ extern "C" k2g_status k2g_text_classify(k2g_text *t, const char *chunk, uint64_t
       v.interleaved = t->cfg.interleaved ? 1 : 0;
       v.quick = t->params.quick ? 1 : 0;
       v.print_names = t->cfg.print_names ? 1 : 0;
-      K2G_CUDA_TRY(cudaMemsetAsync(t->bad.p, 0, 4, st));
-      const unsigned g = grid_for(t, nf, 256);
-      lines::line_len_kernel<<<g, 256, 0, st>>>(v, t->line_len.p);
+      lines::line_len_kernel<<<g, lines::kThreads, 0, st>>>(v, t->line_len.p);
       note_launches();
-      s = exclusive_scan_u32(t->line_len.p, nf, t->line_off.p, t->sums.p, d_tot, st);
+      s = block_scan_u32(t->line_len.p, nf, t->line_off.p, t->sums.p, &info->text_len, st);
       if (s != K2G_OK) return s;
-      K2G_CUDA_TRY(cudaMemcpyAsync(&text_total, d_tot, 8, cudaMemcpyDeviceToHost, st));
-      K2G_CUDA_TRY(cudaStreamSynchronize(st));
-      // the other buffer than the last call's, once its copy out is done
-      const int c = t->text_cur ^ 1;
-      K2G_CUDA_TRY(cudaEventSynchronize(t->text_free[c]));
-      K2G_CUDA_TRY(t->text[c].need(text_total + 1));
-      t->text_cur = c;
-      lines::line_write_kernel<<<g, 256, 0, st>>>(v, t->line_off.p, t->text[c].p);
-      note_launches();
-      K2G_CUDA_TRY(cudaGetLastError());
+      // once the buffer's copy out is done
+      K2G_CUDA_TRY(cudaStreamWaitEvent(st, t->text_free[c], 0));
+      K2G_CUDA_TRY(write_lines());
     }
-    uint32_t status_word = 0;
-    unsigned int bad = 0;
-    K2G_CUDA_TRY(cudaMemcpyAsync(t->h_info, t->info.p, sizeof(ParseInfo), cudaMemcpyDeviceToHost, st));
-    K2G_CUDA_TRY(cudaMemcpyAsync(&status_word, t->status.p, 4, cudaMemcpyDeviceToHost, st));
-    if (t->cfg.lines) K2G_CUDA_TRY(cudaMemcpyAsync(&bad, t->bad.p, 4, cudaMemcpyDeviceToHost, st));
+    K2G_CUDA_TRY(cudaMemcpyAsync(t->h_info, info, sizeof(ParseInfo), cudaMemcpyDeviceToHost, st));
     K2G_CUDA_TRY(cudaStreamSynchronize(st));
-    if (status_word) return fail(K2G_ERR_CAPACITY, "classification buffer overflow");
-    if (bad) return fail(K2G_ERR_FORMAT, "a taxon outside the taxonomy in a kraken line");
-    t->text_len = text_total;
+    if (t->h_info->status) return fail(K2G_ERR_CAPACITY, "classification buffer overflow");
+    if (t->h_info->bad) return fail(K2G_ERR_FORMAT, "a taxon outside the taxonomy in a kraken line");
+    if (t->cfg.lines) {
+      const uint64_t len = t->h_info->text_len;
+      if (len > t->text[c].cap) {   // (the first calls, and longer lines than before)
+        K2G_CUDA_TRY(t->text[c].need(len + len / 8));
+        K2G_CUDA_TRY(write_lines());
+        K2G_CUDA_TRY(cudaStreamSynchronize(st));
+      }
+      t->text_cur = c;
+      t->text_len = len;
+    }
     res->classified = t->h_info->classified;
   }
   res->fragments = nf;
