@@ -1,55 +1,105 @@
-// Sorts many buckets of 64-bit keys (below 2^63) at once, a thread block to a
-// bucket in shared memory, and drops repeats: the library build's sequence
-// blocks and the -K counters' hash ranges.
+// Sorts many buckets of 64-bit keys at once, a thread block to a bucket in
+// shared memory, and drops repeats: the library build's sequence blocks and
+// the -K counters' hash ranges.
 //
-// A bucket's keys go to shared memory by zone -- 256 of them, in the order the
-// caller wants first, spread evenly (a hash or uniform bits) -- and a warp
-// ranks a zone's few keys by comparing all with all: about 5 instructions a
-// key at 25 keys a zone, against a radix pass over memory per 8 bits.
+// A bucket's keys go to shared memory by zone -- 4,096 of them, in the order
+// the caller wants first, spread as evenly as the keys allow (a hash, uniform
+// bits), so that a zone holds about one key and a thread sorts a zone by
+// insertion.  Two passes over the keys and one over the zones: about two warp
+// instructions a key (with 256 zones, ranked by a warp each, it was thirteen).
+// Zones of more than kThreadZone keys -- repeats, uneven keys -- are ranked
+// by a warp.
 #pragma once
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "k2g_device.cuh"
+#include "radix_sort.cuh"
 
 namespace k2g {
 namespace {
 
 constexpr int kSortThreads = 512;
-constexpr int kZones = 256;
+constexpr int kZones = 4096;
+constexpr uint32_t kThreadZone = 20;      // keys of a zone sorted by one thread
 constexpr uint32_t kSmallBlock = 8064;    // keys; three thread blocks to an SM
 constexpr uint32_t kLargeBlock = 25600;   // 200 KB of keys
+constexpr uint32_t kBigZones = kLargeBlock / (kThreadZone + 1) + 1;
 
-inline size_t bucket_sort_smem(uint32_t cap) { return (size_t)cap * 8 + kZones * 12 + 16; }
+// Keys, zone ends (16 bits each), big zones.
+inline size_t bucket_sort_smem(uint32_t cap) {
+  return (size_t)cap * 8 + kZones * 2 + (cap / (kThreadZone + 1) + 1) * 2 + 16;
+}
 
-struct ZoneMurmur {   // MurmurHash3 mod 256
-  __device__ __forceinline__ uint32_t operator()(uint64_t key) const { return (uint32_t)murmur3(key) & 0xFFu; }
-};
-struct ZoneBits {     // eight bits of the key
+struct ZoneMurmur {   // MurmurHash3 mod 256, then the key's four top bits
   int shift;
-  __device__ __forceinline__ uint32_t operator()(uint64_t key) const { return (uint32_t)(key >> shift) & 0xFFu; }
+  __device__ __forceinline__ uint32_t operator()(uint64_t key) const {
+    return ((uint32_t)murmur3(key) & 0xFFu) << 4 | ((uint32_t)(key >> shift) & 15u);
+  }
+};
+struct ZoneBits {     // twelve bits of the key
+  int shift;
+  __device__ __forceinline__ uint32_t operator()(uint64_t key) const { return (uint32_t)(key >> shift) & 0xFFFu; }
 };
 
-// Distinct keys of a zone holding more than 128 keys, one after
-// another from the smallest (warp-wide); out may be null (count only).
-__device__ __forceinline__ uint32_t select_distinct(const uint64_t *z, uint32_t n, uint64_t *out) {
-  const uint32_t lane = threadIdx.x & 31;
-  uint64_t last = 0;
-  uint32_t d = 0;
-  for (;;) {
-    uint64_t best = ~0ull;
-    for (uint32_t i = lane; i < n; i += 32) {
-      const uint64_t x = z[i];
-      if ((!d || x > last) && x < best) best = x;
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) best = min64(best, __shfl_xor_sync(0xffffffffu, best, o));
-    if (best == ~0ull) return d;   // (keys have fewer than 64 bits)
-    if (out && lane == 0) out[d] = best;
-    last = best;
+constexpr uint64_t kNoKey = ~0ull;   // (no key has all bits set)
+
+// One thread: a zone's keys in order, repeats dropped (kNoKey behind them).
+__device__ __forceinline__ void sort_zone(uint64_t *z, uint32_t m) {
+  uint32_t d = 1;
+  for (uint32_t i = 1; i < m; i++) {
+    const uint64_t x = z[i];
+    uint32_t j = d;
+    uint64_t y = 0;
+    while (j && (y = z[j - 1]) > x) j--;
+    if (j && y == x) continue;
+    for (uint32_t t = d; t > j; t--) z[t] = z[t - 1];
+    z[j] = x;
     d++;
+  }
+  for (; d < m; d++) z[d] = kNoKey;
+}
+
+// One warp: the same for a zone of any size, by a bitonic sort whose every
+// exchange puts the lesser key first (keys past m count as the greatest);
+// kNoKey takes the place of repeats.
+__device__ __forceinline__ void sort_big_zone(uint64_t *z, uint32_t m) {
+  const uint32_t lane = threadIdx.x & 31;
+  auto exchange = [&](uint32_t a, uint32_t b) {
+    if (b >= m) return;
+    const uint64_t x = z[a], y = z[b];
+    if (x > y) {
+      z[a] = y;
+      z[b] = x;
+    }
+  };
+  uint32_t half = 1;   // half of m, as a power of two
+  while (2 * half < m) half *= 2;
+  for (uint32_t k = 1; k <= half; k *= 2) {
+    // runs of k are sorted: the second of each two runs backwards, then both apart
+    for (uint32_t i = lane; i < half; i += 32) {
+      const uint32_t t = i & (k - 1), run = (i - t) * 2;
+      exchange(run + t, run + 2 * k - 1 - t);
+    }
+    __syncwarp();
+    for (uint32_t j = k / 2; j; j /= 2) {
+      for (uint32_t i = lane; i < half; i += 32) {
+        const uint32_t t = i & (j - 1), run = (i - t) * 2;
+        exchange(run + t, run + t + j);
+      }
+      __syncwarp();
+    }
+  }
+  uint64_t last = kNoKey;
+  for (uint32_t i0 = 0; i0 < m; i0 += 32) {
+    const uint64_t x = i0 + lane < m ? z[i0 + lane] : kNoKey;
+    uint64_t before = __shfl_up_sync(0xffffffffu, x, 1);
+    if (lane == 0) before = last;
+    last = __shfl_sync(0xffffffffu, x, 31);
+    if (x == before && i0 + lane < m) z[i0 + lane] = kNoKey;
   }
 }
 
@@ -61,113 +111,189 @@ __global__ void __launch_bounds__(kSortThreads)
 bucket_sort_kernel(const uint32_t *start, uint64_t *keys, uint32_t lo, uint32_t cap, uint32_t *n_distinct,
                    Zone zone) {
   extern __shared__ __align__(16) unsigned char smem[];
+  constexpr int kWarps = kSortThreads / 32, kPer = kZones / kSortThreads;
+  static_assert(kPer == 8, "a thread scans its zones as one 16-byte word");
   uint64_t *key = reinterpret_cast<uint64_t *>(smem);
-  uint32_t *hist = reinterpret_cast<uint32_t *>(smem + (size_t)cap * 8), *first = hist + kZones, *dist = first + kZones;
+  uint32_t *count2 = reinterpret_cast<uint32_t *>(smem + (size_t)cap * 8);   // two zones a word
+  uint16_t *end = reinterpret_cast<uint16_t *>(count2);
+  uint16_t *big = end + kZones;
+  __shared__ uint32_t s_warp[kWarps], s_big;
   const uint32_t b = blockIdx.x, base = start[b], n = start[b + 1] - base;
   if (n <= lo && lo) return;
   if (n > cap) return;
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = kSortThreads / 32;
+  const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (!n) {
-    if (threadIdx.x == 0) n_distinct[b] = 0;
+    if (tid == 0) n_distinct[b] = 0;
     return;
   }
-  for (uint32_t i = threadIdx.x; i < kZones; i += kSortThreads) hist[i] = 0;
+  reinterpret_cast<uint4 *>(count2)[tid] = make_uint4(0, 0, 0, 0);
+  if (tid == 0) s_big = 0;
   __syncthreads();
   const uint64_t *x = keys + base;
-  for (uint32_t i = threadIdx.x; i < n; i += kSortThreads) atomicAdd(&hist[zone(x[i])], 1u);
+#pragma unroll 2
+  for (uint32_t i = tid; i < n; i += kSortThreads) {
+    const uint32_t z = zone(x[i]);
+    atomicAdd(&count2[z >> 1], 1u << (16 * (z & 1)));
+  }
   __syncthreads();
-  auto scan = [&](const uint32_t *in, uint32_t *out) {   // exclusive, by the first warp
-    uint32_t carry = 0;
-    for (int i0 = 0; i0 < kZones; i0 += 32) {
-      const uint32_t v = in[i0 + lane];
-      uint32_t x = v;
+  {   // counts to starts
+    uint4 c4 = reinterpret_cast<uint4 *>(count2)[tid];
+    uint32_t c[4] = {c4.x, c4.y, c4.z, c4.w}, sum = 0;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if ((int)lane >= o) x += y;
-      }
-      out[i0 + lane] = carry + x - v;
-      carry += __shfl_sync(0xffffffffu, x, 31);
+    for (int u = 0; u < 4; u++) sum += (c[u] & 0xFFFFu) + (c[u] >> 16);
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if ((int)lane >= o) incl += y;
     }
-    return carry;
-  };
-  if (warp == 0) scan(hist, first);
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint32_t at = incl - sum;
+    for (uint32_t w = 0; w < warp; w++) at += s_warp[w];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const uint32_t lo16 = at, hi16 = at + (c[u] & 0xFFFFu);
+      at = hi16 + (c[u] >> 16);
+      c[u] = lo16 | hi16 << 16;
+    }
+    reinterpret_cast<uint4 *>(count2)[tid] = make_uint4(c[0], c[1], c[2], c[3]);
+  }
   __syncthreads();
-  for (uint32_t i = threadIdx.x; i < kZones; i += kSortThreads) dist[i] = first[i];   // cursors
-  __syncthreads();
-  for (uint32_t i = threadIdx.x; i < n; i += kSortThreads) {
+#pragma unroll 2
+  for (uint32_t i = tid; i < n; i += kSortThreads) {
     const uint64_t v = x[i];
-    key[atomicAdd(&dist[zone(v)], 1u)] = v;
+    const uint32_t z = zone(v), old = atomicAdd(&count2[z >> 1], 1u << (16 * (z & 1)));
+    key[z & 1 ? old >> 16 : old & 0xFFFFu] = v;
+  }
+  __syncthreads();   // (a zone's start is its end now)
+  for (uint32_t z = tid; z < kZones; z += kSortThreads) {
+    const uint32_t from = z ? end[z - 1] : 0, m = end[z] - from;
+    if (m > kThreadZone) big[atomicAdd(&s_big, 1u)] = (uint16_t)z;
+    else if (m > 1) sort_zone(key + from, m);
   }
   __syncthreads();
-  // every zone sorted in place, repeats dropped
-  for (uint32_t z = warp; z < kZones; z += warps) {
-    const uint32_t m = hist[z];
-    uint64_t *zk = key + first[z];
-    uint32_t d = 0;
-    if (m <= 32) {
-      const uint64_t v = lane < m ? zk[lane] : ~0ull;
-      uint32_t less = 0;
-      bool again = false;
-      for (uint32_t j = 0; j < m; j++) {
-        const uint64_t x = __shfl_sync(0xffffffffu, v, j);
-        less |= x < v ? 1u << j : 0u;
-        again |= x == v && j < lane;
-      }
-      const bool own = lane < m && !again;
-      const uint32_t keepers = __ballot_sync(0xffffffffu, own);
-      __syncwarp();
-      if (own) zk[__popc(less & keepers)] = v;
-      d = __popc(keepers);
-    } else if (m <= 128) {
-      uint64_t v[4];
-      uint32_t own = 0, rank[4] = {0, 0, 0, 0};
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        const uint32_t i = 32 * t + lane;
-        v[t] = i < m ? zk[i] : ~0ull;
-        bool again = i >= m;
-        for (uint32_t j = 0; j < i && j < m; j++) again |= zk[j] == v[t];
-        own |= again ? 0u : 1u << t;
-      }
-      __syncwarp();
-      uint32_t keepers[4];
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        keepers[t] = __ballot_sync(0xffffffffu, (own >> t) & 1u);
-        d += __popc(keepers[t]);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-        for (uint32_t k = keepers[u]; k; k &= k - 1) {
-          const uint64_t x = zk[32 * u + __ffs(k) - 1];
-#pragma unroll
-          for (int t = 0; t < 4; t++) rank[t] += x < v[t] ? 1u : 0u;
-        }
-      __syncwarp();
-#pragma unroll
-      for (int t = 0; t < 4; t++)
-        if ((own >> t) & 1u) zk[rank[t]] = v[t];
-    } else {
-      d = select_distinct(zk, m, nullptr);
-    }
-    __syncwarp();
-    if (lane == 0) dist[z] = d;
+  for (uint32_t i = warp; i < s_big; i += kWarps) {
+    const uint32_t z = big[i], from = z ? end[z - 1] : 0;
+    sort_big_zone(key + from, end[z] - from);
   }
   __syncthreads();
-  __shared__ uint32_t place[kZones];
-  if (warp == 0) {
-    const uint32_t total = scan(dist, place);
-    if (lane == 0) n_distinct[b] = total;
-  }
+  // what is left, packed: a run of the keys per warp
+  const uint32_t run = (n + 32 * kWarps - 1) / (32 * kWarps) * 32, r0 = min(n, warp * run), r1 = min(n, r0 + run);
+  uint32_t have = 0;
+  for (uint32_t i0 = r0; i0 < r1; i0 += 32)
+    have += __popc(__ballot_sync(0xffffffffu, i0 + lane < r1 && key[i0 + lane] != kNoKey));
+  if (lane == 0) s_warp[warp] = have;
   __syncthreads();
-  for (uint32_t z = warp; z < kZones; z += warps) {
-    uint64_t *out = keys + base + place[z];
-    const uint64_t *zk = key + first[z];
-    if (hist[z] > 128) select_distinct(zk, hist[z], out);
-    else
-      for (uint32_t i = lane; i < dist[z]; i += 32) out[i] = zk[i];
+  uint32_t at = 0, total = 0;
+  for (uint32_t w = 0; w < kWarps; w++) {
+    if (w < warp) at += s_warp[w];
+    total += s_warp[w];
   }
+  if (tid == 0) n_distinct[b] = total;
+  uint64_t *out = keys + base;
+  for (uint32_t i0 = r0; i0 < r1; i0 += 32) {
+    const uint64_t v = i0 + lane < r1 ? key[i0 + lane] : kNoKey;
+    const uint32_t in = __ballot_sync(0xffffffffu, v != kNoKey);
+    if (v != kNoKey) out[at + __popc(in & ((1u << lane) - 1))] = v;
+    at += __popc(in);
+  }
+}
+
+// Keys are dealt into buckets, by the bits from `shift` up, by two kernels, each
+// thread block on one slice of the keys with a counter per bucket in shared
+// memory (a global atomic per key, counting and dealing, took 0.50 ms each for
+// 28M keys): the first adds up the buckets' sizes, the second takes a place in
+// every bucket for its slice's keys and then writes them there, in any order.
+// The second is bound by these writes, a sector each (0.50 ms; the first
+// 0.04).
+constexpr int kDealThreads = 1024;
+constexpr int kDealBits = 15;   // 2^15 counters are 128 KB
+
+__device__ __forceinline__ void count_slice(const uint64_t *k, uint64_t i0, uint64_t i1, int shift, uint32_t nb,
+                                            uint32_t *h) {
+  for (uint32_t b = threadIdx.x; b < nb; b += kDealThreads) h[b] = 0;
+  __syncthreads();
+#pragma unroll 4
+  for (uint64_t i = i0 + threadIdx.x; i < i1; i += kDealThreads) atomicAdd(&h[k[i] >> shift], 1u);
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(kDealThreads)
+bucket_count_kernel(const uint64_t *k, uint64_t n, uint64_t slice, int shift, uint32_t nb, uint32_t *count) {
+  extern __shared__ uint32_t h[];
+  const uint64_t i0 = min(n, blockIdx.x * slice), i1 = min(n, i0 + slice);
+  count_slice(k, i0, i1, shift, nb, h);
+  for (uint32_t b = threadIdx.x; b < nb; b += kDealThreads)
+    if (h[b]) atomicAdd(&count[b], h[b]);
+}
+
+__global__ void __launch_bounds__(kDealThreads)
+bucket_deal_kernel(const uint64_t *k, uint64_t n, uint64_t slice, int shift, uint32_t nb, uint32_t *cursor,
+                   uint64_t *out) {
+  extern __shared__ uint32_t h[];
+  const uint64_t i0 = min(n, blockIdx.x * slice), i1 = min(n, i0 + slice);
+  count_slice(k, i0, i1, shift, nb, h);
+  for (uint32_t b = threadIdx.x; b < nb; b += kDealThreads)
+    if (h[b]) h[b] = atomicAdd(&cursor[b], h[b]);
+  __syncthreads();
+#pragma unroll 4
+  for (uint64_t i = i0 + threadIdx.x; i < i1; i += kDealThreads) {
+    const uint64_t x = k[i];
+    out[atomicAdd(&h[x >> shift], 1u)] = x;
+  }
+}
+
+__global__ void bucket_largest_kernel(const uint32_t *count, uint32_t n, uint32_t *largest) {
+  uint32_t m = 0;
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) m = max(m, count[i]);
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) atomicMax(largest, m);
+}
+
+// Keys to a bucket, where the number of buckets is free: 2,250 to kBucketKeys,
+// and up to kBucketKeysMost with 2^15 buckets.
+constexpr uint64_t kBucketKeys = 4500, kBucketKeysMost = 6000;
+
+// Device words of a deal over nb buckets.
+struct BucketMem {
+  uint32_t nb;
+  uint32_t *start;      // [nb + 1]
+  uint32_t *largest;    // (behind start[nb])
+  uint32_t *place;      // [nb + 1]
+  uint32_t *distinct;   // [nb]
+  uint32_t *sums;
+  static uint64_t words(uint32_t nb) { return 3ull * nb + 3 + nb / rsort::kScanChunk + 2; }
+  BucketMem(uint32_t *mem, uint32_t n)
+      : nb(n), start(mem), largest(start + n + 1), place(largest + 1), distinct(place + n + 1), sums(distinct + n) {}
+};
+
+// Deals keys[0, n) (n < 2^32, each key >> shift below nb <= 2^15) to out, bucket
+// b at start[b]; got: how many were dealt, and the largest bucket.
+inline cudaError_t deal_to_buckets(const uint64_t *keys, uint64_t n, int shift, const BucketMem &m, int device,
+                                   uint64_t *out, uint32_t got[2], cudaStream_t st) {
+  cudaError_t e;
+#define TRY(x) if ((e = (x)) != cudaSuccess) return e
+  int sms = 0;
+  TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+  // (a slice of several keys per counter)
+  const uint64_t slice = std::max<uint64_t>((n + sms - 1) / sms, 4096);
+  const unsigned g = (unsigned)((n + slice - 1) / slice);
+  const int smem = (int)(m.nb * 4);
+  TRY(cudaFuncSetAttribute(bucket_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 << kDealBits));
+  TRY(cudaFuncSetAttribute(bucket_deal_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 << kDealBits));
+  TRY(cudaMemsetAsync(m.start, 0, (m.nb + 2) * 4ull, st));
+  bucket_count_kernel<<<g, kDealThreads, smem, st>>>(keys, n, slice, shift, m.nb, m.start);
+  bucket_largest_kernel<<<(m.nb + 255) / 256, 256, 0, st>>>(m.start, m.nb, m.largest);
+  note_launches(2);
+  TRY(rsort::exclusive_scan(m.start, m.nb + 1, m.sums, st));
+  TRY(cudaMemcpyAsync(m.place, m.start, m.nb * 4ull, cudaMemcpyDeviceToDevice, st));
+  bucket_deal_kernel<<<g, kDealThreads, smem, st>>>(keys, n, slice, shift, m.nb, m.place, out);
+  note_launches();
+  TRY(cudaGetLastError());
+  TRY(cudaMemcpyAsync(got, m.start + m.nb, 8, cudaMemcpyDeviceToHost, st));
+#undef TRY
+  return cudaStreamSynchronize(st);
 }
 
 // Sorts the buckets; `largest` bounds their sizes (at most kLargeBlock).

@@ -9,9 +9,9 @@
 //                       memory, and mapping it costs more than the scan);
 //   bucket_sort_kernel  (bucket_sort.cuh) one thread block per sequence block:
 //                       its candidates to shared memory by zone (MurmurHash3
-//                       mod 256, the order's first key, so about 22
-//                       candidates a zone at the default block size), each
-//                       zone ranked and freed of repeats by one warp;
+//                       mod 256, the order's first key, then the top bits of
+//                       the value: one or two candidates a zone), each zone
+//                       sorted and freed of repeats by one thread;
 //   block_pack_kernel   the blocks' lists back to back, with their taxa.
 //
 // This replaces eleven radix passes over all (minimizer, block) pairs: for 48

@@ -534,7 +534,7 @@ k2g_status compact(const Gathered &g, Scratch &s, uint64_t **keys, uint32_t **bl
 
 // The distinct (block, minimizer) pairs in the build's order, blocks sorted
 // in shared memory (build_blocks.cuh).
-k2g_status sort_blocks(const Gathered &g, Scratch &s, const uint32_t *block_taxon, uint64_t **keys,
+k2g_status sort_blocks(const k2g_db *db, const Gathered &g, Scratch &s, const uint32_t *block_taxon, uint64_t **keys,
                        uint32_t **taxa, uint64_t *n, cudaStream_t st) {
   const uint32_t nb = (uint32_t)g.block_taxon.size();
   uint32_t *first, *distinct, *place, *sums;   // (first: where a block's candidates start)
@@ -548,7 +548,7 @@ k2g_status sort_blocks(const Gathered &g, Scratch &s, const uint32_t *block_taxo
   K2G_CUDA_TRY(cudaMemcpyAsync(first + nb, &total, 4, cudaMemcpyHostToDevice, st));
   block_start_kernel<<<(unsigned)((g.n_chunks + 255) / 256), 256, 0, st>>>(g.chunks, g.n_chunks, g.offs, first);
   note_launches();
-  K2G_CUDA_TRY(bucket_sort(first, nb, g.largest, g.cand, distinct, ZoneMurmur{}, st));
+  K2G_CUDA_TRY(bucket_sort(first, nb, g.largest, g.cand, distinct, ZoneMurmur{std::max(2 * db->scan_view().l - 4, 0)}, st));
   K2G_CUDA_TRY(cudaMemcpyAsync(place, distinct, nb * 4ull, cudaMemcpyDeviceToDevice, st));
   K2G_CUDA_TRY(rsort::exclusive_scan(place, nb, sums, st));
   block_pack_kernel<<<(unsigned)((nb * 32ull + 255) / 256), 256, 0, st>>>(first, g.cand, distinct, place, nb,
@@ -595,7 +595,7 @@ extern "C" k2g_status k2g_build_sequences(k2g_db *db, const char *bases, const u
   if (scans_by_warps(db->scan_view()) && g.largest <= kLargeBlock) {
     uint64_t *keys = nullptr, n_pairs = 0;
     uint32_t *taxa = nullptr;
-    r = sort_blocks(g, s, d_btax, &keys, &taxa, &n_pairs, st);
+    r = sort_blocks(db, g, s, d_btax, &keys, &taxa, &n_pairs, st);
     s.keep_only(keys, taxa);   // (the insert needs as much again)
     if (r == K2G_OK) r = k2g_build_insert(db, keys, taxa, n_pairs, ordered, st);
     if (r == K2G_OK && n_keys) *n_keys = n_pairs;

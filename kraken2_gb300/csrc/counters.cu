@@ -524,55 +524,6 @@ k2g_status sort_unique(k2g_counters *c, uint64_t *&keys, uint64_t &keys_cap, uin
   return K2G_OK;
 }
 
-// The accumulator's keys are dealt into buckets by two kernels, each thread
-// block on one slice of the keys with a counter per bucket in shared memory
-// (a global atomic per key, counting and dealing, took 0.50 ms each for 28M
-// keys): the first adds up the buckets' sizes, the second takes a place in
-// every bucket for its slice's keys and then writes them there, in any order.
-constexpr int kDealThreads = 1024;
-constexpr int kDealBits = 15;   // 2^15 counters are 128 KB
-
-__device__ __forceinline__ void count_slice(const uint64_t *k, uint64_t i0, uint64_t i1, int shift, uint32_t nb,
-                                            uint32_t *h) {
-  for (uint32_t b = threadIdx.x; b < nb; b += kDealThreads) h[b] = 0;
-  __syncthreads();
-#pragma unroll 4
-  for (uint64_t i = i0 + threadIdx.x; i < i1; i += kDealThreads) atomicAdd(&h[k[i] >> shift], 1u);
-  __syncthreads();
-}
-
-__global__ void __launch_bounds__(kDealThreads)
-bucket_count_kernel(const uint64_t *k, uint64_t n, uint64_t slice, int shift, uint32_t nb, uint32_t *count) {
-  extern __shared__ uint32_t h[];
-  const uint64_t i0 = min(n, blockIdx.x * slice), i1 = min(n, i0 + slice);
-  count_slice(k, i0, i1, shift, nb, h);
-  for (uint32_t b = threadIdx.x; b < nb; b += kDealThreads)
-    if (h[b]) atomicAdd(&count[b], h[b]);
-}
-
-__global__ void __launch_bounds__(kDealThreads)
-bucket_deal_kernel(const uint64_t *k, uint64_t n, uint64_t slice, int shift, uint32_t nb, uint32_t *cursor,
-                   uint64_t *out) {
-  extern __shared__ uint32_t h[];
-  const uint64_t i0 = min(n, blockIdx.x * slice), i1 = min(n, i0 + slice);
-  count_slice(k, i0, i1, shift, nb, h);
-  for (uint32_t b = threadIdx.x; b < nb; b += kDealThreads)
-    if (h[b]) h[b] = atomicAdd(&cursor[b], h[b]);
-  __syncthreads();
-#pragma unroll 4
-  for (uint64_t i = i0 + threadIdx.x; i < i1; i += kDealThreads) {
-    const uint64_t x = k[i];
-    out[atomicAdd(&h[x >> shift], 1u)] = x;
-  }
-}
-
-__global__ void bucket_largest_kernel(const uint32_t *count, uint32_t n, uint32_t *largest) {
-  uint32_t m = 0;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) m = max(m, count[i]);
-  m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0) atomicMax(largest, m);
-}
-
 // One warp per bucket: its distinct keys to their place.
 __global__ void bucket_pack_kernel(const uint32_t *start, const uint64_t *sorted, const uint32_t *n_distinct,
                                    const uint32_t *place, uint32_t n_buckets, uint64_t *out) {
@@ -592,51 +543,31 @@ k2g_status compact_acc(k2g_counters *c, cudaStream_t st) {
   if (c->acc_used == c->acc_compact) return K2G_OK;   // already sorted and unique
   const uint64_t total = c->acc_used;
   int bits = 0;
-  while (bits < kDealBits && (total >> bits) > 4500) bits++;
+  while (bits < kDealBits && (total >> bits) > kBucketKeys) bits++;
   const uint32_t nb = 1u << bits;
   uint64_t n = total;
   bool sorted = false;
-  if (total >= 2 && total < (1ull << 32) && (total >> bits) <= 6000) {
+  if (total >= 2 && total < (1ull << 32) && (total >> bits) <= kBucketKeysMost) {
     const int shift = c->tbits + 32 - bits;
-    uint32_t *mem = nullptr;   // start[nb + 1], cursors and places[nb + 1], distinct[nb], largest, scan sums
-    const uint64_t words = 3ull * nb + 2 + 1 + nb / rsort::kScanChunk + 2;
+    uint32_t *mem = nullptr;
     K2G_CUDA_TRY(reserve(c, st, c->d_alt, c->alt_cap, total));
-    K2G_CUDA_TRY(scratch_alloc(reinterpret_cast<void **>(&mem), words * 4, c->device, st));
-    uint32_t *start = mem, *place = start + nb + 1, *distinct = place + nb + 1, *largest = distinct + nb, *sums = largest + 1;
-    uint32_t most = 0;
+    K2G_CUDA_TRY(scratch_alloc(reinterpret_cast<void **>(&mem), BucketMem::words(nb) * 4, c->device, st));
+    const BucketMem m(mem, nb);
     auto by_buckets = [&]() -> k2g_status {
-      K2G_CUDA_TRY(cudaMemsetAsync(mem, 0, words * 4, st));
-      int sms = 0;
-      K2G_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-      // (a slice of several keys per counter)
-      const uint64_t slice = std::max<uint64_t>((total + sms - 1) / sms, 4096);
-      const unsigned g = (unsigned)((total + slice - 1) / slice);
-      const int smem = (int)(nb * 4);
-      K2G_CUDA_TRY(cudaFuncSetAttribute(bucket_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 << kDealBits));
-      K2G_CUDA_TRY(cudaFuncSetAttribute(bucket_deal_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 << kDealBits));
-      bucket_count_kernel<<<g, kDealThreads, smem, st>>>(c->d_acc, total, slice, shift, nb, start);
-      bucket_largest_kernel<<<(nb + 255) / 256, 256, 0, st>>>(start, nb, largest);
-      note_launches(2);
-      K2G_CUDA_TRY(rsort::exclusive_scan(start, nb + 1, sums, st));
-      K2G_CUDA_TRY(cudaMemcpyAsync(place, start, nb * 4ull, cudaMemcpyDeviceToDevice, st));
-      bucket_deal_kernel<<<g, kDealThreads, smem, st>>>(c->d_acc, total, slice, shift, nb, place, c->d_alt);
-      note_launches();
-      K2G_CUDA_TRY(cudaGetLastError());
-      K2G_CUDA_TRY(cudaMemcpyAsync(&most, largest, 4, cudaMemcpyDeviceToHost, st));
-      K2G_CUDA_TRY(cudaStreamSynchronize(st));
-      if (most > kLargeBlock) return K2G_OK;
-      K2G_CUDA_TRY(bucket_sort(start, nb, most, c->d_alt, distinct, ZoneBits{shift - 8}, st));
-      K2G_CUDA_TRY(cudaMemcpyAsync(place, distinct, nb * 4ull, cudaMemcpyDeviceToDevice, st));
-      K2G_CUDA_TRY(cudaMemsetAsync(place + nb, 0, 4, st));
-      K2G_CUDA_TRY(rsort::exclusive_scan(place, nb + 1, sums, st));
-      bucket_pack_kernel<<<(unsigned)((nb * 32ull + 255) / 256), 256, 0, st>>>(start, c->d_alt, distinct, place, nb,
+      uint32_t got[2] = {0, 0};
+      K2G_CUDA_TRY(deal_to_buckets(c->d_acc, total, shift, m, c->device, c->d_alt, got, st));
+      if (got[1] > kLargeBlock) return K2G_OK;
+      K2G_CUDA_TRY(bucket_sort(m.start, nb, got[1], c->d_alt, m.distinct, ZoneBits{shift - 12}, st));
+      K2G_CUDA_TRY(cudaMemcpyAsync(m.place, m.distinct, nb * 4ull, cudaMemcpyDeviceToDevice, st));
+      K2G_CUDA_TRY(cudaMemsetAsync(m.place + nb, 0, 4, st));
+      K2G_CUDA_TRY(rsort::exclusive_scan(m.place, nb + 1, m.sums, st));
+      bucket_pack_kernel<<<(unsigned)((nb * 32ull + 255) / 256), 256, 0, st>>>(m.start, c->d_alt, m.distinct, m.place, nb,
                                                                               c->d_acc);
       note_launches();
       K2G_CUDA_TRY(cudaGetLastError());
-      uint32_t got = 0;
-      K2G_CUDA_TRY(cudaMemcpyAsync(&got, place + nb, 4, cudaMemcpyDeviceToHost, st));
+      K2G_CUDA_TRY(cudaMemcpyAsync(got, m.place + nb, 4, cudaMemcpyDeviceToHost, st));
       K2G_CUDA_TRY(cudaStreamSynchronize(st));
-      n = got;
+      n = got[0];
       sorted = true;
       return K2G_OK;
     };
