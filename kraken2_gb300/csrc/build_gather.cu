@@ -399,6 +399,10 @@ struct Scratch {
     }
     ptrs.swap(kept);
   }
+  void drop(void *p) {
+    ptrs.erase(std::find(ptrs.begin(), ptrs.end(), p));
+    cudaFreeAsync(p, st);
+  }
   template <class T>
   cudaError_t get(T **p, uint64_t count) {
     *p = nullptr;
@@ -500,6 +504,11 @@ k2g_status gather(const k2g_db *db, const char *bases, const uint64_t *seq_off,
   if (!by_warps) K2G_CUDA_TRY(s.get(&d_cand, extra_slot));
   scan(nullptr);
   K2G_CUDA_TRY(cudaGetLastError());
+  // Random sequence has a new minimizer every three bases (window 5): room for
+  // as many is mapped while the bases are copied and counted.
+  uint64_t *guess = nullptr;
+  const uint64_t guessed = total / 3 + total / 64 + 1024;
+  if (by_warps && s.get(&guess, guessed) != cudaSuccess) cudaGetLastError();
   K2G_CUDA_TRY(cudaMemcpyAsync(d_offs, d_counts, nc * 4, cudaMemcpyDeviceToDevice, st));
   K2G_CUDA_TRY(rsort::exclusive_scan(d_offs, nc, d_sums, st));
   uint32_t last[2] = {0, 0};
@@ -508,7 +517,12 @@ k2g_status gather(const k2g_db *db, const char *bases, const uint64_t *seq_off,
   K2G_CUDA_TRY(cudaStreamSynchronize(st));
   g.n = (uint64_t)last[0] + last[1];
   if (by_warps && g.n) {
-    K2G_CUDA_TRY(s.get(&d_cand, g.n));
+    if (guess && g.n > guessed) {
+      s.drop(guess);
+      guess = nullptr;
+    }
+    if (guess) d_cand = guess;
+    else K2G_CUDA_TRY(s.get(&d_cand, g.n));
     scan(d_offs);
     K2G_CUDA_TRY(cudaGetLastError());
     g.packed = true;
@@ -542,8 +556,6 @@ k2g_status sort_blocks(const k2g_db *db, const Gathered &g, Scratch &s, const ui
   K2G_CUDA_TRY(s.get(&distinct, nb));
   K2G_CUDA_TRY(s.get(&place, nb));
   K2G_CUDA_TRY(s.get(&sums, nb / rsort::kScanChunk + 2));
-  K2G_CUDA_TRY(s.get(keys, g.n));
-  K2G_CUDA_TRY(s.get(taxa, g.n));
   const uint32_t total = (uint32_t)g.n;
   K2G_CUDA_TRY(cudaMemcpyAsync(first + nb, &total, 4, cudaMemcpyHostToDevice, st));
   block_start_kernel<<<(unsigned)((g.n_chunks + 255) / 256), 256, 0, st>>>(g.chunks, g.n_chunks, g.offs, first);
@@ -551,6 +563,10 @@ k2g_status sort_blocks(const k2g_db *db, const Gathered &g, Scratch &s, const ui
   K2G_CUDA_TRY(bucket_sort(first, nb, g.largest, g.cand, distinct, ZoneMurmur{std::max(2 * db->scan_view().l - 4, 0)}, st));
   K2G_CUDA_TRY(cudaMemcpyAsync(place, distinct, nb * 4ull, cudaMemcpyDeviceToDevice, st));
   K2G_CUDA_TRY(rsort::exclusive_scan(place, nb, sums, st));
+  // (before the number is known, while the sort runs: new memory takes 1.5 us
+  // a megabyte to map)
+  K2G_CUDA_TRY(s.get(keys, g.n));
+  K2G_CUDA_TRY(s.get(taxa, g.n));
   block_pack_kernel<<<(unsigned)((nb * 32ull + 255) / 256), 256, 0, st>>>(first, g.cand, distinct, place, nb,
                                                                          block_taxon, *keys, *taxa);
   note_launches();

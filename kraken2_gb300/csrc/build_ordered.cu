@@ -37,12 +37,13 @@ template <class C>
 struct OrderedView {
   TableView t;
   typename C::T *cells;
-  const typename C::T *snap;  // the table before this round
+  const typename C::T *snap;  // the table before this round (null: all zero)
   const uint32_t *occ;        // bitmap: occupied after the unordered pass
   const uint32_t *parent;
   const uint64_t *keys;
   const uint32_t *taxids;
   uint64_t n;
+  __device__ __forceinline__ typename C::T before(uint64_t c) const { return snap ? snap[c] : typename C::T(0); }
 };
 
 template <class C>
@@ -138,7 +139,7 @@ __global__ void replay_kernel(OrderedView<C> v, const uint64_t *sorted, uint64_t
     uint64_t len = 1;
     for (uint64_t c = next_cell(v.t, s); occupied1(v, c) && len < v.t.capacity; c = next_cell(v.t, c))
       len++;
-    for (uint64_t o = 0, c = s; o < len; o++, c = next_cell(v.t, c)) v.cells[c] = v.snap[c];
+    for (uint64_t o = 0, c = s; o < len; o++, c = next_cell(v.t, c)) v.cells[c] = v.before(c);
     uint64_t limit = len;
     bool ok = true;
     for (uint64_t q = p; q < n_sorted && sorted[q] != kNoRegion && (sorted[q] >> kIndexBits) == s; q++) {
@@ -205,7 +206,7 @@ __global__ void fixup_kernel(OrderedView<C> v, const uint64_t *sorted, uint64_t 
         return;
       }
       // restore the extent, gather its pairs
-      for (uint64_t o = 0, x = s0; o < len; o++, x = next_cell(v.t, x)) v.cells[x] = v.snap[x];
+      for (uint64_t o = 0, x = s0; o < len; o++, x = next_cell(v.t, x)) v.cells[x] = v.before(x);
       for (int k = 0; k < ns; k++) {
         for (uint64_t q = lower_bound_region(sorted, n_sorted, starts[k]);
              q < n_sorted && sorted[q] != kNoRegion && (sorted[q] >> kIndexBits) == starts[k]; q++) {
@@ -305,23 +306,28 @@ k2g_status insert_ordered(k2g_db *db, typename C::T *cells, const uint64_t *d_ke
   DevBuf<uint64_t> keys(dev, st), alt(dev, st), flags(dev, st), scratch(dev, st);
   DevBuf<uint32_t> hist(dev, st), sums(dev, st);
   DevBuf<unsigned long long> ctr(dev, st);
-  K2G_CUDA_TRY(snap.alloc(cap));
+  if (!db->blank) K2G_CUDA_TRY(snap.alloc(cap));   // (the first batch of a build needs none)
   K2G_CUDA_TRY(occ.alloc((cap + 31) / 32));
   K2G_CUDA_TRY(status.alloc(1));
   K2G_CUDA_TRY(ctr.alloc(2));
-  K2G_CUDA_TRY(cudaMemcpyAsync(snap.p, cells, cap * sizeof(T), cudaMemcpyDeviceToDevice, st));
+  if (snap.p) K2G_CUDA_TRY(cudaMemcpyAsync(snap.p, cells, cap * sizeof(T), cudaMemcpyDeviceToDevice, st));
+  // 1. unordered pass (validates values and capacity); the memory of the next
+  // steps is mapped while it runs
+  K2G_CUDA_TRY(insert_unordered(db, d_keys, d_taxids, n, status.p, st));
+  K2G_CUDA_TRY(keys.alloc(n));
+  K2G_CUDA_TRY(alt.alloc(n));
+  K2G_CUDA_TRY(hist.alloc(rsort::hist_entries(n)));
+  K2G_CUDA_TRY(sums.alloc(rsort::sum_entries(n) + 1));
+  K2G_CUDA_TRY(flags.alloc(kFlagCap));
+  uint32_t st_word = 0;
+  K2G_CUDA_TRY(cudaMemcpyAsync(&st_word, status.p, 4, cudaMemcpyDeviceToHost, st));
   K2G_CUDA_TRY(cudaStreamSynchronize(st));
-  // 1. unordered pass (validates values and capacity)
-  k2g_status s = k2g_build_insert(db, d_keys, d_taxids, n, 0, st);
+  const k2g_status s = insert_status(st_word);
   if (s != K2G_OK) return s;
   K2G_CUDA_TRY(cudaMemsetAsync(status.p, 0, 4, st));
   K2G_CUDA_TRY(cudaMemsetAsync(ctr.p, 0, 16, st));
   occ_kernel<C><<<grid(db->device, (cap + 31) / 32), 256, 0, st>>>(cells, t, occ.p);
   // 2. cluster of each pair, sorted
-  K2G_CUDA_TRY(keys.alloc(n));
-  K2G_CUDA_TRY(alt.alloc(n));
-  K2G_CUDA_TRY(hist.alloc(rsort::hist_entries(n)));
-  K2G_CUDA_TRY(sums.alloc(rsort::sum_entries(n) + 1));
   OrderedView<C> v{t, cells, snap.p, occ.p, db->d_parent, d_keys, d_taxids, n};
   region_kernel<C><<<grid(db->device, n), 256, 0, st>>>(v, keys.p, status.p);
   note_launches(2);
@@ -332,12 +338,10 @@ k2g_status insert_ordered(k2g_db *db, typename C::T *cells, const uint64_t *d_ke
   // above any cell number)
   K2G_CUDA_TRY(rsort::sort_u64(keys.p, alt.p, n, kIndexBits + bits_of(cap), hist.p, sums.p, st, &sorted, kIndexBits));
   // 3. per-cluster replays
-  K2G_CUDA_TRY(flags.alloc(kFlagCap));
   replay_kernel<C><<<grid(db->device, n), 256, 0, st>>>(v, sorted, n, flags.p, ctr.p);
   note_launches();
   K2G_CUDA_TRY(cudaGetLastError());
   unsigned long long n_flags = 0;
-  uint32_t st_word = 0;
   K2G_CUDA_TRY(cudaMemcpyAsync(&n_flags, ctr.p, 8, cudaMemcpyDeviceToHost, st));
   K2G_CUDA_TRY(cudaMemcpyAsync(&st_word, status.p, 4, cudaMemcpyDeviceToHost, st));
   K2G_CUDA_TRY(cudaStreamSynchronize(st));

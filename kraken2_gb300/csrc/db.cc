@@ -448,6 +448,7 @@ extern "C" k2g_status k2g_db_create(const k2g_index_options *opts, uint64_t capa
   else K2G_CUDA_TRY(cudaMemset(db->d_cells, 0, capacity * sizeof(uint32_t)));
   K2G_CUDA_TRY(cudaMemset(db->d_size, 0, 8));
   db->size = 0;
+  db->blank = true;
   scratch_opened(db->device);
   db->counted = true;
   *out = db.release();

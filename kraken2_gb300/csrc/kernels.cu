@@ -965,7 +965,22 @@ extern "C" k2g_status k2g_build_insert(k2g_db *db, const uint64_t *d_keys, const
   }
   uint32_t *d_status = nullptr;
   K2G_CUDA_TRY(scratch_alloc(reinterpret_cast<void **>(&d_status), 4, db->device, st));
-  K2G_CUDA_TRY(cudaMemsetAsync(d_status, 0, 4, st));
+  uint32_t status = 0;
+  cudaError_t e = insert_unordered(db, d_keys, d_taxids, n, d_status, st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&status, d_status, 4, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  cudaFreeAsync(d_status, st);
+  if (e != cudaSuccess) return cuda_fail(e, "insert_kernel");
+  return insert_status(status);
+}
+
+namespace k2g {
+
+cudaError_t insert_unordered(k2g_db *db, const uint64_t *d_keys, const uint32_t *d_taxids, uint64_t n,
+                             uint32_t *d_status, cudaStream_t st) {
+  const cudaError_t e = cudaMemsetAsync(d_status, 0, 4, st);
+  if (e != cudaSuccess) return e;
+  db->blank = false;
   TableView t = db->table_view();
   uint64_t blocks = std::min<uint64_t>((n + 255) / 256, (uint64_t)sm_count(db->device) * 32);
   const unsigned grid = (unsigned)std::max<uint64_t>(1, blocks);
@@ -977,14 +992,14 @@ extern "C" k2g_status k2g_build_insert(k2g_db *db, const uint64_t *d_keys, const
     insert_kernel<Cell32><<<grid, 256, 0, st>>>(t, db->d_cells, db->d_parent, db->node_count,
                                                 d_keys, d_taxids, n, d_size, d_status);
   note_launches();
-  uint32_t status = 0;
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&status, d_status, 4, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  cudaFreeAsync(d_status, st);
-  if (e != cudaSuccess) return cuda_fail(e, "insert_kernel");
+  return cudaGetLastError();
+}
+
+k2g_status insert_status(uint32_t status) {
   if (status & STATUS_BUILD_FULL) return fail(K2G_ERR_CAPACITY, "compact hash table capacity exceeded");
   if (status & STATUS_BUILD_VALUE)
     return fail(K2G_ERR_ARG, "taxid outside the taxonomy or too wide for the value bits");
   return K2G_OK;
 }
+
+}  // namespace k2g

@@ -93,3 +93,23 @@ def test_list_equals_scan_by_hand(kind, block, sub):
     assert np.array_equal(a[0], b[0]) and a[1] == b[1]
     for x in (db, db1, ref):
         x.close()
+
+
+def test_batches_equal_one_batch():
+    """The second batch starts from a table that is not empty."""
+    rng = np.random.default_rng(5)
+    seqs = library("random", rng)
+    seqs += [s.copy() for s in seqs[-2:]]                                # repeated under other taxa
+    taxa = (np.arange(len(seqs)) + 2).astype(np.uint32)
+    one, two = new_db(len(seqs) + 2), new_db(len(seqs) + 2)
+
+    def add(db, a, b):
+        off = np.concatenate([[0], np.cumsum([len(s) for s in seqs[a:b]])]).astype(np.uint64)
+        return db.build_sequences(np.concatenate(seqs[a:b]), off, taxa[a:b])
+
+    n = add(one, 0, len(seqs))
+    assert add(two, 0, 9) + add(two, 9, 11) + add(two, 11, len(seqs)) == n
+    a, b = one.download(), two.download()
+    assert np.array_equal(a[0], b[0]) and a[1] == b[1]
+    one.close()
+    two.close()
