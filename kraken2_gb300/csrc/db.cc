@@ -135,6 +135,7 @@ k2g_status validate_parents(const uint64_t *parent, uint64_t n) {
 k2g_status upload_parents(k2g_db *db, const uint64_t *parent, uint64_t n) {
   std::vector<uint32_t> p32(n);
   for (uint64_t i = 0; i < n; i++) p32[i] = (uint32_t)parent[i];
+  db->one_root = std::find(p32.begin() + std::min<uint64_t>(n, 2), p32.end(), 0u) == p32.end();
   // Preorder intervals: x is an ancestor of y (or y itself) exactly when y's
   // number lies in x's interval.  parent[i] < i, so one pass from the back
   // gives the subtree sizes and one from the front the numbers.

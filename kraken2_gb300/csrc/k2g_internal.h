@@ -115,6 +115,7 @@ struct k2g_db {
   char *d_names = nullptr;
   uint32_t *d_parent = nullptr;   // node_count entries
   bool blank = false;             // created, and nothing inserted yet: all cells are zero
+  bool one_root = false;          // every taxon but 1 has a parent: no LCA is 0
   uint2 *d_span = nullptr;        // per node: preorder number, one past its subtree's last
                                   // (d_parent follows in the same allocation)
   uint64_t *d_size = nullptr;     // device-side size counter used by builds
@@ -166,10 +167,11 @@ void scratch_closed(int device);
 // Counts each kernel launch issued by the library (k2g_kernel_launches).
 void note_launches(uint64_t n = 1);
 // One round (< 2^30 pairs) of the order-exact build insert (build_ordered.cu).
-// The unordered insert's launch (its status word zeroed first), and what the
-// status word says.
+// The unordered insert's launch (its status word zeroed first; moved, if not
+// null: a bitmap that gets the cells where pairs went past their home), and
+// what the status word says.
 cudaError_t insert_unordered(k2g_db *db, const uint64_t *d_keys, const uint32_t *d_taxids, uint64_t n,
-                             uint32_t *d_status, cudaStream_t st);
+                             uint32_t *d_status, uint32_t *moved, cudaStream_t st);
 k2g_status insert_status(uint32_t status);
 k2g_status build_insert_ordered(k2g_db *db, const uint64_t *d_keys, const uint32_t *d_taxids,
                                 uint64_t n, cudaStream_t st);

@@ -208,7 +208,8 @@ __global__ void scan_kernel(ScanView sv, const uint8_t *bases, const uint64_t *s
 template <class C>
 __device__ __forceinline__ uint32_t insert_lca(const TableView &t, typename C::T *cells,
                                                const uint32_t *parent, uint64_t key,
-                                               uint32_t taxid, uint32_t &added, uint32_t *status) {
+                                               uint32_t taxid, uint32_t &added, uint32_t *status,
+                                               uint32_t *moved) {
   const uint64_t hc = murmur3(key);
   const uint64_t ck = hc >> t.key_shift;
   uint64_t idx = fast_mod(hc, t.div);
@@ -218,14 +219,14 @@ __device__ __forceinline__ uint32_t insert_lca(const TableView &t, typename C::T
     uint32_t v = C::value(cell, t);
     if (!v || C::match(cell, ck, t)) {
       uint32_t want = v ? lca(parent, v, taxid) : taxid;
-      if (v && want == v) return 1;   // already holds the LCA
-      const typename C::T nc = C::make(ck, want, t);
-      const typename C::T prev = atomicCAS(cells + idx, cell, nc);
-      if (prev == cell) {
+      if (!v || want != v) {   // (else it already holds the LCA)
+        const typename C::T nc = C::make(ck, want, t);
+        const typename C::T prev = atomicCAS(cells + idx, cell, nc);
+        if (prev != cell) continue;   // cell changed under us: re-evaluate the same slot
         added += v ? 0u : 1u;
-        return 1;
       }
-      continue;   // cell changed under us: re-evaluate the same slot
+      if (moved && idx != first) atomicOr(&moved[idx >> 5], 1u << (idx & 31));
+      return 1;
     }
     idx = (idx + 1 == t.capacity) ? 0 : idx + 1;
     if (idx == first) {
@@ -238,7 +239,7 @@ __device__ __forceinline__ uint32_t insert_lca(const TableView &t, typename C::T
 template <class C>
 __global__ void insert_kernel(TableView t, typename C::T *cells, const uint32_t *parent,
                               uint64_t node_count, const uint64_t *keys, const uint32_t *taxids,
-                              uint64_t n, unsigned long long *size, uint32_t *status) {
+                              uint64_t n, unsigned long long *size, uint32_t *status, uint32_t *moved) {
   uint32_t added = 0;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
        i += (uint64_t)gridDim.x * blockDim.x) {
@@ -248,7 +249,7 @@ __global__ void insert_kernel(TableView t, typename C::T *cells, const uint32_t 
       atomicOr(status, STATUS_BUILD_VALUE);
       continue;
     }
-    insert_lca<C>(t, cells, parent, keys[i], tx, added, status);
+    insert_lca<C>(t, cells, parent, keys[i], tx, added, status, moved);
   }
   // cells claimed: one addition a warp (one for every cell, all to the same
   // address, was three quarters of this kernel: 16M pairs 1.45 -> 0.35 ms)
@@ -966,7 +967,7 @@ extern "C" k2g_status k2g_build_insert(k2g_db *db, const uint64_t *d_keys, const
   uint32_t *d_status = nullptr;
   K2G_CUDA_TRY(scratch_alloc(reinterpret_cast<void **>(&d_status), 4, db->device, st));
   uint32_t status = 0;
-  cudaError_t e = insert_unordered(db, d_keys, d_taxids, n, d_status, st);
+  cudaError_t e = insert_unordered(db, d_keys, d_taxids, n, d_status, nullptr, st);
   if (e == cudaSuccess) e = cudaMemcpyAsync(&status, d_status, 4, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   cudaFreeAsync(d_status, st);
@@ -977,7 +978,7 @@ extern "C" k2g_status k2g_build_insert(k2g_db *db, const uint64_t *d_keys, const
 namespace k2g {
 
 cudaError_t insert_unordered(k2g_db *db, const uint64_t *d_keys, const uint32_t *d_taxids, uint64_t n,
-                             uint32_t *d_status, cudaStream_t st) {
+                             uint32_t *d_status, uint32_t *moved, cudaStream_t st) {
   const cudaError_t e = cudaMemsetAsync(d_status, 0, 4, st);
   if (e != cudaSuccess) return e;
   db->blank = false;
@@ -987,10 +988,10 @@ cudaError_t insert_unordered(k2g_db *db, const uint64_t *d_keys, const uint32_t 
   unsigned long long *d_size = reinterpret_cast<unsigned long long *>(db->d_size);
   if (db->d_wide)
     insert_kernel<CellWide><<<grid, 256, 0, st>>>(t, db->d_wide, db->d_parent, db->node_count,
-                                                  d_keys, d_taxids, n, d_size, d_status);
+                                                  d_keys, d_taxids, n, d_size, d_status, moved);
   else
     insert_kernel<Cell32><<<grid, 256, 0, st>>>(t, db->d_cells, db->d_parent, db->node_count,
-                                                d_keys, d_taxids, n, d_size, d_status);
+                                                d_keys, d_taxids, n, d_size, d_status, moved);
   note_launches();
   return cudaGetLastError();
 }

@@ -15,9 +15,11 @@ K, L = 35, 31
 TOGGLE = 0xe37e28c4271b5a2d
 
 
-def new_db(nodes, k=K, rv=1, capacity=1_000_003):
-    parent = np.concatenate([[0], np.arange(nodes - 1) // 2]).astype(np.uint64)
-    return k2g.Database.create(k2g.IndexOptions(k, L, 0, TOGGLE, 1, rv, 0), capacity, 20, 12, parent)
+def new_db(nodes, k=K, capacity=1_000_003, key_bits=20, one_root=True):
+    parent = np.arange(nodes, dtype=np.uint64) // 2
+    if not one_root:
+        parent[2] = 0
+    return k2g.Database.create(k2g.IndexOptions(k, L, 0, TOGGLE, 1, 1, 0), capacity, key_bits, 32 - key_bits, parent)
 
 
 def scan(db, bases, k):
@@ -59,7 +61,8 @@ def test_list_equals_scan_by_hand(kind, block, sub):
     rng = np.random.default_rng(block + sub)
     seqs = library(kind, rng)
     nodes = len(seqs) + 2
-    db, db1 = new_db(nodes), new_db(nodes, k=K - 1)
+    one_root = block != 25_000   # (several roots: every pair is sorted and replayed)
+    db, db1 = new_db(nodes, one_root=one_root), new_db(nodes, k=K - 1)
     off = np.concatenate([[0], np.cumsum([len(s) for s in seqs])]).astype(np.uint64)
     taxa = (np.arange(len(seqs)) + 2).astype(np.uint32)
     taxa[-1] = 1
@@ -86,7 +89,7 @@ def test_list_equals_scan_by_hand(kind, block, sub):
             values.append(np.full(len(u), tax, np.uint32))
     keys, values = np.concatenate(keys), np.concatenate(values)
     assert n == len(keys)
-    ref = new_db(nodes)
+    ref = new_db(nodes, one_root=one_root)
     d_k, d_v = to_dev(keys), to_dev(values)
     ref.build_insert(d_k.data_ptr(), d_v.data_ptr(), len(keys), True, torch().cuda.current_stream().cuda_stream)
     a, b = db.download(), ref.download()
@@ -113,3 +116,44 @@ def test_batches_equal_one_batch():
     assert np.array_equal(a[0], b[0]) and a[1] == b[1]
     one.close()
     two.close()
+
+
+@pytest.mark.parametrize("load", [0.05, 0.3, 0.7, 0.95, 1.0])
+@pytest.mark.parametrize("key_bits", [6, 22])            # many and few compacted keys that collide
+@pytest.mark.parametrize("capacity", [33, 1024, 60_001])
+def test_ordered_insert_equals_sequential(load, key_bits, capacity):
+    """Clusters with and without moved pairs, across words and the table's
+    end, in three batches, against a sequential insert."""
+    rng = np.random.default_rng(int(load * 100) + capacity)
+    nodes = 60
+    db = new_db(nodes, capacity=capacity, key_bits=key_bits)
+    distinct = rng.integers(0, 2**62, max(int(capacity * load), 1), dtype=np.int64).astype(np.uint64)
+    keys = distinct[rng.integers(0, len(distinct), 3 * len(distinct) + 5)]
+    keys[:len(distinct)] = distinct
+    taxa = rng.integers(0, nodes, len(keys)).astype(np.uint32)
+    parent = np.arange(nodes) // 2
+    cells = np.zeros(capacity, np.uint32)
+    hc = murmur3_np(keys)
+    size = 0
+    for h, t in zip(hc.tolist(), taxa.tolist()):
+        if not t:
+            continue
+        at, ck = h % capacity, h >> (64 - key_bits)
+        while cells[at] and int(cells[at]) >> (32 - key_bits) != ck:
+            at = (at + 1) % capacity
+        a, b = int(cells[at]) & ((1 << (32 - key_bits)) - 1), t
+        size += not a
+        while a and a != b:
+            a, b = (int(parent[a]), b) if a > b else (a, int(parent[b]))
+        cells[at] = ck << (32 - key_bits) | b
+    st = torch().cuda.current_stream().cuda_stream
+    cut = [0, len(keys) // 3, 2 * len(keys) // 3, len(keys)]
+    if size == capacity:   # a full table is refused by the insert
+        cut = cut[:1]
+    for x, y in zip(cut, cut[1:]):
+        d_k, d_t = to_dev(keys[x:y]), to_dev(taxa[x:y])
+        db.build_insert(d_k.data_ptr(), d_t.data_ptr(), y - x, True, st)
+    if size < capacity:
+        got, n = db.download()
+        assert np.array_equal(got, cells) and n == size
+    db.close()
