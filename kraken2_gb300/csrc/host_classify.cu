@@ -1,9 +1,12 @@
 // k2g_classify_host: classification of reads held in host memory.
 //
-// The input is cut into chunks of about an eighth of the call.  Each chunk is
-// copied in, classified and its results copied out on one of three streams,
-// so its copies overlap the kernels of the others, and the host waits for a
-// chunk only when the two after it are under way.  Hit-list runs are
+// The input is cut into chunks of about a twelfth of the call.  Each chunk has
+// one of three slots, with a stream for its copies in and its classification
+// and one for what follows, so its copies overlap the kernels of the others,
+// and the host waits for a chunk only when the two after it are under way.
+// The second stream has the higher priority: its short kernels would wait
+// behind the classification of the next two chunks, and the slot with them
+// (2M x 150 bp: 3.6 ms, 2.9 with it).  Hit-list runs are
 // compacted on the device (exclusive scan of the per-fragment run counts,
 // then a gather) so only the used runs cross back to the host.
 #include <cuda_runtime.h>
@@ -152,8 +155,10 @@ namespace {
 // calls (grown when a call needs more), so a call allocates nothing once
 // the sizes have been seen.
 struct Slot {
-  cudaStream_t st = nullptr;
-  cudaEvent_t done = nullptr;
+  cudaStream_t st = nullptr, out = nullptr;   // in and classified; counted, compacted and out
+  cudaEvent_t classified = nullptr;
+  cudaEvent_t done = nullptr;      // compacted: the input buffers are free, the number of runs known
+  cudaEvent_t left = nullptr;      // copied out: all are
   char *bases = nullptr, *quals = nullptr;
   uint64_t *off = nullptr;
   uint32_t *call = nullptr, *hg = nullptr, *hlen = nullptr;
@@ -192,8 +197,12 @@ cudaError_t fit_slot(Slot &s, uint64_t bb, uint64_t fb, int per, bool quals, uin
   cudaError_t e;
 #define TRY(x) if ((e = (x)) != cudaSuccess) return e
   if (!s.st) {
+    int low = 0, high = 0;
+    TRY(cudaDeviceGetStreamPriorityRange(&low, &high));
+    for (cudaEvent_t *e1 : {&s.classified, &s.done, &s.left})
+      TRY(cudaEventCreateWithFlags(e1, cudaEventDisableTiming));
+    TRY(cudaStreamCreateWithPriority(&s.out, cudaStreamNonBlocking, high));
     TRY(cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking));
-    TRY(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
     TRY(cudaHostAlloc(&s.h_total, 16, cudaHostAllocDefault));
     TRY(cudaMalloc(&s.total, 16));
     TRY(cudaMalloc(&s.hits_used, 8));
@@ -266,14 +275,17 @@ static k2g_status host_classify(const k2g_db *db, const char *bases, const char 
   K2G_CUDA_TRY(cudaSetDevice(db->device));
   const int per = params->paired ? 2 : 1;
 
-  // Chunk plan: about an eighth of the call (a quarter with hit events, whose
-  // counting makes the host wait), 16 MB of bases at least -- below that a
-  // chunk's launches and copies outweigh what overlaps -- and 128 MB (64 MB
-  // with hit events) or 2M fragments at most.  2M x 150 bp: 8 chunks 3.5 ms,
-  // 2 of 256 MB 5.6.
+  // Chunk plan: about a twelfth of the call (a quarter with hit events, whose
+  // counting makes the host wait), 128 MB (64 MB with hit events) of bases or
+  // 2M fragments at most, and 16 MB at least, 20 where most are long -- below
+  // that a chunk's launches and copies outweigh what overlaps.  2M x 150 bp:
+  // 6 chunks 3.01 ms, 8 2.96, 12 2.89, 16 2.90; 117 MB of mixed long ones: 16
+  // MB 2.81, 20 MB 2.54, 24 MB 2.60; with hit events 1M x 150 bp: 3 to 5
+  // chunks 4.9 to 5.0, 8 5.3.
   const uint64_t all_bases = seq_off[n_frags * per] - seq_off[0];
+  const uint64_t least = (long_batch(all_bases, n_frags) ? 20ull : 16ull) << 20;
   const uint64_t max_bases = std::min<uint64_t>(counters ? 64ull << 20 : 128ull << 20,
-                                                std::max<uint64_t>(16ull << 20, all_bases / (counters ? 4 : 8) + 1)),
+                                                std::max<uint64_t>(least, all_bases / (counters ? 4 : 12) + 1)),
                  max_frags = 2ull << 20;
   std::vector<uint64_t> cuts{0};
   while (cuts.back() < n_frags) {
@@ -334,6 +346,7 @@ static k2g_status host_classify(const k2g_db *db, const char *bases, const char 
     const uint64_t b0 = seq_off[f0 * per], nb = seq_off[(f0 + nf) * per] - b0;
     s.f0 = f0;
     s.nf = nf;
+    K2G_CUDA_TRY(cudaStreamWaitEvent(s.st, s.done, 0));
     if (counters) {
       K2G_CUDA_TRY(cudaMemcpyAsync(s.blocks, frag_block + f0, nf * 4, cudaMemcpyHostToDevice, s.st));
       K2G_CUDA_TRY(cudaMemsetAsync(s.hits_used, 0, 8, s.st));
@@ -355,6 +368,7 @@ static k2g_status host_classify(const k2g_db *db, const char *bases, const char 
     const uint64_t f0 = s.f0, nf = s.nf, b0 = seq_off[f0 * per], nb = seq_off[(f0 + nf) * per] - b0;
     // (after the copies: a kernel waits for the blocks of the chunk before,
     // and copies behind it would too)
+    K2G_CUDA_TRY(cudaStreamWaitEvent(s.st, s.left, 0));
     rebase_kernel<<<(unsigned)((nf * per + 1 + 255) / 256), 256, 0, s.st>>>(s.off, nf * per + 1, b0);
     note_launches();
     s.rd = k2g_reads{};
@@ -385,24 +399,28 @@ static k2g_status host_classify(const k2g_db *db, const char *bases, const char 
     // them only adds interference); long-read chunks overlap their tails
     // (the one-launch form has no state)
     const void *key = long_batch(nb, nf) ? (const void *)s.st : (const void *)&hc;
-    return classify_keyed(db, &s.rd, params, &s.rs, K2G_MODE_PIPELINED, s.st, key);
+    const k2g_status r = classify_keyed(db, &s.rd, params, &s.rs, K2G_MODE_PIPELINED, s.st, key);
+    if (r != K2G_OK) return r;
+    K2G_CUDA_TRY(cudaEventRecord(s.classified, s.st));
+    return K2G_OK;
   };
   // Stage 3: count the events, compact the runs, copy the fixed-size results.
   auto copy_out = [&](size_t c) -> k2g_status {
     Slot &s = slots[c % n_slots];
+    K2G_CUDA_TRY(cudaStreamWaitEvent(s.out, s.classified, 0));
     if (counters) {
-      const k2g_status r = k2g_counters_add(counters, &s.rd, &s.rs, s.st);
+      const k2g_status r = k2g_counters_add(counters, &s.rd, &s.rs, s.out);
       if (r != K2G_OK) return r;
     }
-    const k2g_status r = compact_runs(s.sparse, s.off, per, s.hlen, s.nf, s.excl, s.sums, s.total, s.dense, s.st);
+    const k2g_status r = compact_runs(s.sparse, s.off, per, s.hlen, s.nf, s.excl, s.sums, s.total, s.dense, s.out);
     if (r != K2G_OK) return r;
-    K2G_CUDA_TRY(cudaMemcpyAsync(s.h_total, s.total, 16, cudaMemcpyDeviceToHost, s.st));
-    K2G_CUDA_TRY(cudaEventRecord(s.done, s.st));
-    K2G_CUDA_TRY(cudaMemcpyAsync(call + s.f0, s.call, s.nf * 4, cudaMemcpyDeviceToHost, s.st));
+    K2G_CUDA_TRY(cudaMemcpyAsync(s.h_total, s.total, 16, cudaMemcpyDeviceToHost, s.out));
+    K2G_CUDA_TRY(cudaEventRecord(s.done, s.out));
+    K2G_CUDA_TRY(cudaMemcpyAsync(call + s.f0, s.call, s.nf * 4, cudaMemcpyDeviceToHost, s.out));
     if (hit_groups)
-      K2G_CUDA_TRY(cudaMemcpyAsync(hit_groups + s.f0, s.hg, s.nf * 4, cudaMemcpyDeviceToHost, s.st));
+      K2G_CUDA_TRY(cudaMemcpyAsync(hit_groups + s.f0, s.hg, s.nf * 4, cudaMemcpyDeviceToHost, s.out));
     if (hitlist_len)
-      K2G_CUDA_TRY(cudaMemcpyAsync(hitlist_len + s.f0, s.hlen, s.nf * 4, cudaMemcpyDeviceToHost, s.st));
+      K2G_CUDA_TRY(cudaMemcpyAsync(hitlist_len + s.f0, s.hlen, s.nf * 4, cudaMemcpyDeviceToHost, s.out));
     s.copied = true;
     return K2G_OK;
   };
@@ -418,15 +436,17 @@ static k2g_status host_classify(const k2g_db *db, const char *bases, const char 
     const uint64_t nr = s.h_total[0];
     if (runs) {
       if (runs_written + nr > runs_cap) return fail(K2G_ERR_CAPACITY, "runs buffer too small");
-      K2G_CUDA_TRY(cudaMemcpyAsync(runs + runs_written, s.dense, nr * 8, cudaMemcpyDeviceToHost, s.st));
+      K2G_CUDA_TRY(cudaMemcpyAsync(runs + runs_written, s.dense, nr * 8, cudaMemcpyDeviceToHost, s.out));
     }
+    K2G_CUDA_TRY(cudaEventRecord(s.left, s.out));
     runs_written += nr;
     return K2G_OK;
   };
   auto all_chunks = [&]() -> k2g_status {
     // with counters, stage 3 of a chunk makes the host wait for its kernels:
     // the next chunk's are in the queue and the copies of the one after it on
-    // their way before that (1M x 150 bp: 4.2 -> 2.9 ms)
+    // their way before that (1M x 150 bp: 4.2 -> 2.9 ms
+    // for the classification)
     const size_t lag = counters ? 1 : 0, ahead = counters && n_slots > 2 ? 1 : 0;
     for (size_t c = 0; c < n_chunks + ahead + lag; c++) {
       k2g_status r = K2G_OK;
@@ -449,8 +469,10 @@ static k2g_status host_classify(const k2g_db *db, const char *bases, const char 
   // every copy is done (on an error too: the slots are free for the next call)
   cudaError_t e = cudaSuccess;
   for (int i = 0; i < used; i++) {
-    const cudaError_t es = cudaStreamSynchronize(slots[i].st);
-    if (es != cudaSuccess) e = es;
+    for (cudaStream_t x : {slots[i].st, slots[i].out}) {
+      const cudaError_t es = cudaStreamSynchronize(x);
+      if (es != cudaSuccess) e = es;
+    }
     slots[i].copied = false;
   }
   if (status != K2G_OK) return status;
