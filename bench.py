@@ -947,7 +947,7 @@ def translated_run(log, n_reads: int = 500_000, parity_reads: int = 20_000) -> d
                        "protein fixture (k=15, l=12)",
            "mreads_min": round(n_reads / t * 60 / 1e6, 1),
            "g_bases_per_s": round(n_reads * L / t / 1e9, 3), "s": round(t, 4),
-           "form": "one MODE_PIPELINED call (translated search: one thread per fragment)",
+           "form": "one MODE_PIPELINED call (translated search: a warp per group of fragments)",
            "parity": {"reads": ns, "classified": classified, **_parity(gpu, oo, ns)}}
     log(f"translated: {out['mreads_min']} Mreads/min")
     return out
@@ -1556,13 +1556,13 @@ def random_sector_rate(wl, n_loads: int = 1 << 30) -> dict:
 
 
 # DRAM bytes per 150 bp read of the classification step, from one ncu capture
-# (dram__bytes_read.sum + dram__bytes_write.sum over every beat of one call)
-# of the 2 GB-table / 5M-read case of this workload:
+# (dram__bytes_read.sum + dram__bytes_write.sum of one call's launch) of the
+# 2 GB-table / 5M-read case of this workload:
 #   python bench.py --scale 0.05 --profile  under
 #   ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum
-#       --clock-control none -k regex:pipe_step -s <beats of the first call> -c <beats of one call>
+#       --clock-control none -k regex:warp_classify -s 1 -c 1
 # Traffic grows in proportion to the reads, so it scales to a full call.
-DRAM_BYTES_PER_READ = 7752.0
+DRAM_BYTES_PER_READ = 5776.0
 
 
 def value_counts_run(wl: Workload, reps: int = 5) -> dict:

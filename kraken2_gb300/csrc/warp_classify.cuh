@@ -25,12 +25,12 @@
 //            (src/classify.cc:710-762) needs no walks to the root.
 //
 // What bounds it: on tables beyond L2 the random 32-byte table loads and the
-// integer ALU together (150 bp reads on a 2 GB table: DRAM 59 % busy, ALU pipe
-// 57 %, 730 warp instructions a read); where the table fits L2 the ALU alone.
+// integer ALU together (150 bp reads on a 2 GB table: DRAM 68 % busy, ALU pipe
+// 62 %, 696 warp instructions a read); where the table fits L2 the ALU alone.
 // Against the staged scan / probe / resolve kernels it replaces for such
-// calls: 8M x 150 bp on a 16 GB table 16.56 -> 9.82 ms (37 G sectors/s of the
-// 48 G/s a bare random gather reaches), 500k pairs over related genomes 2.75
-// -> 1.42 ms, 1,000 reads 118 -> 18 us (one launch instead of seven).
+// calls: 8M x 150 bp on a 16 GB table 16.5 -> 9.4 ms (39 G sectors/s of the
+// 49 G/s a bare random gather reaches), 500k pairs over related genomes 2.75
+// -> 1.34 ms, 1,000 reads 118 -> 18 us (one launch instead of seven).
 #pragma once
 
 #include "classify_core.cuh"
