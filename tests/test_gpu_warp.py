@@ -132,7 +132,7 @@ def test_edge_lengths_equal_the_oracle(params, wide, many):
     check(db, o, bases, q, off, len(lens) // (2 if params.get("paired") else 1), params)
 
 
-@pytest.mark.parametrize("n,hi", [(3_800, 200), (9_000, 260), (16_000, 200), (40_001, 190), (40_000, 36)])
+@pytest.mark.parametrize("n,hi", [(3_800, 200), (5_000, 330), (9_000, 260), (16_000, 200), (40_001, 190), (40_000, 36)])
 @pytest.mark.parametrize("paired", [False, True])
 def test_groups_of_several_fragments_equal_the_oracle(n, hi, paired):
     """Calls large enough that a warp takes 1, 2, 4 and 8 fragments."""
