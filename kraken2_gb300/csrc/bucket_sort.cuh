@@ -200,48 +200,29 @@ bucket_sort_kernel(const uint32_t *start, uint64_t *keys, uint32_t lo, uint32_t 
   }
 }
 
-// Keys are dealt into buckets, by the bits from `shift` up, by two kernels, each
-// thread block on one slice of the keys with a counter per bucket in shared
-// memory (a global atomic per key, counting and dealing, took 0.50 ms each for
-// 28M keys): the first adds up the buckets' sizes, the second takes a place in
-// every bucket for its slice's keys and then writes them there, in any order.
-// The second is bound by these writes, a sector each (0.50 ms; the first
-// 0.04).
+// Keys are dealt into buckets by the bits from `shift` up.  A pass over slices
+// of the keys with a counter per bucket in shared memory counts them (a global
+// atomic per key took 0.50 ms for 28M keys, this 0.04).  Then they are dealt
+// to at most 2^kDealDigit places at a time -- in two steps where there are
+// more buckets -- tile by tile: a tile's keys are put in the order of their
+// places in shared memory and written out run by run.  (Straight to 2^13
+// buckets, a random sector a key, took 0.57 ms for 28M keys; 0.21 both steps.)
 constexpr int kDealThreads = 1024;
 constexpr int kDealBits = 15;   // 2^15 counters are 128 KB
-
-__device__ __forceinline__ void count_slice(const uint64_t *k, uint64_t i0, uint64_t i1, int shift, uint32_t nb,
-                                            uint32_t *h) {
-  for (uint32_t b = threadIdx.x; b < nb; b += kDealThreads) h[b] = 0;
-  __syncthreads();
-#pragma unroll 4
-  for (uint64_t i = i0 + threadIdx.x; i < i1; i += kDealThreads) atomicAdd(&h[k[i] >> shift], 1u);
-  __syncthreads();
-}
+constexpr int kDealDigit = 7, kDealDigitMost = kDealBits - kDealDigit;
+constexpr int kDealPer = 8, kDealTile = kDealThreads * kDealPer;
 
 __global__ void __launch_bounds__(kDealThreads)
 bucket_count_kernel(const uint64_t *k, uint64_t n, uint64_t slice, int shift, uint32_t nb, uint32_t *count) {
   extern __shared__ uint32_t h[];
   const uint64_t i0 = min(n, blockIdx.x * slice), i1 = min(n, i0 + slice);
-  count_slice(k, i0, i1, shift, nb, h);
-  for (uint32_t b = threadIdx.x; b < nb; b += kDealThreads)
-    if (h[b]) atomicAdd(&count[b], h[b]);
-}
-
-__global__ void __launch_bounds__(kDealThreads)
-bucket_deal_kernel(const uint64_t *k, uint64_t n, uint64_t slice, int shift, uint32_t nb, uint32_t *cursor,
-                   uint64_t *out) {
-  extern __shared__ uint32_t h[];
-  const uint64_t i0 = min(n, blockIdx.x * slice), i1 = min(n, i0 + slice);
-  count_slice(k, i0, i1, shift, nb, h);
-  for (uint32_t b = threadIdx.x; b < nb; b += kDealThreads)
-    if (h[b]) h[b] = atomicAdd(&cursor[b], h[b]);
+  for (uint32_t b = threadIdx.x; b < nb; b += kDealThreads) h[b] = 0;
   __syncthreads();
 #pragma unroll 4
-  for (uint64_t i = i0 + threadIdx.x; i < i1; i += kDealThreads) {
-    const uint64_t x = k[i];
-    out[atomicAdd(&h[x >> shift], 1u)] = x;
-  }
+  for (uint64_t i = i0 + threadIdx.x; i < i1; i += kDealThreads) atomicAdd(&h[k[i] >> shift], 1u);
+  __syncthreads();
+  for (uint32_t b = threadIdx.x; b < nb; b += kDealThreads)
+    if (h[b]) atomicAdd(&count[b], h[b]);
 }
 
 __global__ void bucket_largest_kernel(const uint32_t *count, uint32_t n, uint32_t *largest) {
@@ -249,6 +230,76 @@ __global__ void bucket_largest_kernel(const uint32_t *count, uint32_t n, uint32_
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) m = max(m, count[i]);
   m = __reduce_max_sync(0xffffffffu, m);
   if ((threadIdx.x & 31) == 0) atomicMax(largest, m);
+}
+
+// First places of the `n` groups of `per` buckets.
+__global__ void bucket_cursor_kernel(const uint32_t *start, uint32_t per, uint32_t n, uint32_t *cursor) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) cursor[i] = start[i * per];
+}
+
+// Parent p holds keys[start[p * per], start[(p + 1) * per]); its keys go to the
+// `digits` (a power of two) cursors cursor[p * digits ..] by the bits from
+// shift up.  Block b works on parent b % parents.
+__global__ void __launch_bounds__(kDealThreads)
+bucket_deal_kernel(const uint64_t *keys, const uint32_t *start, uint32_t parents, uint32_t per, int shift,
+                   uint32_t digits, uint32_t *cursor, uint64_t *out) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  uint64_t *s_key = reinterpret_cast<uint64_t *>(smem);
+  constexpr int kMost = 1 << (kDealDigit > kDealDigitMost ? kDealDigit : kDealDigitMost);
+  __shared__ uint32_t s_count[kMost], s_first[kMost], s_warp[kMost / 32];
+  const uint32_t tid = threadIdx.x, lane = tid & 31, p = blockIdx.x % parents;
+  const uint32_t lo = start[p * per], hi = start[(p + 1) * per];
+  const uint64_t stride = (uint64_t)(gridDim.x / parents) * kDealTile;
+  for (uint64_t t0 = lo + (uint64_t)(blockIdx.x / parents) * kDealTile; t0 < hi; t0 += stride) {
+    const uint32_t n = (uint32_t)min((uint64_t)kDealTile, hi - t0);
+    __syncthreads();   // (the tile before is done with)
+    if (tid < digits) s_count[tid] = 0;
+    __syncthreads();
+    uint64_t x[kDealPer];
+    uint32_t at[kDealPer];
+#pragma unroll
+    for (int u = 0; u < kDealPer; u++) {
+      const uint32_t i = u * kDealThreads + tid;
+      if (i < n) x[u] = keys[t0 + i];
+    }
+#pragma unroll
+    for (int u = 0; u < kDealPer; u++)
+      if (u * kDealThreads + tid < n) at[u] = atomicAdd(&s_count[(uint32_t)(x[u] >> shift) & (digits - 1)], 1u);
+    __syncthreads();
+    // where each digit's keys lie in the tile (s_first) and, less that, go to
+    uint32_t c = 0, incl = 0;
+    if (tid < kMost) {
+      c = tid < digits ? s_count[tid] : 0;
+      incl = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if ((int)lane >= o) incl += y;
+      }
+      if (lane == 31) s_warp[tid >> 5] = incl;
+    }
+    __syncthreads();
+    if (tid < digits) {
+      uint32_t first = incl - c;
+      for (uint32_t w = 0; w < tid >> 5; w++) first += s_warp[w];
+      s_first[tid] = first;
+      s_count[tid] = (c ? atomicAdd(&cursor[p * digits + tid], c) : 0u) - first;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kDealPer; u++)
+      if (u * kDealThreads + tid < n) s_key[s_first[(uint32_t)(x[u] >> shift) & (digits - 1)] + at[u]] = x[u];
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kDealPer; u++) {
+      const uint32_t i = u * kDealThreads + tid;
+      if (i < n) {
+        const uint64_t v = s_key[i];
+        out[s_count[(uint32_t)(v >> shift) & (digits - 1)] + i] = v;   // (modulo 2^32)
+      }
+    }
+  }
 }
 
 // Keys to a bucket, where the number of buckets is free: 2,250 to kBucketKeys,
@@ -268,30 +319,41 @@ struct BucketMem {
       : nb(n), start(mem), largest(start + n + 1), place(largest + 1), distinct(place + n + 1), sums(distinct + n) {}
 };
 
-// Deals keys[0, n) (n < 2^32, each key >> shift below nb <= 2^15) to out, bucket
-// b at start[b]; got: how many were dealt, and the largest bucket.
-inline cudaError_t deal_to_buckets(const uint64_t *keys, uint64_t n, int shift, const BucketMem &m, int device,
-                                   uint64_t *out, uint32_t got[2], cudaStream_t st) {
+// Deals keys[0, n) (n < 2^32, each key >> shift below nb = 2^bits, bits <=
+// kDealBits) into buckets, bucket b at start[b]: in alt, or back in keys where
+// that took two steps (*dealt).  *largest: the largest bucket.
+inline cudaError_t deal_to_buckets(uint64_t *keys, uint64_t *alt, uint64_t n, int shift, int bits, const BucketMem &m,
+                                   int device, uint64_t **dealt, uint32_t *largest, cudaStream_t st) {
   cudaError_t e;
 #define TRY(x) if ((e = (x)) != cudaSuccess) return e
   int sms = 0;
   TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
   // (a slice of several keys per counter)
   const uint64_t slice = std::max<uint64_t>((n + sms - 1) / sms, 4096);
-  const unsigned g = (unsigned)((n + slice - 1) / slice);
-  const int smem = (int)(m.nb * 4);
   TRY(cudaFuncSetAttribute(bucket_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 << kDealBits));
-  TRY(cudaFuncSetAttribute(bucket_deal_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 << kDealBits));
+  TRY(cudaFuncSetAttribute(bucket_deal_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDealTile * 8));
   TRY(cudaMemsetAsync(m.start, 0, (m.nb + 2) * 4ull, st));
-  bucket_count_kernel<<<g, kDealThreads, smem, st>>>(keys, n, slice, shift, m.nb, m.start);
+  bucket_count_kernel<<<(unsigned)((n + slice - 1) / slice), kDealThreads, m.nb * 4, st>>>(keys, n, slice, shift, m.nb,
+                                                                                         m.start);
   bucket_largest_kernel<<<(m.nb + 255) / 256, 256, 0, st>>>(m.start, m.nb, m.largest);
   note_launches(2);
   TRY(rsort::exclusive_scan(m.start, m.nb + 1, m.sums, st));
-  TRY(cudaMemcpyAsync(m.place, m.start, m.nb * 4ull, cudaMemcpyDeviceToDevice, st));
-  bucket_deal_kernel<<<g, kDealThreads, smem, st>>>(keys, n, slice, shift, m.nb, m.place, out);
-  note_launches();
+  const int low = bits > kDealDigit ? bits - kDealDigit : 0;   // bits left for the second step
+  auto step = [&](const uint64_t *in, uint64_t *out, uint32_t parents, int digit_bits, int at) {
+    const uint32_t digits = 1u << digit_bits, cursors = parents * digits;
+    bucket_cursor_kernel<<<(cursors + 255) / 256, 256, 0, st>>>(m.start, m.nb / cursors, cursors, m.place);
+    // (two blocks to an SM, and a few for every parent)
+    const uint64_t tiles = n / parents / kDealTile + 1;
+    const uint32_t each = (uint32_t)std::min<uint64_t>(tiles, (2 * sms + parents - 1) / parents);
+    bucket_deal_kernel<<<parents * each, kDealThreads, kDealTile * 8, st>>>(in, m.start, parents, m.nb / parents, at,
+                                                                            digits, m.place, out);
+    note_launches(2);
+  };
+  step(keys, alt, 1, bits - low, shift + low);
+  if (low) step(alt, keys, 1u << kDealDigit, low, shift);
+  *dealt = low ? keys : alt;
   TRY(cudaGetLastError());
-  TRY(cudaMemcpyAsync(got, m.start + m.nb, 8, cudaMemcpyDeviceToHost, st));
+  TRY(cudaMemcpyAsync(largest, m.largest, 4, cudaMemcpyDeviceToHost, st));
 #undef TRY
   return cudaStreamSynchronize(st);
 }

@@ -554,20 +554,25 @@ k2g_status compact_acc(k2g_counters *c, cudaStream_t st) {
     K2G_CUDA_TRY(scratch_alloc(reinterpret_cast<void **>(&mem), BucketMem::words(nb) * 4, c->device, st));
     const BucketMem m(mem, nb);
     auto by_buckets = [&]() -> k2g_status {
-      uint32_t got[2] = {0, 0};
-      K2G_CUDA_TRY(deal_to_buckets(c->d_acc, total, shift, m, c->device, c->d_alt, got, st));
-      if (got[1] > kLargeBlock) return K2G_OK;
-      K2G_CUDA_TRY(bucket_sort(m.start, nb, got[1], c->d_alt, m.distinct, ZoneBits{shift - 12}, st));
+      uint64_t *dealt = nullptr;
+      uint32_t largest = 0, got = 0;
+      K2G_CUDA_TRY(deal_to_buckets(c->d_acc, c->d_alt, total, shift, bits, m, c->device, &dealt, &largest, st));
+      if (largest > kLargeBlock) return K2G_OK;
+      K2G_CUDA_TRY(bucket_sort(m.start, nb, largest, dealt, m.distinct, ZoneBits{shift - 12}, st));
       K2G_CUDA_TRY(cudaMemcpyAsync(m.place, m.distinct, nb * 4ull, cudaMemcpyDeviceToDevice, st));
       K2G_CUDA_TRY(cudaMemsetAsync(m.place + nb, 0, 4, st));
       K2G_CUDA_TRY(rsort::exclusive_scan(m.place, nb + 1, m.sums, st));
-      bucket_pack_kernel<<<(unsigned)((nb * 32ull + 255) / 256), 256, 0, st>>>(m.start, c->d_alt, m.distinct, m.place, nb,
+      if (dealt == c->d_acc) {
+        std::swap(c->d_acc, c->d_alt);
+        std::swap(c->acc_cap, c->alt_cap);
+      }
+      bucket_pack_kernel<<<(unsigned)((nb * 32ull + 255) / 256), 256, 0, st>>>(m.start, dealt, m.distinct, m.place, nb,
                                                                               c->d_acc);
       note_launches();
       K2G_CUDA_TRY(cudaGetLastError());
-      K2G_CUDA_TRY(cudaMemcpyAsync(got, m.place + nb, 4, cudaMemcpyDeviceToHost, st));
+      K2G_CUDA_TRY(cudaMemcpyAsync(&got, m.place + nb, 4, cudaMemcpyDeviceToHost, st));
       K2G_CUDA_TRY(cudaStreamSynchronize(st));
-      n = got[0];
+      n = got;
       sorted = true;
       return K2G_OK;
     };
