@@ -507,7 +507,8 @@ k2g_status gather(const k2g_db *db, const char *bases, const uint64_t *seq_off,
   // Random sequence has a new minimizer every three bases (window 5): room for
   // as many is mapped while the bases are copied and counted.
   uint64_t *guess = nullptr;
-  const uint64_t guessed = total / 3 + total / 64 + 1024;
+  const uint64_t share = sample_below ? sample_below : 1024;   // (of 1,024 minimizers, those kept)
+  const uint64_t guessed = (total / 3 + total / 64) / 1024 * share + 4096;
   if (by_warps && s.get(&guess, guessed) != cudaSuccess) cudaGetLastError();
   K2G_CUDA_TRY(cudaMemcpyAsync(d_offs, d_counts, nc * 4, cudaMemcpyDeviceToDevice, st));
   K2G_CUDA_TRY(rsort::exclusive_scan(d_offs, nc, d_sums, st));
