@@ -73,18 +73,19 @@ __global__ void scan_sums_kernel(uint64_t *sums, uint64_t nb, uint64_t *total) {
   if (threadIdx.x == 0) *total = carry;
 }
 
-// Adds block offsets and gathers each fragment's runs into the dense array: a
-// thread copies a short list, a warp the long ones of its 32 fragments one
-// after another (a thread each for all took 0.72 ms for 120k fragments of up
-// to 50 kb).
+// Adds block offsets and gathers each fragment's runs into the dense array.  A
+// warp takes `each` fragments: a thread copies a short list, the warp the long
+// ones one after another.  (A thread for every list took 0.72 ms for 120k
+// fragments of up to 50 kb.  4 fragments a warp where most bases are in long
+// ones, not 32, which are six long lists: that host call 2.38 -> 2.32 ms.)
 constexpr uint32_t kShortList = 16;
 
 __global__ void gather_runs_kernel(const uint64_t *sparse, const uint64_t *seq_off, int per,
-                                   const uint32_t *len, uint64_t *excl, const uint64_t *sums,
-                                   uint64_t n, uint64_t *dense) {
-  const uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+                                   const uint32_t *len, const uint64_t *excl, const uint64_t *sums,
+                                   uint64_t n, uint32_t each, uint64_t *dense) {
   const uint32_t lane = threadIdx.x & 31;
-  const bool in = i < n;
+  const uint64_t i = ((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5) * each + lane;
+  const bool in = i < n && lane < each;
   const uint32_t m = in ? len[i] : 0;
   const uint64_t to = in ? excl[i] + sums[i / kScanBlock] : 0, from = in ? seq_off[i * per] + 2 * i : 0;
   if (m <= kShortList)
@@ -134,13 +135,14 @@ k2g_status exclusive_scan_u32(const uint32_t *d_in, uint64_t n, uint64_t *d_out,
 
 k2g_status compact_runs(const uint64_t *d_sparse, const uint64_t *d_seq_off, int per,
                         const uint32_t *d_len, uint64_t n, uint64_t *d_excl, uint64_t *d_sums,
-                        uint64_t *d_total, uint64_t *d_dense, cudaStream_t st) {
+                        uint64_t *d_total, uint64_t *d_dense, bool long_lists, cudaStream_t st) {
   uint64_t nb = (n + kScanBlock - 1) / kScanBlock;
   scan_blocks_kernel<<<(unsigned)nb, kScanBlock, 0, st>>>(d_len, d_excl, d_sums, n);
   scan_sums_kernel<<<1, kScanBlock, 0, st>>>(d_sums, nb, d_total);
   note_launches(3);
-  gather_runs_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(d_sparse, d_seq_off, per, d_len,
-                                                                 d_excl, d_sums, n, d_dense);
+  const uint32_t each = long_lists ? 4 : 32;
+  gather_runs_kernel<<<(unsigned)((n + 8 * each - 1) / (8 * each)), 256, 0, st>>>(d_sparse, d_seq_off, per, d_len, d_excl,
+                                                                                d_sums, n, each, d_dense);
   K2G_CUDA_TRY(cudaGetLastError());
   return K2G_OK;
 }
@@ -415,7 +417,8 @@ static k2g_status host_classify(const k2g_db *db, const char *bases, const char 
       const k2g_status r = k2g_counters_add(counters, &s.rd, &s.rs, s.out);
       if (r != K2G_OK) return r;
     }
-    const k2g_status r = compact_runs(s.sparse, s.off, per, s.hlen, s.nf, s.excl, s.sums, s.total, s.dense, s.out);
+    const k2g_status r = compact_runs(s.sparse, s.off, per, s.hlen, s.nf, s.excl, s.sums, s.total, s.dense,
+                                      long_batch(s.rd.total_bases, s.nf), s.out);
     if (r != K2G_OK) return r;
     K2G_CUDA_TRY(cudaMemcpyAsync(s.h_total, s.total, 16, cudaMemcpyDeviceToHost, s.out));
     K2G_CUDA_TRY(cudaEventRecord(s.done, s.out));

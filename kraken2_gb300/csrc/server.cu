@@ -33,7 +33,7 @@
 namespace k2g {
 k2g_status compact_runs(const uint64_t *d_sparse, const uint64_t *d_seq_off, int per,
                         const uint32_t *d_len, uint64_t n, uint64_t *d_excl, uint64_t *d_sums,
-                        uint64_t *d_total, uint64_t *d_dense, cudaStream_t st);
+                        uint64_t *d_total, uint64_t *d_dense, bool long_lists, cudaStream_t st);
 }
 
 namespace {
@@ -258,7 +258,7 @@ k2g_status launch(k2g_server *sv, Slot &s) {
   k2g_status st = classify_keyed(sv->db, &rd, &sv->params, &rs, K2G_MODE_PIPELINED, s.st, key);
   if (st != K2G_OK) return st;
   st = compact_runs(s.d_sparse, s.d_off, sv->per, s.d_hlen, fb, s.d_excl, s.d_sums, s.d_total,
-                    s.d_dense, s.st);
+                    s.d_dense, long_batch(bb, fb), s.st);
   if (st != K2G_OK) return st;
   K2G_CUDA_TRY(cudaMemcpyAsync(s.h_total, s.d_total, 8, cudaMemcpyDeviceToHost, s.st));
   K2G_CUDA_TRY(cudaMemcpyAsync(s.h_call, s.d_call, fb * 4, cudaMemcpyDeviceToHost, s.st));
