@@ -575,6 +575,7 @@ struct k2g_text {
   DBuf<char> text[2];             // kraken lines of the last two calls
   int text_cur = 0;               // the buffer of the last call
   cudaStream_t fetch_st = nullptr;
+  cudaEvent_t parsed = nullptr;   // the last call's counts are on the host
   cudaEvent_t text_free[2] = {nullptr, nullptr};   // the last copy out of each buffer
   DBuf<ParseInfo> info;
   ParseInfo *h_info = nullptr;    // pinned
@@ -623,6 +624,7 @@ k2g_status text_alloc(k2g_text *t) {
   K2G_CUDA_TRY(t->hits_used.need(1));
   K2G_CUDA_TRY(cudaStreamCreateWithFlags(&t->copy_st, cudaStreamNonBlocking));
   K2G_CUDA_TRY(cudaStreamCreateWithFlags(&t->fetch_st, cudaStreamNonBlocking));
+  K2G_CUDA_TRY(cudaEventCreateWithFlags(&t->parsed, cudaEventDisableTiming));
   for (auto &e : t->text_free) K2G_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   for (auto &a : t->ahead) K2G_CUDA_TRY(cudaEventCreateWithFlags(&a.done, cudaEventDisableTiming));
   return K2G_OK;
@@ -641,6 +643,7 @@ void text_free(k2g_text *t) {
   if (t->copy_st) cudaStreamSynchronize(t->copy_st);
   if (t->fetch_st) cudaStreamSynchronize(t->fetch_st);
   for (auto &b : t->text) b.free();
+  if (t->parsed) cudaEventDestroy(t->parsed);
   for (auto &e : t->text_free)
     if (e) cudaEventDestroy(e);
   if (t->fetch_st) cudaStreamDestroy(t->fetch_st);
@@ -783,15 +786,17 @@ extern "C" k2g_status k2g_text_classify(k2g_text *t, const char *chunk, uint64_t
   note_launches(8);
   K2G_CUDA_TRY(cudaGetLastError());
   K2G_CUDA_TRY(cudaMemcpyAsync(t->h_info, info, sizeof(ParseInfo), cudaMemcpyDeviceToHost, st));
-  K2G_CUDA_TRY(cudaStreamSynchronize(st));
+  K2G_CUDA_TRY(cudaEventRecord(t->parsed, st));
+  // 5. gather (while the host learns of the counts), classify, count and format
+  gather_kernel<<<grid_for(t, (W / 256 + 1) * 32, 256), 256, 0, st>>>(wd, t->contrib.p, t->line_pos.p, t->rec_line.p,
+                                                                      t->params.min_quality, t->bases.p);
+  note_launches();
+  K2G_CUDA_TRY(cudaGetLastError());
+  K2G_CUDA_TRY(cudaEventSynchronize(t->parsed));
   const ParseInfo pi = *t->h_info;
   if (pi.too_many) return hand_off(0);   // lines too short for the buffers
   const uint64_t nf = pi.n_frags;
-  // 5. gather, classify, count and format
   if (nf) {
-    gather_kernel<<<grid_for(t, pi.n_take * 32, 256), 256, 0, st>>>(
-        wd, t->contrib.p, t->line_pos.p, t->rec_line.p, t->params.min_quality, t->bases.p);
-    note_launches();
     k2g_classify_params cp = t->params;
     cp.min_quality = 0;   // masked while gathering
     k2g_reads rd{};
