@@ -40,6 +40,7 @@ struct LinesView {
   const uint64_t *ext;         // external id per internal taxon
   const uint64_t *name_off;    // scientific name of taxon t at names + name_off[t]
   const char *names;
+  unsigned long long *classified;   // fragments with a call are added to it (may be null)
   uint64_t n;
   int paired, interleaved, quick, print_names;
 };
@@ -209,9 +210,14 @@ constexpr int kThreads = 256;
 constexpr uint32_t kStage = 4096;   // bytes of a warp's lines in shared memory
 
 static __global__ void line_len_kernel(LinesView v, uint32_t *len) {
+  uint32_t calls = 0;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < v.n;
-       i += (uint64_t)gridDim.x * blockDim.x)
+       i += (uint64_t)gridDim.x * blockDim.x) {
     len[i] = (uint32_t)line<false>(v, i, nullptr);
+    calls += v.call[i] != 0;
+  }
+  calls = __reduce_add_sync(0xffffffffu, calls);
+  if (v.classified && (threadIdx.x & 31) == 0 && calls) atomicAdd(v.classified, (unsigned long long)calls);
 }
 
 // Line i goes to text + off[i] + sums[i / 1024] (block_scan_u32 of the

@@ -832,9 +832,11 @@ extern "C" k2g_status k2g_text_classify(k2g_text *t, const char *chunk, uint64_t
       s = k2g_counters_add(counters, &rd, &rs, st);
       if (s != K2G_OK) return s;
     }
-    count_classified_kernel<<<grid_for(t, nf, 256), 256, 0, st>>>(t->call.p, info);
-    note_launches();
-    K2G_CUDA_TRY(cudaGetLastError());
+    if (!t->cfg.lines) {   // (line_len_kernel counts them too)
+      count_classified_kernel<<<grid_for(t, nf, 256), 256, 0, st>>>(t->call.p, info);
+      note_launches();
+      K2G_CUDA_TRY(cudaGetLastError());
+    }
     lines::LinesView v{};
     const unsigned g = grid_for(t, nf, lines::kThreads);
     const int c = t->text_cur ^ 1;   // the other buffer than the last call's
@@ -859,6 +861,7 @@ extern "C" k2g_status k2g_text_classify(k2g_text *t, const char *chunk, uint64_t
       v.n_runs = t->runs.cap;
       v.node_count = t->db->node_count;
       v.bad = &info->bad;
+      v.classified = &info->classified;
       v.ext = t->db->d_ext;
       v.name_off = t->db->d_name_off;
       v.names = t->db->d_names;
