@@ -159,6 +159,15 @@ k2g_status upload_parents(k2g_db *db, const uint64_t *parent, uint64_t n) {
   return K2G_OK;
 }
 
+// A handle's tables are cleared and copied on the legacy stream, by calls that
+// may return before the device is done (cudaMemset, copies from pageable
+// memory).  Callers' streams need not wait for that stream, so a call that
+// hands a table out waits here.
+k2g_status legacy_stream_done() {
+  K2G_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
+  return K2G_OK;
+}
+
 k2g_status upload_names(k2g_db *db, const std::vector<uint64_t> &ext,
                         const std::vector<uint64_t> &name_off, const std::vector<char> &names) {
   K2G_CUDA_TRY(cudaMalloc(&db->d_ext, ext.size() * 8));
@@ -167,7 +176,7 @@ k2g_status upload_names(k2g_db *db, const std::vector<uint64_t> &ext,
   K2G_CUDA_TRY(cudaMemcpy(db->d_name_off, name_off.data(), name_off.size() * 8, cudaMemcpyHostToDevice));
   K2G_CUDA_TRY(cudaMalloc(&db->d_names, names.size()));
   K2G_CUDA_TRY(cudaMemcpy(db->d_names, names.data(), names.size(), cudaMemcpyHostToDevice));
-  return K2G_OK;
+  return legacy_stream_done();
 }
 
 k2g_status alloc_table(k2g_db *db, uint64_t capacity) {
@@ -412,6 +421,8 @@ extern "C" k2g_status k2g_db_open(const char *hash_k2d, const char *taxo_k2d,
   }
   ce = cudaMemcpy(db->d_size, &db->size, 8, cudaMemcpyHostToDevice);
   if (ce != cudaSuccess) { destroy(db.release()); return cuda_fail(ce, "size upload"); }
+  s = legacy_stream_done();
+  if (s != K2G_OK) { destroy(db.release()); return s; }
   scratch_opened(db->device);
   db->counted = true;
   *out = db.release();
@@ -441,13 +452,18 @@ extern "C" k2g_status k2g_db_create(const k2g_index_options *opts, uint64_t capa
   db->key_bits = key_bits;
   db->value_bits = value_bits;
   db->cell_bytes = key_bits + value_bits == 40 ? 5 : 4;
-  s = upload_parents(db.get(), parent, node_count);
+  auto fill = [&]() -> k2g_status {
+    k2g_status r = alloc_table(db.get(), capacity);
+    if (r != K2G_OK) return r;
+    if (db->d_wide) K2G_CUDA_TRY(cudaMemset(db->d_wide, 0, capacity * 8));
+    else K2G_CUDA_TRY(cudaMemset(db->d_cells, 0, capacity * sizeof(uint32_t)));
+    K2G_CUDA_TRY(cudaMemset(db->d_size, 0, 8));
+    // (prepared on the host while the cells are cleared)
+    r = upload_parents(db.get(), parent, node_count);
+    return r != K2G_OK ? r : legacy_stream_done();
+  };
+  s = fill();
   if (s != K2G_OK) { destroy(db.release()); return s; }
-  s = alloc_table(db.get(), capacity);
-  if (s != K2G_OK) { destroy(db.release()); return s; }
-  if (db->d_wide) K2G_CUDA_TRY(cudaMemset(db->d_wide, 0, capacity * 8));
-  else K2G_CUDA_TRY(cudaMemset(db->d_cells, 0, capacity * sizeof(uint32_t)));
-  K2G_CUDA_TRY(cudaMemset(db->d_size, 0, 8));
   db->size = 0;
   db->blank = true;
   scratch_opened(db->device);
