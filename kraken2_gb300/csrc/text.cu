@@ -617,7 +617,8 @@ k2g_status text_alloc(k2g_text *t) {
   K2G_CUDA_TRY(t->hlen.need(t->rec_cap));
   K2G_CUDA_TRY(t->runs.need(W + 2 * t->rec_cap + 8));
   K2G_CUDA_TRY(t->taxon_reads.need(t->db->node_count));
-  K2G_CUDA_TRY(cudaMemset(t->taxon_reads.p, 0, t->db->node_count * 8));
+  // (on the stream of the calls that count: it does not wait for another)
+  K2G_CUDA_TRY(cudaMemsetAsync(t->taxon_reads.p, 0, t->db->node_count * 8, t->st));
   K2G_CUDA_TRY(t->line_len.need(t->rec_cap));
   K2G_CUDA_TRY(t->line_off.need(t->rec_cap));
   K2G_CUDA_TRY(t->info.need(1));

@@ -34,3 +34,19 @@ def test_an_opened_table_is_loaded_when_the_call_returns(name):
         assert f.pending() == 0
         db.close()
         assert f.faults() == []
+
+
+def text_reader(db, **kw):
+    return k2g.TextReader(db, k2g.ClassifyParams(0.1, 2, 0, 0, 0), chunk_cap=1 << 16, **kw)
+
+
+def test_a_new_text_reader_leaves_nothing_on_the_legacy_stream():
+    """(its per-taxon counts are cleared there or on its own stream, which its
+    kernels run on)"""
+    with fake_cuda() as f:
+        db = k2g.Database.open(os.path.join(GOLDEN, "db_a"))
+        t = text_reader(db)
+        assert f.pending() == 0
+        t.close()
+        db.close()
+        assert f.faults() == []
