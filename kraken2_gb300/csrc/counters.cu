@@ -700,7 +700,9 @@ extern "C" k2g_status k2g_counters_create(const k2g_db *db, k2g_counters **out) 
   std::copy(node_of.begin(), node_of.end(), all.begin() + 2 * n);
   if (e != cudaSuccess || (e = cudaMemset(mem, 0, tables)) != cudaSuccess ||
       (e = cudaMemset(c->d_dense, 0, n)) != cudaSuccess ||
-      (e = cudaMemcpy(c->d_pre, all.data(), 12 * n, cudaMemcpyHostToDevice)) != cudaSuccess)
+      (e = cudaMemcpy(c->d_pre, all.data(), 12 * n, cudaMemcpyHostToDevice)) != cudaSuccess ||
+      // (callers' streams need not wait for this one)
+      (e = cudaStreamSynchronize(cudaStreamLegacy)) != cudaSuccess)
     return bad(cuda_fail(e, "counter set-up"));
   // a quarter of the free memory for the accumulator and its sort buffer
   size_t free_b = 0, total_b = 0;

@@ -50,3 +50,13 @@ def test_a_new_text_reader_leaves_nothing_on_the_legacy_stream():
         t.close()
         db.close()
         assert f.faults() == []
+
+
+def test_new_counters_are_ready_when_the_call_returns():
+    with fake_cuda() as f:
+        db = k2g.Database.open(os.path.join(GOLDEN, "db_a"))
+        c = k2g.Counters(db)
+        assert f.pending() == 0
+        c.close()
+        db.close()
+        assert f.faults() == []
