@@ -498,7 +498,8 @@ k2g_status insert_ordered(k2g_db *db, typename C::T *cells, const uint64_t *d_ke
     K2G_CUDA_TRY(cudaMemcpyAsync(fl.data(), flags.p, n_flags * 8, cudaMemcpyDeviceToHost, st));
     K2G_CUDA_TRY(cudaStreamSynchronize(st));
     std::sort(fl.begin(), fl.end());
-    K2G_CUDA_TRY(cudaMemcpy(flags.p, fl.data(), n_flags * 8, cudaMemcpyHostToDevice));
+    // (on this stream: the kernel below need not wait for another's copy)
+    K2G_CUDA_TRY(cudaMemcpyAsync(flags.p, fl.data(), n_flags * 8, cudaMemcpyHostToDevice, st));
     const uint64_t scratch_cap = std::min<uint64_t>(n, 1ull << 24);
     K2G_CUDA_TRY(scratch.alloc(scratch_cap));
     fixup_kernel<C><<<1, 32, 0, st>>>(v, sorted, n_sorted, flags.p, n_flags, scratch.p, scratch_cap, status.p);

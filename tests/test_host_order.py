@@ -2,6 +2,7 @@
 runtime: calls that hand out an object work on the legacy stream, which streams
 of other calls (non-blocking ones) do not wait for, so none of that work may
 be under way when they return."""
+import ctypes as C
 import os
 
 import numpy as np
@@ -58,5 +59,30 @@ def test_new_counters_are_ready_when_the_call_returns():
         c = k2g.Counters(db)
         assert f.pending() == 0
         c.close()
+        db.close()
+        assert f.faults() == []
+
+
+def test_merged_replays_start_after_their_flags_have_arrived():
+    """The order-exact insert sorts the flagged clusters on the host and sends
+    them back: on the stream of the kernel that reads them."""
+    with fake_cuda() as f:
+        db = k2g.Database.create(OPTS, 100_003, 22, 10, np.array([0, 0, 0, 1, 2], np.uint64))   # two roots
+        st = f.stream()
+        seen = []
+
+        def launch(name, args):
+            def arg(i, ty):
+                return C.cast(args[i], C.POINTER(ty))[0]
+            if "replay_kernel" in name:          # (view, sorted, n, flags, counter): one flagged cluster
+                C.cast(arg(3, C.c_void_p), C.POINTER(C.c_uint64))[0] = 7
+                C.cast(arg(4, C.c_void_p), C.POINTER(C.c_uint64))[0] = 1
+            if "fixup_kernel" in name:
+                seen.append((C.cast(arg(3, C.c_void_p), C.POINTER(C.c_uint64))[0], f.pending()))
+
+        f.hook(launch)
+        n = 1000
+        db.build_insert(f.device(np.arange(n, dtype=np.uint64)), f.device(np.ones(n, np.uint32)), n, True, st)
+        assert seen == [(7, 0)]
         db.close()
         assert f.faults() == []
