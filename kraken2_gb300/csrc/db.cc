@@ -30,6 +30,8 @@ k2g_status fail(k2g_status s, const std::string &msg) {
 }
 
 k2g_status cuda_fail(int err, const char *what) {
+  // (reported now: the runtime would hand it to the next call's launch check)
+  (void)cudaGetLastError();
   g_last_error = std::string(what) + ": " + cudaGetErrorString((cudaError_t)err);
   if (err == cudaErrorMemoryAllocation) return K2G_ERR_NOMEM;
   return K2G_ERR_CUDA;
