@@ -431,7 +431,8 @@ namespace k2g {
 namespace {
 
 // Buffers come from the device's scratch pool, on the calling stream: every
-// entry point leaves its stream synchronised, so the next may use another.
+// entry point leaves its stream synchronised, also where it fails (settled),
+// so the next may use another.
 // (cudaMalloc and cudaFree here stopped all other streams.)
 template <class T>
 cudaError_t reserve(k2g_counters *c, cudaStream_t st, T *&p, uint64_t &cap, uint64_t want) {
@@ -724,15 +725,14 @@ extern "C" k2g_status k2g_counters_destroy(k2g_counters *c) {
   return K2G_OK;
 }
 
-extern "C" k2g_status k2g_counters_add(k2g_counters *c, const k2g_reads *reads,
-                                       const k2g_results *res, void *stream) {
+static k2g_status counters_add(k2g_counters *c, const k2g_reads *reads, const k2g_results *res,
+                               cudaStream_t st) {
   if (!c || !reads || !res) return fail(K2G_ERR_ARG, "null argument");
   if (!res->d_hit_keys || !res->d_hit_taxa || !res->d_hit_order || !res->d_hits_used)
     return fail(K2G_ERR_ARG, "k2g_counters_add needs the hit event buffers");
   if (!reads->n_frags) return K2G_OK;
   if (!reads->d_frag_block) return fail(K2G_ERR_ARG, "k2g_counters_add needs d_frag_block");
   K2G_CUDA_TRY(cudaSetDevice(c->device));
-  cudaStream_t st = (cudaStream_t)stream;
   uint64_t used = 0;
   uint32_t b_first = 0, b_last = 0;
   K2G_CUDA_TRY(cudaMemcpyAsync(&used, res->d_hits_used, 8, cudaMemcpyDeviceToHost, st));
@@ -815,12 +815,17 @@ extern "C" k2g_status k2g_counters_add(k2g_counters *c, const k2g_reads *reads,
   return K2G_OK;
 }
 
-extern "C" k2g_status k2g_counters_export(k2g_counters *c, uint64_t *entries, uint64_t cap,
-                                          uint64_t *n_entries, uint64_t *taxon_kmers,
-                                          uint8_t *dense, void *stream) {
+extern "C" k2g_status k2g_counters_add(k2g_counters *c, const k2g_reads *reads,
+                                       const k2g_results *res, void *stream) {
+  cudaStream_t st = (cudaStream_t)stream;
+  return settled(counters_add(c, reads, res, st), st);
+}
+
+static k2g_status counters_export(k2g_counters *c, uint64_t *entries, uint64_t cap,
+                                  uint64_t *n_entries, uint64_t *taxon_kmers, uint8_t *dense,
+                                  cudaStream_t st) {
   if (!c || !n_entries) return fail(K2G_ERR_ARG, "null argument");
   K2G_CUDA_TRY(cudaSetDevice(c->device));
-  cudaStream_t st = (cudaStream_t)stream;
   k2g_status s = compact_acc(c, st);
   if (s != K2G_OK) return s;
   *n_entries = c->acc_used;
@@ -837,12 +842,18 @@ extern "C" k2g_status k2g_counters_export(k2g_counters *c, uint64_t *entries, ui
   return K2G_OK;
 }
 
-extern "C" k2g_status k2g_counters_import(k2g_counters *c, const uint64_t *entries,
-                                          uint64_t n_entries, const uint64_t *taxon_kmers,
-                                          const uint8_t *dense, void *stream) {
+extern "C" k2g_status k2g_counters_export(k2g_counters *c, uint64_t *entries, uint64_t cap,
+                                          uint64_t *n_entries, uint64_t *taxon_kmers,
+                                          uint8_t *dense, void *stream) {
+  cudaStream_t st = (cudaStream_t)stream;
+  return settled(counters_export(c, entries, cap, n_entries, taxon_kmers, dense, st), st);
+}
+
+static k2g_status counters_import(k2g_counters *c, const uint64_t *entries, uint64_t n_entries,
+                                  const uint64_t *taxon_kmers, const uint8_t *dense,
+                                  cudaStream_t st) {
   if (!c || !taxon_kmers || !dense || (n_entries && !entries)) return fail(K2G_ERR_ARG, "null argument");
   K2G_CUDA_TRY(cudaSetDevice(c->device));
-  cudaStream_t st = (cudaStream_t)stream;
   // an entry is (encoding << tbits | preorder number of its taxon)
   const uint64_t pmask = (1ull << c->tbits) - 1;
   for (uint64_t i = 0; i < n_entries; i++)
@@ -879,12 +890,17 @@ extern "C" k2g_status k2g_counters_import(k2g_counters *c, const uint64_t *entri
   return K2G_OK;
 }
 
-extern "C" k2g_status k2g_counters_finish(k2g_counters *c, uint64_t *taxon_kmers,
-                                          uint64_t *clade_kmers, uint64_t *clade_distinct,
-                                          void *stream) {
+extern "C" k2g_status k2g_counters_import(k2g_counters *c, const uint64_t *entries,
+                                          uint64_t n_entries, const uint64_t *taxon_kmers,
+                                          const uint8_t *dense, void *stream) {
+  cudaStream_t st = (cudaStream_t)stream;
+  return settled(counters_import(c, entries, n_entries, taxon_kmers, dense, st), st);
+}
+
+static k2g_status counters_finish(k2g_counters *c, uint64_t *taxon_kmers, uint64_t *clade_kmers,
+                                  uint64_t *clade_distinct, cudaStream_t st) {
   if (!c || !clade_kmers || !clade_distinct) return fail(K2G_ERR_ARG, "null argument");
   K2G_CUDA_TRY(cudaSetDevice(c->device));
-  cudaStream_t st = (cudaStream_t)stream;
   const uint64_t n = c->node_count;
   k2g_status s = compact_acc(c, st);
   if (s != K2G_OK) return s;
@@ -975,4 +991,11 @@ extern "C" k2g_status k2g_counters_finish(k2g_counters *c, uint64_t *taxon_kmers
     }
   }
   return K2G_OK;
+}
+
+extern "C" k2g_status k2g_counters_finish(k2g_counters *c, uint64_t *taxon_kmers,
+                                          uint64_t *clade_kmers, uint64_t *clade_distinct,
+                                          void *stream) {
+  cudaStream_t st = (cudaStream_t)stream;
+  return settled(counters_finish(c, taxon_kmers, clade_kmers, clade_distinct, st), st);
 }

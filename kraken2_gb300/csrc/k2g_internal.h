@@ -164,6 +164,13 @@ cudaError_t scratch_alloc_now(void **p, size_t bytes, int device);
 void scratch_free_now(void *p, int device);
 void scratch_opened(int device);
 void scratch_closed(int device);
+// The end of a call that works on `st` and waits for it: one that fails waits
+// too, since its buffers are on their way back to the pool (cudaFreeAsync does
+// not wait as cudaFree does) and the caller may free its own.
+inline k2g_status settled(k2g_status s, cudaStream_t st) {
+  if (s != K2G_OK && cudaStreamSynchronize(st) != cudaSuccess) (void)cudaGetLastError();
+  return s;
+}
 // Counts each kernel launch issued by the library (k2g_kernel_launches).
 void note_launches(uint64_t n = 1);
 // One round (< 2^30 pairs) of the order-exact build insert (build_ordered.cu).

@@ -8,6 +8,7 @@ from fake_cuda import fake_cuda
 
 OPTS = k2g.IndexOptions(35, 31, 0, 0xe37e28c4271b5a2d, 1, 1, 0)
 PARENT = np.array([0, 0, 1, 1, 2], np.uint64)
+FALLIBLE = ["cudaMallocFromPoolAsync", "cudaMemcpyAsync", "cudaMemsetAsync", "launch", "cudaStreamSynchronize"]
 
 
 def test_an_error_that_was_reported_is_not_reported_again():
@@ -24,3 +25,57 @@ def test_an_error_that_was_reported_is_not_reported_again():
         db.build_insert(keys, taxa, 100, False, st)
         db.lookup(keys, taxa, 100, st)
         db.close()
+
+
+def every_failure(f, call, fn):
+    """call() with the 1st, 2nd ... use of fn failing, until it needs no more."""
+    for i in range(400):
+        f.fail(fn, i)
+        try:
+            call()
+        except k2g.K2GError:
+            assert f.failed(), "an error without a cause"
+            assert f.pending_all() == 0, (fn, i)
+            continue
+        assert not f.failed(), (fn, i, "a failure that was not reported")
+        f.fail("", -1)
+        return i
+    raise AssertionError("too many calls")
+
+
+def events(f, n):
+    """k2g_counters_add's inputs: n events of 40 fragments in two blocks."""
+    frags = 40
+    d_blocks = f.device((np.arange(frags) // 20).astype(np.uint32))
+    reads = k2g.Reads(None, None, None, frags, 0, 0, d_blocks, 0)
+    res = k2g.Results()
+    res.d_hit_keys, res.d_hit_order = f.device(np.arange(n, dtype=np.uint64)), f.device(np.zeros(n, np.uint64))
+    res.d_hit_taxa, res.hits_cap = f.device(np.ones(n, np.uint32)), n
+    res.d_hits_used = f.device(np.array([n], np.uint64))
+    return reads, res
+
+
+@pytest.mark.parametrize("fn", FALLIBLE)
+@pytest.mark.parametrize("what", ["add", "import", "export", "finish"])
+def test_counters(what, fn):
+    with fake_cuda() as f:
+        db = k2g.Database.create(OPTS, 100_003, 22, 10, PARENT)
+        st = f.stream()
+        n = 20_000
+        state = {"entries": np.arange(n, dtype=np.uint64) << np.uint64(3), "taxon_kmers": np.ones(5, np.uint64),
+                 "dense": np.zeros(5, np.uint8)}
+        c = k2g.Counters(db)
+
+        def one():
+            if what == "add":
+                c.add(*events(f, n), stream=st)
+            elif what == "import":
+                c.import_state(state, stream=st)
+            else:
+                c.import_state(state, stream=st)
+                c.export(st) if what == "export" else c.finish(st)
+
+        every_failure(f, one, fn)
+        c.close()
+        db.close()
+        assert f.faults() == []
