@@ -585,18 +585,10 @@ k2g_status sort_blocks(const k2g_db *db, const Gathered &g, Scratch &s, const ui
 
 using namespace k2g;
 
-extern "C" k2g_status k2g_build_sequences(k2g_db *db, const char *bases, const uint64_t *seq_off,
-                                          const uint32_t *taxids, uint64_t n_seqs,
-                                          uint64_t block_size, uint64_t subblock_size, int ordered,
-                                          uint64_t *n_keys) {
-  if (n_keys) *n_keys = 0;
-  if (!db || (n_seqs && (!bases || !seq_off || !taxids))) return fail(K2G_ERR_ARG, "null argument");
-  if (!block_size || !subblock_size) return fail(K2G_ERR_ARG, "block sizes must be positive");
-  if (!n_seqs) return K2G_OK;
-  K2G_CUDA_TRY(cudaSetDevice(db->device));
-  StreamGuard guard;
-  K2G_CUDA_TRY(cudaStreamCreateWithFlags(&guard.s, cudaStreamNonBlocking));
-  cudaStream_t st = guard.s;
+static k2g_status build_sequences(k2g_db *db, const char *bases, const uint64_t *seq_off,
+                                  const uint32_t *taxids, uint64_t n_seqs, uint64_t block_size,
+                                  uint64_t subblock_size, int ordered, uint64_t *n_keys,
+                                  cudaStream_t st) {
   Scratch s{db->device, st};
   Gathered g;
   k2g_status r = gather(db, bases, seq_off, taxids, n_seqs, block_size, subblock_size, 0, s, st, g);
@@ -671,18 +663,24 @@ extern "C" k2g_status k2g_build_sequences(k2g_db *db, const char *bases, const u
   return K2G_OK;
 }
 
-extern "C" k2g_status k2g_sample_minimizers(const k2g_db *db, const char *bases,
-                                            const uint64_t *seq_off, uint64_t n_seqs,
-                                            uint32_t sample_below, uint64_t *keys, uint64_t keys_cap,
-                                            uint64_t *n_keys) {
-  if (!db || !n_keys || (n_seqs && (!bases || !seq_off))) return fail(K2G_ERR_ARG, "null argument");
-  *n_keys = 0;
-  if (sample_below < 1 || sample_below > 1024) return fail(K2G_ERR_ARG, "sample_below must be in [1, 1024]");
+extern "C" k2g_status k2g_build_sequences(k2g_db *db, const char *bases, const uint64_t *seq_off,
+                                          const uint32_t *taxids, uint64_t n_seqs,
+                                          uint64_t block_size, uint64_t subblock_size, int ordered,
+                                          uint64_t *n_keys) {
+  if (n_keys) *n_keys = 0;
+  if (!db || (n_seqs && (!bases || !seq_off || !taxids))) return fail(K2G_ERR_ARG, "null argument");
+  if (!block_size || !subblock_size) return fail(K2G_ERR_ARG, "block sizes must be positive");
   if (!n_seqs) return K2G_OK;
   K2G_CUDA_TRY(cudaSetDevice(db->device));
   StreamGuard guard;
   K2G_CUDA_TRY(cudaStreamCreateWithFlags(&guard.s, cudaStreamNonBlocking));
-  cudaStream_t st = guard.s;
+  return settled(build_sequences(db, bases, seq_off, taxids, n_seqs, block_size, subblock_size, ordered, n_keys,
+                                 guard.s), guard.s);
+}
+
+static k2g_status sample_minimizers(const k2g_db *db, const char *bases, const uint64_t *seq_off,
+                                    uint64_t n_seqs, uint32_t sample_below, uint64_t *keys,
+                                    uint64_t keys_cap, uint64_t *n_keys, cudaStream_t st) {
   Scratch s{db->device, st};
   Gathered g;
   // whole sequences: one block, no subblocks (MinimizerScanner::LoadSequence(seq))
@@ -722,4 +720,18 @@ extern "C" k2g_status k2g_sample_minimizers(const k2g_db *db, const char *bases,
     K2G_CUDA_TRY(cudaMemcpy(keys, d_out, n_unique * 8, cudaMemcpyDeviceToHost));
   }
   return K2G_OK;
+}
+
+extern "C" k2g_status k2g_sample_minimizers(const k2g_db *db, const char *bases,
+                                            const uint64_t *seq_off, uint64_t n_seqs,
+                                            uint32_t sample_below, uint64_t *keys, uint64_t keys_cap,
+                                            uint64_t *n_keys) {
+  if (!db || !n_keys || (n_seqs && (!bases || !seq_off))) return fail(K2G_ERR_ARG, "null argument");
+  *n_keys = 0;
+  if (sample_below < 1 || sample_below > 1024) return fail(K2G_ERR_ARG, "sample_below must be in [1, 1024]");
+  if (!n_seqs) return K2G_OK;
+  K2G_CUDA_TRY(cudaSetDevice(db->device));
+  StreamGuard guard;
+  K2G_CUDA_TRY(cudaStreamCreateWithFlags(&guard.s, cudaStreamNonBlocking));
+  return settled(sample_minimizers(db, bases, seq_off, n_seqs, sample_below, keys, keys_cap, n_keys, guard.s), guard.s);
 }

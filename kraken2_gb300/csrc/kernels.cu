@@ -949,12 +949,8 @@ k2g_status k2g::classify_keyed(const k2g_db *db, const k2g_reads *reads,
   return run_classify(db, a, mode, reads->max_seq_len, total, st, state_key, tn);
 }
 
-extern "C" k2g_status k2g_build_insert(k2g_db *db, const uint64_t *d_keys, const uint32_t *d_taxids,
-                                       uint64_t n, int ordered, void *stream) {
-  if (!db || (n && (!d_keys || !d_taxids))) return fail(K2G_ERR_ARG, "null argument");
-  if (!n) return K2G_OK;
-  K2G_CUDA_TRY(cudaSetDevice(db->device));
-  cudaStream_t st = (cudaStream_t)stream;
+static k2g_status build_insert(k2g_db *db, const uint64_t *d_keys, const uint32_t *d_taxids, uint64_t n,
+                               int ordered, cudaStream_t st) {
   if (ordered) {
     // sequential insertion of the whole list = rounds of it in order
     const uint64_t round = (1ull << 30) - 1;
@@ -973,6 +969,15 @@ extern "C" k2g_status k2g_build_insert(k2g_db *db, const uint64_t *d_keys, const
   cudaFreeAsync(d_status, st);
   if (e != cudaSuccess) return cuda_fail(e, "insert_kernel");
   return insert_status(status);
+}
+
+extern "C" k2g_status k2g_build_insert(k2g_db *db, const uint64_t *d_keys, const uint32_t *d_taxids,
+                                       uint64_t n, int ordered, void *stream) {
+  if (!db || (n && (!d_keys || !d_taxids))) return fail(K2G_ERR_ARG, "null argument");
+  if (!n) return K2G_OK;
+  K2G_CUDA_TRY(cudaSetDevice(db->device));
+  cudaStream_t st = (cudaStream_t)stream;
+  return settled(build_insert(db, d_keys, d_taxids, n, ordered, st), st);
 }
 
 namespace k2g {

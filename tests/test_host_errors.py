@@ -1,5 +1,7 @@
 """Calls of the CUDA runtime that fail, under the library's entry points (on
 the fake runtime)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -8,6 +10,7 @@ from fake_cuda import fake_cuda
 
 OPTS = k2g.IndexOptions(35, 31, 0, 0xe37e28c4271b5a2d, 1, 1, 0)
 PARENT = np.array([0, 0, 1, 1, 2], np.uint64)
+ROOTS = {True: PARENT, False: np.array([0, 0, 0, 1, 2], np.uint64)}
 FALLIBLE = ["cudaMallocFromPoolAsync", "cudaMemcpyAsync", "cudaMemsetAsync", "launch", "cudaStreamSynchronize"]
 
 
@@ -27,7 +30,7 @@ def test_an_error_that_was_reported_is_not_reported_again():
         db.close()
 
 
-def every_failure(f, call, fn):
+def every_failure(f, call, fn, optional=None):
     """call() with the 1st, 2nd ... use of fn failing, until it needs no more."""
     for i in range(400):
         f.fail(fn, i)
@@ -37,7 +40,10 @@ def every_failure(f, call, fn):
             assert f.failed(), "an error without a cause"
             assert f.pending_all() == 0, (fn, i)
             continue
-        assert not f.failed(), (fn, i, "a failure that was not reported")
+        if f.failed():
+            # only room asked for ahead of its size, which a build can do without
+            assert fn == "cudaMallocFromPoolAsync" and i == optional, (fn, i, "a failure that was not reported")
+            continue
         f.fail("", -1)
         return i
     raise AssertionError("too many calls")
@@ -77,5 +83,38 @@ def test_counters(what, fn):
 
         every_failure(f, one, fn)
         c.close()
+        db.close()
+        assert f.faults() == []
+
+
+@pytest.mark.parametrize("fn", FALLIBLE)
+@pytest.mark.parametrize("one_root", [True, False])
+@pytest.mark.parametrize("what", ["unordered", "ordered", "sequences", "sample"])
+def test_builds(what, one_root, fn):
+    with fake_cuda() as f:
+        db = k2g.Database.create(OPTS, 100_003, 22, 10, ROOTS[one_root])
+        st = f.stream()
+        n = 5000
+        keys, taxa = f.device(np.arange(n, dtype=np.uint64)), f.device(np.ones(n, np.uint32))
+        seq = np.frombuffer(b"ACGT" * 10_000, np.uint8)
+        off = np.array([0, 15_000, 40_000], np.uint64)
+
+        def count(name, args):   # (the scan finds a candidate, so that what follows it runs)
+            if "block_scan_kernel" in name:
+                counts = C.cast(args[5], C.POINTER(C.c_void_p))[0]
+                C.cast(counts, C.POINTER(C.c_uint32))[0] = 1
+
+        f.hook(count)
+
+        def one():
+            if what == "sequences":
+                db.build_sequences(seq, off, np.array([3, 4], np.uint32))
+            elif what == "sample":
+                db.sample_minimizers(seq, off)
+            else:
+                db.build_insert(keys, taxa, n, what == "ordered", st)
+
+        # (the seventh allocation of a library scan: bases, chunks, blocks, counts, offsets, sums, then it)
+        every_failure(f, one, fn, optional=6 if what in ("sequences", "sample") else None)
         db.close()
         assert f.faults() == []
