@@ -198,21 +198,24 @@ cudaError_t regrow(T *&p, uint64_t n) {
 cudaError_t fit_slot(Slot &s, uint64_t bb, uint64_t fb, int per, bool quals, uint64_t hits) {
   cudaError_t e;
 #define TRY(x) if ((e = (x)) != cudaSuccess) return e
-  if (!s.st) {
+  if (!s.hits_used) {   // (the last of them: after a failure the rest is made)
     int low = 0, high = 0;
     TRY(cudaDeviceGetStreamPriorityRange(&low, &high));
     for (cudaEvent_t *e1 : {&s.classified, &s.done, &s.left})
-      TRY(cudaEventCreateWithFlags(e1, cudaEventDisableTiming));
-    TRY(cudaStreamCreateWithPriority(&s.out, cudaStreamNonBlocking, high));
-    TRY(cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking));
-    TRY(cudaHostAlloc(&s.h_total, 16, cudaHostAllocDefault));
-    TRY(cudaMalloc(&s.total, 16));
+      if (!*e1) TRY(cudaEventCreateWithFlags(e1, cudaEventDisableTiming));
+    if (!s.out) TRY(cudaStreamCreateWithPriority(&s.out, cudaStreamNonBlocking, high));
+    if (!s.st) TRY(cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking));
+    if (!s.h_total) TRY(cudaHostAlloc(&s.h_total, 16, cudaHostAllocDefault));
+    if (!s.total) TRY(cudaMalloc(&s.total, 16));
     TRY(cudaMalloc(&s.hits_used, 8));
   }
   if (bb > s.cap_bases || fb > s.cap_frags) {
     bb = std::max(bb, s.cap_bases);
     fb = std::max(fb, s.cap_frags);
     const uint64_t sparse_cap = bb + 2 * fb + 8;
+    // (until all of them are there, the slot holds nothing: a call that runs
+    // out of memory here leaves it to the next to start over)
+    s.cap_bases = s.cap_frags = s.cap_quals = s.cap_hits = 0;
     TRY(regrow(s.bases, bb + 16));
     TRY(regrow(s.off, fb * 2 + 1));
     TRY(regrow(s.call, fb));
@@ -225,14 +228,14 @@ cudaError_t fit_slot(Slot &s, uint64_t bb, uint64_t fb, int per, bool quals, uin
     TRY(regrow(s.blocks, fb));
     s.cap_bases = bb;
     s.cap_frags = fb;
-    s.cap_quals = 0;
-    s.cap_hits = 0;
   }
   if (quals && s.cap_quals < s.cap_bases) {
+    s.cap_quals = 0;
     TRY(regrow(s.quals, s.cap_bases + 16));
     s.cap_quals = s.cap_bases;
   }
   if (hits > s.cap_hits) {
+    s.cap_hits = 0;
     TRY(regrow(s.hit_keys, hits));
     TRY(regrow(s.hit_taxa, hits));
     TRY(regrow(s.hit_order, hits));
@@ -333,6 +336,7 @@ static k2g_status host_classify(const k2g_db *db, const char *bases, const char 
   unsigned long long *d_taxon_reads = nullptr;
   if (taxon_reads) {
     if (hc.taxon_cap < db->node_count) {
+      hc.taxon_cap = 0;
       K2G_CUDA_TRY(regrow(hc.taxon_reads, db->node_count));
       hc.taxon_cap = db->node_count;
     }

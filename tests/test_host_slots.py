@@ -1,0 +1,73 @@
+"""The buffers that k2g_classify_host keeps between calls, on the fake runtime:
+after an allocation that failed, the next call, of any size, finds buffers that
+are as large as it takes them to be."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import kraken2_gb300 as k2g
+from fake_cuda import fake_cuda
+
+OPTS = k2g.IndexOptions(35, 31, 0, 0xe37e28c4271b5a2d, 1, 1, 0)
+PARENT = np.array([0, 0, 1, 1, 2], np.uint64)
+
+
+def classify(db, n, length=150, counters=None, quals=True, nodes=len(PARENT)):
+    bases = np.full(n * length + 16, ord("A"), np.uint8)
+    off = np.arange(n + 1, dtype=np.uint64) * np.uint64(length)
+    call, hg, hlen = (np.zeros(n, np.uint32) for _ in range(3))
+    runs, tr = np.zeros(16, np.uint64), np.zeros(nodes, np.uint64)
+    nr = C.c_uint64(len(runs))
+    cp = k2g.ClassifyParams(0.0, 2, 0, 0, 10)
+    args = [db.h, bases.ctypes.data, bases.ctypes.data if quals else None, off.ctypes.data, n]
+    out = [C.byref(cp), call.ctypes.data, hg.ctypes.data, hlen.ctypes.data, runs.ctypes.data, C.byref(nr),
+           tr.ctypes.data]
+    if counters is None:
+        return k2g.lib().k2g_classify_host(*args, *out)
+    blocks = (np.arange(n) // 100).astype(np.uint32)
+    return k2g.lib().k2g_classify_host_blocks(*args, blocks.ctypes.data, counters.h, *out)
+
+
+@pytest.mark.parametrize("with_counters", [False, True])
+def test_a_failed_allocation_leaves_no_capacity_behind(with_counters):
+    with fake_cuda() as f:
+        small = k2g.Database.create(OPTS, 100_003, 22, 10, PARENT, device=11 + with_counters)
+        large = k2g.Database.create(OPTS, 100_003, 22, 10, np.arange(1000, dtype=np.uint64) // 2, device=11 + with_counters)
+        cs = [k2g.Counters(db) if with_counters else None for db in (small, large)]
+        n = 500
+        for i in range(60):
+            k2g.check(classify(small, n, counters=cs[0]))
+            n += 50                                  # every buffer has to grow
+            f.fail("cudaMalloc", i)
+            status = classify(large, n, counters=cs[1], nodes=1000)
+            assert (status != 0) == f.failed()
+            f.fail("", -1)
+            k2g.check(classify(small, 500, counters=cs[0]))
+            k2g.check(classify(large, 500, counters=cs[1], nodes=1000))
+            assert f.faults() == []
+            if status == 0:
+                break
+        assert status == 0 and i > 10
+
+
+@pytest.mark.parametrize("fn", ["cudaMalloc", "cudaHostAlloc", "cudaStreamCreateWithFlags",
+                                "cudaStreamCreateWithPriority", "cudaEventCreateWithFlags"])
+def test_a_first_call_that_failed_half_way(fn):
+    with fake_cuda() as f:
+        # (a device of its own for each of the calls made to fail)
+        first = 20 + 8 * ["cudaHostAlloc", "cudaStreamCreateWithFlags", "cudaStreamCreateWithPriority",
+                          "cudaEventCreateWithFlags", "cudaMalloc"].index(fn)
+        for i in range(8):
+            db = k2g.Database.create(OPTS, 100_003, 22, 10, PARENT, device=first + i)
+            f.fail(fn, i)
+            status = classify(db, 500)
+            assert (status != 0) == f.failed()
+            f.fail("", -1)
+            k2g.check(classify(db, 500))
+            k2g.check(classify(db, 700))
+            db.close()
+            assert f.faults() == []
+            if status == 0:
+                break
+        assert i > 0
