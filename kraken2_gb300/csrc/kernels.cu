@@ -383,22 +383,25 @@ static k2g_status ctx_reserve(ExecCtx &c, uint64_t frags, uint64_t slots, size_t
     K2G_CUDA_TRY(cudaMalloc(&c.slow, slow_bytes));
     c.slow_bytes = slow_bytes;
   }
+  // (a capacity that several buffers share is none until all of them are there)
   if (pipeline && c.cap_slots < slots) {
-    uint64_t cs = c.cap_slots;
+    c.cap_slots = 0;
+    uint64_t cs = 0;
     K2G_CUDA_TRY(grow(c.gstream, cs, slots));
-    cs = c.cap_slots;
+    cs = 0;
     K2G_CUDA_TRY(grow(c.gtax, cs, slots));
-    cs = c.cap_slots;
+    cs = 0;
     K2G_CUDA_TRY(grow(c.rkey, cs, slots));
-    cs = c.cap_slots;
+    cs = 0;
     K2G_CUDA_TRY(grow(c.rslot, cs, slots));
     c.cap_slots = slots;
   }
   if (pipeline && keys) K2G_CUDA_TRY(grow(c.gkey, c.cap_gkey, slots));
   if (pipeline && c.cap_frags < frags) {
-    uint64_t cf = c.cap_frags;
+    c.cap_frags = 0;
+    uint64_t cf = 0;
     K2G_CUDA_TRY(grow(c.gcount, cf, frags));
-    cf = c.cap_frags;
+    cf = 0;
     K2G_CUDA_TRY(grow(c.bcount, cf, frags));
     c.cap_frags = frags;
   }

@@ -71,3 +71,50 @@ def test_a_first_call_that_failed_half_way(fn):
             if status == 0:
                 break
         assert i > 0
+
+
+def test_staged_buffers_after_a_failed_allocation():
+    """k2g_classify on a table that the staged kernels take (k = l): whatever
+    failed in between, a call's kernels get every pointer they got before."""
+    with fake_cuda() as f:
+        db = k2g.Database.create(k2g.IndexOptions(31, 31, 0, 0xe37e28c4271b5a2d, 1, 1, 0), 100_003, 22, 10, PARENT,
+                                 device=61)
+        st = f.stream()
+
+        def call(n, events):
+            bases = f.device(np.full(150 * n, ord("A"), np.uint8))
+            off = f.device(np.arange(n + 1, dtype=np.uint64) * np.uint64(150))
+            out = f.device(np.zeros(400 * n, np.uint64))
+            reads = k2g.Reads(bases, None, off, n, 150, 150 * n, None, 0)
+            res = k2g.Results(out, None, None, None, out, 152 * n, None, out if events else None, out, out, n, out, out)
+            try:
+                db.classify(reads, k2g.ClassifyParams(0.0, 2, 0, 0, 0), res, mode=k2g.MODE_PIPELINED, stream=st)
+                return True
+            except k2g.K2GError:
+                return False
+            finally:
+                for p in (bases, off, out):
+                    f.lib.cudaFree(C.c_void_p(p))
+
+        given = []
+
+        def launch(name, args):              # which words of a launch's argument are null
+            if "pipe_step_kernel" in name:
+                words = C.cast(args[0], C.POINTER(C.c_uint64))[:128]
+                given.append([w != 0 for w in words])
+
+        f.hook(launch)
+        assert call(1000, True) and call(1000, True)
+        want = given[len(given) // 2:]
+        n = 1000
+        for i in range(60):
+            n += 500
+            f.fail("cudaMalloc", i + 3)          # (three are the caller's)
+            done = call(n, True)
+            assert done != f.failed()
+            f.fail("", -1)
+            given.clear()
+            assert call(1000, True) and given == want
+            if done:
+                break
+        assert done and i > 3
