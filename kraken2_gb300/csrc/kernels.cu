@@ -396,7 +396,8 @@ static k2g_status ctx_reserve(ExecCtx &c, uint64_t frags, uint64_t slots, size_t
     K2G_CUDA_TRY(grow(c.rslot, cs, slots));
     c.cap_slots = slots;
   }
-  if (pipeline && keys) K2G_CUDA_TRY(grow(c.gkey, c.cap_gkey, slots));
+  // (as many as the kernels take there to be: a larger call may have come before)
+  if (pipeline && keys) K2G_CUDA_TRY(grow(c.gkey, c.cap_gkey, c.cap_slots));
   if (pipeline && c.cap_frags < frags) {
     c.cap_frags = 0;
     uint64_t cf = 0;

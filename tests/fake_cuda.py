@@ -54,6 +54,7 @@ class Fake:
         for f in ("fake_pending", "fake_pending_all", "fake_used", "fake_launches"):
             getattr(lib, f).restype = C.c_uint64
         lib.fake_tail_of_copy.argtypes, lib.fake_tail_of_copy.restype = [C.c_size_t], C.c_long
+        lib.fake_room.argtypes, lib.fake_room.restype = [C.c_void_p], C.c_long
         lib.fake_limit.argtypes = [C.c_uint64]
         lib.fake_fail.argtypes = [C.c_char_p, C.c_long, C.c_int]
         lib.fake_launches.argtypes = [C.c_char_p]
@@ -82,6 +83,10 @@ class Fake:
 
     def used(self) -> int:
         return self.lib.fake_used()
+
+    def room(self, p: int) -> int:
+        """Bytes from p to the end of its allocation (-1: none)."""
+        return self.lib.fake_room(p)
 
     def tail_of_copy(self, n: int) -> int:
         """Bytes of the allocation behind the last host-to-device copy of n bytes (-1: none)."""

@@ -191,6 +191,11 @@ API uint64_t fake_launches(const char *part) {
 }
 API long fake_faults() { return (long)F().faults.size(); }
 API const char *fake_fault(long i) { return F().faults[i].c_str(); }
+// Bytes from p to the end of its allocation (-1: none).
+API long fake_room(const void *p) {
+  auto it = find(p);
+  return it == F().mem.end() ? -1 : (long)(it->first + it->second.size - (uintptr_t)p);
+}
 API long fake_tail_of_copy(size_t bytes) { return F().tails.count(bytes) ? (long)F().tails[bytes] : -1; }
 API void fake_hook(LaunchHook h) { F().hook = h; }
 

@@ -73,6 +73,23 @@ def test_a_first_call_that_failed_half_way(fn):
         assert i > 0
 
 
+def staged_call(f, db, st, n, events):
+    """k2g_classify of n fragments of 150 bases; whether it succeeded."""
+    bases = f.device(np.full(150 * n, ord("A"), np.uint8))
+    off = f.device(np.arange(n + 1, dtype=np.uint64) * np.uint64(150))
+    out = f.device(np.zeros(400 * n, np.uint64))
+    reads = k2g.Reads(bases, None, off, n, 150, 150 * n, None, 0)
+    res = k2g.Results(out, None, None, None, out, 152 * n, None, out if events else None, out, out, n, out, out)
+    try:
+        db.classify(reads, k2g.ClassifyParams(0.0, 2, 0, 0, 0), res, mode=k2g.MODE_PIPELINED, stream=st)
+        return True
+    except k2g.K2GError:
+        return False
+    finally:
+        for p in (bases, off, out):
+            f.lib.cudaFree(C.c_void_p(p))
+
+
 def test_staged_buffers_after_a_failed_allocation():
     """k2g_classify on a table that the staged kernels take (k = l): whatever
     failed in between, a call's kernels get every pointer they got before."""
@@ -82,19 +99,7 @@ def test_staged_buffers_after_a_failed_allocation():
         st = f.stream()
 
         def call(n, events):
-            bases = f.device(np.full(150 * n, ord("A"), np.uint8))
-            off = f.device(np.arange(n + 1, dtype=np.uint64) * np.uint64(150))
-            out = f.device(np.zeros(400 * n, np.uint64))
-            reads = k2g.Reads(bases, None, off, n, 150, 150 * n, None, 0)
-            res = k2g.Results(out, None, None, None, out, 152 * n, None, out if events else None, out, out, n, out, out)
-            try:
-                db.classify(reads, k2g.ClassifyParams(0.0, 2, 0, 0, 0), res, mode=k2g.MODE_PIPELINED, stream=st)
-                return True
-            except k2g.K2GError:
-                return False
-            finally:
-                for p in (bases, off, out):
-                    f.lib.cudaFree(C.c_void_p(p))
+            return staged_call(f, db, st, n, events)
 
         given = []
 
@@ -118,3 +123,23 @@ def test_staged_buffers_after_a_failed_allocation():
             if done:
                 break
         assert done and i > 3
+
+
+def test_staged_hit_keys_have_room_for_every_slot():
+    """A call with hit events behind a larger one without: the slots are still
+    those of the larger one."""
+    with fake_cuda() as f:
+        db = k2g.Database.create(k2g.IndexOptions(31, 31, 0, 0xe37e28c4271b5a2d, 1, 1, 0), 100_003, 22, 10, PARENT,
+                                 device=62)
+        st = f.stream()
+        seen = []
+
+        def launch(name, args):
+            if "pipe_step_kernel" in name:       # the scan role's view: its last two words
+                gkey, cap_slots = C.cast(args[0], C.POINTER(C.c_uint64))[58:60]
+                seen.append((f.room(gkey), 8 * cap_slots))
+
+        assert staged_call(f, db, st, 20_000, False)
+        f.hook(launch)
+        assert staged_call(f, db, st, 1000, True)
+        assert seen and all(have >= need > 0 for have, need in seen)
