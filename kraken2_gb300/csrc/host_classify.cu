@@ -246,6 +246,17 @@ cudaError_t fit_slot(Slot &s, uint64_t bb, uint64_t fb, int per, bool quals, uin
   return cudaSuccess;
 }
 
+// Gives a slot's buffers back.
+void empty_slot(Slot &s) {
+  auto drop = [](auto *&p) {
+    if (p) cudaFree(p);
+    p = nullptr;
+  };
+  drop(s.bases); drop(s.quals); drop(s.off); drop(s.call); drop(s.hg); drop(s.hlen); drop(s.sparse); drop(s.dense);
+  drop(s.excl); drop(s.sums); drop(s.blocks); drop(s.hit_keys); drop(s.hit_taxa); drop(s.hit_order);
+  s.cap_bases = s.cap_frags = s.cap_quals = s.cap_hits = 0;
+}
+
 // Largest g in [f, n] with seq_off[g * per] - seq_off[f * per] <= max_bases
 // (offsets are non-decreasing).
 uint64_t cut_by_bases(const uint64_t *seq_off, int per, uint64_t f, uint64_t n,
@@ -329,10 +340,26 @@ static k2g_status host_classify(const k2g_db *db, const char *bases, const char 
   // chunks' classification (120k mixed ones: 2.54 -> 2.38 ms; short ones the
   // same, with hit events 4.52 -> 4.59).  A third as large as one huge sequence
   // would be memory for nothing.
-  const size_t n_slots = chunk_bases > (256ull << 20) ? 2 : long_batch(all_bases, n_frags) && !counters ? kSlots : 3;
-  const int used = (int)std::min(n_chunks, n_slots);
-  for (int i = 0; i < used; i++)
-    K2G_CUDA_TRY(fit_slot(slots[i], chunk_bases, chunk_frags, per, quals != nullptr, hits_cap));
+  size_t n_slots = chunk_bases > (256ull << 20) ? 2 : long_batch(all_bases, n_frags) && !counters ? kSlots : 3;
+  int used = (int)std::min(n_chunks, n_slots);
+  auto fit = [&]() {
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < used && e == cudaSuccess; i++)
+      e = fit_slot(slots[i], chunk_bases, chunk_frags, per, quals != nullptr, hits_cap);
+    return e;
+  };
+  cudaError_t fitted = fit();
+  bool more = used > 2;
+  for (int i = 2; i < kSlots; i++) more = more || slots[i].bases || slots[i].sparse;
+  if (fitted == cudaErrorMemoryAllocation && more) {
+    // two slots do, where the others' memory is needed or not there
+    (void)cudaGetLastError();
+    for (int i = 2; i < kSlots; i++) empty_slot(slots[i]);
+    n_slots = 2;
+    used = (int)std::min(n_chunks, n_slots);
+    fitted = fit();
+  }
+  K2G_CUDA_TRY(fitted);
   unsigned long long *d_taxon_reads = nullptr;
   if (taxon_reads) {
     if (hc.taxon_cap < db->node_count) {

@@ -143,3 +143,37 @@ def test_staged_hit_keys_have_room_for_every_slot():
         f.hook(launch)
         assert staged_call(f, db, st, 1000, True)
         assert seen and all(have >= need > 0 for have, need in seen)
+
+
+@pytest.mark.parametrize("with_counters", [False, True])
+@pytest.mark.parametrize("length", [150, 5000])      # three slots, and four for long fragments
+def test_a_device_with_room_for_two_slots(length, with_counters):
+    """Calls of several chunks take more slots than two for speed alone: where
+    memory is short, two do, also when others hold some from an earlier call."""
+    with fake_cuda() as f:
+        n = (400 << 20 if with_counters else 130 << 20) // length        # five chunks and more
+        slots = 4 if length == 5000 and not with_counters else 3
+
+        def call(db, frags):
+            c = k2g.Counters(db) if with_counters else None
+            return classify(db, frags, length, c, quals=False)
+
+        first = 30 + 6 * (length == 5000) + 3 * with_counters            # (devices of their own)
+        dbs = [k2g.Database.create(OPTS, 100_003, 22, 10, PARENT, device=first + i) for i in range(3)]
+        base = f.used()
+        k2g.check(call(dbs[0], n))
+        slot = (f.used() - base) // slots
+        base = f.used()
+        f.limit(base + 5 * slot // 2)
+        k2g.check(call(dbs[1], n // 2))                                  # (fewer, or smaller, chunks)
+        for _ in range(2):
+            k2g.check(call(dbs[1], n))
+        f.limit(1 << 60)
+        k2g.check(call(dbs[1], n))
+        # with room for one there is an error, which leaves the next call whole
+        base = f.used()
+        f.limit(base + 3 * slot // 2)
+        assert call(dbs[2], n) == 5
+        f.limit(1 << 60)
+        k2g.check(call(dbs[2], n))
+        assert f.faults() == []
