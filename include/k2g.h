@@ -221,27 +221,33 @@ k2g_status k2g_classify(const k2g_db *db, const k2g_reads *reads,
  * prefetch distance at src/compact_hash.h:380-392).  Each table keeps one
  * set of values per (single-end or paired, length class) of a batch; every
  * k2g_classify call uses the set of its batch's class.  The values change
- * only how the work is scheduled, never a result.  The one-launch form of
- * K2G_MODE_PIPELINED uses piece_len only (a warp's pieces are four times as
- * long, up to 8192).  A table starts with
+ * only how the work is scheduled, never a result.  Which of them a call
+ * uses depends on its kernels: the one-launch form of K2G_MODE_PIPELINED
+ * (tables with k - l = 4) uses piece_len only, translated search none; the
+ * staged and fused kernels use all of them.  A table starts with
  * pipeline 1 for short batches and 0 otherwise, probe_split 2,
  * sub_batch_mb 256, piece_len 512 and graphs 0 in every class. */
 typedef struct {
-  /* 1: K2G_MODE_PIPELINED runs scan / probe / resolve beats over
-   * sub-batches; 0: it runs the fused work-stealing kernel instead */
+  /* staged and fused kernels: 1: K2G_MODE_PIPELINED runs scan / probe /
+   * resolve beats over sub-batches; 0: it runs the fused work-stealing
+   * kernel instead */
   uint32_t pipeline;
-  /* table-probe blocks per 128-fragment group in a beat (1..4): the probe
-   * lanes, and so the table loads in flight, per fragment scanned */
+  /* staged kernels: table-probe blocks per 128-fragment group in a beat
+   * (1..4): the probe lanes, and so the table loads in flight, per fragment
+   * scanned */
   uint32_t probe_split;
-  /* most bases of one pipeline sub-batch, in MiB (16..1024) */
+  /* staged kernels: most bases of one pipeline sub-batch, in MiB (16..1024) */
   uint32_t sub_batch_mb;
   /* nominal piece length (256..8192, a power of two): single-end fragments
    * of twice this length and more are cut into pieces that separate lanes
-   * classify, so a read of L bases gets about L / piece_len lanes */
+   * classify, so a read of L bases gets about L / piece_len lanes.  The
+   * one-launch form gives a piece to a warp, four times as long, up to 8192
+   * bases */
   uint32_t piece_len;
-  /* 1: each call's launch sequence is captured as a CUDA graph and launched
-   * as one (the last graph is kept and updated in place for a batch of the
-   * same shape); 0: the launches are issued one by one */
+  /* staged and fused kernels: 1: each call's launch sequence is captured as
+   * a CUDA graph and launched as one (the last graph is kept and updated in
+   * place for a batch of the same shape); 0: the launches are issued one by
+   * one */
   uint32_t graphs;
 } k2g_tuning;
 
@@ -253,14 +259,16 @@ k2g_status k2g_tuning_get(const k2g_db *db, int paired, int length_class, k2g_tu
 /* Rejects values outside the ranges above (K2G_ERR_ARG). */
 k2g_status k2g_tuning_set(k2g_db *db, int paired, int length_class, const k2g_tuning *in);
 /* Times k2g_classify (K2G_MODE_PIPELINED) on the given batch under each
- * candidate set of values for the batch's class -- probe split and
- * sub-batch size for short reads; pipeline or fused kernel and piece length
- * otherwise, then the fastest with and without graph capture -- `trials`
- * timed calls per candidate after one warm-up, keeps
- * the fastest for that class of this table and returns it in *chosen and
- * its time in *best_ms (either may be NULL).  The batch's outputs are
- * written many times over; the last call leaves them as k2g_classify
- * would.  Synchronises `stream`. */
+ * candidate set of values that changes how the batch runs -- by the
+ * one-launch form, the piece lengths that cut its fragments differently
+ * (only the defaults for pairs, quick mode, short fragments and translated
+ * search); by the staged and fused kernels, probe split and sub-batch size
+ * for short reads, pipeline or fused kernel and piece length otherwise, then
+ * the fastest with and without graph capture -- `trials` timed calls per
+ * candidate after one warm-up, keeps the fastest for that class of this
+ * table and returns it in *chosen and its time in *best_ms (either may be
+ * NULL).  The batch's outputs are written many times over; the last call
+ * leaves them as k2g_classify would.  Synchronises `stream`. */
 k2g_status k2g_autotune(k2g_db *db, const k2g_reads *reads, const k2g_classify_params *params,
                         k2g_results *out, int trials, k2g_tuning *chosen, double *best_ms,
                         void *stream);

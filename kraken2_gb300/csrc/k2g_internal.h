@@ -148,11 +148,13 @@ k2g_status classify_translated(const k2g_db *db, const k2g_reads *reads,
                                const k2g_classify_params *params, k2g_results *out,
                                cudaStream_t st);
 // Classification by warps on the caller's stream (warp_classify.cu): whether
-// it takes a call, and the call itself.
+// it takes a call, the pieces it cuts the call's long fragments into under a
+// tuned piece length (0: it cuts none), and the call itself.
 struct ClassifyArgs;
 void set_classify_args(ClassifyArgs &a, const k2g_db *db, const k2g_reads *reads,
                        const k2g_classify_params *params, const k2g_results *out);
 bool warp_classify_takes(const ClassifyArgs &a, uint64_t max_len);
+uint32_t warp_piece(int paired, int quick, uint64_t max_len, uint32_t piece_len);
 cudaError_t warp_classify(const ClassifyArgs &a, const uint2 *span, uint64_t max_len, uint64_t total_bases,
                           uint32_t piece_len, int device, int sms, cudaStream_t st);
 // Device scratch of one call, allocated on its stream (given back by

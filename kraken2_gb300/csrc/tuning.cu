@@ -4,13 +4,17 @@
 // The reference fixes its scheduling: reader blocks of 3 MiB
 // (src/classify.cc:527, src/seqreader.h:101-119) and a GetBatch prefetch
 // distance of 8 keys (src/compact_hash.h:380-392).  Here the corresponding
-// choices -- how many fragments a pipeline sub-batch holds, how many probe
-// lanes serve each scanned fragment, whether a batch runs as pipeline beats
-// or on the fused work-stealing kernel, and how many lanes share a long read
-// -- depend on the table and the read lengths, so they are measured: every
-// candidate is a complete classification of the caller's batch, timed with
-// CUDA events, and the fastest is kept for that table and batch class.  No
-// value changes a result (the GPU tests compare every candidate's outputs).
+// choices depend on the table and the read lengths, so they are measured:
+// every candidate is a complete classification of the caller's batch, timed
+// with CUDA events, and the fastest is kept for that table and batch class.
+// Which choices there are depends on the kernels that take the call.  Calls
+// on tables with the default window run as one launch, whose only value is
+// the length of the pieces that long single fragments are cut into; the
+// staged and fused kernels, for other tables, take all of them: how many
+// fragments a pipeline sub-batch holds, how many probe lanes serve each
+// scanned fragment, whether a batch runs as pipeline beats or on the fused
+// work-stealing kernel, and how many lanes share a long read.  No value
+// changes a result (the GPU tests compare every candidate's outputs).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -49,14 +53,45 @@ Tuning from_abi(const k2g_tuning &t) {
   return r;
 }
 
-// The candidates for one batch class: for short reads the pipeline's probe
-// lanes per fragment and sub-batch size (and the fused kernel once); for
-// mixed and long batches the choice of pipeline or fused kernel and the
-// piece length, i.e. the lanes that share one long read.
-std::vector<Tuning> candidates(int length_class) {
+// Whether the call goes to kernels that take the staged and fused kernels'
+// values; if not, `piece` says whether they take a piece length.
+struct Route {
+  bool staged = false, piece = false;
+};
+Route route_of(const k2g_db *db, const k2g_reads *reads, const k2g_classify_params *params,
+               const k2g_results *out) {
+  Route r;
+  if (!db->opts.dna_db) return r;   // translated search takes none
+  ClassifyArgs a{};
+  set_classify_args(a, db, reads, params, out);
+  r.piece = warp_classify_takes(a, reads->max_seq_len);
+  r.staged = !r.piece;
+  return r;
+}
+
+// The candidates for one batch, the defaults of its class first.  By warps:
+// a piece length for each length that they would cut into, none among them.
+// Staged and fused: for short reads the pipeline's probe lanes per fragment
+// and sub-batch size (and the fused kernel once); for mixed and long batches
+// the choice of pipeline or fused kernel and the piece length, i.e. the lanes
+// that share one long read.
+std::vector<Tuning> candidates(int length_class, const Route &route, const k2g_reads *reads,
+                               const k2g_classify_params *params) {
   std::vector<Tuning> out;
   const Tuning base = default_tuning(length_class);
-  if (length_class == 0) {
+  if (!route.staged) {
+    std::vector<uint32_t> pieces;
+    auto add = [&](uint32_t piece_len) {
+      const uint32_t piece = warp_piece(params->paired, params->quick, reads->max_seq_len, piece_len);
+      if (std::find(pieces.begin(), pieces.end(), piece) != pieces.end()) return;
+      pieces.push_back(piece);
+      Tuning t = base;
+      t.piece_len = piece_len;
+      out.push_back(t);
+    };
+    add(base.piece_len);
+    for (uint32_t len = kPieceLenMin; route.piece && len <= kPieceLenMax; len *= 2) add(len);
+  } else if (length_class == 0) {
     for (uint32_t split : {1u, 2u, 3u})
       for (uint32_t mb : {64u, 128u, 256u, 512u}) {
         Tuning t = base;
@@ -141,10 +176,11 @@ extern "C" k2g_status k2g_autotune(k2g_db *db, const k2g_reads *reads,
   k2g_status s = K2G_OK;
   Tuning best = before;
   float best_t = -1.0f;
-  std::vector<Tuning> cands = candidates(cls);
-  // the last candidate is the best one so far with graph capture switched
-  // (added once the others have run)
-  for (size_t ci = 0; ci <= cands.size(); ci++) {
+  const Route route = route_of(db, reads, params, &trial);
+  const std::vector<Tuning> cands = candidates(cls, route, reads, params);
+  // the last candidate of the staged and fused kernels is the best one so far
+  // with graph capture switched (added once the others have run)
+  for (size_t ci = 0; ci < cands.size() + (route.staged ? 1 : 0); ci++) {
     Tuning cand;
     if (ci < cands.size()) {
       cand = cands[ci];

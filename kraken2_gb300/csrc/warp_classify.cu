@@ -37,13 +37,18 @@ bool warp_classify_takes(const ClassifyArgs &a, uint64_t max_len) {
   return a.scan.w == 5 && a.scan.revcom_version != 0 && max_len <= kWcMaxLen && sectors < (1ull << 32);
 }
 
+// Single fragments of two pieces and more are cut (quick mode stops inside a
+// fragment, and a pair carries a mate border: those stay whole).
+uint32_t warp_piece(int paired, int quick, uint64_t max_len, uint32_t piece_len) {
+  const uint32_t piece = std::min(kWarpPieces * piece_len, kPieceLenMax);
+  return !paired && !quick && max_len >= 2ull * piece ? piece : 0;
+}
+
 cudaError_t warp_classify(const ClassifyArgs &a, const uint2 *span, uint64_t max_len, uint64_t total_bases,
                           uint32_t piece_len, int device, int sms, cudaStream_t st) {
   WcArgs wa{a, span, 0, 0, 0};
-  // Single fragments of two pieces and more are cut (quick mode stops inside
-  // a fragment, and a pair carries a mate border: those stay whole).
-  const uint32_t piece = std::min(kWarpPieces * piece_len, kPieceLenMax);
-  const bool split = !a.cls.paired && !a.cls.quick && max_len >= 2ull * piece;
+  const uint32_t piece = warp_piece(a.cls.paired, a.cls.quick, max_len, piece_len);
+  const bool split = piece != 0;
   // Fragments per group: as many as keep every warp slot of the device busy
   // (kWcWarps * kWcBlocks per SM), up to about 1,600 bases (their entries
   // fill the shared-memory list once); 4 where long fragments are cut, since
