@@ -471,7 +471,7 @@ k2g_status gather(const k2g_db *db, const char *bases, const uint64_t *seq_off,
   Chunk *d_chunks;
   uint64_t *d_cand = nullptr;
   uint32_t *d_counts, *d_offs, *d_sums;
-  K2G_CUDA_TRY(s.get(&d_bases, total + 8));
+  K2G_CUDA_TRY(s.get(&d_bases, total + 16));   // (read as the 16-byte chunks that hold them)
   K2G_CUDA_TRY(s.get(&d_chunks, nc));
   K2G_CUDA_TRY(s.get(&d_blocks, blocks.size()));
   K2G_CUDA_TRY(s.get(&d_counts, nc));
