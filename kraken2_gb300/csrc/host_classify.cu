@@ -295,9 +295,12 @@ static k2g_status host_classify(const k2g_db *db, const char *bases, const char 
   // counting makes the host wait), 128 MB (64 MB with hit events) of bases or
   // 2M fragments at most, and 16 MB at least, 20 where most are long -- below
   // that a chunk's launches and copies outweigh what overlaps.  2M x 150 bp:
-  // 6 chunks 3.01 ms, 8 2.96, 12 2.89, 16 2.90; 117 MB of mixed long ones: 16
-  // MB 2.81, 20 MB 2.54, 24 MB 2.60; with hit events 1M x 150 bp: 3 to 5
-  // chunks 4.9 to 5.0, 8 5.3.
+  // 6 chunks 3.01 ms, 8 2.96, 12 2.89, 16 2.90; with hit events 1M x 150 bp: 3
+  // to 5 chunks 4.9 to 5.0, 8 5.3.  Long ones (mean 5 kb) among 150 bp, four
+  // slots, chunks of 16, 20 and 24 MB at least: 20k and 100k 2.39, 2.30, 2.28
+  // ms; 20k and 1k 2.07, 2.03, 1.99; 10k and 50k of 100 bp 1.43, 1.38, 1.42; 8k
+  // and 1k 1.06, 1.05, 1.06; 5k and 500k 2.13, 2.11, 2.12; 3k and 20k 0.74,
+  // 0.73, 0.73; 20k and 300k of 251 bp 3.24, 3.24, 3.29: 20 is never behind 16.
   const uint64_t all_bases = seq_off[n_frags * per] - seq_off[0];
   const uint64_t least = (long_batch(all_bases, n_frags) ? 20ull : 16ull) << 20;
   const uint64_t max_bases = std::min<uint64_t>(counters ? 64ull << 20 : 128ull << 20,

@@ -49,13 +49,17 @@ cudaError_t warp_classify(const ClassifyArgs &a, const uint2 *span, uint64_t max
   WcArgs wa{a, span, 0, 0, 0};
   const uint32_t piece = warp_piece(a.cls.paired, a.cls.quick, max_len, piece_len);
   const bool split = piece != 0;
-  // Fragments per group: as many as keep every warp slot of the device busy
-  // (kWcWarps * kWcBlocks per SM), up to about 1,600 bases (their entries
-  // fill the shared-memory list once); 4 where long fragments are cut, since
-  // the average says nothing of the others then.  Two that fit one scan pass
-  // cost little more than one: half the slots will do for them (5,000 x 150
-  // bp 21.1 -> 18.5 us, 8,000 of 30 to 301 bases 37.8 -> 30.7; from 3,000
-  // down no difference).
+  // Fragments per group: as many as leave 28 groups an SM, up to about 1,600
+  // bases (their entries fill the shared-memory list once); 4 where long
+  // fragments are cut, since the average says nothing of the others then.
+  // (28 an SM, two more than it holds at a time: with 26 a second wave that is
+  // nearly empty is avoided at some sizes, 7,904 x 250 bp 29.1 -> 27.0 us and
+  // 16,000 x 150 on a table within L2 31.1 -> 29.0, but the larger groups cost
+  // more at others, 16,000 x 150 on 400 MB 34.2 -> 36.7 and x 250 51.3 -> 56.0,
+  // 31,616 x 150 44.2 -> 47.1.)  Two of up to 170 bases, which one scan pass
+  // holds (two of 158) or nearly so, cost little more than one: half as many
+  // groups will do for them (5,000 x 150 bp 21.1 -> 18.5 us, x 165 20.7 -> 18.7,
+  // 8,000 of 30 to 301 bases 37.8 -> 30.7; from 3,000 down no difference).
   const double avg = (double)total_bases / (double)a.n_frags;
   const uint64_t slots = (uint64_t)sms * kWcWarps * kWcBlocks;
   while ((2u << wa.log_reads) <= (uint32_t)(split ? 4 : kWcReads) &&

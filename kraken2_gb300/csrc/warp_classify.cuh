@@ -38,9 +38,11 @@
 
 namespace k2g {
 
-// Warps per block and blocks per SM, and table sectors in flight per lane of
-// a probe: 2 x 14 and 3.  On 2M x 150 bp reads, 4 GB table: 2.30 ms; 2 x 12
-// and 4: 2.37, 2 x 12 and 5: 2.51, 2 x 16 and 2 (with half the entries): 2.38.
+// Warps per block and blocks per SM that the registers are fitted to, and table
+// sectors in flight per lane of a probe: 2 x 14 and 3.  On 2M x 150 bp reads, 4
+// GB table: 2.30 ms; 2 x 12 and 4: 2.37, 2 x 12 and 5: 2.51, 2 x 16 and 2 (with
+// half the entries): 2.38.  An SM holds 13 blocks of them, 26 warps: a block's
+// shared memory is 15.6 KB and 1 KB goes with it, of 228.
 constexpr int kWcWarps = 2, kWcBlocks = 14;
 constexpr int kWcReads = 8;           // most fragments per group
 constexpr int kWcEntries = 320;       // entries held before a probe and replay
