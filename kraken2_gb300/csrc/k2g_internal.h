@@ -115,7 +115,7 @@ struct k2g_db {
   char *d_names = nullptr;
   uint32_t *d_parent = nullptr;   // node_count entries
   bool blank = false;             // created, and nothing inserted yet: all cells are zero
-  bool one_root = false;          // every taxon but 1 has a parent: no LCA is 0
+  bool one_root = false;          // every taxon but 1 has a parent: no LCA of two is 0
   uint2 *d_span = nullptr;        // per node: preorder number, one past its subtree's last
                                   // (d_parent follows in the same allocation)
   uint64_t *d_size = nullptr;     // device-side size counter used by builds
@@ -153,7 +153,7 @@ k2g_status classify_translated(const k2g_db *db, const k2g_reads *reads,
 struct ClassifyArgs;
 void set_classify_args(ClassifyArgs &a, const k2g_db *db, const k2g_reads *reads,
                        const k2g_classify_params *params, const k2g_results *out);
-bool warp_classify_takes(const ClassifyArgs &a, uint64_t max_len);
+bool warp_classify_takes(const k2g_db *db, const ClassifyArgs &a, uint64_t max_len);
 uint32_t warp_piece(int paired, int quick, uint64_t max_len, uint32_t piece_len);
 cudaError_t warp_classify(const ClassifyArgs &a, const uint2 *span, uint64_t max_len, uint64_t total_bases,
                           uint32_t piece_len, int device, int sms, cudaStream_t st);

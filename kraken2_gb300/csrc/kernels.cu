@@ -945,7 +945,7 @@ k2g_status k2g::classify_keyed(const k2g_db *db, const k2g_reads *reads,
     total = ends[1] - ends[0];
   }
   const Tuning tn = db->tuning(params->paired != 0, total, reads->n_frags);
-  if (mode == K2G_MODE_PIPELINED && warp_classify_takes(a, reads->max_seq_len)) {
+  if (mode == K2G_MODE_PIPELINED && warp_classify_takes(db, a, reads->max_seq_len)) {
     K2G_CUDA_TRY(warp_classify(a, db->d_span, reads->max_seq_len, total, tn.piece_len, db->device,
                                sm_count(db->device), st));
     return K2G_OK;

@@ -103,14 +103,15 @@ cudaError_t launch_warp(const TxWarpArgs &wa, cudaStream_t st) {
 
 // The warp form (warp_translated.cuh) takes the default window (k - l = 3);
 // it reads bases and qualities as the same 16-byte chunks.
-bool warp_takes(const TableView &t, const ScanView &sv, const k2g_reads *reads,
+bool warp_takes(const k2g_db *db, const TableView &t, const ScanView &sv, const k2g_reads *reads,
                 const k2g_classify_params *params) {
   const uint64_t max_len = reads->max_seq_len;
   if (reads->d_quals && params->min_quality > 0 &&
       (((uintptr_t)reads->d_bases - (uintptr_t)reads->d_quals) & 15u))
     return false;
-  // (a walk that goes on keeps its sector's number in 32 bits)
-  return sv.w == 4 && max_len <= kTxMaxLen && t.capacity / (t.wide ? 4 : 8) < (1ull << 32);
+  // (a walk that goes on keeps its sector's number in 32 bits; several roots
+  // are resolved taxon by taxon, as in warp_classify_takes)
+  return db->one_root && sv.w == 4 && max_len <= kTxMaxLen && t.capacity / (t.wide ? 4 : 8) < (1ull << 32);
 }
 
 }  // namespace
@@ -123,7 +124,7 @@ k2g_status classify_translated(const k2g_db *db, const k2g_reads *reads,
   if (reads->max_seq_len > (1u << 30)) return fail(K2G_ERR_ARG, "sequence too long");
   int sms = 0;
   K2G_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, db->device));
-  if (warp_takes(db->table_view(), sv, reads, params)) {
+  if (warp_takes(db, db->table_view(), sv, reads, params)) {
     ClassifyArgs c{};
     set_classify_args(c, db, reads, params, out);
     TxWarpArgs wa{c, db->d_span, 0, 0, reads->max_seq_len};

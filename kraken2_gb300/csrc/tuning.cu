@@ -64,7 +64,7 @@ Route route_of(const k2g_db *db, const k2g_reads *reads, const k2g_classify_para
   if (!db->opts.dna_db) return r;   // translated search takes none
   ClassifyArgs a{};
   set_classify_args(a, db, reads, params, out);
-  r.piece = warp_classify_takes(a, reads->max_seq_len);
+  r.piece = warp_classify_takes(db, a, reads->max_seq_len);
   r.staged = !r.piece;
   return r;
 }

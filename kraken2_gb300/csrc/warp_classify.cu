@@ -31,10 +31,12 @@ cudaError_t launch(const WcArgs &wa, cudaStream_t st) {
 
 }  // namespace
 
-bool warp_classify_takes(const ClassifyArgs &a, uint64_t max_len) {
-  // (a walk that goes on keeps its sector's number in 32 bits)
+bool warp_classify_takes(const k2g_db *db, const ClassifyArgs &a, uint64_t max_len) {
+  // (a walk that goes on keeps its sector's number in 32 bits; with several
+  // roots the LCA of taxa one after another is not that of all: an LCA of 0
+  // and the next taxon give the taxon)
   const uint64_t sectors = a.table.capacity / (a.table.wide ? 4 : 8);
-  return a.scan.w == 5 && a.scan.revcom_version != 0 && max_len <= kWcMaxLen && sectors < (1ull << 32);
+  return db->one_root && a.scan.w == 5 && a.scan.revcom_version != 0 && max_len <= kWcMaxLen && sectors < (1ull << 32);
 }
 
 // Single fragments of two pieces and more are cut (quick mode stops inside a
