@@ -93,12 +93,21 @@ __global__ void translated_kernel(TxArgs a) {
   }
 }
 
-template <bool WIDE, bool HITS>
+template <bool WIDE, bool HITS, class Shared>
 cudaError_t launch_warp(const TxWarpArgs &wa, cudaStream_t st) {
   const uint64_t blocks = (wa.n_groups + kWcWarps - 1) / kWcWarps;
-  warp_translated_kernel<WIDE, HITS><<<(unsigned)blocks, kWcWarps * 32, kWcWarps * sizeof(TxShared), st>>>(wa);
+  warp_translated_kernel<WIDE, HITS, Shared>
+      <<<(unsigned)blocks, kWcWarps * 32, kWcWarps * sizeof(Shared), st>>>(wa);
   note_launches();
   return cudaGetLastError();
+}
+
+template <class Shared>
+cudaError_t launch(const TxWarpArgs &wa, cudaStream_t st) {
+  const bool hits = wa.a.hit_keys != nullptr;
+  if (wa.a.table.wide)
+    return hits ? launch_warp<true, true, Shared>(wa, st) : launch_warp<true, false, Shared>(wa, st);
+  return hits ? launch_warp<false, true, Shared>(wa, st) : launch_warp<false, false, Shared>(wa, st);
 }
 
 // The warp form (warp_translated.cuh) takes the default window (k - l = 3);
@@ -133,9 +142,8 @@ k2g_status classify_translated(const k2g_db *db, const k2g_reads *reads,
     if (!params->paired && reads->max_seq_len <= 200 && reads->n_frags / 2 >= (uint64_t)sms * kWcWarps * 10)
       wa.log_reads = 1;
     wa.n_groups = (reads->n_frags + (1ull << wa.log_reads) - 1) >> wa.log_reads;
-    const bool hits = c.hit_keys != nullptr;
-    const cudaError_t e = c.table.wide ? (hits ? launch_warp<true, true>(wa, st) : launch_warp<true, false>(wa, st))
-                                       : (hits ? launch_warp<false, true>(wa, st) : launch_warp<false, false>(wa, st));
+    const bool many = reads->max_seq_len * (params->paired ? 2 : 1) >= kTxManyBases;
+    const cudaError_t e = many ? launch<TxSharedMany>(wa, st) : launch<TxShared>(wa, st);
     return e == cudaSuccess ? K2G_OK : cuda_fail(e, "warp_translated_kernel");
   }
   TxArgs a{};

@@ -13,20 +13,21 @@ namespace {
 // the others of its SM, so the last pieces to run do not keep the device long.
 constexpr uint32_t kWarpPieces = 4;
 
-template <bool WIDE, bool HITS, bool LONG>
+template <bool WIDE, bool HITS, bool LONG, class Shared>
 cudaError_t launch_warp(const WcArgs &wa, cudaStream_t st) {
   const uint64_t blocks = (wa.piece_slots + wa.n_groups + kWcWarps - 1) / kWcWarps;
-  warp_classify_kernel<WIDE, HITS, LONG>
-      <<<(unsigned)blocks, kWcWarps * 32, kWcWarps * sizeof(WcShared), st>>>(wa);
+  warp_classify_kernel<WIDE, HITS, LONG, Shared>
+      <<<(unsigned)blocks, kWcWarps * 32, kWcWarps * sizeof(Shared), st>>>(wa);
   note_launches();
   return cudaGetLastError();
 }
 
-template <bool LONG>
+template <bool LONG, class Shared>
 cudaError_t launch(const WcArgs &wa, cudaStream_t st) {
   const bool hits = wa.a.hit_keys != nullptr;
-  if (wa.a.table.wide) return hits ? launch_warp<true, true, LONG>(wa, st) : launch_warp<true, false, LONG>(wa, st);
-  return hits ? launch_warp<false, true, LONG>(wa, st) : launch_warp<false, false, LONG>(wa, st);
+  if (wa.a.table.wide)
+    return hits ? launch_warp<true, true, LONG, Shared>(wa, st) : launch_warp<true, false, LONG, Shared>(wa, st);
+  return hits ? launch_warp<false, true, LONG, Shared>(wa, st) : launch_warp<false, false, LONG, Shared>(wa, st);
 }
 
 }  // namespace
@@ -69,7 +70,8 @@ cudaError_t warp_classify(const ClassifyArgs &a, const uint2 *span, uint64_t max
          (split || avg * (double)(2u << wa.log_reads) <= 1600.0))
     wa.log_reads++;
   wa.n_groups = (a.n_frags + (1ull << wa.log_reads) - 1) >> wa.log_reads;
-  if (!split) return launch<false>(wa, st);
+  if (!split && max_len * (a.cls.paired ? 2 : 1) >= kManyBases) return launch<false, WcSharedMany>(wa, st);
+  if (!split) return launch<false, WcShared>(wa, st);
 
   const uint64_t pc = split_pieces_cap(total_bases, piece), fc = split_frags_cap(total_bases, piece);
   const size_t at_pieces = 64, at_frags = at_pieces + pc * sizeof(SplitPiece),
@@ -87,7 +89,7 @@ cudaError_t warp_classify(const ClassifyArgs &a, const uint2 *span, uint64_t max
     wa.a.n_pieces = b.ctr;
     wa.a.split_mark = b.mark;
     wa.piece_slots = pc;
-    e = launch<true>(wa, st);
+    e = launch<true, WcShared>(wa, st);
   }
   if (e == cudaSuccess) {
     const uint64_t blocks = std::min<uint64_t>((fc + kMergeWarps - 1) / kMergeWarps, (uint64_t)sms * 12);

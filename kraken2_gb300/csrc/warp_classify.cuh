@@ -86,12 +86,23 @@ struct WcBase {
 // ... and the packed bases of the nucleotide scan.  After a scan the same
 // words list the entries whose walk goes on (16 bits each).
 struct WcShared : WcBase {
-  static constexpr bool kFrames = false;
+  static constexpr bool kFrames = false, kMany = false;
   uint32_t be[kWcWindow / 16 + 4];
   uint32_t le[kWcWindow / 16 + 4];    // [3] holds the window's first word
   uint32_t inv[kWcWindow / 32 + 4];   // bit per base: not A/C/G/T; [2] is the first word
   __device__ __forceinline__ uint16_t *list() { return reinterpret_cast<uint16_t *>(be); }
 };
+
+// The same for fragments of kManyBases and more that stay whole (pairs): those
+// with more taxa than a map in shared memory holds are resolved from a map in
+// their run region (wc_resolve_many).  A type of its own, since the mere call
+// made the other kernels up to 1 % slower; shorter ones gain nothing by it
+// (5,000 pairs of 2 x 2 kb with a taxon a k-mer 1.11 and 1.12 ms, 1,000 of 2 x
+// 10 kb 41.9 and 10.5).
+struct WcSharedMany : WcShared {
+  static constexpr bool kMany = true;
+};
+constexpr uint64_t kManyBases = 8192;
 
 __device__ __forceinline__ uint32_t below(int n) { return n >= 32 ? 0xFFFFFFFFu : (1u << n) - 1u; }
 __device__ __forceinline__ int last_bit(uint32_t m) { return 31 - __clz(m); }
@@ -397,6 +408,40 @@ __device__ __forceinline__ uint32_t wc_resolve_slots(const uint32_t *parent, con
   __syncwarp();
   const uint2 x = (int)lane < n ? list[lane] : make_uint2(0, 0);
   return wc_resolve(parent, span, x.x, x.y, n, required);
+}
+
+// ResolveTree from a fragment's runs, for one with more taxa than any map in
+// shared memory holds: a map in the unused part of its run region of `region`
+// words -- left zero -- or, where that is too small, the runs themselves (200
+// pairs of 2 x 50 kb with thousands of taxa each: 905 ms from the runs alone,
+// 42 with the map).
+static __device__ __noinline__ uint32_t wc_resolve_many(const uint32_t *parent, const uint2 *span, uint64_t *runs,
+                                                        uint32_t count, uint32_t region, uint32_t required) {
+  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t room = region > count ? region - count : 0;
+  uint32_t slots = 32;
+  while (slots < 65536 && 2 * slots <= room) slots *= 2;
+  if (slots <= room) {
+    uint64_t *at = runs + count;
+    uint32_t *mem = reinterpret_cast<uint32_t *>(at);
+    const WcMap big{mem, mem + 1, slots - 1, 2};
+    for (uint32_t i = lane; i < slots; i += 32) at[i] = 0;
+    __syncwarp();
+    bool full = false;
+    for (uint32_t i = lane; i < count; i += 32) {
+      const uint2 x = wc_run(runs, i);
+      if (x.x && big.add(x.x, x.y) == 0xFFFFFFFFu) full = true;
+    }
+    __syncwarp();
+    uint32_t call = 0;
+    full = __any_sync(0xffffffffu, full);
+    if (!full) call = wc_resolve_map(parent, span, big, required);
+    __syncwarp();
+    for (uint32_t i = lane; i < slots; i += 32) at[i] = 0;
+    __syncwarp();
+    if (!full) return call;
+  }
+  return wc_resolve_runs(parent, span, runs, count, required);
 }
 
 // ---- the kernel --------------------------------------------------------------
@@ -783,8 +828,17 @@ struct Wc {
         }
         __syncwarp();
         added = __reduce_add_sync(0xffffffffu, added);
-        if (__any_sync(0xffffffffu, full)) got = wc_resolve_runs(a.parent, span, a.runs + base, n, need);
-        else got = wc_resolve_slots(a.parent, span, big, added, list, need);
+        if (__any_sync(0xffffffffu, full)) {
+          if constexpr (Shared::kMany) {
+            const uint64_t f = f0 + r, per = a.cls.paired ? 2 : 1;
+            const uint64_t end = base + (a.seq_off[(f + 1) * per] - a.seq_off[f * per]) + 2;
+            got = wc_resolve_many(a.parent, span, a.runs + base, n, (uint32_t)(min(end, a.runs_cap) - base), need);
+          } else {
+            got = wc_resolve_runs(a.parent, span, a.runs + base, n, need);
+          }
+        } else {
+          got = wc_resolve_slots(a.parent, span, big, added, list, need);
+        }
       }
       __syncwarp();
       if (lane == (int)r) call = got;
@@ -802,8 +856,9 @@ struct Wc {
   }
 };
 
-// LONG: the call's long fragments come as pieces.
-template <bool WIDE, bool HITS, bool LONG>
+// LONG: the call's long fragments come as pieces.  Shared: WcShared, or
+// WcSharedMany where long ones stay whole.
+template <bool WIDE, bool HITS, bool LONG, class Shared>
 __global__ void __launch_bounds__(kWcWarps * 32, kWcBlocks) warp_classify_kernel(WcArgs wa) {
   extern __shared__ __align__(16) unsigned char smem[];
   const ClassifyArgs &a = wa.a;
@@ -826,14 +881,14 @@ __global__ void __launch_bounds__(kWcWarps * 32, kWcBlocks) warp_classify_kernel
     if (task >= wa.n_groups) return;
     f0 = task << wa.log_reads;
   }
-  WcShared &s = reinterpret_cast<WcShared *>(smem)[threadIdx.x >> 5];
+  Shared &s = reinterpret_cast<Shared *>(smem)[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const uint32_t lt = (1u << lane) - 1u, le = lt | (1u << lane);
   const int k = a.scan.k, l = a.scan.l;
   const int nr = piece ? 1 : (int)min((uint64_t)1 << wa.log_reads, a.n_frags - f0);
   const int per = a.cls.paired ? 2 : 1, ns = nr * per;
   const uint32_t key_shift = 64u - 2u * (uint32_t)l;
-  Wc<WIDE, HITS, WcShared> w{a, s, lane, lt, f0, piece ? kWcLogSlots : kWcLogSlots - wa.log_reads, first_pos, key_shift,
+  Wc<WIDE, HITS, Shared> w{a, s, lane, lt, f0, piece ? kWcLogSlots : kWcLogSlots - wa.log_reads, first_pos, key_shift,
                    a.scan.toggle << key_shift};
   const uint64_t mask_top = (a.scan.spaced_mask ? a.scan.spaced_mask & a.scan.lmer_mask : a.scan.lmer_mask)
                             << key_shift;
@@ -1137,27 +1192,9 @@ warp_merge_kernel(ClassifyArgs a, const uint2 *span, SplitBufs b) {
     added = __reduce_add_sync(0xffffffffu, added);
     uint32_t call = 0;
     if (__any_sync(0xffffffffu, full)) {
-      // too many taxa for the map: one in the unused part of the run region
-      const uint64_t end = min(base + len + 2, a.runs_cap), free0 = base + w;
-      const uint64_t room = end > free0 ? end - free0 : 0;
-      uint32_t slots = 32;
-      while (slots < 65536 && 2ull * slots <= room) slots *= 2;
       const uint32_t n = base >= a.runs_cap ? 0u : (uint32_t)min((uint64_t)w, a.runs_cap - base);
-      bool over = slots > room;
-      if (!over) {
-        uint32_t *mem = reinterpret_cast<uint32_t *>(a.runs + free0);
-        const WcMap big{mem, mem + 1, slots - 1, 2};
-        for (uint32_t i = lane; i < slots; i += 32) a.runs[free0 + i] = 0;
-        __syncwarp();
-        for (uint32_t i = lane; i < n; i += 32) {
-          const uint2 x = wc_run(a.runs + base, i);
-          if (x.x && big.add(x.x, x.y) == 0xFFFFFFFFu) over = true;
-        }
-        __syncwarp();
-        over = __any_sync(0xffffffffu, over);
-        if (!over) call = wc_resolve_map(a.parent, span, big, required);
-      }
-      if (over) call = wc_resolve_runs(a.parent, span, a.runs + base, n, required);
+      call = wc_resolve_many(a.parent, span, a.runs + base, n, base < a.runs_cap ? (uint32_t)(min(base + len + 2, a.runs_cap) - base) : 0u,
+                             required);
     } else if (added) {
       call = wc_resolve_slots(a.parent, span, small, added, s.list, required);
     }

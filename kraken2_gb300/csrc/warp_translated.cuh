@@ -31,7 +31,7 @@ constexpr int kTxWords = kTxResidues / 8;
 constexpr uint64_t kTxMaxLen = 1ull << 24;
 
 struct TxShared : WcBase {
-  static constexpr bool kFrames = true;
+  static constexpr bool kFrames = true, kMany = false;
   uint32_t bases[kTxBases / 16 + 4];              // 2 bits per base, first base low
   uint32_t inv[kTxBases / 32 + 4];                // bit per base: not A/C/G/T
   // per class: residues of the codons (8 a word, the first one high; [4] is
@@ -44,6 +44,12 @@ struct TxShared : WcBase {
   uint32_t mate_len[4];
   __device__ __forceinline__ uint16_t *list() { return reinterpret_cast<uint16_t *>(fwd); }
 };
+
+// (as WcSharedMany, from kTxManyBases on: six frames give more runs a base)
+struct TxSharedMany : TxShared {
+  static constexpr bool kMany = true;
+};
+constexpr uint64_t kTxManyBases = 4096;
 
 struct TxWarpArgs {
   ClassifyArgs a;
@@ -119,7 +125,7 @@ __device__ __forceinline__ void tx_pack_residues(S &s, const uint8_t *lut, uint3
   }
 }
 
-template <bool WIDE, bool HITS>
+template <bool WIDE, bool HITS, class Shared>
 __global__ void __launch_bounds__(kWcWarps * 32, 10) warp_translated_kernel(TxWarpArgs wa) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ uint8_t lut[64];   // codon (first base low) -> residue, and of its complement << 4
@@ -136,7 +142,7 @@ __global__ void __launch_bounds__(kWcWarps * 32, 10) warp_translated_kernel(TxWa
   const ClassifyArgs &a = wa.a;
   const uint64_t group = blockIdx.x * (uint64_t)kWcWarps + (threadIdx.x >> 5);
   if (group >= wa.n_groups) return;
-  TxShared &s = reinterpret_cast<TxShared *>(smem)[threadIdx.x >> 5];
+  Shared &s = reinterpret_cast<Shared *>(smem)[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const uint32_t lt = (1u << lane) - 1u, le = lt | (1u << lane);
   const int k = a.scan.k, l = a.scan.l;
@@ -144,7 +150,7 @@ __global__ void __launch_bounds__(kWcWarps * 32, 10) warp_translated_kernel(TxWa
   const int nr = (int)min((uint64_t)1 << wa.log_reads, a.n_frags - f0);
   const int per = a.cls.paired ? 2 : 1, nm = nr * per, ns = 6 * nm;
   const uint32_t key_shift = 64u - 4u * (uint32_t)l;
-  Wc<WIDE, HITS, TxShared> w{a, s, lane, lt, f0, kWcLogSlots - wa.log_reads, 0u, key_shift,
+  Wc<WIDE, HITS, Shared> w{a, s, lane, lt, f0, kWcLogSlots - wa.log_reads, 0u, key_shift,
                              a.scan.toggle << key_shift};
   const uint64_t mask_top = (a.scan.spaced_mask ? a.scan.spaced_mask & a.scan.lmer_mask : a.scan.lmer_mask)
                             << key_shift;
