@@ -599,9 +599,14 @@ static k2g_status build_sequences(k2g_db *db, const char *bases, const uint64_t 
   uint32_t *d_btax;
   K2G_CUDA_TRY(s.get(&d_btax, nb));
   K2G_CUDA_TRY(cudaMemcpyAsync(d_btax, g.block_taxon.data(), nb * 4, cudaMemcpyHostToDevice, st));
-  // (a thread block holds the candidates of a sequence block up to 25,600,
-  // at least those of 16,384 k-mer starts; larger ones go to radix passes)
-  if (scans_by_warps(db->scan_view()) && g.largest <= kLargeBlock) {
+  // A thread block holds the candidates of a sequence block up to 25,600, at
+  // least those of 16,384 k-mer starts; larger ones go to radix passes.  So do
+  // batches of short sequences, where a thread block has little to sort: 400k
+  // of 60 bases (9 candidates each) take 8.2 ms by blocks and 6.5 by passes,
+  // 240k of 100 (22 each) 5.2 and 5.0, 80k of 300 (88) 2.3 and 3.4, 24k of
+  // 1,000 (318) 1.4 and 2.9.
+  constexpr uint64_t kFewCandidates = 24;   // a block
+  if (scans_by_warps(db->scan_view()) && g.largest <= kLargeBlock && n >= kFewCandidates * nb) {
     uint64_t *keys = nullptr, n_pairs = 0;
     uint32_t *taxa = nullptr;
     r = sort_blocks(db, g, s, d_btax, &keys, &taxa, &n_pairs, st);
