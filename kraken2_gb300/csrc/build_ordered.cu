@@ -27,10 +27,12 @@
 // unordered pass marks the cells that pairs were moved to, and only the pairs
 // of clusters with marks are sorted and replayed: three in ten of the 15.7M of
 // 48 Mbp at a load of 0.26 (whole build 4.9 -> 3.9 ms), nearly all at 0.85
-// (14.7 -> 14.3).
+// (14.7 -> 14.3) -- unless step 4 is likely, which needs all of them
+// (merges_expected).
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <vector>
 
 #include "k2g_device.cuh"
@@ -370,6 +372,22 @@ int bits_of(uint64_t x) {
   return b;
 }
 
+// Whether some cluster of a batch of n pairs is likely to need a merged replay,
+// for which all pairs have to be sorted; then the pairs of clusters with marks
+// are not sorted first.  Where the first such clusters appear at loads of 0.40,
+// 0.66 and 0.85, for 1.3M to 157M pairs and 10 to 22 key bits, fits their number
+// going with n / 4^key_bits and the power 5.3 of 1 / (1 - load).  The line lies
+// where the sort in vain costs as much as the picking gains: of 15.7M pairs at
+// 0.66 the picking took 6.6 ms with 12 bits, where some need it, 5.1 all sorted;
+// with 13, where none do, 5.0 and 5.1; at 0.85 14.1 and 11.4 with 16 bits, 10.2
+// and 11.1 with 22; at 0.40 4.5 and 3.9 with 10, 3.2 and 3.7 with 11; of 157M at
+// 0.66 72.6 and 61.2 with 13, 58.8 and 60.3 with 14.
+bool merges_expected(uint64_t n, uint64_t size, uint64_t capacity, uint32_t key_bits) {
+  const double free_share = std::max(1.0 - (double)size / (double)capacity, 0.01);
+  const double expected = 0.005 * std::ldexp((double)n, -2 * (int)key_bits) / std::pow(free_share, 5.3);
+  return expected > 0.38;
+}
+
 template <class T>
 struct DevBuf {
   int device;
@@ -419,10 +437,13 @@ k2g_status insert_ordered(k2g_db *db, typename C::T *cells, const uint64_t *d_ke
   K2G_CUDA_TRY(insert_unordered(db, d_keys, d_taxids, n, status.p, moved.p, st));
   uint32_t st_word = 0;
   unsigned long long n_flags = 0;
+  uint64_t size = 0;
   K2G_CUDA_TRY(cudaMemcpyAsync(&st_word, status.p, 4, cudaMemcpyDeviceToHost, st));
+  K2G_CUDA_TRY(cudaMemcpyAsync(&size, db->d_size, 8, cudaMemcpyDeviceToHost, st));
   K2G_CUDA_TRY(cudaStreamSynchronize(st));
   const k2g_status s = insert_status(st_word);
   if (s != K2G_OK) return s;
+  const bool pick = db->one_root && !merges_expected(n, size, cap, (uint32_t)db->key_bits);
   K2G_CUDA_TRY(cudaMemsetAsync(status.p, 0, 4, st));
   K2G_CUDA_TRY(cudaMemsetAsync(ctr.p, 0, 16, st));
   occ_kernel<C><<<grid(db->device, 8 * words), 256, 0, st>>>(cells, t, occ.p);
@@ -471,7 +492,7 @@ k2g_status insert_ordered(k2g_db *db, typename C::T *cells, const uint64_t *d_ke
     K2G_CUDA_TRY(cudaGetLastError());
     return sort_pairs();
   };
-  const k2g_status by = db->one_root ? sort_picked() : sort_all();
+  const k2g_status by = pick ? sort_picked() : sort_all();
   if (by != K2G_OK) return by;
   // 3. per-cluster replays
   if (n_sorted) {
@@ -486,7 +507,7 @@ k2g_status insert_ordered(k2g_db *db, typename C::T *cells, const uint64_t *d_ke
   if (n_flags > kFlagCap) return fail(K2G_ERR_BUDGET, "too many clusters need a merged replay");
   // 4. merged replays of flagged clusters, in cluster order
   if (n_flags) {
-    if (db->one_root) {   // (their neighbours may be clusters without marks)
+    if (pick) {   // (their neighbours may be clusters without marks)
       keys.free();
       alt.free();
       hist.free();

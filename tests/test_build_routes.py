@@ -30,3 +30,25 @@ def test_sort_by_candidates_a_block(per_block, by_blocks):
         assert (f.launches("bucket_sort_kernel") > 0) == by_blocks
         assert (f.launches("pair_scatter_kernel") > 0) == (not by_blocks)
         db.close()
+
+
+@pytest.mark.parametrize("key_bits,load,n,pick", [
+    (22, 0.26, 20_000, True), (22, 0.85, 20_000, True), (8, 0.4, 20_000, True), (6, 0.4, 40_000, False),
+    (10, 0.66, 20_000, True), (8, 0.66, 20_000, False), (12, 0.85, 20_000, True), (9, 0.85, 20_000, False),
+    (10, 0.66, 400_000, False), (22, 1.0, 20_000, True), (6, 1.0, 20_000, False)])
+def test_pairs_are_picked_unless_merges_are_expected(key_bits, load, n, pick):
+    with fake_cuda() as f:
+        capacity = 1_000_003
+        db = k2g.Database.create(k2g.IndexOptions(35, 31, 0, 0, 1, 1, 0), capacity, key_bits, 32 - key_bits, PARENT,
+                                 device=59)
+
+        def inserted(name, args):    # the size after the unordered pass
+            if "13insert_kernel" in name:
+                size = C.cast(args[7], C.POINTER(C.c_void_p))[0]
+                C.cast(size, C.POINTER(C.c_uint64))[0] = int(load * capacity)
+
+        f.hook(inserted)
+        db.build_insert(f.device(np.arange(n, dtype=np.uint64)), f.device(np.ones(n, np.uint32)), n, True, f.stream())
+        assert (f.launches("11pick_kernel") > 0) == pick
+        assert (f.launches("13region_kernel") > 0) == (not pick)
+        db.close()
