@@ -63,11 +63,38 @@ __device__ __forceinline__ void sort_zone(uint64_t *z, uint32_t m) {
   for (; d < m; d++) z[d] = kNoKey;
 }
 
-// One warp: the same for a zone of any size, by a bitonic sort whose every
-// exchange puts the lesser key first (keys past m count as the greatest);
-// kNoKey takes the place of repeats.
+// One warp: the same for a zone of any size.  Most are large by repeats of a few
+// keys, which are taken out first, one after another, as long as each makes up a
+// sixteenth of what is left (28M keys of 10,000 distinct ones 5.69 -> 0.81 ms); the
+// rest and one of each are sorted by a bitonic sort whose every exchange puts the
+// lesser key first (keys past m count as the greatest); kNoKey takes the place of
+// repeats.
 __device__ __forceinline__ void sort_big_zone(uint64_t *z, uint32_t m) {
   const uint32_t lane = threadIdx.x & 31;
+  {
+    uint32_t left = m, taken = 0, gone = m;
+    uint64_t mine = kNoKey;   // lane i: the i-th key taken out
+    while (left > 32 && taken < 32 && gone * 16 >= left) {
+      const uint64_t key = z[0];
+      __syncwarp();
+      uint32_t kept = 0;
+      for (uint32_t i0 = 0; i0 < left; i0 += 32) {
+        const uint64_t x = i0 + lane < left ? z[i0 + lane] : key;
+        const uint32_t others = __ballot_sync(0xffffffffu, x != key);
+        if (x != key) z[kept + __popc(others & ((1u << lane) - 1))] = x;
+        kept += __popc(others);
+        __syncwarp();
+      }
+      if (lane == taken) mine = key;
+      taken++;
+      gone = left - kept;
+      left = kept;
+    }
+    if (lane < taken) z[left + lane] = mine;
+    for (uint32_t i = left + taken + lane; i < m; i += 32) z[i] = kNoKey;
+    m = left + taken;
+    __syncwarp();
+  }
   auto exchange = [&](uint32_t a, uint32_t b) {
     if (b >= m) return;
     const uint64_t x = z[a], y = z[b];
@@ -218,8 +245,20 @@ bucket_count_kernel(const uint64_t *k, uint64_t n, uint64_t slice, int shift, ui
   const uint64_t i0 = min(n, blockIdx.x * slice), i1 = min(n, i0 + slice);
   for (uint32_t b = threadIdx.x; b < nb; b += kDealThreads) h[b] = 0;
   __syncthreads();
+  // (a thread adds up a bucket's keys while they follow one another: one key
+  // over and over would leave the additions to one address)
+  uint32_t last = 0, run = 0;
 #pragma unroll 4
-  for (uint64_t i = i0 + threadIdx.x; i < i1; i += kDealThreads) atomicAdd(&h[k[i] >> shift], 1u);
+  for (uint64_t i = i0 + threadIdx.x; i < i1; i += kDealThreads) {
+    const uint32_t b = (uint32_t)(k[i] >> shift);
+    if (b != last) {
+      if (run) atomicAdd(&h[last], run);
+      last = b;
+      run = 0;
+    }
+    run++;
+  }
+  if (run) atomicAdd(&h[last], run);
   __syncthreads();
   for (uint32_t b = threadIdx.x; b < nb; b += kDealThreads)
     if (h[b]) atomicAdd(&count[b], h[b]);
@@ -240,10 +279,12 @@ __global__ void bucket_cursor_kernel(const uint32_t *start, uint32_t per, uint32
 
 // Parent p holds keys[start[p * per], start[(p + 1) * per]); its keys go to the
 // `digits` (a power of two) cursors cursor[p * digits ..] by the bits from
-// shift up.  Block b works on parent b % parents.
+// shift up.  Block b works on parent b % parents.  Nothing is dealt where the
+// largest bucket is too large to be sorted.
 __global__ void __launch_bounds__(kDealThreads)
 bucket_deal_kernel(const uint64_t *keys, const uint32_t *start, uint32_t parents, uint32_t per, int shift,
-                   uint32_t digits, uint32_t *cursor, uint64_t *out) {
+                   uint32_t digits, const uint32_t *largest, uint32_t *cursor, uint64_t *out) {
+  if (*largest > kLargeBlock) return;
   extern __shared__ __align__(16) unsigned char smem[];
   uint64_t *s_key = reinterpret_cast<uint64_t *>(smem);
   constexpr int kMost = 1 << (kDealDigit > kDealDigitMost ? kDealDigit : kDealDigitMost);
@@ -321,7 +362,8 @@ struct BucketMem {
 
 // Deals keys[0, n) (n < 2^32, each key >> shift below nb = 2^bits, bits <=
 // kDealBits) into buckets, bucket b at start[b]: in alt, or back in keys where
-// that took two steps (*dealt).  *largest: the largest bucket.
+// that took two steps (*dealt).  *largest: the largest bucket; above kLargeBlock
+// the keys stay where they are.
 inline cudaError_t deal_to_buckets(uint64_t *keys, uint64_t *alt, uint64_t n, int shift, int bits, const BucketMem &m,
                                    int device, uint64_t **dealt, uint32_t *largest, cudaStream_t st) {
   cudaError_t e;
@@ -346,7 +388,7 @@ inline cudaError_t deal_to_buckets(uint64_t *keys, uint64_t *alt, uint64_t n, in
     const uint64_t tiles = n / parents / kDealTile + 1;
     const uint32_t each = (uint32_t)std::min<uint64_t>(tiles, (2 * sms + parents - 1) / parents);
     bucket_deal_kernel<<<parents * each, kDealThreads, kDealTile * 8, st>>>(in, m.start, parents, m.nb / parents, at,
-                                                                            digits, m.place, out);
+                                                                            digits, m.largest, m.place, out);
     note_launches(2);
   };
   step(keys, alt, 1, bits - low, shift + low);
