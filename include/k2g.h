@@ -175,7 +175,8 @@ typedef struct {
   /* Hit-list runs, (code << 32 | count), the RLE of the per-k-mer taxa list
    * printed by AddHitlistString.  Fragment i's runs start at index
    * d_seq_off[i * (paired ? 2 : 1)] + 2 * i, so runs_cap must be at least
-   * d_seq_off[n_seqs] + 2 * n_frags. */
+   * d_seq_off[n_seqs] + 2 * n_frags.  What lies behind a fragment's runs, up
+   * to the next fragment's, is scratch of the call. */
   uint64_t *d_runs;
   uint64_t runs_cap;
   uint64_t *d_taxon_reads;    /* [node_count] += calls per taxon, or NULL   */
@@ -196,9 +197,10 @@ typedef enum {
   K2G_MODE_PLAIN = 0,         /* fused kernel, one thread per fragment      */
   K2G_MODE_PERSISTENT = 1,    /* fused kernel, work-stealing lanes          */
   K2G_MODE_PIPELINED = 2      /* the fastest form.  Tables with k - l = 4
-                                 (the default): one launch on the caller's
-                                 stream, a warp per group of fragments, long
-                                 single fragments in pieces.  Other tables:
+                                 (the default) and a taxonomy of one root:
+                                 one launch on the caller's stream, a warp
+                                 per group of fragments, long single
+                                 fragments in pieces.  Other tables:
                                  scan / probe / resolve stages over
                                  overlapping sub-batches; long fragments go
                                  to the fused kernel, and a batch averaging
@@ -223,7 +225,7 @@ k2g_status k2g_classify(const k2g_db *db, const k2g_reads *reads,
  * k2g_classify call uses the set of its batch's class.  The values change
  * only how the work is scheduled, never a result.  Which of them a call
  * uses depends on its kernels: the one-launch form of K2G_MODE_PIPELINED
- * (tables with k - l = 4) uses piece_len only, translated search none; the
+ * (see k2g_mode) uses piece_len only, translated search none; the
  * staged and fused kernels use all of them.  A table starts with
  * pipeline 1 for short batches and 0 otherwise, probe_split 2,
  * sub_batch_mb 256, piece_len 512 and graphs 0 in every class. */

@@ -1,5 +1,7 @@
 // Instantiations of the classify kernels for the default window
-// (k = 35, l = 31: five l-mers per k-mer).
+// (k = 35, l = 31: five l-mers per k-mer).  The warp kernels take most calls of
+// such tables; the staged step has those on taxonomies with several roots, on
+// tables of 2^32 sectors and more and with sequences above 2^26 bases.
 #include "classify_kernels.cuh"
 #include "pipeline.cuh"
 

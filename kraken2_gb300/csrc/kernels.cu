@@ -80,7 +80,7 @@ k2g_status max_table_value(const k2g_db *db, uint32_t *out) {
 // the walks that go on (one in five at load 0.7) from a list in shared memory,
 // a thread each -- in their own threads they kept whole warps waiting for a
 // few lanes.  Bound by the random sectors: 16.8M keys, 2 GB table 0.67 ->
-// 0.40 ms (54 G sectors/s).
+// 0.40 to 0.43 ms (50 to 54 G sectors/s).
 constexpr int kLookupThreads = 256;
 
 template <bool WIDE, int K>
