@@ -715,9 +715,8 @@ extern "C" k2g_status k2g_text_reset(k2g_text *t, uint32_t first_block, uint64_t
   return K2G_OK;
 }
 
-extern "C" k2g_status k2g_text_classify(k2g_text *t, const char *chunk, uint64_t len, int at_eof,
-                                        k2g_counters *counters, k2g_text_result *res) {
-  if (!t || !res || (len && !chunk)) return fail(K2G_ERR_ARG, "null argument");
+static k2g_status text_classify(k2g_text *t, const char *chunk, uint64_t len, int at_eof,
+                                k2g_counters *counters, k2g_text_result *res) {
   memset(res, 0, sizeof(*res));
   t->text_len = 0;
   if (t->handed_off) return fail(K2G_ERR_ARG, "the input was handed off; reset first");
@@ -916,6 +915,12 @@ extern "C" k2g_status k2g_text_classify(k2g_text *t, const char *chunk, uint64_t
   t->stream_pos += consumed;
   res->consumed = t->stream_pos;
   return K2G_OK;
+}
+
+extern "C" k2g_status k2g_text_classify(k2g_text *t, const char *chunk, uint64_t len, int at_eof,
+                                        k2g_counters *counters, k2g_text_result *res) {
+  if (!t || !res || (len && !chunk)) return fail(K2G_ERR_ARG, "null argument");
+  return settled(text_classify(t, chunk, len, at_eof, counters, res), t->st);
 }
 
 extern "C" k2g_status k2g_text_prefetch(k2g_text *t, const char *chunk, uint64_t len) {

@@ -118,3 +118,33 @@ def test_builds(what, one_root, fn):
         every_failure(f, one, fn, optional=6 if what in ("sequences", "sample") else None)
         db.close()
         assert f.faults() == []
+
+
+@pytest.mark.parametrize("fn", ["cudaMalloc", *FALLIBLE, "cudaEventSynchronize"])
+def test_text(fn):
+    """(the caller's chunk is on its way to the device when the call fails)"""
+    with fake_cuda() as f:
+        db = k2g.Database.create(OPTS, 100_003, 22, 10, PARENT)
+        n = 100
+        chunk = b"".join(b"@r%d\n%s\n+\n%s\n" % (i, b"ACGT" * 30, b"I" * 120) for i in range(n))
+
+        def launch(name, args):      # what the parser finds: the whole chunk's records, one block
+            if "11frag_kernel" in name:
+                info = C.cast(C.cast(args[5], C.POINTER(C.c_void_p))[0], C.POINTER(C.c_uint64))
+                for word, value in ((0, 2**64 - 1), (1, 120), (2, n), (3, n), (4, 1), (5, len(chunk)), (6, 120 * n)):
+                    info[word] = value
+
+        f.hook(launch)
+        t = k2g.TextReader(db, k2g.ClassifyParams(0.1, 2, 0, 0, 0), chunk_cap=1 << 16, lines=False)
+        counters = k2g.Counters(db)
+
+        def one():
+            t.reset()
+            res, _ = t.classify(chunk, True, counters)
+            assert (res.fragments, res.handoff) == (n, 0)
+
+        every_failure(f, one, fn)
+        t.close()
+        counters.close()
+        db.close()
+        assert f.faults() == []
