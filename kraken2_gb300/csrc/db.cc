@@ -380,6 +380,7 @@ extern "C" k2g_status k2g_db_open(const char *hash_k2d, const char *taxo_k2d,
       if (pin[0]) cudaFreeHost(pin[0]);
       if (pin[1]) cudaFreeHost(pin[1]);
       destroy(db.release());
+      (void)cudaGetLastError();
       return fail(K2G_ERR_NOMEM, "pinned staging allocation failed");
     }
     cudaEvent_t ev[2];
@@ -388,18 +389,21 @@ extern "C" k2g_status k2g_db_open(const char *hash_k2d, const char *taxo_k2d,
     uint64_t total = hdr[0] * 4, done = 0;
     int b = 0;
     bool ok = true;
+    cudaError_t copied = cudaSuccess;
     bool used[2] = {false, false};
     while (done < total) {
       size_t n = (size_t)std::min<uint64_t>(chunk, total - done);
-      if (used[b]) cudaEventSynchronize(ev[b]);
+      if (used[b] && (copied = cudaEventSynchronize(ev[b])) != cudaSuccess) break;
       if (!read_exact(fd, pin[b], n)) { ok = false; break; }
-      cudaMemcpyAsync((char *)db->d_cells + done, pin[b], n, cudaMemcpyHostToDevice, st);
-      cudaEventRecord(ev[b], st);
+      copied = cudaMemcpyAsync((char *)db->d_cells + done, pin[b], n, cudaMemcpyHostToDevice, st);
+      if (copied == cudaSuccess) copied = cudaEventRecord(ev[b], st);
+      if (copied != cudaSuccess) break;
       used[b] = true;
       done += n;
       b ^= 1;
     }
     cudaError_t e = cudaStreamSynchronize(st);
+    if (copied != cudaSuccess) e = copied;
     cudaEventDestroy(ev[0]);
     cudaEventDestroy(ev[1]);
     cudaStreamDestroy(st);

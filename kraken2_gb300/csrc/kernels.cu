@@ -62,11 +62,14 @@ __global__ void max_value_kernel(const uint32_t *cells, const unsigned long long
 k2g_status max_table_value(const k2g_db *db, uint32_t *out) {
   unsigned int *d = nullptr;
   K2G_CUDA_TRY(cudaMalloc(&d, 4));
-  K2G_CUDA_TRY(cudaMemset(d, 0, 4));
-  max_value_kernel<<<1216, 256>>>(db->d_cells, db->d_wide, db->capacity,
-                                  (uint32_t)((1ull << db->value_bits) - 1), d);
-  note_launches();
-  cudaError_t e = cudaMemcpy(out, d, 4, cudaMemcpyDeviceToHost);
+  cudaError_t e = cudaMemset(d, 0, 4);
+  if (e == cudaSuccess) {
+    max_value_kernel<<<1216, 256>>>(db->d_cells, db->d_wide, db->capacity,
+                                    (uint32_t)((1ull << db->value_bits) - 1), d);
+    note_launches();
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(out, d, 4, cudaMemcpyDeviceToHost);
   cudaFree(d);
   if (e != cudaSuccess) return cuda_fail(e, "max_value_kernel");
   return K2G_OK;

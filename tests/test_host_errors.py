@@ -1,12 +1,14 @@
 """Calls of the CUDA runtime that fail, under the library's entry points (on
 the fake runtime)."""
 import ctypes as C
+import os
 
 import numpy as np
 import pytest
 
 import kraken2_gb300 as k2g
 from fake_cuda import fake_cuda
+from kraken_io import GOLDEN
 
 OPTS = k2g.IndexOptions(35, 31, 0, 0xe37e28c4271b5a2d, 1, 1, 0)
 PARENT = np.array([0, 0, 1, 1, 2], np.uint64)
@@ -148,3 +150,41 @@ def test_text(fn):
         counters.close()
         db.close()
         assert f.faults() == []
+
+
+MAKING = ["cudaMalloc", "cudaMallocFromPoolAsync", "cudaMemcpy", "cudaMemset", "cudaMemcpyAsync", "cudaMemsetAsync",
+          "launch", "cudaStreamSynchronize", "cudaEventRecord", "cudaEventSynchronize", "cudaStreamCreate",
+          "cudaStreamCreateWithFlags", "cudaHostAlloc", "cudaEventCreateWithFlags"]
+
+
+def every_failure_in_making(f, make):
+    """make() with each call of the runtime failing in turn: it says so, and
+    keeps no memory."""
+    for fn in MAKING:
+        for i in range(200):
+            held = f.used()
+            f.fail(fn, i)
+            try:
+                made = make()
+            except k2g.K2GError:
+                assert f.failed() and f.used() == held, (fn, i)
+                continue
+            assert not f.failed(), (fn, i, "a failure that was not reported")
+            f.fail("", -1)
+            made.close()
+            assert f.used() == held, fn
+            break
+        else:
+            raise AssertionError("too many calls")
+    assert f.faults() == []
+
+
+@pytest.mark.parametrize("key_bits", [22, 30])
+def test_tables(key_bits):
+    with fake_cuda() as f:
+        every_failure_in_making(f, lambda: k2g.Database.create(OPTS, 100_003, key_bits, 10, PARENT))
+
+
+def test_opened_tables():
+    with fake_cuda() as f:
+        every_failure_in_making(f, lambda: k2g.Database.open(os.path.join(GOLDEN, "db_a")))
