@@ -59,8 +59,14 @@ cudaError_t scratch_alloc_now(void **p, size_t bytes, int device) {
       if (e != cudaSuccess) return e;
     }
   }
-  const cudaError_t e = scratch_alloc(p, bytes, device, d.st);
-  return e != cudaSuccess ? e : cudaStreamSynchronize(d.st);
+  cudaError_t e = scratch_alloc(p, bytes, device, d.st);
+  if (e != cudaSuccess) return e;
+  e = cudaStreamSynchronize(d.st);
+  if (e != cudaSuccess) {
+    cudaFreeAsync(*p, d.st);
+    *p = nullptr;
+  }
+  return e;
 }
 
 void scratch_free_now(void *p, int device) {

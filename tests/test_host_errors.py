@@ -188,3 +188,15 @@ def test_tables(key_bits):
 def test_opened_tables():
     with fake_cuda() as f:
         every_failure_in_making(f, lambda: k2g.Database.open(os.path.join(GOLDEN, "db_a")))
+
+
+@pytest.mark.parametrize("what", ["counters", "text", "server"])
+def test_objects(what):
+    with fake_cuda() as f:
+        db = k2g.Database.open(os.path.join(GOLDEN, "db_a"))
+        cp = k2g.ClassifyParams(0.1, 2, 0, 0, 0)
+        make = {"counters": lambda: k2g.Counters(db), "text": lambda: k2g.TextReader(db, cp, chunk_cap=1 << 16),
+                "server": lambda: k2g.Server(db, cp, 64 << 20)}[what]
+        make().close()               # (the pool's stream)
+        every_failure_in_making(f, make)
+        db.close()
