@@ -185,12 +185,12 @@ k2g_status alloc_table(k2g_db *db, uint64_t capacity) {
   if (capacity == 0) return fail(K2G_ERR_FORMAT, "table capacity is zero");
   if (db->cell_bytes == 5) {
     uint64_t padded = (capacity + 3) & ~3ull;   // whole 32-byte sectors
-    K2G_CUDA_TRY(cudaMalloc(&db->d_wide, padded * 8));
+    K2G_CUDA_TRY(device_alloc(&db->d_wide, padded * 8));
     if (padded != capacity)
       K2G_CUDA_TRY(cudaMemset(db->d_wide + capacity, 0, (padded - capacity) * 8));
   } else {
     uint64_t padded = (capacity + 7) & ~7ull;   // whole 32-byte sectors
-    K2G_CUDA_TRY(cudaMalloc(&db->d_cells, padded * sizeof(uint32_t)));
+    K2G_CUDA_TRY(device_alloc(&db->d_cells, padded * sizeof(uint32_t)));
     if (padded != capacity)
       K2G_CUDA_TRY(cudaMemset(db->d_cells + capacity, 0, (padded - capacity) * sizeof(uint32_t)));
   }

@@ -31,7 +31,7 @@ struct Buf {
     if (p) cudaFree(p);
     p = nullptr;
     cap = 0;
-    cudaError_t e = cudaMalloc(&p, std::max<size_t>(n, 64));
+    cudaError_t e = device_alloc(&p, std::max<size_t>(n, 64));
     if (e == cudaSuccess) cap = std::max<size_t>(n, 64);
     return e;
   }

@@ -191,7 +191,7 @@ template <class T>
 cudaError_t regrow(T *&p, uint64_t n) {
   if (p) cudaFree(p);
   p = nullptr;
-  return cudaMalloc(&p, std::max<uint64_t>(n, 1) * sizeof(T));
+  return device_alloc(&p, std::max<uint64_t>(n, 1) * sizeof(T));
 }
 
 // Makes the slot hold chunks of up to fb fragments / bb bases.

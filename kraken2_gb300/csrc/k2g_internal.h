@@ -165,6 +165,13 @@ cudaError_t scratch_alloc(void **p, size_t bytes, int device, cudaStream_t st);
 cudaError_t scratch_alloc_now(void **p, size_t bytes, int device);
 void scratch_free_now(void *p, int device);
 void scratch_opened(int device);
+// cudaMalloc on the current device; where memory is short, with what the pool
+// keeps given back first.
+cudaError_t device_alloc(void **p, size_t bytes);
+template <class T>
+cudaError_t device_alloc(T **p, size_t bytes) {
+  return device_alloc(reinterpret_cast<void **>(p), bytes);
+}
 void scratch_closed(int device);
 // The end of a call that works on `st` and waits for it: one that fails waits
 // too, since its buffers are on their way back to the pool (cudaFreeAsync does

@@ -370,7 +370,7 @@ static cudaError_t grow(T *&p, uint64_t &cap, uint64_t want) {
   if (p) cudaFree(p);
   p = nullptr;
   cap = 0;
-  cudaError_t e = cudaMalloc(&p, want * sizeof(T));
+  cudaError_t e = device_alloc(&p, want * sizeof(T));
   if (e == cudaSuccess) cap = want;
   return e;
 }
@@ -383,7 +383,7 @@ static k2g_status ctx_reserve(ExecCtx &c, uint64_t frags, uint64_t slots, size_t
     if (c.slow) cudaFree(c.slow);
     c.slow = nullptr;
     c.slow_bytes = 0;
-    K2G_CUDA_TRY(cudaMalloc(&c.slow, slow_bytes));
+    K2G_CUDA_TRY(device_alloc(&c.slow, slow_bytes));
     c.slow_bytes = slow_bytes;
   }
   // (a capacity that several buffers share is none until all of them are there)
@@ -799,8 +799,8 @@ extern "C" k2g_status k2g_lookup_host(const k2g_db *db, const uint64_t *keys, ui
   K2G_CUDA_TRY(cudaSetDevice(db->device));
   uint64_t *dk = nullptr;
   uint32_t *dv = nullptr;
-  K2G_CUDA_TRY(cudaMalloc(&dk, n * 8));
-  cudaError_t e = cudaMalloc(&dv, n * 4);
+  K2G_CUDA_TRY(device_alloc(&dk, n * 8));
+  cudaError_t e = device_alloc(&dv, n * 4);
   if (e != cudaSuccess) { cudaFree(dk); return cuda_fail(e, "cudaMalloc"); }
   e = cudaMemcpy(dk, keys, n * 8, cudaMemcpyHostToDevice);
   k2g_status s = K2G_OK;

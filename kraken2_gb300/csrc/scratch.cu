@@ -5,7 +5,7 @@
 // graph.  The pool keeps up to kKeep bytes between calls (a pool that keeps
 // nothing maps the memory anew after every synchronisation, about 0.8 ms a
 // call) and gives everything back when the device's last database or counter
-// set is closed.
+// set is closed, or when the library needs it for something else (device_alloc).
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -71,6 +71,21 @@ cudaError_t scratch_alloc_now(void **p, size_t bytes, int device) {
 
 void scratch_free_now(void *p, int device) {
   if (p) cudaFreeAsync(p, g_pools[device & 63].st);
+}
+
+cudaError_t device_alloc(void **p, size_t bytes) {
+  const cudaError_t e = cudaMalloc(p, bytes);
+  int device = 0;
+  if (e != cudaErrorMemoryAllocation || cudaGetDevice(&device) != cudaSuccess) return e;
+  Pool &d = g_pools[device & 63];
+  {
+    std::lock_guard<std::mutex> lock(d.mu);
+    if (!d.pool) return e;
+    // (what was given back on a stream counts once its end has been waited for)
+    if (cudaDeviceSynchronize() != cudaSuccess || cudaMemPoolTrimTo(d.pool, 0) != cudaSuccess) return e;
+  }
+  (void)cudaGetLastError();
+  return cudaMalloc(p, bytes);
 }
 
 void scratch_opened(int device) {

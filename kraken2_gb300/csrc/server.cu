@@ -159,18 +159,18 @@ cudaError_t alloc_slot(Slot &s, uint64_t cb, uint64_t cf, int per, bool quals) {
   TRY(cudaHostAlloc(&s.h_call, cf * 4, cudaHostAllocDefault));
   TRY(cudaHostAlloc(&s.h_hg, cf * 4, cudaHostAllocDefault));
   TRY(cudaHostAlloc(&s.h_hlen, cf * 4, cudaHostAllocDefault));
-  TRY(cudaMalloc(&s.d_bases, cb + 16));
-  if (quals) TRY(cudaMalloc(&s.d_quals, cb + 16));
-  TRY(cudaMalloc(&s.d_off, (cf * per + 1) * 8));
-  TRY(cudaMalloc(&s.d_sparse, runs_cap * 8));
-  TRY(cudaMalloc(&s.d_dense, runs_cap * 8));
-  TRY(cudaMalloc(&s.d_excl, cf * 8));
-  TRY(cudaMalloc(&s.d_sums, ((cf + kScanBlock - 1) / kScanBlock + 1) * 8));
-  TRY(cudaMalloc(&s.d_total, 8));
-  TRY(cudaMalloc(&s.d_call, cf * 4));
-  TRY(cudaMalloc(&s.d_hg, cf * 4));
-  TRY(cudaMalloc(&s.d_hlen, cf * 4));
-  TRY(cudaMalloc(&s.d_status, 4));
+  TRY(device_alloc(&s.d_bases, cb + 16));
+  if (quals) TRY(device_alloc(&s.d_quals, cb + 16));
+  TRY(device_alloc(&s.d_off, (cf * per + 1) * 8));
+  TRY(device_alloc(&s.d_sparse, runs_cap * 8));
+  TRY(device_alloc(&s.d_dense, runs_cap * 8));
+  TRY(device_alloc(&s.d_excl, cf * 8));
+  TRY(device_alloc(&s.d_sums, ((cf + kScanBlock - 1) / kScanBlock + 1) * 8));
+  TRY(device_alloc(&s.d_total, 8));
+  TRY(device_alloc(&s.d_call, cf * 4));
+  TRY(device_alloc(&s.d_hg, cf * 4));
+  TRY(device_alloc(&s.d_hlen, cf * 4));
+  TRY(device_alloc(&s.d_status, 4));
 #undef TRY
   return cudaSuccess;
 }

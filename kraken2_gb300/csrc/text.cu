@@ -535,7 +535,7 @@ struct DBuf {
     if (p) cudaFree(p);
     p = nullptr;
     cap = 0;
-    cudaError_t e = cudaMalloc(&p, std::max<uint64_t>(n, 16) * sizeof(T));
+    cudaError_t e = device_alloc(&p, std::max<uint64_t>(n, 16) * sizeof(T));
     if (e == cudaSuccess) cap = std::max<uint64_t>(n, 16);
     return e;
   }

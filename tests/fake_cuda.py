@@ -19,6 +19,7 @@ from kraken2_gb300 import build as kb
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 OUT_OF_MEMORY = 2           # cudaErrorMemoryAllocation
+UNKNOWN = 999               # cudaErrorUnknown: nothing that asking again would mend
 _HOOK = C.CFUNCTYPE(None, C.c_char_p, C.POINTER(C.c_void_p))
 _built = None
 
@@ -51,7 +52,7 @@ class Fake:
         self.lib = lib
         lib.fake_fault.restype = C.c_char_p
         lib.fake_pending.argtypes = [C.c_void_p]
-        for f in ("fake_pending", "fake_pending_all", "fake_used", "fake_launches"):
+        for f in ("fake_pending", "fake_pending_all", "fake_used", "fake_kept", "fake_launches"):
             getattr(lib, f).restype = C.c_uint64
         lib.fake_tail_of_copy.argtypes, lib.fake_tail_of_copy.restype = [C.c_size_t], C.c_long
         lib.fake_room.argtypes, lib.fake_room.restype = [C.c_void_p], C.c_long
@@ -71,7 +72,7 @@ class Fake:
     def launches(self, part: str) -> int:
         return self.lib.fake_launches(part.encode())
 
-    def fail(self, fn: str, skip: int, err: int = OUT_OF_MEMORY):
+    def fail(self, fn: str, skip: int, err: int = UNKNOWN):
         self.lib.fake_fail(fn.encode(), skip, err)
 
     def failed(self) -> bool:
@@ -82,7 +83,12 @@ class Fake:
         self.lib.fake_limit(bytes_)
 
     def used(self) -> int:
+        """Device memory held, without what the pool keeps."""
         return self.lib.fake_used()
+
+    def kept(self) -> int:
+        """What the pool keeps of the memory given back to it."""
+        return self.lib.fake_kept()
 
     def room(self, p: int) -> int:
         """Bytes from p to the end of its allocation (-1: none)."""
@@ -109,6 +115,7 @@ class Fake:
         """The array in an allocation of the fake device."""
         p = C.c_void_p()
         self.lib.cudaMalloc(C.byref(p), C.c_size_t(max(a.nbytes, 1) + 16))
+        assert p.value
         if a.nbytes:
             C.memmove(p.value, a.ctypes.data, a.nbytes)
         return p.value

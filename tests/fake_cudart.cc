@@ -4,7 +4,8 @@
 // choose: work queued on a stream stays pending until the host waits for it,
 // and a host copy from pageable memory may still be on its way when the call
 // returns.  Calls can be made to fail, and a copy or fill outside the
-// allocations is recorded instead of done.
+// allocations is recorded instead of done.  A pool keeps up to 1 GB of what was
+// freed, as the library asks, until it is trimmed.
 #include <cuda_runtime_api.h>
 
 #include <cstdint>
@@ -50,7 +51,7 @@ struct Fake {
   long fail_at = -1;
   int fail_err = 0;
   cudaError_t last = cudaSuccess;
-  uint64_t limit = ~0ull, used = 0;
+  uint64_t limit = ~0ull, used = 0, kept = 0;   // kept: by the pool (in used)
   LaunchHook hook = nullptr;
 };
 
@@ -171,9 +172,11 @@ API void fake_fail(const char *fn, long skip, int err) {
   F().fail_at = skip;
   F().fail_err = err;
 }
+API uint64_t fake_kept() { return F().kept; }
 API int fake_failed() { return F().fail_at < 0; }
 API void fake_limit(uint64_t bytes) { F().limit = bytes; }
-API uint64_t fake_used() { return F().used; }
+// Device memory held, without what the pool keeps.
+API uint64_t fake_used() { return F().used - F().kept; }
 API uint64_t fake_pending(void *st) {
   Stream *s = stream_of((cudaStream_t)st);
   return s->issued - s->done;
@@ -207,8 +210,9 @@ API cudaError_t cudaGetLastError() {
   return e;
 }
 API const char *cudaGetErrorString(cudaError_t e) { return e == cudaErrorMemoryAllocation ? "out of memory" : "error"; }
-API cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
-API cudaError_t cudaSetDevice(int) { return cudaSuccess; }
+static thread_local int t_device = 0;
+API cudaError_t cudaGetDevice(int *d) { *d = t_device; return cudaSuccess; }
+API cudaError_t cudaSetDevice(int d) { t_device = d; return cudaSuccess; }
 API cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr a, int) {
   *v = a == cudaDevAttrMultiProcessorCount ? 152 : 0;
   return cudaSuccess;
@@ -228,13 +232,30 @@ API cudaError_t cudaFree(void *p) { Lock lock(F().mu); complete_all(); release(p
 API cudaError_t cudaFreeHost(void *p) { Lock lock(F().mu); complete_all(); release(p, "cudaFreeHost of no allocation"); return cudaSuccess; }
 API cudaError_t cudaMemPoolCreate(cudaMemPool_t *p, const cudaMemPoolProps *) { FAILS(cudaMemPoolCreate) *p = (cudaMemPool_t)8; return cudaSuccess; }
 API cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void *) { return cudaSuccess; }
-API cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) { return cudaSuccess; }
+API cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t) {
+  Lock lock(F().mu);
+  F().used -= F().kept;
+  F().kept = 0;
+  return cudaSuccess;
+}
+API cudaError_t cudaDeviceSynchronize() { Lock lock(F().mu); complete_all(); return cudaSuccess; }
 API cudaError_t cudaMallocFromPoolAsync(void **p, size_t n, cudaMemPool_t pool, cudaStream_t) {
   FAILS(cudaMallocFromPoolAsync)
   if (!pool) fault("allocation from no pool");
+  const uint64_t reused = F().kept < n ? F().kept : n;
+  F().kept -= reused;
+  F().used -= reused;
   return allocate(p, n, false);
 }
-API cudaError_t cudaFreeAsync(void *p, cudaStream_t) { Lock lock(F().mu); release(p, "cudaFreeAsync of no allocation"); return cudaSuccess; }
+API cudaError_t cudaFreeAsync(void *p, cudaStream_t) {
+  Lock lock(F().mu);
+  const uint64_t before = F().used;
+  release(p, "cudaFreeAsync of no allocation");
+  const uint64_t size = before - F().used, room = (1ull << 30) - F().kept, keep = size < room ? size : room;
+  F().kept += keep;
+  F().used += keep;
+  return cudaSuccess;
+}
 
 API cudaError_t cudaMemcpy(void *d, const void *s, size_t n, cudaMemcpyKind k) {
   FAILS(cudaMemcpy)

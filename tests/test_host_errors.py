@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 import kraken2_gb300 as k2g
-from fake_cuda import fake_cuda
+from fake_cuda import OUT_OF_MEMORY, fake_cuda
 from kraken_io import GOLDEN
 
 OPTS = k2g.IndexOptions(35, 31, 0, 0xe37e28c4271b5a2d, 1, 1, 0)
@@ -23,7 +23,7 @@ def test_an_error_that_was_reported_is_not_reported_again():
         db = k2g.Database.create(OPTS, 100_003, 22, 10, PARENT)
         keys, taxa = f.device(np.arange(100, dtype=np.uint64)), f.device(np.ones(100, np.uint32))
         st = f.stream()
-        f.fail("cudaMallocFromPoolAsync", 0)
+        f.fail("cudaMallocFromPoolAsync", 0, OUT_OF_MEMORY)
         with pytest.raises(k2g.K2GError) as e:
             db.build_insert(keys, taxa, 100, False, st)
         assert e.value.status == 5               # K2G_ERR_NOMEM

@@ -177,3 +177,43 @@ def test_a_device_with_room_for_two_slots(length, with_counters):
         f.limit(1 << 60)
         k2g.check(call(dbs[2], n))
         assert f.faults() == []
+
+
+@pytest.mark.parametrize("what", ["table", "wide table", "host", "staged", "text", "server", "lines"])
+def test_memory_that_the_pool_keeps_is_there_for_others(what):
+    """(up to 1 GB, which a program that needs it for a table or a call gets)"""
+    with fake_cuda() as f:
+        staged = k2g.IndexOptions(31, 31, 0, 0xe37e28c4271b5a2d, 1, 1, 0)
+        roots = np.array([0, 0, 0, 1, 2], np.uint64)             # (an ordered insert sorts all pairs)
+        db = k2g.Database.create(staged if what == "staged" else OPTS, 100_003, 22, 10, roots, device=63)
+        if what in ("text", "lines"):
+            db.set_names(np.arange(5), [b"x"] * 5)
+        n = 20_000_000
+        keys, taxa = f.device(np.zeros(n, np.uint64)), f.device(np.zeros(n, np.uint32))
+        db.build_insert(keys, taxa, n, True, f.stream())
+        assert f.kept() > 100 << 20
+        cp = k2g.ClassifyParams(0.0, 2, 0, 0, 0)
+
+        def call():
+            if what == "table":
+                k2g.Database.create(OPTS, 40_000_003, 22, 10, PARENT, device=63).close()
+            elif what == "wide table":
+                k2g.Database.create(OPTS, 20_000_003, 30, 10, PARENT, device=63).close()
+            elif what == "host":
+                k2g.check(classify(db, 5000, quals=False))
+            elif what == "staged":
+                assert staged_call(f, db, f.stream(), 2000, False)
+            elif what == "text":
+                k2g.TextReader(db, cp, chunk_cap=1 << 20).close()
+            elif what == "server":
+                k2g.Server(db, cp, 64 << 20).close()
+            else:
+                m = 1_000_000
+                db.format_lines(np.zeros(m, np.uint32), np.zeros(m, np.uint32), np.zeros(0, np.uint64), [b"r"] * m,
+                                np.full(m, 150))
+
+        f.limit(f.used() + f.kept() + (16 << 20))    # (the call needs more than that, and less than what is kept)
+        call()
+        assert f.kept() < 100 << 20 and f.faults() == []
+        f.limit(1 << 60)
+        db.close()
