@@ -409,7 +409,8 @@ cudaError_t bucket_sort(const uint32_t *start, uint32_t n_buckets, uint64_t larg
     if (i > 1 && largest <= caps[i - 1]) break;
     const size_t smem = bucket_sort_smem(caps[i]);
     auto kern = bucket_sort_kernel<Zone>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // (the limit is the kernel's, whichever thread calls: always the largest)
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bucket_sort_smem(kLargeBlock));
     if (e != cudaSuccess) return e;
     kern<<<n_buckets, kSortThreads, smem, st>>>(start, keys, caps[i - 1], caps[i], n_distinct, zone);
     note_launches();

@@ -93,8 +93,9 @@ extern "C" k2g_status k2g_db_value_counts(const k2g_db *db, uint64_t *counts, ui
     const uint64_t lo = 1 + p * kMaxBins;
     const uint32_t bins = (uint32_t)std::min<uint64_t>(kMaxBins, ids - std::min(ids, p * kMaxBins));
     const size_t smem = std::max<size_t>((size_t)bins * 4, 4);
+    // (the limit is the kernel's, whichever thread calls: always the largest)
     if ((e = cudaFuncSetAttribute(value_hist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem)) != cudaSuccess)
+                                  (int)(kMaxBins * 4))) != cudaSuccess)
       break;
     int per_sm = 0;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, value_hist_kernel, kHistThreads,

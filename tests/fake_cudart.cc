@@ -43,6 +43,7 @@ struct Fake {
   std::map<uintptr_t, Alloc> mem;
   std::map<const void *, std::string> kernels;
   std::map<std::string, uint64_t> launches;
+  std::map<const void *, int> smem;   // limits of dynamic shared memory
   std::vector<Stream *> streams;
   Stream legacy;
   std::vector<std::string> faults;
@@ -219,7 +220,14 @@ API cudaError_t cudaDeviceGetAttribute(int *v, cudaDeviceAttr a, int) {
 }
 API cudaError_t cudaDeviceGetStreamPriorityRange(int *lo, int *hi) { *lo = 0; *hi = -5; return cudaSuccess; }
 API cudaError_t cudaMemGetInfo(size_t *free_b, size_t *total) { *free_b = *total = 1ull << 38; return cudaSuccess; }
-API cudaError_t cudaFuncSetAttribute(const void *, cudaFuncAttribute, int) { return cudaSuccess; }
+// (one limit a kernel for all threads: lowered by one call, it fails another's launch)
+API cudaError_t cudaFuncSetAttribute(const void *fn, cudaFuncAttribute a, int v) {
+  Lock lock(F().mu);
+  if (a != cudaFuncAttributeMaxDynamicSharedMemorySize) return cudaSuccess;
+  if (F().smem.count(fn) && F().smem[fn] > v) fault(("limit of shared memory lowered: " + F().kernels[fn]).c_str());
+  F().smem[fn] = v;
+  return cudaSuccess;
+}
 API cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int *n, const void *, int, size_t, unsigned) {
   *n = 8;
   return cudaSuccess;
@@ -351,11 +359,14 @@ API cudaError_t __cudaPopCallConfiguration(dim3 *grid, dim3 *block, size_t *smem
   return cudaSuccess;
 }
 API cudaError_t __cudaGetKernel(cudaKernel_t *k, const void *fn) { *k = (cudaKernel_t)fn; return cudaSuccess; }
-API cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 grid, dim3 block, void **args, size_t, cudaStream_t st) {
+API cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 grid, dim3 block, void **args, size_t smem, cudaStream_t st) {
   FAILS(launch)
   const std::string &name = F().kernels[(const void *)k];
   F().launches[name]++;
   if (!grid.x || !grid.y || !grid.z || !block.x) fault(("empty launch of " + name).c_str());
+  const void *fn = (const void *)k;
+  if (smem > 48 * 1024 && (!F().smem.count(fn) || (size_t)F().smem[fn] < smem))
+    fault(("shared memory above its limit: " + name).c_str());
   stream_of(st)->issued++;
   if (F().hook) F().hook(name.c_str(), args);
   return cudaSuccess;
